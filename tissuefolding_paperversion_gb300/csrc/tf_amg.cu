@@ -25,7 +25,8 @@
 //   lambda_max of D^-1 A by power iteration (smoother weight and prolongator
 //   smoothing weight omega = 4 / (3.15 lambda)); P; T = A P; A_{l+1} = P^T T;
 //   6x6 block inverses; Gauss-Jordan inverse of the coarsest level per
-//   instance (<= 16 nodes).
+//   instance (<= 16 nodes); the explicit dense operator of the levels whose
+//   matrices are small enough (k_dense_build).
 // Application (one V-cycle per preconditioner call, all kernels, capturable
 // in a CUDA graph): damped block-Jacobi pre- and post-smoothing (one sweep
 // each way at level 0, kCoarseSweeps on the coarser levels), residual,
@@ -57,9 +58,23 @@ namespace {
 constexpr int kT = 256;
 constexpr int kCoarseNodes = 16;  // nodes per instance at the coarsest level (96 DOFs)
 constexpr int kCoarseDofs = 6 * kCoarseNodes;
+constexpr int kInvThreads = 512;  // of the coarsest level's inverse
 constexpr int kPowerIters = 16;
-constexpr int kTailNodes = 256;   // levels with at most this many nodes per instance run fused
-constexpr int kTailThreads = 1024;
+// The first level whose dense operators (one m x m FP32 matrix per instance,
+// m = 6 nodes) fit these bytes, and every level below it, is applied as one
+// matrix-vector product: reading 64 MB takes ~10 us at the HBM rate, where a
+// level run kernel by kernel takes eight launches (~40 us on the 391-node
+// level of the 320,000-prism sheet) and the levels below another ~20 us.
+constexpr int64_t kDenseBytes = 64 << 20;
+constexpr int kDenseThreads = 512;
+constexpr int kDenseCols = 16;    // columns of the dense operator built together by one CTA
+constexpr int kDenseQuads = kDenseCols / 4;  // lanes per row, four columns each
+// Three V-cycles instead of one cost nothing per application and leave the
+// coarse levels nearly solved: 95 -> 70 CG iterations per 1.0M-prism wing step,
+// 42 -> 39 BiCGStab iterations on the 320,000-prism sheet (two cycles: 78 and 41).
+constexpr int kDenseRows = 3600;  // rows of an instance: its vectors have to fit shared memory, 64 bytes a row
+constexpr int kDenseSweeps = 3;  // their sweeps each way
+constexpr int kDenseCycles = 3;   // V-cycles the dense operator stands for
 // damped block-Jacobi sweeps before and after the coarse correction on the
 // levels >= 1 (level 0 sweeps once each way): more sweeps on the small,
 // launch-bound coarse levels cut the Krylov iterations (320,000-prism sheet:
@@ -175,6 +190,9 @@ tf_status zeros(T** dst, size_t n) {
     } while (0)
 
 
+struct DenseBuild;
+__global__ void k_dense_build(DenseBuild B);
+
 }  // namespace
 
 // Device view of one level: what the V-cycle reads and writes, all FP32
@@ -264,7 +282,18 @@ struct Amg {
     bool coarse_exact = true;
     int max_cm = 0;
     int v0_smem = 0;           // shared memory of the level-0 prolongation (3 floats per block of a CTA)
-    int tail = 0;              // levels tail..nlev-1 run in one kernel (one CTA per instance); 0: none
+    // levels dense..nlev-1 are applied as one dense operator per instance
+    // (0: none, the coarsest level has too many DOFs for an exact inverse)
+    int dense = 0;
+    float* dmat = nullptr;     // the operators, m_g x m_g row-major (cinv when dense is the coarsest level)
+    int* doff = nullptr;       // [nseg+1] their offsets
+    int2* dgroup = nullptr;    // column groups (instance, first column) of their construction
+    int ndgroup = 0;
+    float* dwork = nullptr;    // work vectors of the construction, per CTA
+    int dgrid = 0;             // its CTAs
+    int dlvl[kAmgMaxLevels] = {};  // offset of each level's vectors within a CTA's work
+    int64_t dstride = 0;
+    int dsmem = 0;             // its shared memory
     int smooth_unroll = 4;     // slots in flight per lane in the level-0 smoother's row product (2, 4, 8)
     std::vector<int> h_n;      // nodes per level (host)
     std::vector<int> h_prow[kAmgMaxLevels], h_pcol[kAmgMaxLevels];  // prolongator patterns (host)
@@ -291,8 +320,10 @@ void amg_free(Amg* a) {
         for (void* p : sptrs)
             if (p) cudaFree(p);
     }
+    if (a->dmat != a->cinv && a->dmat) cudaFree(a->dmat);
+    if (a->doff != a->cinv0 && a->doff) cudaFree(a->doff);
     void* ptrs[] = {a->omega, a->pscal, a->pv, a->pw, a->part, a->ticket, a->cnode0, a->cinv0, a->cinv,
-                    a->val32, a->dinv32, a->valh, a->diag32};
+                    a->val32, a->dinv32, a->valh, a->diag32, a->dgroup, a->dwork};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     delete a;
@@ -645,18 +676,55 @@ tf_status amg_build(tf_handle* h, const double* pos) {
         cinv0[g + 1] = cinv0[g] + m * m;
     }
     a->coarse_exact = a->max_cm <= kCoarseDofs;
-    // the levels whose instances all have at most kTailNodes nodes run as
-    // one kernel per V-cycle, one CTA per instance
-    a->tail = a->coarse_exact ? a->nlev - 1 : 0;
-    for (int l = a->nlev - 1; l >= 1 && a->coarse_exact; --l) {
-        int maxn = 0;
-        for (int g = 0; g < d.nseg; ++g) maxn = std::max(maxn, H[l].seg0[g + 1] - H[l].seg0[g]);
-        if (maxn > kTailNodes) break;
-        a->tail = l;
-    }
     AMG_TRY(up(&a->cnode0, CH.seg0));
     AMG_TRY(up(&a->cinv0, cinv0));
     AMG_TRY(zeros(&a->cinv, (size_t)std::max(cinv0[d.nseg], 1)));
+    if (!a->coarse_exact) return TF_OK;
+    // the dense operator: from the finest level that fits down (the coarsest
+    // level's inverse exists anyway)
+    a->dense = a->nlev - 1;
+    std::vector<int> doff = cinv0;
+    for (int l = a->nlev - 2; l >= 1; --l) {
+        std::vector<int> off(d.nseg + 1, 0);
+        int64_t total = 0;
+        bool fits = true;
+        for (int g = 0; g < d.nseg; ++g) {
+            const int64_t m = 6 * (int64_t)(H[l].seg0[g + 1] - H[l].seg0[g]);
+            total += m * m;
+            fits = fits && total * (int64_t)sizeof(float) <= kDenseBytes && m <= kDenseRows;
+            if (!fits) break;
+            off[g + 1] = static_cast<int>(total);
+        }
+        if (!fits) break;
+        a->dense = l;
+        doff = off;
+    }
+    if (a->dense == a->nlev - 1) {
+        a->dmat = a->cinv;
+        a->doff = a->cinv0;
+        return TF_OK;
+    }
+    std::vector<int2> group;
+    std::vector<int> maxn(a->nlev, 0);
+    for (int l = a->dense; l < a->nlev; ++l)
+        for (int g = 0; g < d.nseg; ++g) maxn[l] = std::max(maxn[l], H[l].seg0[g + 1] - H[l].seg0[g]);
+    for (int g = 0; g < d.nseg; ++g) {
+        const int m = 6 * (H[a->dense].seg0[g + 1] - H[a->dense].seg0[g]);
+        for (int c = 0; c < m; c += kDenseCols) group.push_back(make_int2(g, c));
+    }
+    a->dsmem = static_cast<int>(sizeof(float) * 6 * (size_t)maxn[a->dense] * kDenseCols);
+    TF_CUDA(cudaFuncSetAttribute(k_dense_build, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)(sizeof(float) * kDenseRows * kDenseCols)));
+    for (int l = a->dense; l < a->nlev; ++l) {  // r, x, t, e per level, the result too at the first
+        a->dlvl[l] = static_cast<int>(a->dstride);
+        a->dstride += (int64_t)(l == a->dense ? 5 : 4) * 6 * maxn[l] * kDenseCols;
+    }
+    a->ndgroup = static_cast<int>(group.size());
+    a->dgrid = std::min(a->ndgroup, 152);
+    AMG_TRY(up(&a->dgroup, group));
+    AMG_TRY(up(&a->doff, doff));
+    AMG_TRY(zeros(&a->dmat, (size_t)doff[d.nseg]));
+    AMG_TRY(zeros(&a->dwork, (size_t)a->dgrid * (size_t)a->dstride));
     return TF_OK;
 }
 
@@ -1273,29 +1341,32 @@ __global__ void k_pw_step6(AmgLevel L, const float* __restrict__ v, float* __res
     if (grid_sum(s, part, ticket, &tot)) pw_finish(tot, scal, omega);
 }
 
-// Gauss-Jordan inverse of the coarsest matrix of each instance (one CTA
-// each, FP64 work, FP32 result)
-__global__ void k_coarse_invert(AmgLevel L, const int* __restrict__ cnode0, const int* __restrict__ cinv0,
-                                float* __restrict__ cinv) {
-    extern __shared__ double M[];  // m x 2m
-    __shared__ double f[kCoarseDofs];
+// Gauss-Jordan inverse of the coarsest matrix of each instance, in place
+// (one CTA each, FP64 work, FP32 result).  Bound by the m^2 FP64 updates of
+// each of the m steps on one SM (m <= 96: 0.2 ms); the pivot is found by one
+// warp.  1.26 -> 0.3 ms at m = 90 against an m x 2m form with a serial pivot
+// search.
+__global__ void __launch_bounds__(kInvThreads) k_coarse_invert(AmgLevel L, const int* __restrict__ cnode0,
+                                                               const int* __restrict__ cinv0,
+                                                               float* __restrict__ cinv) {
+    extern __shared__ double M[];  // m x m
+    __shared__ double f[kCoarseDofs], prow[kCoarseDofs];
+    __shared__ int swapped[kCoarseDofs];  // row exchanged with row k at step k
     __shared__ int piv;
-    __shared__ double tiny;
+    __shared__ double tiny, pval;
     const int g = blockIdx.x;
     const int n0 = cnode0[g], n1 = cnode0[g + 1];
-    const int m = 6 * (n1 - n0), w = 2 * m;
+    const int m = 6 * (n1 - n0);
     if (m == 0) return;
-    for (int k = threadIdx.x; k < m * w; k += blockDim.x) {
-        const int r = k / w, c = k - r * w;
-        M[k] = (c - m == r) ? 1.0 : 0.0;
-    }
+    const int lane = threadIdx.x & 31;
+    for (int k = threadIdx.x; k < m * m; k += blockDim.x) M[k] = 0.0;
     __syncthreads();
     for (int I = n0 + threadIdx.x; I < n1; I += blockDim.x) {
         for (int p = L.rowptr[I]; p < L.rowptr[I + 1]; ++p) {
             const int J = L.colidx[p] - n0;
             const float* v = L.val + 36 * (size_t)p;
             for (int a = 0; a < 6; ++a)
-                for (int b = 0; b < 6; ++b) M[(6 * (I - n0) + a) * w + 6 * J + b] = (double)v[6 * a + b];
+                for (int b = 0; b < 6; ++b) M[(6 * (I - n0) + a) * m + 6 * J + b] = (double)v[6 * a + b];
         }
         if (L.xrow)
             for (int q = L.xrow[I]; q < L.xrow[I + 1]; ++q) {
@@ -1303,61 +1374,86 @@ __global__ void k_coarse_invert(AmgLevel L, const int* __restrict__ cnode0, cons
                 if (J < 0 || J >= n1 - n0) continue;  // couples another instance: outside this inverse
                 const float* v = L.xval + 36 * (size_t)q;
                 for (int a = 0; a < 6; ++a)
-                    for (int b = 0; b < 6; ++b) M[(6 * (I - n0) + a) * w + 6 * J + b] += (double)v[6 * a + b];
+                    for (int b = 0; b < 6; ++b) M[(6 * (I - n0) + a) * m + 6 * J + b] += (double)v[6 * a + b];
             }
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (threadIdx.x < 32) {
         double dmax = 0.0;
-        for (int r = 0; r < m; ++r) dmax = fmax(dmax, fabs(M[r * w + r]));
-        tiny = 1e-12 * dmax;
+        for (int r = lane; r < m; r += 32) dmax = fmax(dmax, fabs(M[r * m + r]));
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) dmax = fmax(dmax, __shfl_xor_sync(0xffffffffu, dmax, o));
+        if (lane == 0) tiny = 1e-12 * dmax;
     }
     __syncthreads();
     for (int k = 0; k < m; ++k) {
-        if (threadIdx.x == 0) {
-            int best = k;
-            double bv = fabs(M[k * w + k]);
-            for (int r = k + 1; r < m; ++r)
-                if (fabs(M[r * w + k]) > bv) {
-                    bv = fabs(M[r * w + k]);
+        if (threadIdx.x < 32) {  // the largest entry of column k from row k down, the first of equal ones
+            double bv = -1.0;
+            int best = m;
+            for (int r = k + lane; r < m; r += 32) {
+                const double v = fabs(M[r * m + k]);
+                if (v > bv) {
+                    bv = v;
                     best = r;
                 }
-            piv = bv > tiny ? best : -1;
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                const double ov = __shfl_xor_sync(0xffffffffu, bv, o);
+                const int ob = __shfl_xor_sync(0xffffffffu, best, o);
+                if (ov > bv || (ov == bv && ob < best)) {
+                    bv = ov;
+                    best = ob;
+                }
+            }
+            if (lane == 0) {
+                piv = bv > tiny ? best : -1;
+                swapped[k] = bv > tiny ? best : k;
+                pval = bv > tiny ? M[best * m + k] : 0.0;
+            }
         }
         __syncthreads();
-        if (piv < 0) {
+        const int pr = piv;
+        if (pr < 0) {
             // (numerically) singular direction, e.g. a free rigid mode of an
             // unconstrained sheet: no coarse correction along it
-            for (int c = threadIdx.x; c < w; c += blockDim.x) M[k * w + c] = 0.0;
-            for (int r = threadIdx.x; r < m; r += blockDim.x) M[r * w + k] = 0.0;
+            for (int c = threadIdx.x; c < m; c += blockDim.x) M[k * m + c] = M[c * m + k] = 0.0;
             __syncthreads();
             continue;
         }
-        const int pr = piv;
-        if (pr != k)
-            for (int c = threadIdx.x; c < w; c += blockDim.x) {
-                const double tmp = M[k * w + c];
-                M[k * w + c] = M[pr * w + c];
-                M[pr * w + c] = tmp;
-            }
+        // the pivot row scaled (unit column in place of column k), the rest of
+        // column k as the multipliers
+        const double rinv = 1.0 / pval;
+        for (int c = threadIdx.x; c < m; c += blockDim.x) {
+            const double v = M[pr * m + c];
+            if (pr != k) M[pr * m + c] = M[k * m + c];
+            prow[c] = (c == k ? 1.0 : v) * rinv;
+        }
         __syncthreads();
-        const double dk = M[k * w + k];
-        const double rinv = 1.0 / dk;
+        for (int r = threadIdx.x; r < m; r += blockDim.x) {
+            f[r] = r == k ? 0.0 : M[r * m + k];
+            if (r != k) M[r * m + k] = 0.0;
+        }
         __syncthreads();
-        for (int c = threadIdx.x; c < w; c += blockDim.x) M[k * w + c] *= rinv;
-        for (int r = threadIdx.x; r < m; r += blockDim.x) f[r] = M[r * w + k];
+        for (int q = threadIdx.x; q < m * m; q += blockDim.x) {
+            const int r = q / m, c = q - r * m;
+            M[q] = r == k ? prow[c] : fma(-f[r], prow[c], M[q]);
+        }
         __syncthreads();
-        for (int q = threadIdx.x; q < m * w; q += blockDim.x) {
-            const int r = q / w, c = q - r * w;
-            if (r != k) M[q] = fma(-f[r], M[k * w + c], M[q]);
+    }
+    // the row exchanges of A are column exchanges of its inverse, last first
+    for (int k = m - 1; k >= 0; --k) {
+        const int pr = swapped[k];
+        if (pr == k) continue;
+        for (int r = threadIdx.x; r < m; r += blockDim.x) {
+            const double tmp = M[r * m + k];
+            M[r * m + k] = M[r * m + pr];
+            M[r * m + pr] = tmp;
         }
         __syncthreads();
     }
     float* out = cinv + cinv0[g];
-    for (int q = threadIdx.x; q < m * m; q += blockDim.x) {
-        const int r = q / m, c = q - r * m;
-        out[q] = (float)M[r * w + m + c];
-    }
+    for (int q = threadIdx.x; q < m * m; q += blockDim.x) out[q] = (float)M[q];
 }
 
 // ---- V-cycle (FP32) -------------------------------------------------------------
@@ -1602,80 +1698,266 @@ __host__ __device__ __forceinline__ float* post_sweep_out(const AmgLevel& L, con
     return cur == L.x ? L.t : L.x;
 }
 
-// e = C^-1 r on the coarsest level, one CTA per instance
-__global__ void k_coarse_solve(AmgLevel L, const double* __restrict__ scal, const int* __restrict__ cnode0,
-                               const int* __restrict__ cinv0, const float* __restrict__ cinv) {
+// e = M r on level `dense`, M the explicit operator of the V-cycles from that
+// level down (k_dense_build), one warp per row.  Bound by reading M (22 MB at
+// the 391-node level of the 320,000-prism sheet); it replaces the three sweeps
+// each way, residual, restriction and prolongation of that level and the
+// levels below.
+__global__ void k_dense(AmgLevel L, const double* __restrict__ scal, const int* __restrict__ doff,
+                        const float* __restrict__ mat) {
     pdl_enter();
-    const int g = blockIdx.x;
+    const int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;  // row over all instances
+    if (k >= 6 * L.n) return;
+    const int g = L.seg[k / 6];
     if (seg_stopped(scal, g)) return;
-    const int n0 = cnode0[g], m = 6 * (cnode0[g + 1] - n0);
-    const float* __restrict__ Mi = cinv + cinv0[g];
-    const float* __restrict__ r = L.r + 6 * (size_t)n0;
-    for (int k = threadIdx.x; k < m; k += blockDim.x) {
-        float s = 0.f;
-        for (int j = 0; j < m; ++j) s = fmaf(__ldg(&Mi[(size_t)k * m + j]), r[j], s);
-        L.e[6 * (size_t)n0 + k] = s;
+    const int lane = threadIdx.x & 31;
+    const int k0 = 6 * L.seg0[g];
+    const int m2 = 3 * (L.seg0[g + 1] - L.seg0[g]);  // pairs of a row: m is even, rows are 8-byte aligned
+    const float2* __restrict__ M = reinterpret_cast<const float2*>(mat + doff[g] + (size_t)(k - k0) * (2 * m2));
+    const float2* __restrict__ r = reinterpret_cast<const float2*>(L.r + k0);
+    float s = 0.f;
+#pragma unroll 8
+    for (int q = lane; q < m2; q += 32) {
+        const float2 a = __ldg(&M[q]), b = r[q];
+        s = fmaf(a.x, b.x, fmaf(a.y, b.y, s));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) L.e[k] = s;
+}
+
+// The dense operator column by column: kDenseCycles V-cycles (each on the
+// residual the one before left) of the levels first..last applied to the unit
+// vectors, in FP32 with the FP32 operators.  A CTA builds kDenseCols columns
+// at once, four lanes per row with four columns each, so a lane uses every
+// matrix value it loads four times (one column per lane, sixteen lanes per
+// row, spent its time handing the same values to every lane: 1.83 against
+// 1.10 ms at 286 nodes, three cycles).  Its vectors live in its own slice of `work`,
+// [component][column]; the one the row products read is staged in shared
+// memory.  Run when the coarse levels are rebuilt.
+struct DenseBuild {
+    AmgLevel L[kAmgMaxLevels];
+    const double* omega;
+    const int* cinv0;
+    const float* cinv;
+    int first, last, sweeps;
+    const int2* group;
+    int ngroup;
+    float* work;
+    int64_t stride;
+    int off[kAmgMaxLevels];
+    float* mat;
+    const int* doff;
+};
+
+__device__ __forceinline__ float4 fma4(float a, float4 x, float4 y) {
+    return make_float4(fmaf(a, x.x, y.x), fmaf(a, x.y, y.y), fmaf(a, x.z, y.z), fmaf(a, x.w, y.w));
+}
+
+// y += s M x for a 6x6 block M (row-major) and this lane's columns
+__device__ __forceinline__ void block6(const float* __restrict__ M, float s, const float4* x, float4 (&y)[6]) {
+    const float4* __restrict__ v = reinterpret_cast<const float4*>(M);
+    float4 xv[6];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+        const float4 f = x[k * kDenseQuads];
+        xv[k] = make_float4(s * f.x, s * f.y, s * f.z, s * f.w);
+    }
+#pragma unroll
+    for (int u = 0; u < 9; ++u) {
+        const float4 f = __ldg(&v[u]);
+        y[(4 * u) / 6] = fma4(f.x, xv[(4 * u) % 6], y[(4 * u) / 6]);
+        y[(4 * u + 1) / 6] = fma4(f.y, xv[(4 * u + 1) % 6], y[(4 * u + 1) / 6]);
+        y[(4 * u + 2) / 6] = fma4(f.z, xv[(4 * u + 2) % 6], y[(4 * u + 2) / 6]);
+        y[(4 * u + 3) / 6] = fma4(f.w, xv[(4 * u + 3) % 6], y[(4 * u + 3) / 6]);
+    }
+}
+__device__ __forceinline__ void load6(const float4* x, float4 (&y)[6]) {
+#pragma unroll
+    for (int k = 0; k < 6; ++k) y[k] = x[k * kDenseQuads];
+}
+__device__ __forceinline__ void store6(float4* x, const float4 (&y)[6]) {
+#pragma unroll
+    for (int k = 0; k < 6; ++k) x[k * kDenseQuads] = y[k];
+}
+
+// acc -= (A x)_i; x: the vector of the instance (first node n0) in shared memory
+__device__ __forceinline__ void dense_row(const AmgLevel& L, int i, int n0, int n1, const float4* x, int c,
+                                          float4 (&acc)[6]) {
+    const int p1 = __ldg(&L.rowptr[i + 1]);
+    for (int p = __ldg(&L.rowptr[i]); p < p1; ++p)
+        block6(L.val + 36 * (size_t)p, -1.f, x + 6 * (__ldg(&L.colidx[p]) - n0) * kDenseQuads + c, acc);
+    if (!L.xrow) return;
+    for (int q = L.xrow[i]; q < L.xrow[i + 1]; ++q) {
+        const int j = L.xcol[q] - n0;
+        if (j < 0 || j >= n1 - n0) continue;  // couples another instance: outside this operator
+        block6(L.xval + 36 * (size_t)q, -1.f, x + 6 * j * kDenseQuads + c, acc);
     }
 }
 
-// The coarse tail of a V-cycle: levels T.first .. T.last of one instance
-// (one CTA each), block barriers instead of kernel boundaries.  Level
-// T.first arrives restricted and pre-smoothed; its corrected x goes out in e.
-struct Tail {
-    AmgLevel L[kAmgMaxLevels];
-    const double* omega;
-    const double* scal;
-    const int* cinv0;
-    const float* cinv;
-    int first, last;
-    int sweeps;  // pre- and post-smoothing sweeps per level
-};
+// out_i = (x_i or 0) + omega D_i^-1 acc
+__device__ __forceinline__ void dense_smooth(const AmgLevel& L, int i, float om, const float4 (&acc)[6],
+                                             const float4* x, float4* out) {
+    const float* __restrict__ Di = L.dinv + 36 * (size_t)i;
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+        float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int m = 0; m < 6; ++m) s = fma4(__ldg(&Di[6 * k + m]), acc[m], s);
+        out[k * kDenseQuads] = fma4(om, s, x ? x[k * kDenseQuads] : make_float4(0.f, 0.f, 0.f, 0.f));
+    }
+}
 
-__global__ void __launch_bounds__(kTailThreads) k_tail(Tail T) {
-    pdl_enter();
-    const int g = blockIdx.x;
-    if (seg_stopped(T.scal, g)) return;
-    const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    float* cur[kAmgMaxLevels];
-    for (int l = T.first; l < T.last; ++l) {
-        const AmgLevel& F = T.L[l];
-        const AmgLevel& C = T.L[l + 1];
-        float* x = F.x;
-        for (int s = 2; s <= T.sweeps; ++s) {
-            float* out = pre_sweep_out(F, x);
-            for (int i = F.seg0[g] + warp; i < F.seg0[g + 1]; i += nw) post_row(F, T.omega + l, x, out, i);
-            __syncthreads();
-            x = out;
-        }
-        cur[l] = x;
-        for (int i = F.seg0[g] + warp; i < F.seg0[g + 1]; i += nw) resid_row(F, x, i);
-        __syncthreads();
-        for (int I = C.seg0[g] + warp; I < C.seg0[g + 1]; I += nw)
-            restrict_node<6>(F, C, F.t, I, T.omega + l + 1, l + 1 < T.last ? 1 : 0);
-        __syncthreads();
-    }
-    {
-        const AmgLevel& C = T.L[T.last];
-        const int n0 = C.seg0[g], m = 6 * (C.seg0[g + 1] - n0);
-        const float* __restrict__ Mi = T.cinv + T.cinv0[g];
-        for (int k = threadIdx.x; k < m; k += blockDim.x) {
-            float s2 = 0.f;
-            for (int j = 0; j < m; ++j) s2 = fmaf(__ldg(&Mi[(size_t)k * m + j]), C.r[6 * (size_t)n0 + j], s2);
-            C.e[6 * (size_t)n0 + k] = s2;
-        }
-    }
+// The vector a pass of row products reads, brought into shared memory.
+__device__ __forceinline__ void dense_stage(const float4* x, float4* xs, int n) {
+    for (int q = threadIdx.x; q < n * kDenseQuads; q += kDenseThreads) xs[q] = x[q];
     __syncthreads();
-    for (int l = T.last - 1; l >= T.first; --l) {
-        const AmgLevel& F = T.L[l];
-        float* x = cur[l];
-        for (int i = F.seg0[g] + threadIdx.x; i < F.seg0[g + 1]; i += blockDim.x) prolong_node(F, T.L[l + 1].e, i, x);
-        __syncthreads();
-        for (int s = 1; s <= T.sweeps; ++s) {
-            float* out = post_sweep_out(F, x, s, T.sweeps);
-            for (int i = F.seg0[g] + warp; i < F.seg0[g + 1]; i += nw) post_row(F, T.omega + l, x, out, i);
-            __syncthreads();
-            x = out;
+}
+
+__global__ void __launch_bounds__(kDenseThreads) k_dense_build(DenseBuild B) {
+    extern __shared__ __align__(16) float4 xs[];  // [6 nodes][kDenseCols] of the largest instance
+    const int c = threadIdx.x % kDenseQuads, h = threadIdx.x / kDenseQuads;
+    constexpr int nh = kDenseThreads / kDenseQuads;  // rows in flight
+    float4* work = reinterpret_cast<float4*>(B.work + (int64_t)blockIdx.x * B.stride);
+    for (int gi = blockIdx.x; gi < B.ngroup; gi += gridDim.x) {
+        const int g = B.group[gi].x, col0 = B.group[gi].y;
+        float4 *r[kAmgMaxLevels], *x[kAmgMaxLevels], *t[kAmgMaxLevels], *e[kAmgMaxLevels];
+        for (int l = B.first; l <= B.last; ++l) {
+            const size_t n = (size_t)6 * (B.L[l].seg0[g + 1] - B.L[l].seg0[g]) * kDenseQuads;
+            r[l] = work + B.off[l] / 4;
+            x[l] = r[l] + n;
+            t[l] = x[l] + n;
+            e[l] = t[l] + n;
         }
+        const AmgLevel& L1 = B.L[B.first];
+        const int m = 6 * (L1.seg0[g + 1] - L1.seg0[g]);
+        float4* y = e[B.first] + (size_t)m * kDenseQuads;
+        for (int k = h; k < m; k += nh) {
+            const int u = k - col0 - 4 * c;  // the unit column of this row among the lane's four
+            r[B.first][k * kDenseQuads + c] = make_float4(u == 0, u == 1, u == 2, u == 3);
+            y[k * kDenseQuads + c] = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        __syncthreads();
+        for (int cyc = 0; cyc < kDenseCycles; ++cyc) {
+            for (int l = B.first; l < B.last; ++l) {  // down
+                const AmgLevel& F = B.L[l];
+                const AmgLevel& C = B.L[l + 1];
+                const int f0 = F.seg0[g], f1 = F.seg0[g + 1], c0 = C.seg0[g], c1 = C.seg0[g + 1];
+                const float om = (float)__ldg(B.omega + l);
+                for (int i = f0 + h; i < f1; i += nh) {
+                    const size_t q = (size_t)6 * (i - f0) * kDenseQuads + c;
+                    float4 acc[6];
+                    load6(r[l] + q, acc);
+                    dense_smooth(F, i, om, acc, nullptr, x[l] + q);
+                }
+                __syncthreads();
+                float4 *cur = x[l], *oth = e[l];
+                for (int s = 2; s <= B.sweeps + 1; ++s) {  // the last pass leaves the residual in t
+                    dense_stage(cur, xs, 6 * (f1 - f0));
+                    for (int i = f0 + h; i < f1; i += nh) {
+                        const size_t q = (size_t)6 * (i - f0) * kDenseQuads + c;
+                        float4 acc[6];
+                        load6(r[l] + q, acc);
+                        dense_row(F, i, f0, f1, xs, c, acc);
+                        if (s <= B.sweeps) dense_smooth(F, i, om, acc, cur + q, oth + q);
+                        else store6(t[l] + q, acc);
+                    }
+                    __syncthreads();
+                    if (s <= B.sweeps) {
+                        float4* sw = cur;
+                        cur = oth;
+                        oth = sw;
+                    }
+                }
+                x[l] = cur;
+                e[l] = oth;
+                for (int I = c0 + h; I < c1; I += nh) {
+                    float4 acc[6];
+#pragma unroll
+                    for (int b = 0; b < 6; ++b) acc[b] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    for (int p = __ldg(&F.pcptr[I]); p < __ldg(&F.pcptr[I + 1]); ++p) {
+                        const float* __restrict__ P = F.Pc + 36 * (size_t)p;
+                        const float4* ti = t[l] + (size_t)6 * (__ldg(&F.pcrow[p]) - f0) * kDenseQuads + c;
+#pragma unroll
+                        for (int k = 0; k < 6; ++k) {
+                            const float4 tk = ti[k * kDenseQuads];
+#pragma unroll
+                            for (int b = 0; b < 6; ++b) acc[b] = fma4(__ldg(&P[6 * k + b]), tk, acc[b]);
+                        }
+                    }
+                    store6(r[l + 1] + (size_t)6 * (I - c0) * kDenseQuads + c, acc);
+                }
+                __syncthreads();
+            }
+            {  // coarsest level
+                const AmgLevel& C = B.L[B.last];
+                const int mc = 6 * (C.seg0[g + 1] - C.seg0[g]);
+                const float* __restrict__ Mi = B.cinv + B.cinv0[g];
+                for (int k = h; k < mc; k += nh) {
+                    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+                    for (int j = 0; j < mc; ++j)
+                        s = fma4(__ldg(&Mi[(size_t)k * mc + j]), r[B.last][j * kDenseQuads + c], s);
+                    e[B.last][k * kDenseQuads + c] = s;
+                }
+                __syncthreads();
+            }
+            for (int l = B.last - 1; l >= B.first; --l) {  // up
+                const AmgLevel& F = B.L[l];
+                const int f0 = F.seg0[g], f1 = F.seg0[g + 1], c0 = B.L[l + 1].seg0[g];
+                const float om = (float)__ldg(B.omega + l);
+                for (int i = f0 + h; i < f1; i += nh) {
+                    float4* xi = x[l] + (size_t)6 * (i - f0) * kDenseQuads + c;
+                    float4 s[6];
+                    load6(xi, s);
+                    for (int b = __ldg(&F.prow[i]); b < __ldg(&F.prow[i + 1]); ++b)
+                        block6(F.Pv + 36 * (size_t)b, 1.f,
+                               e[l + 1] + (size_t)6 * (__ldg(&F.pcol[b]) - c0) * kDenseQuads + c, s);
+                    store6(xi, s);
+                }
+                __syncthreads();
+                float4 *cur = x[l], *oth = e[l];
+                for (int s = 1; s <= B.sweeps; ++s) {
+                    dense_stage(cur, xs, 6 * (f1 - f0));
+                    for (int i = f0 + h; i < f1; i += nh) {
+                        const size_t q = (size_t)6 * (i - f0) * kDenseQuads + c;
+                        float4 acc[6];
+                        load6(r[l] + q, acc);
+                        dense_row(F, i, f0, f1, xs, c, acc);
+                        dense_smooth(F, i, om, acc, cur + q, oth + q);
+                    }
+                    __syncthreads();
+                    float4* sw = cur;
+                    cur = oth;
+                    oth = sw;
+                }
+                x[l] = oth;
+                e[l] = cur;  // the level's correction
+            }
+            for (int k = h; k < m; k += nh) {
+                const size_t q = (size_t)k * kDenseQuads + c;
+                y[q] = fma4(1.f, e[B.first][q], y[q]);
+            }
+            if (cyc + 1 == kDenseCycles) break;
+            const int f0 = L1.seg0[g], f1 = L1.seg0[g + 1];
+            dense_stage(e[B.first], xs, m);
+            for (int i = f0 + h; i < f1; i += nh) {  // r -= A e
+                const size_t q = (size_t)6 * (i - f0) * kDenseQuads + c;
+                float4 acc[6];
+                load6(r[B.first] + q, acc);
+                dense_row(L1, i, f0, f1, xs, c, acc);
+                store6(r[B.first] + q, acc);
+            }
+            __syncthreads();
+        }
+        for (int k = h; k < m; k += nh) {
+            const float4 v = y[(size_t)k * kDenseQuads + c];
+            const float o[4] = {v.x, v.y, v.z, v.w};
+            float* out = B.mat + B.doff[g] + (size_t)k * m + col0 + 4 * c;
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (col0 + 4 * c + u < m) out[u] = o[u];
+        }
+        __syncthreads();
     }
 }
 
@@ -1798,15 +2080,34 @@ tf_status amg_numeric(tf_handle* h) {
     }
     if (a->coarse_exact) {
         AmgLevel& L = a->L[a->nlev - 1];
-        const size_t smem = sizeof(double) * (size_t)a->max_cm * 2 * a->max_cm;
+        const size_t smem = sizeof(double) * (size_t)a->max_cm * a->max_cm;
         static bool configured = false;
         if (!configured) {
             TF_CUDA(cudaFuncSetAttribute(k_coarse_invert, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)(sizeof(double) * 2 * kCoarseDofs * kCoarseDofs)));
+                                         (int)(sizeof(double) * kCoarseDofs * kCoarseDofs)));
             configured = true;
         }
-        k_coarse_invert<<<a->nseg, kT, smem, st>>>(L, a->cnode0, a->cinv0, a->cinv);
+        k_coarse_invert<<<a->nseg, kInvThreads, smem, st>>>(L, a->cnode0, a->cinv0, a->cinv);
         TF_LAUNCH_CHECK(h);
+        if (a->dense < a->nlev - 1) {
+            DenseBuild B;
+            for (int l = 0; l < a->nlev; ++l) B.L[l] = a->L[l];
+            B.omega = a->omega;
+            B.cinv0 = a->cinv0;
+            B.cinv = a->cinv;
+            B.first = a->dense;
+            B.last = a->nlev - 1;
+            B.sweeps = kDenseSweeps;
+            B.group = a->dgroup;
+            B.ngroup = a->ndgroup;
+            B.work = a->dwork;
+            B.stride = a->dstride;
+            for (int l = 0; l < a->nlev; ++l) B.off[l] = a->dlvl[l];
+            B.mat = a->dmat;
+            B.doff = a->doff;
+            k_dense_build<<<a->dgrid, kDenseThreads, a->dsmem, st>>>(B);
+            TF_LAUNCH_CHECK(h);
+        }
     }
     a->stale = 0;
     return TF_OK;
@@ -1848,22 +2149,22 @@ int amg_smoother_unroll(const tf_handle* h) { return h->amg ? h->amg->smooth_unr
 int amg_vcycle_kernels(const tf_handle* h) {
     const Amg* a = h->amg;
     const int per = 2 * kCoarseSweeps + 2;  // kernels of a coarse level run kernel by kernel
-    if (a->tail > 0) return 5 + per * (a->tail - 1) + 1;
-    return 5 + per * (a->nlev - 2) + (a->coarse_exact ? 1 : 3);
+    if (a->dense > 0) return 5 + per * (a->dense - 1) + 1;
+    return 5 + per * (a->nlev - 2) + 3;
 }
 
 // out = M^-1 r: one V-cycle (all launches on h->stream, no host work).
-// Levels below `tail` run kernel by kernel over all instances; the tail runs
-// as one kernel with a CTA per instance.
+// Levels above `dense` run kernel by kernel over all instances; `dense` and
+// the levels below it are one product with their dense operator.
 void amg_vcycle(tf_handle* h, const double* r, double* out) {
     Amg* a = h->amg;
     Device& d = h->d;
     cudaStream_t st = h->stream;
     const int nl = a->nlev;
-    const int stop = a->tail > 0 ? a->tail : nl - 1;  // first level not handled kernel by kernel
+    const int stop = a->dense > 0 ? a->dense : nl - 1;  // first level not handled kernel by kernel
     V0 v0{d, a->omega, a->dinv32, a->valh, a->diag32};
     AmgLevel& L0 = a->L[0];
-    auto presmooth = [&](int l) { return (l < nl - 1 || !a->coarse_exact) ? 1 : 0; };
+    auto presmooth = [&](int l) { return l == a->dense ? 0 : 1; };
     launch_pdl(k_v0_pre, d.ncta, kNodeThreads, st, v0, r, L0.x);
     switch (a->smooth_unroll) {
         case 2: launch_pdl(k_v0_resid<2>, d.ncta, kNodeThreads, st, v0, r, L0.x, L0.t); break;
@@ -1888,28 +2189,17 @@ void amg_vcycle(tf_handle* h, const double* r, double* out) {
         launch_pdl(k_restrict<6>, cdiv(32 * (int64_t)a->L[l + 1].n, kT), kT, st, L, a->L[l + 1], (const float*)L.t,
                    (const double*)d.scal, (const double*)(a->omega + l + 1), presmooth(l + 1));
     }
-    if (a->tail > 0) {
-        Tail T;
-        for (int l = 0; l < nl; ++l) T.L[l] = a->L[l];
-        T.omega = a->omega;
-        T.scal = d.scal;
-        T.cinv0 = a->cinv0;
-        T.cinv = a->cinv;
-        T.first = a->tail;
-        T.last = nl - 1;
-        T.sweeps = kCoarseSweeps;
-        launch_pdl(k_tail, a->nseg, kTailThreads, st, T);
+    if (a->dense > 0) {
+        AmgLevel& LD = a->L[stop];
+        launch_pdl(k_dense, cdiv(32 * 6 * (int64_t)LD.n, kT), kT, st, LD, (const double*)d.scal, (const int*)a->doff,
+                   (const float*)a->dmat);
     } else {
+        // x from the restriction's pre-smoothing; three more sweeps into e
         AmgLevel& LC = a->L[nl - 1];
-        if (a->coarse_exact) {
-            launch_pdl(k_coarse_solve, a->nseg, 128, st, LC, d.scal, a->cnode0, a->cinv0, a->cinv);
-        } else {
-            // x from the restriction's pre-smoothing; three more sweeps into e
-            const int nbc = cdiv(32 * (int64_t)LC.n, kT);
-            launch_pdl(k_v6_post, nbc, kT, st, LC, d.scal, a->omega + nl - 1, LC.x, LC.e);
-            launch_pdl(k_v6_post, nbc, kT, st, LC, d.scal, a->omega + nl - 1, LC.e, LC.t);
-            launch_pdl(k_v6_post, nbc, kT, st, LC, d.scal, a->omega + nl - 1, LC.t, LC.e);
-        }
+        const int nbc = cdiv(32 * (int64_t)LC.n, kT);
+        launch_pdl(k_v6_post, nbc, kT, st, LC, d.scal, a->omega + nl - 1, LC.x, LC.e);
+        launch_pdl(k_v6_post, nbc, kT, st, LC, d.scal, a->omega + nl - 1, LC.e, LC.t);
+        launch_pdl(k_v6_post, nbc, kT, st, LC, d.scal, a->omega + nl - 1, LC.t, LC.e);
     }
     for (int l = stop - 1; l >= 1; --l) {
         AmgLevel& L = a->L[l];
