@@ -891,7 +891,7 @@ def main():
     ap.add_argument("--adj-fd-default", type=int, default=2,
                     help="central-difference directions of the adjoint sub-measurement of the plain workload")
     ap.add_argument("--precond", type=int, default=0,
-                    help="0 auto (smoothed-aggregation multigrid from 20,000 nodes), 1 block-Jacobi, "
+                    help="0 auto (smoothed-aggregation multigrid), 1 block-Jacobi, "
                          "2 smoothed-aggregation multigrid, 3 plain-aggregation multigrid")
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--mg-reuse", type=int, default=0,

@@ -75,7 +75,9 @@ typedef struct tf_options {
     int32_t deterministic;   /* 1: order-fixed assembly (no atomics); 0: atomic scatter */
     int32_t device;          /* CUDA device ordinal */
     int32_t autotune_off;    /* 1: keep 16 prisms per CTA instead of timing 8/16/32 on the mesh */
-    int32_t precond;         /* 0 auto (smoothed-aggregation multigrid from 20,000 nodes on,
+    int32_t precond;         /* 0 auto (smoothed-aggregation multigrid from 20,000 nodes on
+                                and, with the atomic assembly, on smaller meshes too, there
+                                with block-Jacobi in its place once a solve with it fails;
                                 else block-Jacobi), 1 block-Jacobi, 2 smoothed-aggregation
                                 multigrid, 3 plain-aggregation multigrid (no reference
                                 counterpart for 2 and 3); other values: TF_BAD_INPUT */

@@ -69,3 +69,60 @@ def test_dense_coarse_operators_of_a_ragged_batch():
     ts = [_sheet(3, 3, 2, 0.0), _sheet(12, 13, 2, 0.0, 4), _sheet(8, 8, 1, 0.0, 5), _sheet(25, 9, 3, 0.0, 6)]
     with api.Batch(ts, precond=2, krylov_rtol=RTOL) as s:
         _solve(s, ts)
+
+
+# The multigrid of the small meshes (auto, atomic assembly) against the general
+# path there, block-Jacobi: the same Newton counts, positions to the parity
+# tests' 1e-8.  A mesh of 12 nodes has no hierarchy.
+@pytest.mark.parametrize("eta", [0.0, 100.0])
+@pytest.mark.parametrize("nx,ny,layers,coarsens", [(2, 1, 1, False), (3, 3, 1, True), (9, 7, 3, True), (40, 11, 4, True)])
+def test_small_meshes_take_the_multigrid(nx, ny, layers, coarsens, eta):
+    t = _sheet(nx, ny, layers, eta)
+    t.rates = np.tile([4e-6, 3e-6, 0.0], t.n_elems)
+    res = []
+    for pc in (0, 1):
+        with api.Solver(t, precond=pc) as s:
+            s.set_growth_rates(t.rates)
+            its = [s.newton_step(t.dt, allow_not_converged=False)["iters"] for _ in range(3)]
+            res.append((its, s.positions(), bool(s.multigrid_info()[0])))
+    assert res[0][0] == res[1][0]
+    assert np.abs(res[0][1] - res[1][1]).max() <= 1e-8 * np.abs(res[1][1]).max()
+    assert (res[0][2], res[1][2]) == (coarsens, False)
+
+
+def test_order_fixed_small_meshes_keep_block_jacobi_for_steps():
+    t = _sheet(9, 7, 3, 0.0)
+    with api.Solver(t, deterministic=True) as s:
+        assert s.multigrid_info()[0] == []
+        lv, sv = s.adjoint_forward(np.full(t.n_elems, 1e-6), np.log(t.E), 1, t.dt, 1, np.array([20.0, 20.0, 5.0, 40.0]))
+        sv.free()
+        assert s.multigrid_info()[0] == []
+
+
+def test_singular_system_goes_to_block_jacobi():
+    """No external viscosity: the in-plane rigid motions have no stiffness.
+    Block-Jacobi solves the (consistent) system, the multigrid may not; then
+    the handle stays with block-Jacobi."""
+    t = _sheet(12, 12, 2, 0.0)
+    t.ext_visc[:] = 0.0
+    uk, un = mesh.perturbed_state(t, seed=8, amp=0.005)
+    res = []
+    for pc in (0, 1):
+        with api.Solver(t, precond=pc) as s:
+            for _ in range(2):
+                s.set_state(uk, un, t.dt)
+                s.assemble()
+                out = s.solve()
+                assert out["relres"] <= 1e-8
+            res.append(s.residual())
+    np.testing.assert_allclose(res[0], res[1], rtol=0, atol=1e-12 * np.abs(res[1]).max())
+
+
+def test_iteration_cap_is_the_callers():
+    t = _sheet(12, 12, 2, 100.0)
+    uk, un = mesh.perturbed_state(t, seed=8)
+    with api.Solver(t, krylov_max_iter=3) as s:
+        s.set_state(uk, un, t.dt)
+        s.assemble()
+        out = s.solve(allow_not_converged=True)
+        assert out["status"] == api.TF_KRYLOV_NOT_CONVERGED and out["iters"] == 3

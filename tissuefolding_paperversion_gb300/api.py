@@ -219,8 +219,8 @@ def _mesh_structs(t):
 class Solver:
     """One GPU Newton solver over one tissue (a ``tf_handle``).  The keyword
     arguments are the fields of ``tf_options``.  ``precond``: 0 auto
-    (smoothed-aggregation multigrid from 20,000 nodes on, else block-Jacobi),
-    1 block-Jacobi, 2 smoothed-aggregation multigrid, 3 plain-aggregation
+    (smoothed-aggregation multigrid from 20,000 nodes on and, unless
+    ``deterministic``, below that too; else block-Jacobi), 1 block-Jacobi, 2 smoothed-aggregation multigrid, 3 plain-aggregation
     multigrid.  ``update_atol``: the absolute accuracy a Newton update needs
     (0: newton_tol x 1e-4, negative: every solve to krylov_rtol).
     ``host_loops``: host-driven Newton iterations and host-checked Krylov

@@ -443,6 +443,27 @@ struct CoarseRebuiltEachStep {
     ~CoarseRebuiltEachStep() { h->opt.multigrid_reuse_steps = keep; }
 };
 
+// The solves of the adjoint on a handle that uses block-Jacobi for its steps
+// only so that a batched instance reproduces its plain run (the order-fixed
+// assembly on a small mesh): a batch has no adjoint, so there they use the
+// multigrid, built at the first such call (3,200 prisms, 6 steps, every solve
+// to 1e-13: forward and backward 587 -> 113 ms).
+struct AdjointMultigrid {
+    tf_handle* h;
+    bool on;
+    explicit AdjointMultigrid(tf_handle* hh) : h(hh), on(hh->amg_adjoint && !hh->amg_failed) {
+        if (!on) return;
+        destroy_graphs(h);
+        h->amg_off = false;
+        amg_mark_stale(h, 2);
+    }
+    ~AdjointMultigrid() {
+        if (!on) return;
+        destroy_graphs(h);
+        h->amg_off = true;
+    }
+};
+
 }  // namespace
 
 extern "C" {
@@ -475,6 +496,18 @@ TF_API tf_status tf_adj_forward(tf_handle* h, const double* rate, const double* 
     a->dt = dt;
     a->device = h->device;
     std::memcpy(a->params, loss_params, sizeof(a->params));
+    if (h->amg_trial && !h->amg) {
+        const tf_status b = amg_build(h, h->h_pos0.data());
+        if (b != TF_OK) {
+            amg_free(h->amg);
+            h->amg = nullptr;
+            tf_adj_free(a);
+            return b;
+        }
+        h->amg_adjoint = h->amg != nullptr;
+        h->amg_off = true;
+    }
+    AdjointMultigrid multigrid(h);
     CoarseRebuiltEachStep rebuilt(h);
     const tf_status s = adj_forward(h, a, rate, logE);
     if (s != TF_OK && s != TF_NOT_CONVERGED) {
@@ -496,6 +529,7 @@ TF_API tf_status tf_adj_backward(tf_handle* h, tf_adjoint* a, double dloss, doub
         return TF_BAD_INPUT;
     }
     TF_CUDA(cudaSetDevice(h->device));
+    AdjointMultigrid multigrid(h);
     CoarseRebuiltEachStep rebuilt(h);
     return adj_backward(h, a, dloss, grad_rate, grad_logE);
 }

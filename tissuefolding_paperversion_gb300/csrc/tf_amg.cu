@@ -1971,7 +1971,7 @@ bool amg_reused(const tf_handle* h) { return h->amg && h->amg->reused; }
 
 long amg_rebuilds(const tf_handle* h) { return h->amg ? h->amg->rebuilds : 0; }
 
-bool use_multigrid(const tf_handle* h) { return h->amg != nullptr; }
+bool use_multigrid(const tf_handle* h) { return h->amg != nullptr && !h->amg_off; }
 
 // Numeric phase for the current matrix.  Within a time step the matrix of
 // a later Newton iteration differs little from the first one's, so a new
@@ -2144,7 +2144,7 @@ tf_status amg_autotune(tf_handle* h) {
     return TF_OK;
 }
 
-int amg_smoother_unroll(const tf_handle* h) { return h->amg ? h->amg->smooth_unroll : 0; }
+int amg_smoother_unroll(const tf_handle* h) { return use_multigrid(h) ? h->amg->smooth_unroll : 0; }
 
 int amg_vcycle_kernels(const tf_handle* h) {
     const Amg* a = h->amg;
@@ -2228,7 +2228,7 @@ extern "C" TF_API tf_status tf_multigrid_blocks(tf_handle* h, int64_t* blocks, i
         tf::set_error("tf_multigrid_blocks: bad arguments");
         return TF_BAD_INPUT;
     }
-    tf::Amg* a = h->amg;
+    tf::Amg* a = tf::use_multigrid(h) ? h->amg : nullptr;
     for (int l = 0; l < (a ? a->nlev : 0); ++l) {
         blocks[l] = a->L[l].nnzb;
         prolongator_blocks[l] = a->L[l].npb;
@@ -2241,7 +2241,7 @@ extern "C" TF_API tf_status tf_multigrid_info(tf_handle* h, int32_t* levels, int
         tf::set_error("tf_multigrid_info: bad arguments");
         return TF_BAD_INPUT;
     }
-    tf::Amg* a = h->amg;
+    tf::Amg* a = tf::use_multigrid(h) ? h->amg : nullptr;
     *levels = a ? a->nlev : 0;
     if (!a) return TF_OK;
     if (nodes)

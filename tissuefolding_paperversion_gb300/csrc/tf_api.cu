@@ -530,7 +530,16 @@ tf_status cuda_fail(cudaError_t e, const char* what) {
 }
 
 
-// Meshes from this many nodes on use the multigrid preconditioner by default.
+// Meshes from this many nodes on use the multigrid preconditioner by default
+// whatever the assembly, smaller ones with the atomic assembly only: the
+// order-fixed assembly promises that a batched instance reproduces its own
+// plain run bit for bit, and the hierarchy of a batch is not made of its
+// instances' own (one smoother weight, one dense level).  The multigrid is the
+// faster one at every size it can coarsen (ms per step with block-Jacobi /
+// multigrid, eta = 0 and 100): 36 prisms 4.3 / 2.1 and 7.1 / 2.3, 256 prisms
+// 9.1 / 2.8 and 13.4 / 3.1, 1,600 prisms 18 / 3.0 and 31 / 3.9, 9,176 prisms
+// 36 / 4.6 and 48 / 3.4.  Below the line it is on trial: a system that it does
+// not solve (a singular one, say) goes to block-Jacobi (krylov_solve).
 constexpr int kAutoMultigridNodes = 20000;
 // Time steps the multigrid's coarse levels are kept for by default.
 constexpr int kDefaultMultigridReuse = 4;
@@ -579,7 +588,9 @@ tf_status create_handle(const tf_mesh* mesh, const tf_material* mat, const tf_op
         return s;
     }
     tf_status s = build(h, mesh, mat, seg_node0, seg_elem0);
-    const bool amg = h->opt.precond >= 2 || (h->opt.precond == 0 && mesh->n_nodes >= kAutoMultigridNodes);
+    const bool large = mesh->n_nodes >= kAutoMultigridNodes;
+    const bool amg = h->opt.precond >= 2 || (h->opt.precond == 0 && (large || !h->opt.deterministic));
+    h->amg_trial = h->opt.precond == 0 && !large;
     if (s == TF_OK && amg) s = amg_build(h, mesh->node_pos);
     if (s != TF_OK) {
         free_all(h);

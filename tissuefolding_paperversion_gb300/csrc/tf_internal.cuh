@@ -423,6 +423,10 @@ struct tf_handle {
     double* du0 = nullptr;                      // the first Newton update of the last step (start of the next)
     bool have_du0 = false;
     tf::Amg* amg = nullptr;                     // multigrid preconditioner (null: block-Jacobi)
+    bool amg_off = false;                       // ... built, but block-Jacobi is used
+    bool amg_trial = false;                     // ... chosen by size: block-Jacobi where a solve with it fails
+    bool amg_failed = false;                    // ... and one has: block-Jacobi from then on
+    bool amg_adjoint = false;                   // ... built for the adjoint's solves only
     tf::Packing* pk = nullptr;                  // packing between tissue surfaces (null: off)
     tf::Growth* growth = nullptr;               // growth functions (null: none added yet)
     double time = 0.0;                          // simulation time (currSimTimeSec), advanced by tf_end_step

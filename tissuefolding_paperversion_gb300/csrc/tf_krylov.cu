@@ -821,6 +821,15 @@ bool build_krylov_loop(tf_handle* h, const Ctx& c, int method) {
     return ok;
 }
 
+// Iterations of a multigrid solve on trial: several times what the hardest
+// systems it suits have needed (packed sheets to 1e-12: 1,400), so a solve that
+// will not converge does not run to the caller's cap first.
+constexpr int kTrialIters = 2000;
+
+int krylov_cap(const tf_handle* h) {
+    return h->amg_trial && use_multigrid(h) ? std::min(h->opt.krylov_max_iter, kTrialIters) : h->opt.krylov_max_iter;
+}
+
 tf_status krylov_run(tf_handle* h, int method, int keep, int* iters, double* relres) {
     Device& d = h->d;
     const Ctx c = make_ctx(h);
@@ -858,7 +867,7 @@ tf_status krylov_run(tf_handle* h, int method, int keep, int* iters, double* rel
         }
     }
     TF_LAUNCH_CHECK(h);
-    const int maxit = h->opt.krylov_max_iter;
+    const int maxit = krylov_cap(h);
     const size_t nscal = (size_t)d.nseg * S_COUNT;
     // Iterations run in graph chunks of 4/8/16/32/64 with a flag check after
     // each batch.  The solve of a step's k-th Newton iteration needs about as
@@ -965,7 +974,7 @@ tf_status krylov_run(tf_handle* h, int method, int keep, int* iters, double* rel
 // geometric stiffness term), so the instances whose CG breaks down are solved
 // again with BiCGStab -- the others keep their CG result -- as the
 // reference's direct LU would not care.
-tf_status krylov_solve(tf_handle* h, int* iters, double* relres) {
+static tf_status krylov_attempt(tf_handle* h, int* iters, double* relres) {
     Device& d = h->d;
     TF_CUDA(cudaMemcpyAsync(d.seg_solve, d.seg_active, sizeof(int) * (size_t)d.nseg, cudaMemcpyDeviceToDevice,
                             h->stream));
@@ -1004,6 +1013,25 @@ tf_status krylov_solve(tf_handle* h, int* iters, double* relres) {
         *iters += it2;
     }
     return s;
+}
+
+// A solve with the multigrid on trial (chosen by size where block-Jacobi is
+// the general path) that fails is done again with block-Jacobi, which then
+// stays for the handle; where that fails too, the system is to blame and its
+// answer is the one block-Jacobi gives.
+tf_status krylov_solve(tf_handle* h, int* iters, double* relres) {
+    const tf_status s = krylov_attempt(h, iters, relres);
+    if (s == TF_OK || !h->amg_trial || !use_multigrid(h) || s == TF_CUDA_ERROR || s == TF_OUT_OF_MEMORY) return s;
+    destroy_graphs(h);  // they hold the multigrid's kernels
+    h->amg_off = true;
+    const tf_status t = krylov_attempt(h, iters, relres);
+    if (t == TF_OK) {
+        h->amg_failed = true;
+    } else {
+        destroy_graphs(h);
+        h->amg_off = false;
+    }
+    return t;
 }
 
 tf_status launch_update(tf_handle* h) {
@@ -1188,7 +1216,7 @@ bool issue_newton_iteration(tf_handle* h, cudaGraphConditionalHandle newton) {
     }
     cudaGraphConditionalHandle kc = 0;
     if (!capture_handle(h, &kc)) return false;
-    k_krylov_arm<<<1, 1, 0, st>>>(h->kloop_ctl, h->opt.krylov_max_iter, kc, 1);
+    k_krylov_arm<<<1, 1, 0, st>>>(h->kloop_ctl, krylov_cap(h), kc, 1);
     bool ok = capture_while(h, kc, [&] {
         issue_iterations(h, c, method, 1);
         k_krylov_ctl<<<1, 32, 0, h->stream>>>(d.scal, d.nseg, h->kloop_ctl, kc);
