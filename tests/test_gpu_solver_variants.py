@@ -126,3 +126,29 @@ def test_iteration_cap_is_the_callers():
         s.assemble()
         out = s.solve(allow_not_converged=True)
         assert out["status"] == api.TF_KRYLOV_NOT_CONVERGED and out["iters"] == 3
+
+
+# The level-0 transfers with the smoothing folded in against the kernels that
+# systems with extra blocks use: an added entry of zero between two far nodes
+# makes such a system of the same matrix.  Both solve it, with Krylov counts
+# within a quarter of each other (the two cycles differ by rounding and the
+# tangent's small asymmetry only).  Sizes: one CTA of nodes, its edge, two
+# with a remainder, and a coarse level that runs kernel by kernel (forked).
+@pytest.mark.parametrize("eta", [0.0, 100.0])
+@pytest.mark.parametrize("nx,ny,layers", [(9, 7, 2), (15, 7, 1), (10, 10, 2), (83, 70, 4)])
+def test_folded_transfers_match_the_kernels_of_extra_blocks(nx, ny, layers, eta):
+    t = _sheet(nx, ny, layers, eta)
+    its = []
+    for extra in (False, True):
+        with api.Solver(t, precond=2, krylov_rtol=RTOL) as s:
+            uk, un = mesh.perturbed_state(t, seed=5)
+            s.set_positions(un)
+            s.begin_step(t.dt)
+            s.set_state(uk, un, t.dt)
+            s.assemble()
+            if extra:
+                s.add_K_triplets([0], [3 * (t.n_nodes - 1)], [0.0])
+            out = s.solve()
+            _check_solution(s, out, [(0, 3 * t.n_nodes)])
+            its.append(out["iters"])
+    assert abs(its[0] - its[1]) <= 0.25 * its[1] + 1, its

@@ -49,13 +49,14 @@
 
 #include <cuda_fp16.h>
 
-#include "tf_internal.cuh"
+#include "tf_reduce.cuh"
 
 namespace tf {
 
 namespace {
 
 constexpr int kT = 256;
+constexpr int kRestrictThreads = 128;  // per coarse node in the level-0 restriction
 constexpr int kCoarseNodes = 16;  // nodes per instance at the coarsest level (96 DOFs)
 constexpr int kCoarseDofs = 6 * kCoarseNodes;
 constexpr int kInvThreads = 512;  // of the coarsest level's inverse
@@ -234,6 +235,25 @@ struct AmgLevel {
     int* check = nullptr;    // checked build: failed index checks
 };
 
+// The level-0 transfer of the V-cycle with the smoothing folded in,
+// Q = (I - omega S) P (pattern of T = A P, 3x6 blocks, FP16 like P's own copy
+// for the transfers): by row in the 32-row slices of the node-parallel kernels
+// (entries 0-15 of a lane's block as two 16-byte packs, 16-17 as one word), and
+// by coarse column.
+struct AmgQ {
+    int* slot0 = nullptr;    // [ncta * kWarps + 1] first slot of each warp's rows
+    int* col = nullptr;      // [nslots * 32] coarse node of each slot and lane
+    uint4* v16 = nullptr;    // [nslots * 2 * 32]
+    uint32_t* v2 = nullptr;  // [nslots * 32]
+    int* cptr = nullptr;     // [n_1 + 1] blocks of each coarse node
+    int* crow = nullptr;     // [nT] fine node of each
+    uint32_t* cval = nullptr;  // [nT][9]
+    // set-up: per T block its P block (-1: none), slice position and column position
+    int* tp = nullptr;
+    int* pos = nullptr;
+    int* cpos = nullptr;
+};
+
 // Lists of the numeric set-up of the transfer from level l to l + 1
 // (device arrays, built once on the host from the block patterns).
 struct AmgSetup {
@@ -261,8 +281,10 @@ struct Amg {
     bool smooth = true;        // smoothed (true) or plain (false) aggregation
     AmgLevel L[kAmgMaxLevels];
     AmgSetup S[kAmgMaxLevels];
+    AmgQ Q;
     double* omega = nullptr;   // [nlev] smoother weights
     double* pscal = nullptr;   // [nlev][2] power-iteration scalars (scale, lambda)
+    float* x1 = nullptr;       // [3 n] the smoothed part of a V-cycle's result (k_q_smooth)
     float* pv = nullptr;       // power-iteration vectors (max n*bs each)
     float* pw = nullptr;
     double* part = nullptr;    // per-CTA partial sums
@@ -323,10 +345,65 @@ void amg_free(Amg* a) {
     if (a->dmat != a->cinv && a->dmat) cudaFree(a->dmat);
     if (a->doff != a->cinv0 && a->doff) cudaFree(a->doff);
     void* ptrs[] = {a->omega, a->pscal, a->pv, a->pw, a->part, a->ticket, a->cnode0, a->cinv0, a->cinv,
-                    a->val32, a->dinv32, a->valh, a->diag32, a->dgroup, a->dwork};
+                    a->val32, a->dinv32, a->valh, a->diag32, a->dgroup, a->dwork,
+                    a->Q.slot0, a->Q.col, a->Q.v16, a->Q.v2, a->Q.cptr, a->Q.crow, a->Q.cval, a->Q.tp, a->Q.pos,
+                    a->Q.cpos, a->x1};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     delete a;
+}
+
+// Layouts of Q (see AmgQ) from the pattern of T = A P.
+static tf_status build_q(const Device& d, AmgQ* q, const std::vector<int>& trowptr, const std::vector<int>& tcol,
+                         const std::vector<int>& prow, const std::vector<int>& pcol, int nc) {
+    const int n = d.nn;
+    const int64_t nT = (int64_t)tcol.size();
+    std::vector<int> c0(d.ncta), c1(d.ncta);
+    TF_CUDA(cudaMemcpy(c0.data(), d.cta_node0, sizeof(int) * (size_t)d.ncta, cudaMemcpyDeviceToHost));
+    TF_CUDA(cudaMemcpy(c1.data(), d.cta_node1, sizeof(int) * (size_t)d.ncta, cudaMemcpyDeviceToHost));
+    std::vector<int> slot0((size_t)d.ncta * kWarps + 1, 0), tp(nT, -1), pos(nT), cpos(nT), cptr(nc + 1, 0), crow(nT);
+    int ns = 0;
+    for (int c = 0; c < d.ncta; ++c)
+        for (int w = 0; w < kWarps; ++w) {
+            const int r0 = c0[c] + 32 * w, r1 = std::min(r0 + 32, c1[c]);
+            slot0[(size_t)c * kWarps + w] = ns;
+            int most = 0;
+            for (int i = r0; i < r1; ++i) {
+                most = std::max(most, trowptr[i + 1] - trowptr[i]);
+                for (int t = trowptr[i]; t < trowptr[i + 1]; ++t) pos[t] = (ns + t - trowptr[i]) * 32 + (i - r0);
+            }
+            ns += most;
+        }
+    slot0[(size_t)d.ncta * kWarps] = ns;
+    std::vector<int> col((size_t)ns * 32, 0);
+    for (int64_t t = 0; t < nT; ++t) {
+        col[pos[t]] = tcol[t];
+        cptr[tcol[t] + 1]++;
+    }
+    for (int J = 0; J < nc; ++J) cptr[J + 1] += cptr[J];
+    {
+        std::vector<int> fill(cptr.begin(), cptr.end() - 1);
+        for (int i = 0; i < n; ++i) {
+            int b = prow[i];
+            for (int t = trowptr[i]; t < trowptr[i + 1]; ++t) {
+                cpos[t] = fill[tcol[t]]++;
+                crow[cpos[t]] = i;
+                while (b < prow[i + 1] && pcol[b] < tcol[t]) ++b;  // both sorted by column
+                if (b < prow[i + 1] && pcol[b] == tcol[t]) tp[t] = b;
+            }
+        }
+    }
+    AMG_TRY(up(&q->slot0, slot0));
+    AMG_TRY(up(&q->col, col));
+    AMG_TRY(zeros(&q->v16, (size_t)ns * 64));
+    AMG_TRY(zeros(&q->v2, (size_t)ns * 32));
+    AMG_TRY(up(&q->cptr, cptr));
+    AMG_TRY(up(&q->crow, crow));
+    AMG_TRY(zeros(&q->cval, (size_t)nT * 9));
+    AMG_TRY(up(&q->tp, tp));
+    AMG_TRY(up(&q->pos, pos));
+    AMG_TRY(up(&q->cpos, cpos));
+    return TF_OK;
 }
 
 // Symbolic set-up from the level-0 pattern, the reference positions and the
@@ -504,6 +581,7 @@ tf_status amg_build(tf_handle* h, const double* pos) {
                 }
             }
         }
+        if (lev == 0) AMG_TRY(build_q(d, &a->Q, trowptr, tcol, prow, pcol, na));
         // coarse pattern: row I joins the T rows of the fine nodes with a
         // block in column I
         HostLevel C;
@@ -659,7 +737,14 @@ tf_status amg_build(tf_handle* h, const double* pos) {
     AMG_TRY(zeros(&a->valh, (size_t)d.nval));
     AMG_TRY(zeros(&a->dinv32, 9 * (size_t)d.nn));
     AMG_TRY(zeros(&a->diag32, 9 * (size_t)d.nn));
+    AMG_TRY(zeros(&a->x1, 3 * (size_t)d.nn));
     AMG_TRY(zeros(&a->pscal, 2 * (size_t)a->nlev));
+    if (!h->side_stream) {
+        TF_CUDA(cudaStreamCreateWithFlags(&h->side_stream, cudaStreamNonBlocking));
+        TF_CUDA(cudaStreamCreateWithFlags(&h->cap_side, cudaStreamNonBlocking));
+        TF_CUDA(cudaEventCreateWithFlags(&h->fork_ev, cudaEventDisableTiming));
+        TF_CUDA(cudaEventCreateWithFlags(&h->join_ev, cudaEventDisableTiming));
+    }
     AMG_TRY(zeros(&a->pv, maxv));
     AMG_TRY(zeros(&a->pw, maxv));
     int64_t maxc = 0;  // CTAs of the warp-per-row power iteration on the coarse levels
@@ -1163,6 +1248,40 @@ __global__ void k_ap(AmgLevel F, AmgSetup S, const int* __restrict__ bofs0, cons
     for (int c = 0; c < 6; ++c) out[c] = acc[c];
 }
 
+// Q = (I - omega S) P in its two layouts, one thread per block (i, J):
+// P_iJ - omega D_i^-1 T_iJ.
+__global__ void k_make_q(AmgQ Q, AmgSetup S, const float* __restrict__ Pv, const float* __restrict__ dinv,
+                         const double* __restrict__ omega) {
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= S.nT) return;
+    const int i = S.trow[t], b = Q.tp[t];
+    const float om = (float)__ldg(omega);
+    const float* __restrict__ T = S.T + 18 * (size_t)t;
+    const float* __restrict__ D = dinv + 9 * (size_t)i;
+    float v[18];
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+#pragma unroll
+        for (int c = 0; c < 6; ++c) {
+            const float s = fmaf(__ldg(&D[3 * r]), __ldg(&T[c]),
+                                 fmaf(__ldg(&D[3 * r + 1]), __ldg(&T[6 + c]), __ldg(&D[3 * r + 2]) * __ldg(&T[12 + c])));
+            v[6 * r + c] = fmaf(-om, s, b >= 0 ? __ldg(&Pv[18 * (size_t)b + 6 * r + c]) : 0.f);
+        }
+    uint32_t w[9];
+#pragma unroll
+    for (int k = 0; k < 9; ++k)
+        w[k] = (uint32_t)__half_as_ushort(__float2half_rn(v[2 * k])) |
+               ((uint32_t)__half_as_ushort(__float2half_rn(v[2 * k + 1])) << 16);
+    const int p = Q.pos[t], lane = p & 31;
+    const size_t s = (size_t)(p >> 5);
+    Q.v16[64 * s + lane] = make_uint4(w[0], w[1], w[2], w[3]);
+    Q.v16[64 * s + 32 + lane] = make_uint4(w[4], w[5], w[6], w[7]);
+    Q.v2[32 * s + lane] = w[8];
+    uint32_t* __restrict__ o = Q.cval + 9 * (size_t)Q.cpos[t];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) o[k] = w[k];
+}
+
 // Coarse block c = (I, J), row p: sum over its pairs (P_iI, T_iJ) of
 // (P_iI^T T_iJ)(p, :).
 template <int BS>
@@ -1466,16 +1585,145 @@ struct V0 {  // level-0 operands
     const float* diag32;  // diagonal blocks D, FP32 [9 n]
 };
 
-// x = omega D^-1 r  (r is the Krylov method's FP64 vector)
-__global__ void k_v0_pre(V0 a, const double* __restrict__ r, float* __restrict__ x) {
+// The level-0 part of a V-cycle: pre-sweep from zero x = omega D^-1 r, residual
+// t = r - A x, coarse correction x += P e, post-sweep x += omega D^-1 (r - A x).
+// With S = D^-1 A and z = omega D^-1 r the result is
+//     (2 z - omega S z) + Q e,   Q = (I - omega S) P,
+// and the restricted residual P^T (r - A z) is Q^T r for a symmetric A (the
+// viscous tangent's asymmetry, of the order of eta |grad v| / E, only changes
+// the preconditioner).  So the smoother's matrix is read once instead of twice,
+// and that product does not wait for the coarse levels: k_q_restrict (Q^T r),
+// the coarse levels, k_q_post; k_q_smooth runs beside the coarse levels where
+// those are a chain of launches, and is part of k_q_post where they are one
+// dense product.  Bound by reading S (66 MB at 320,000 prisms) and Q twice (52 MB
+// each): 77 us of kernels before (pre, residual, restriction, prolongation,
+// post), 19 + 14 us now with 16 us beside the coarse levels; 32.3 -> 30.3 ms per
+// 320,000-prism step, 46.6 -> 38.2 ms per step of 32 batched tissues.  Systems
+// with extra blocks (packing couples, added entries) keep the kernels that apply
+// the current matrix: k_v0_resid .. k_v0_post below.
+
+// r_C(I) = sum over the blocks (i, I) of Q_iI^T r_i, and the coarse level's first
+// sweep; one CTA of kRestrictThreads per coarse node, its threads striding over
+// the (block, row) pairs of the column, stored contiguously.
+__global__ void __launch_bounds__(kRestrictThreads) k_q_restrict(AmgQ Q, AmgLevel C, int nf, int* check,
+                                                                 const float* __restrict__ r,
+                                                                 const double* __restrict__ scal,
+                                                                 const double* __restrict__ omegaC, int presmooth) {
+    __shared__ float sm[kRestrictThreads / 32][6];
+    pdl_enter();
+    const int I = blockIdx.x;
+    if (seg_stopped(scal, C.seg[I])) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int q0 = __ldg(&Q.cptr[I]), np = 3 * (__ldg(&Q.cptr[I + 1]) - q0);
+    float rc[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+    for (int q = threadIdx.x; q < np; q += kRestrictThreads) {
+        const int m = q / 3, k = q - 3 * m;
+        const int i = __ldg(&Q.crow[q0 + m]);
+        if (!TF_IN(check, i, nf, CK_RESTRICT_ROW)) continue;
+        const float t = r[3 * (size_t)i + k];
+        const __half2* __restrict__ P = reinterpret_cast<const __half2*>(Q.cval + 9 * (size_t)(q0 + m) + 3 * k);
+#pragma unroll
+        for (int b = 0; b < 3; ++b) {
+            const float2 f = __half22float2(__ldg(&P[b]));
+            rc[2 * b] = fmaf(f.x, t, rc[2 * b]);
+            rc[2 * b + 1] = fmaf(f.y, t, rc[2 * b + 1]);
+        }
+    }
+#pragma unroll
+    for (int b = 0; b < 6; ++b)
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) rc[b] += __shfl_xor_sync(0xffffffffu, rc[b], o);
+    if (lane < 6) sm[warp][lane] = pick6(rc, lane);
+    __syncthreads();
+    if (warp > 0) return;
+#pragma unroll
+    for (int b = 0; b < 6; ++b) {
+        rc[b] = 0.f;
+#pragma unroll
+        for (int w = 0; w < kRestrictThreads / 32; ++w) rc[b] += sm[w][b];
+    }
+    if (lane < 6) {
+        C.r[6 * I + lane] = pick6(rc, lane);
+        if (presmooth) C.x[6 * I + lane] = (float)__ldg(omegaC) * lane_mul6(C.dinv + 36 * (size_t)I, rc, lane);
+    }
+}
+
+// x = 2 z - omega S z
+template <int U>
+__global__ void k_q_smooth(V0 a, const float* __restrict__ z, float* __restrict__ x) {
     pdl_enter();
     const Node0 q = node0(a.d);
     if (!q.valid || seg_stopped(a.d.scal, q.seg)) return;
+    float y[3];
+    row0s<U>(a.d, a.valh, a.dinv32, z, q.i, y);
     const float om = (float)__ldg(a.omega);
-    float rr[3] = {(float)r[3 * q.i], (float)r[3 * q.i + 1], (float)r[3 * q.i + 2]}, z[3];
-    mul3(a.dinv32 + 9 * (size_t)q.i, rr, z);
 #pragma unroll
-    for (int k = 0; k < 3; ++k) x[3 * q.i + k] = om * z[k];
+    for (int k = 0; k < 3; ++k) x[3 * q.i + k] = fmaf(-om, y[k], 2.f * z[3 * q.i + k]);
+}
+
+// (Q e)_i added to x
+__device__ __forceinline__ void row_q(const AmgQ& Q, const float* __restrict__ e, int nc, int* check, float x[3]) {
+    const int lane = threadIdx.x & 31;
+    const int wg = blockIdx.x * kWarps + (threadIdx.x >> 5);
+    const int s0 = __ldg(&Q.slot0[wg]), s1 = __ldg(&Q.slot0[wg + 1]);
+#pragma unroll 4
+    for (int s = s0; s < s1; ++s) {
+        const int J = __ldg(&Q.col[32 * (size_t)s + lane]);
+        if (!TF_IN(check, J, nc, CK_PROLONG_COL)) continue;
+        const uint4 a = __ldg(&Q.v16[64 * (size_t)s + lane]), b = __ldg(&Q.v16[64 * (size_t)s + 32 + lane]);
+        const uint32_t c = __ldg(&Q.v2[32 * (size_t)s + lane]);
+        const float2* __restrict__ ej = reinterpret_cast<const float2*>(e + 6 * (size_t)J);
+        const float2 e0 = ej[0], e1 = ej[1], e2 = ej[2];
+        const uint32_t w[9] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, c};
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const float2 f0 = __half22float2(*reinterpret_cast<const __half2*>(&w[3 * k]));
+            const float2 f1 = __half22float2(*reinterpret_cast<const __half2*>(&w[3 * k + 1]));
+            const float2 f2 = __half22float2(*reinterpret_cast<const __half2*>(&w[3 * k + 2]));
+            x[k] = fmaf(f0.x, e0.x, fmaf(f0.y, e0.y, fmaf(f1.x, e1.x, fmaf(f1.y, e1.y,
+                   fmaf(f2.x, e2.x, fmaf(f2.y, e2.y, x[k]))))));
+        }
+    }
+}
+
+// out = x + Q e, x = 2 z - omega S z read from k_q_smooth (SMOOTH: formed here
+// from z), as the FP64 preconditioned vector.  DOT: with (r, out) and CG's beta
+// (start: the first of a solve, which also sets p = out).
+template <int U, bool SMOOTH, bool DOT>
+__global__ void k_q_post(V0 a, Ctx c, AmgQ Q, int nc, const float* __restrict__ zx, const float* __restrict__ e,
+                         double* __restrict__ out, const double* __restrict__ r, double* __restrict__ p, int start) {
+    pdl_enter();
+    const Node0 q = node0(a.d);
+    if (seg_stopped(a.d.scal, q.seg)) return;
+    double v[1] = {0.0};
+    if (q.valid) {
+        float x[3];
+        if constexpr (SMOOTH) {
+            row0s<U>(a.d, a.valh, a.dinv32, zx, q.i, x);
+            const float om = (float)__ldg(a.omega);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) x[k] = fmaf(-om, x[k], 2.f * zx[3 * q.i + k]);
+        } else {
+#pragma unroll
+            for (int k = 0; k < 3; ++k) x[k] = zx[3 * q.i + k];
+        }
+        row_q(Q, e, nc, a.d.check, x);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const double o = (double)x[k];
+            out[3 * q.i + k] = o;
+            if constexpr (DOT) {
+                if (start) p[3 * q.i + k] = o;
+                v[0] = fma(r[3 * q.i + k], o, v[0]);
+            }
+        }
+    }
+    if constexpr (DOT) {
+        double tot[1];
+        if (reduce_seg<1>(c, q.seg, v, tot) && threadIdx.x == 0)
+            cg_rz(a.d.scal + (size_t)q.seg * S_COUNT, tot[0], start != 0);
+    }
 }
 
 // t = r - A x
@@ -2065,6 +2313,10 @@ tf_status amg_numeric(tf_handle* h) {
             k_f32_to_h<<<4 * 152, kT, 0, st>>>(L.npb * L.bs * 6, L.Pc, L.Pch);
             TF_LAUNCH_CHECK(h);
         }
+        if (l == 0 && d.nxb == 0) {  // a new extra-block layout rebuilds everything
+            k_make_q<<<cdiv(S.nT, kT), kT, 0, st>>>(a->Q, S, L.Pv, a->dinv32, a->omega);
+            TF_LAUNCH_CHECK(h);
+        }
         if (l == 0) k_ptap<3><<<cdiv(C.nnzb * 6, kT), kT, 0, st>>>(L, S, C);
         else k_ptap<6><<<cdiv(C.nnzb * 6, kT), kT, 0, st>>>(L, S, C);
         TF_LAUNCH_CHECK(h);
@@ -2146,17 +2398,60 @@ tf_status amg_autotune(tf_handle* h) {
 
 int amg_smoother_unroll(const tf_handle* h) { return use_multigrid(h) ? h->amg->smooth_unroll : 0; }
 
+// Level 0 through Q (k_q_restrict ..): every system without extra blocks.
+static bool uses_q(const tf_handle* h) { return h->d.nxb == 0; }
+
+// k_q_smooth beside the coarse levels: where those are a chain of launches
+// (level 1 kernel by kernel) there is time to hide it in.
+static bool forks(const Amg* a) { return a->dense != 1; }
+
+bool amg_fuses_dot(const tf_handle* h) { return use_multigrid(h) && uses_q(h); }
+
+AmgPre amg_pre(const tf_handle* h) {
+    if (!use_multigrid(h)) return AmgPre{nullptr, nullptr, nullptr, nullptr};
+    const Amg* a = h->amg;
+    return AmgPre{a->dinv32, a->omega, a->L[0].x, a->L[0].t};
+}
+
 int amg_vcycle_kernels(const tf_handle* h) {
     const Amg* a = h->amg;
     const int per = 2 * kCoarseSweeps + 2;  // kernels of a coarse level run kernel by kernel
-    if (a->dense > 0) return 5 + per * (a->dense - 1) + 1;
-    return 5 + per * (a->nlev - 2) + 3;
+    const int fine = uses_q(h) ? (forks(a) ? 3 : 2) : 4;
+    if (a->dense > 0) return fine + per * (a->dense - 1) + 1;
+    return fine + per * (a->nlev - 2) + 3;
 }
 
-// out = M^-1 r: one V-cycle (all launches on h->stream, no host work).
-// Levels above `dense` run kernel by kernel over all instances; `dense` and
-// the levels below it are one product with their dense operator.
-void amg_vcycle(tf_handle* h, const double* r, double* out) {
+template <int U>
+static void launch_q_smooth(tf_handle* h, cudaStream_t st, const V0& v0, const float* z, float* x) {
+    k_q_smooth<U><<<h->d.ncta, kNodeThreads, 0, st>>>(v0, z, x);
+}
+
+// The last kernel of a V-cycle through Q.  After k_q_smooth on the side
+// stream it has two predecessors, so it is an ordinary launch there.
+template <int U, bool SMOOTH>
+static void launch_q_post(tf_handle* h, const V0& v0, const float* zx, double* out, const double* r, double* p,
+                          int dot) {
+    Amg* a = h->amg;
+    const Ctx c = make_ctx(h);
+    const int nb = h->d.ncta, nc = a->L[1].n;
+    const float* e = a->L[1].e;
+    if constexpr (SMOOTH) {
+        if (dot) launch_pdl(k_q_post<U, true, true>, nb, kNodeThreads, h->stream, v0, c, a->Q, nc, zx, e, out, r, p,
+                            dot == kVcycleStart ? 1 : 0);
+        else launch_pdl(k_q_post<U, true, false>, nb, kNodeThreads, h->stream, v0, c, a->Q, nc, zx, e, out, r, p, 0);
+    } else {
+        if (dot) k_q_post<U, false, true><<<nb, kNodeThreads, 0, h->stream>>>(v0, c, a->Q, nc, zx, e, out, r, p,
+                                                                            dot == kVcycleStart ? 1 : 0);
+        else k_q_post<U, false, false><<<nb, kNodeThreads, 0, h->stream>>>(v0, c, a->Q, nc, zx, e, out, r, p, 0);
+    }
+}
+
+// out = M^-1 r: one V-cycle (all launches on h->stream and, joined to it, the
+// side stream; no host work).  The input's FP32 copy and first sweep are in
+// place (AmgPre).  Levels above `dense` run kernel by kernel over all
+// instances; `dense` and the levels below it are one product with their dense
+// operator.
+void amg_vcycle(tf_handle* h, const double* r, double* out, int dot, double* p) {
     Amg* a = h->amg;
     Device& d = h->d;
     cudaStream_t st = h->stream;
@@ -2165,14 +2460,29 @@ void amg_vcycle(tf_handle* h, const double* r, double* out) {
     V0 v0{d, a->omega, a->dinv32, a->valh, a->diag32};
     AmgLevel& L0 = a->L[0];
     auto presmooth = [&](int l) { return l == a->dense ? 0 : 1; };
-    launch_pdl(k_v0_pre, d.ncta, kNodeThreads, st, v0, r, L0.x);
-    switch (a->smooth_unroll) {
-        case 2: launch_pdl(k_v0_resid<2>, d.ncta, kNodeThreads, st, v0, r, L0.x, L0.t); break;
-        case 8: launch_pdl(k_v0_resid<8>, d.ncta, kNodeThreads, st, v0, r, L0.x, L0.t); break;
-        default: launch_pdl(k_v0_resid<4>, d.ncta, kNodeThreads, st, v0, r, L0.x, L0.t); break;
+    const bool q = uses_q(h), fork = q && forks(a);
+    if (q) {
+        if (fork) {
+            cudaEventRecord(h->fork_ev, st);
+            cudaStreamWaitEvent(h->side_stream, h->fork_ev, 0);
+            switch (a->smooth_unroll) {
+                case 2: launch_q_smooth<2>(h, h->side_stream, v0, L0.x, a->x1); break;
+                case 8: launch_q_smooth<8>(h, h->side_stream, v0, L0.x, a->x1); break;
+                default: launch_q_smooth<4>(h, h->side_stream, v0, L0.x, a->x1); break;
+            }
+            cudaEventRecord(h->join_ev, h->side_stream);
+        }
+        launch_pdl(k_q_restrict, a->L[1].n, kRestrictThreads, st, a->Q, a->L[1], L0.n, L0.check, (const float*)L0.t,
+                   (const double*)d.scal, (const double*)(a->omega + 1), presmooth(1));
+    } else {
+        switch (a->smooth_unroll) {
+            case 2: launch_pdl(k_v0_resid<2>, d.ncta, kNodeThreads, st, v0, r, L0.x, L0.t); break;
+            case 8: launch_pdl(k_v0_resid<8>, d.ncta, kNodeThreads, st, v0, r, L0.x, L0.t); break;
+            default: launch_pdl(k_v0_resid<4>, d.ncta, kNodeThreads, st, v0, r, L0.x, L0.t); break;
+        }
+        launch_pdl(k_restrict<3>, cdiv(32 * (int64_t)a->L[1].n, kT), kT, st, L0, a->L[1], (const float*)L0.t,
+                   (const double*)d.scal, (const double*)(a->omega + 1), presmooth(1));
     }
-    launch_pdl(k_restrict<3>, cdiv(32 * (int64_t)a->L[1].n, kT), kT, st, L0, a->L[1], (const float*)L0.t,
-               (const double*)d.scal, (const double*)(a->omega + 1), presmooth(1));
     float* cur[kAmgMaxLevels] = {};
     for (int l = 1; l < stop; ++l) {
         AmgLevel& L = a->L[l];
@@ -2211,6 +2521,19 @@ void amg_vcycle(tf_handle* h, const double* r, double* out) {
                        (const double*)(a->omega + l), (const float*)x, o);
             x = o;
         }
+    }
+    if (q) {
+        if (fork) {
+            cudaStreamWaitEvent(st, h->join_ev, 0);
+            launch_q_post<4, false>(h, v0, a->x1, out, r, p, dot);
+        } else {
+            switch (a->smooth_unroll) {
+                case 2: launch_q_post<2, true>(h, v0, L0.x, out, r, p, dot); break;
+                case 8: launch_q_post<8, true>(h, v0, L0.x, out, r, p, dot); break;
+                default: launch_q_post<4, true>(h, v0, L0.x, out, r, p, dot); break;
+            }
+        }
+        return;
     }
     launch_pdl_smem(k_v0_prolong, d.ncta, kNodeThreads, (size_t)a->v0_smem, st, v0, L0, (const float*)a->L[1].e,
                     L0.x);

@@ -130,6 +130,13 @@ void free_all(tf_handle* h) {
     if (h->nd_seg) cudaFree(h->nd_seg);
     if (h->nd_seg_host) cudaFreeHost(h->nd_seg_host);
     if (h->cap_stream) cudaStreamDestroy(h->cap_stream);
+    if (h->side_stream) cudaStreamDestroy(h->side_stream);
+    if (h->cap_side) cudaStreamDestroy(h->cap_side);
+    h->cap_side = nullptr;
+    if (h->fork_ev) cudaEventDestroy(h->fork_ev);
+    if (h->join_ev) cudaEventDestroy(h->join_ev);
+    h->side_stream = nullptr;
+    h->fork_ev = h->join_ev = nullptr;
     h->nd = nullptr;
     h->nd_host = nullptr;
     h->nd_seg = nullptr;

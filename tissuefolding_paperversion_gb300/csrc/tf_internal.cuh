@@ -408,6 +408,9 @@ struct tf_handle {
     bool nloop_off = false;                     // that graph could not be built here: host-driven iterations
     int64_t nloop_kernels = 0;                  // kernels of one of its Newton iterations outside the Krylov loop
     cudaStream_t cap_stream = nullptr;          // second stream for capturing nested loop bodies
+    cudaStream_t side_stream = nullptr;         // branch of the V-cycle beside its coarse levels
+    cudaStream_t cap_side = nullptr;            // its partner while nested loop bodies are captured
+    cudaEvent_t fork_ev = nullptr, join_ev = nullptr;
     tf::NewtonDev* nd = nullptr;                // device Newton-loop state and its pinned mirror
     tf::NewtonDev* nd_host = nullptr;
     int* nd_seg = nullptr;                      // device [3][nseg]: Newton iterations, converged, capped
@@ -475,8 +478,21 @@ void amg_refresh(tf_handle* h);     // launches the level-0 smoother copies of t
 tf_status amg_autotune(tf_handle* h);  // picks the level-0 smoother's row-product variant by timing
 int amg_smoother_unroll(const tf_handle* h);
 void amg_refreshed(tf_handle* h);   // records that amg_refresh ran for the current assembly
-void amg_vcycle(tf_handle* h, const double* r, double* out);
+// out = M^-1 r; dot: what the last kernel does besides (CG): (r, out) with beta,
+// or the same at the start of a solve with p = out (amg_fuses_dot).
+enum VcycleDot { kVcyclePlain = 0, kVcycleDot = 1, kVcycleStart = 2 };
+void amg_vcycle(tf_handle* h, const double* r, double* out, int dot = kVcyclePlain, double* p = nullptr);
+bool amg_fuses_dot(const tf_handle* h);
 int amg_vcycle_kernels(const tf_handle* h);
+// Where the kernel that makes a V-cycle's input leaves it and its first sweep
+// (z null: no multigrid).
+struct AmgPre {
+    const float* dinv32;
+    const double* omega;
+    float* z;
+    float* r;
+};
+AmgPre amg_pre(const tf_handle* h);
 void amg_free(Amg* a);
 void amg_mark_stale(tf_handle* h, int level);  // 1: new assembly, 2: rebuild the hierarchy
 tf_status packing_setup(tf_handle* h, int flags); // switch packing on (device tables)

@@ -22,112 +22,11 @@
 #include <cstring>
 #include <vector>
 
-#include "tf_internal.cuh"
+#include "tf_reduce.cuh"
 
 namespace tf {
 
 namespace {
-
-constexpr int kThreads = kNodeThreads;
-
-enum Flag { F_RUNNING = 0, F_CONVERGED = 1, F_BREAKDOWN = 2, F_NAN = 3 };
-// Cause of a breakdown (S_WHY): which denominator vanished.
-enum Why { W_NONE = 0, W_CG_PAP = 1, W_CG_RZ = 2, W_BI_RV = 3, W_BI_OMEGA = 4, W_BI_RHO = 5 };
-const char* const kWhy[] = {"", "(p, Ap) <= 0", "(r, M^-1 r) <= 0", "(rhat, A phat) = 0", "omega = 0",
-                            "(rhat, r) = 0"};
-
-struct Ctx {
-    const int* __restrict__ wslot0;
-    const int* __restrict__ scol;
-    const double* __restrict__ val;
-    const double* __restrict__ dinv;
-    double* scal;               // [nseg][S_COUNT]
-    double* part;               // [3][ncta]
-    unsigned* tickets;          // [nseg]
-    int ncta;
-    const int* __restrict__ cta_seg;
-    const int* __restrict__ cta_node0;
-    const int* __restrict__ cta_node1;
-    const int* __restrict__ seg_cta0;
-    const int* __restrict__ seg_solve;
-    const int* __restrict__ xrow;     // extra blocks (tf_add_K_triplets), null: none
-    const int* __restrict__ xcol;
-    const double* __restrict__ xval;
-    int nn;
-    int* check;                       // checked build: failed index checks
-};
-
-struct Where {
-    int node;    // node of this thread
-    bool valid;  // node inside this CTA's range
-    int seg;     // instance of this CTA
-    double* s;   // its scalars
-};
-
-__device__ __forceinline__ Where where(const Ctx& c) {
-    Where w;
-    w.seg = c.cta_seg[blockIdx.x];
-    w.node = c.cta_node0[blockIdx.x] + threadIdx.x;
-    w.valid = w.node < c.cta_node1[blockIdx.x];
-    w.s = c.scal + (size_t)w.seg * S_COUNT;
-    return w;
-}
-
-template <int NV>
-__device__ __forceinline__ void block_sum(double (&v)[NV], double (*sm)[kThreads / 32]) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int k = 0; k < NV; ++k) {
-        double x = v[k];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-        if (lane == 0) sm[k][warp] = x;
-    }
-    __syncthreads();
-    if (warp == 0) {
-#pragma unroll
-        for (int k = 0; k < NV; ++k) {
-            double x = lane < kThreads / 32 ? sm[k][lane] : 0.0;
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-            v[k] = x;  // valid in thread 0
-        }
-    }
-    __syncthreads();
-}
-
-// Writes this CTA's partial sums; returns true in the CTA of the instance
-// that arrives last, whose thread 0 then holds the fixed-order totals.
-template <int NV>
-__device__ bool reduce_seg(const Ctx& c, int seg, double (&v)[NV], double (&tot)[NV]) {
-    __shared__ double sm[NV][kThreads / 32];
-    __shared__ bool last;
-    block_sum<NV>(v, sm);
-    const int b0 = c.seg_cta0[seg], b1 = c.seg_cta0[seg + 1];
-    if (threadIdx.x == 0) {
-#pragma unroll
-        for (int k = 0; k < NV; ++k) c.part[(size_t)k * c.ncta + blockIdx.x] = v[k];
-        __threadfence();
-        const unsigned ticket = atomicAdd(&c.tickets[seg], 1u);
-        last = (ticket == (unsigned)(b1 - b0 - 1));
-    }
-    __syncthreads();
-    if (!last) return false;
-    __threadfence();
-    double acc[NV];
-#pragma unroll
-    for (int k = 0; k < NV; ++k) {
-        acc[k] = 0.0;
-        for (int b = b0 + threadIdx.x; b < b1; b += kThreads) acc[k] += __ldcg(&c.part[(size_t)k * c.ncta + b]);
-    }
-    block_sum<NV>(acc, sm);
-#pragma unroll
-    for (int k = 0; k < NV; ++k) tot[k] = acc[k];
-    if (threadIdx.x == 0) c.tickets[seg] = 0u;
-    return true;
-}
-
-__device__ __forceinline__ bool stopped(const Where& w) { return __ldcg(&w.s[S_FLAG]) != 0.0; }
 
 __device__ __forceinline__ void apply_dinv(const double* __restrict__ D, const double r[3], double z[3]) {
     z[0] = fma(D[0], r[0], fma(D[1], r[1], D[2] * r[2]));
@@ -171,6 +70,21 @@ __device__ __forceinline__ void start_flags(double* s, double bb, double tol2, d
     s[S_FLAG] = (bb == 0.0 || rr <= tol2 * bb) ? F_CONVERGED : (isfinite(bb) && isfinite(rr) ? F_RUNNING : F_NAN);
 }
 
+// What the V-cycle starts from, written by the kernel that makes its input v:
+// v in FP32 and the first sweep z = omega D^-1 v (nothing with block-Jacobi).
+__device__ __forceinline__ void pre_smooth(const AmgPre& a, int i, const double v[3]) {
+    if (!a.z) return;
+    const float om = (float)__ldg(a.omega);
+    const float f[3] = {(float)v[0], (float)v[1], (float)v[2]};
+    const float* __restrict__ D = a.dinv32 + 9 * (size_t)i;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        a.r[3 * i + k] = f[k];
+        a.z[3 * i + k] =
+            om * fmaf(__ldg(&D[3 * k]), f[0], fmaf(__ldg(&D[3 * k + 1]), f[1], __ldg(&D[3 * k + 2]) * f[2]));
+    }
+}
+
 // ---- CG -------------------------------------------------------------------
 
 // r = b, z = M^-1 r, p = z, x = 0;  rz = (r,z), bb = (b,b).  Instances left
@@ -179,7 +93,7 @@ __device__ __forceinline__ void start_flags(double* s, double bb, double tol2, d
 // Newton loop has stopped); both are flagged done at once.
 __global__ void k_cg_init(Ctx c, const double* __restrict__ b, double* __restrict__ x, double* __restrict__ r,
                           double* __restrict__ z, double* __restrict__ p, double tol2, double atol, int keep,
-                          int jac, const double* __restrict__ x0) {
+                          int jac, const double* __restrict__ x0, AmgPre pre) {
     const Where w = where(c);
     const bool active = c.seg_solve[w.seg] != 0;
     if (!active && keep) {
@@ -209,6 +123,7 @@ __global__ void k_cg_init(Ctx c, const double* __restrict__ b, double* __restric
                 v[0] = fma(rr[d], zz[d], v[0]);
             }
         }
+        pre_smooth(pre, i, rr);
 #pragma unroll
         for (int d = 0; d < 3; ++d) v[1] = fma(rr[d], rr[d], v[1]);
     }
@@ -250,7 +165,7 @@ __global__ void k_cg_spmv(Ctx c, const double* __restrict__ p, double* __restric
 
 // x += alpha p; r -= alpha q; z = M^-1 r;  beta = (r,z)_new / (r,z)
 __global__ void k_cg_update(Ctx c, double* __restrict__ x, double* __restrict__ r, double* __restrict__ z,
-                            const double* __restrict__ p, const double* __restrict__ q, int jac) {
+                            const double* __restrict__ p, const double* __restrict__ q, int jac, AmgPre pre) {
     pdl_enter();
     const Where w = where(c);
     if (stopped(w)) return;
@@ -274,6 +189,7 @@ __global__ void k_cg_update(Ctx c, double* __restrict__ x, double* __restrict__ 
                 v[0] = fma(rr[d], zz[d], v[0]);
             }
         }
+        pre_smooth(pre, i, rr);
 #pragma unroll
         for (int d = 0; d < 3; ++d) v[1] = fma(rr[d], rr[d], v[1]);
     }
@@ -296,7 +212,8 @@ __global__ void k_cg_update(Ctx c, double* __restrict__ x, double* __restrict__ 
     }
 }
 
-// With the multigrid preconditioner (z = M^-1 r computed between kernels):
+// With the multigrid preconditioner (z = M^-1 r computed between kernels), where
+// its last kernel does not do it (systems with extra blocks):
 // rz = (r, z), beta = rz / rz_old; start != 0 also sets p = z (first step).
 __global__ void k_cg_rz(Ctx c, const double* __restrict__ r, const double* __restrict__ z, double* __restrict__ p,
                         int start) {
@@ -312,18 +229,7 @@ __global__ void k_cg_rz(Ctx c, const double* __restrict__ r, const double* __res
             if (start) p[k] = z[k];
         }
     double tot[1];
-    if (reduce_seg<1>(c, w.seg, v, tot) && threadIdx.x == 0) {
-        double* s = w.s;
-        const double rz = tot[0];
-        if (!start) s[S_BETA] = rz / s[S_RZ];
-        s[S_RZ] = rz;
-        if (!isfinite(rz)) {
-            s[S_FLAG] = F_NAN;
-        } else if (!(rz > 0.0)) {
-            s[S_FLAG] = F_BREAKDOWN;
-            s[S_WHY] = W_CG_RZ;
-        }
-    }
+    if (reduce_seg<1>(c, w.seg, v, tot) && threadIdx.x == 0) cg_rz(w.s, tot[0], start);
 }
 
 // p = z + beta p
@@ -381,7 +287,7 @@ __global__ void k_bi_init(Ctx c, const double* __restrict__ b, double* __restric
 
 // p = r + beta (p - omega v); phat = M^-1 p
 __global__ void k_bi_dir(Ctx c, const double* __restrict__ r, const double* __restrict__ v, double* __restrict__ p,
-                         double* __restrict__ phat, int jac) {
+                         double* __restrict__ phat, int jac, AmgPre pre) {
     pdl_enter();
     const Where w = where(c);
     if (stopped(w) || !w.valid) return;
@@ -394,6 +300,7 @@ __global__ void k_bi_dir(Ctx c, const double* __restrict__ r, const double* __re
         pp[d] = fma(beta, fma(-omega, v[k], p[k]), r[k]);
         p[k] = pp[d];
     }
+    pre_smooth(pre, i, pp);
     if (!jac) return;
     apply_dinv(c.dinv + 9 * (size_t)i, pp, z);
 #pragma unroll
@@ -430,10 +337,10 @@ __global__ void k_bi_spmv1(Ctx c, const double* __restrict__ phat, const double*
 }
 
 // s = r - alpha v; shat = M^-1 s; |s|^2.  When |s| already meets the
-// tolerance the half step is the solution: x += alpha phat and stop (t and
-// omega would otherwise be formed from a vanishing s).
+// tolerance the half step is the solution: k_bi_spmv2 then does x += alpha phat
+// and stops (t and omega would otherwise be formed from a vanishing s).
 __global__ void k_bi_s(Ctx c, const double* __restrict__ r, const double* __restrict__ v, double* __restrict__ s,
-                       double* __restrict__ shat, double* __restrict__ x, const double* __restrict__ phat, int jac) {
+                       double* __restrict__ shat, int jac, AmgPre pre) {
     pdl_enter();
     const Where w = where(c);
     if (stopped(w)) return;
@@ -454,6 +361,7 @@ __global__ void k_bi_s(Ctx c, const double* __restrict__ r, const double* __rest
 #pragma unroll
             for (int d = 0; d < 3; ++d) shat[3 * i + d] = z[d];
         }
+        pre_smooth(pre, i, ss);
     }
     double tot[1];
     if (reduce_seg<1>(c, w.seg, acc, tot) && threadIdx.x == 0) {
@@ -465,33 +373,30 @@ __global__ void k_bi_s(Ctx c, const double* __restrict__ r, const double* __rest
     }
 }
 
-// Applies the half step x += alpha phat of instances flagged -1 by k_bi_s
-// and marks them converged.
-__global__ void k_bi_half(Ctx c, double* __restrict__ x, const double* __restrict__ phat) {
-    pdl_enter();
-    const Where w = where(c);
-    if (__ldcg(&w.s[S_FLAG]) != -1.0) return;
-    const double alpha = __ldcg(&w.s[S_ALPHA]);
-    if (w.valid)
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            const int k = 3 * w.node + d;
-            x[k] = fma(alpha, phat[k], x[k]);
-        }
-    double tot[1] = {0.0}, v[1] = {0.0};
-    if (reduce_seg<1>(c, w.seg, v, tot) && threadIdx.x == 0) {
-        w.s[S_ITER] += 1.0;
-        w.s[S_FLAG] = F_CONVERGED;
-    }
-}
-
-// t = A shat; omega = (t, s) / (t, t)
+// t = A shat; omega = (t, s) / (t, t).  An instance flagged -1 by k_bi_s takes
+// its half step x += alpha phat here and is marked converged.
 template <int U>
 __global__ void k_bi_spmv2(Ctx c, const double* __restrict__ shat, const double* __restrict__ s,
-                           double* __restrict__ t) {
+                           double* __restrict__ t, double* __restrict__ x, const double* __restrict__ phat) {
     pdl_enter();
     const Where w = where(c);
-    if (stopped(w)) return;
+    const double flag = __ldcg(&w.s[S_FLAG]);
+    if (flag == -1.0) {
+        const double alpha = __ldcg(&w.s[S_ALPHA]);
+        if (w.valid)
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                const int k = 3 * w.node + d;
+                x[k] = fma(alpha, phat[k], x[k]);
+            }
+        double none[1] = {0.0}, all[1];
+        if (reduce_seg<1>(c, w.seg, none, all) && threadIdx.x == 0) {
+            w.s[S_ITER] += 1.0;
+            w.s[S_FLAG] = F_CONVERGED;
+        }
+        return;
+    }
+    if (flag != 0.0) return;
     double acc[2] = {0.0, 0.0};
     if (w.valid) {
         double y[3];
@@ -618,30 +523,6 @@ __global__ void k_update(Ctx c, double* __restrict__ uk, const double* __restric
     }
 }
 
-Ctx make_ctx(tf_handle* h) {
-    Device& d = h->d;
-    Ctx c;
-    c.wslot0 = d.wslot0;
-    c.scol = d.scol;
-    c.val = d.val;
-    c.dinv = d.dinv;
-    c.scal = d.scal;
-    c.part = d.part;
-    c.tickets = d.tickets;
-    c.ncta = d.ncta;
-    c.cta_seg = d.cta_seg;
-    c.cta_node0 = d.cta_node0;
-    c.cta_node1 = d.cta_node1;
-    c.seg_cta0 = d.seg_cta0;
-    c.seg_solve = d.seg_solve;
-    c.xrow = d.nxb > 0 ? d.xrow : nullptr;
-    c.xcol = d.xcol;
-    c.xval = d.xval;
-    c.nn = d.nn;
-    c.check = d.check;
-    return c;
-}
-
 // Issues n iterations of `method` on the stream (no host interaction).
 template <int U>
 void issue_iterations_u(tf_handle* h, const Ctx& c, int method, int n) {
@@ -649,23 +530,23 @@ void issue_iterations_u(tf_handle* h, const Ctx& c, int method, int n) {
     cudaStream_t st = h->stream;
     const int nb = d.ncta;
     const int jac = use_multigrid(h) ? 0 : 1;
+    const AmgPre pre = amg_pre(h);
     for (int it = 0; it < n; ++it) {
         if (method == 1) {
             launch_pdl(k_cg_spmv<U>, nb, kThreads, st, c, d.p, d.q);
-            launch_pdl(k_cg_update, nb, kThreads, st, c, d.du, d.r, d.z, d.p, d.q, jac);
+            launch_pdl(k_cg_update, nb, kThreads, st, c, d.du, d.r, d.z, d.p, d.q, jac, pre);
             if (!jac) {
-                amg_vcycle(h, d.r, d.z);
-                launch_pdl(k_cg_rz, nb, kThreads, st, c, d.r, d.z, d.p, 0);
+                amg_vcycle(h, d.r, d.z, kVcycleDot, d.p);
+                if (!amg_fuses_dot(h)) launch_pdl(k_cg_rz, nb, kThreads, st, c, d.r, d.z, d.p, 0);
             }
             launch_pdl(k_cg_direction, nb, kThreads, st, c, d.z, d.p);
         } else {
-            launch_pdl(k_bi_dir, nb, kThreads, st, c, d.r, d.q, d.p, d.z, jac);
+            launch_pdl(k_bi_dir, nb, kThreads, st, c, d.r, d.q, d.p, d.z, jac, pre);
             if (!jac) amg_vcycle(h, d.p, d.z);
             launch_pdl(k_bi_spmv1<U>, nb, kThreads, st, c, d.z, d.rhat, d.q);
-            launch_pdl(k_bi_s, nb, kThreads, st, c, d.r, d.q, d.s, d.sh, d.du, d.z, jac);
+            launch_pdl(k_bi_s, nb, kThreads, st, c, d.r, d.q, d.s, d.sh, jac, pre);
             if (!jac) amg_vcycle(h, d.s, d.sh);
-            launch_pdl(k_bi_half, nb, kThreads, st, c, d.du, d.z);
-            launch_pdl(k_bi_spmv2<U>, nb, kThreads, st, c, d.sh, d.s, d.t);
+            launch_pdl(k_bi_spmv2<U>, nb, kThreads, st, c, d.sh, d.s, d.t, d.du, d.z);
             launch_pdl(k_bi_x, nb, kThreads, st, c, d.du, d.r, d.rhat, d.z, d.sh, d.s, d.t);
         }
     }
@@ -729,9 +610,9 @@ tf_status autotune_solve(tf_handle* h) {
 }
 
 int kernels_per_iteration(const tf_handle* h, int method) {
-    if (!use_multigrid(h)) return method == 1 ? 3 : 6;
+    if (!use_multigrid(h)) return method == 1 ? 3 : 5;
     const int v = amg_vcycle_kernels(h);
-    return method == 1 ? 4 + v : 6 + 2 * v;
+    return method == 1 ? 3 + (amg_fuses_dot(h) ? 0 : 1) + v : 5 + 2 * v;
 }
 
 constexpr int kChunk0 = 4;  // iterations of the smallest graph chunk
@@ -855,12 +736,15 @@ tf_status krylov_run(tf_handle* h, int method, int keep, int* iters, double* rel
             if (su != TF_OK) return su;
         }
         if (method == 1) {
-            k_cg_init<<<d.ncta, kThreads, 0, st>>>(c, d.g, d.du, d.r, d.z, d.p, tol2, h->solve_atol, keep, jac, x0);
+            k_cg_init<<<d.ncta, kThreads, 0, st>>>(c, d.g, d.du, d.r, d.z, d.p, tol2, h->solve_atol, keep, jac, x0,
+                                                   amg_pre(h));
             if (!jac) {
-                TF_LAUNCH_CHECK(h);
-                amg_vcycle(h, d.r, d.z);
+                amg_vcycle(h, d.r, d.z, kVcycleStart, d.p);
                 h->launches += amg_vcycle_kernels(h);
-                k_cg_rz<<<d.ncta, kThreads, 0, st>>>(c, d.r, d.z, d.p, 1);
+                if (!amg_fuses_dot(h)) {
+                    k_cg_rz<<<d.ncta, kThreads, 0, st>>>(c, d.r, d.z, d.p, 1);
+                    TF_LAUNCH_CHECK(h);
+                }
             }
         } else {
             k_bi_init<<<d.ncta, kThreads, 0, st>>>(c, d.g, d.du, d.r, d.rhat, d.p, d.q, tol2, h->solve_atol, keep, x0);
@@ -1178,9 +1062,13 @@ bool capture_while(tf_handle* h, cudaGraphConditionalHandle hc, Body body) {
     if (cudaStreamBeginCaptureToGraph(h->cap_stream, bg, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal) !=
         cudaSuccess)
         return false;
+    // a stream stays in the capture it joined until that one ends, so the
+    // nested body gets a side stream of its own
     std::swap(h->stream, h->cap_stream);
+    std::swap(h->side_stream, h->cap_side);
     body();
     std::swap(h->stream, h->cap_stream);
+    std::swap(h->side_stream, h->cap_side);
     cudaGraph_t out = nullptr;
     return cudaStreamEndCapture(h->cap_stream, &out) == cudaSuccess;
 }
@@ -1205,10 +1093,10 @@ bool issue_newton_iteration(tf_handle* h, cudaGraphConditionalHandle newton) {
     const int jac = mg ? 0 : 1;
     if (method == 1) {
         k_cg_init<<<d.ncta, kThreads, 0, st>>>(c, d.g, d.du, d.r, d.z, d.p, tol2, h->opt.update_atol, 0, jac,
-                                                nullptr);
+                                                nullptr, amg_pre(h));
         if (mg) {
-            amg_vcycle(h, d.r, d.z);
-            k_cg_rz<<<d.ncta, kThreads, 0, st>>>(c, d.r, d.z, d.p, 1);
+            amg_vcycle(h, d.r, d.z, kVcycleStart, d.p);
+            if (!amg_fuses_dot(h)) k_cg_rz<<<d.ncta, kThreads, 0, st>>>(c, d.r, d.z, d.p, 1);
         }
     } else {
         k_bi_init<<<d.ncta, kThreads, 0, st>>>(c, d.g, d.du, d.r, d.rhat, d.p, d.q, tol2, h->opt.update_atol, 0,
@@ -1258,7 +1146,8 @@ bool build_newton_loop(tf_handle* h) {
             // test and the update
             const bool mg = use_multigrid(h);
             h->nloop_kernels = 2 + 2 + (h->opt.deterministic ? 2 : 0) + 1 + (mg ? 3 : 0) +
-                               (h->method == 1 && mg ? 2 + amg_vcycle_kernels(h) : 1) + 1 + 3;
+                               (h->method == 1 && mg ? 1 + (amg_fuses_dot(h) ? 0 : 1) + amg_vcycle_kernels(h) : 1) +
+                               1 + 3;
             cudaGraph_t out = nullptr;
             ok = (cudaStreamEndCapture(h->stream, &out) == cudaSuccess) && ok;
         }
