@@ -152,3 +152,38 @@ def test_folded_transfers_match_the_kernels_of_extra_blocks(nx, ny, layers, eta)
             _check_solution(s, out, [(0, 3 * t.n_nodes)])
             its.append(out["iters"])
     assert abs(its[0] - its[1]) <= 0.25 * its[1] + 1, its
+
+
+# The element kernel's tile edges: prism counts around multiples of the tiles (8,
+# 16, 32), one and several layers, both stiffness paths and both assemblies,
+# strongly deformed.  K (FP64 sums of double-float blocks) and g against the
+# element routine that the parity tests pin to the oracle (tf_element_eval, FP64),
+# summed here: 1e-11 of the largest entry, the parity tests' bound.
+@pytest.mark.parametrize("deterministic", [False, True])
+@pytest.mark.parametrize("eta", [0.0, 100.0])
+@pytest.mark.parametrize("nx,ny,layers", [(1, 1, 1), (1, 2, 1), (2, 2, 1), (3, 3, 1), (1, 5, 3), (5, 3, 2), (4, 4, 1)])
+def test_element_tiles(nx, ny, layers, eta, deterministic):
+    t = _sheet(nx, ny, layers, eta)
+    if eta:
+        t.eta[::3] = 0.0  # prisms without viscosity among the others
+    uk, un = mesh.perturbed_state(t, seed=9, amp=0.8)
+    with api.Solver(t, deterministic=deterministic) as s:
+        s.set_Fg(mesh.growth_Fg(t, seed=10, amp=0.05))
+        s.set_state(uk, un, t.dt)  # no viscosity surfaces yet: element terms only
+        s.assemble()
+        ia, ja, a = s.export_csr(0.0)
+        g = s.residual()
+        ev = s.element_eval()
+    n = 3 * t.n_nodes
+    K, f = np.zeros((n, n)), np.zeros(n)
+    free = t.fixed == 0
+    for e, nodes in enumerate(t.conn.reshape(-1, 6)):
+        dof = (3 * nodes[:, None] + np.arange(3)).reshape(-1)
+        K[np.ix_(dof, dof)] += ev["Ke"][e] + ev["Kv"][e]
+        f[dof] += (ev["fe"][e] + ev["fv"][e]).reshape(-1)
+    K *= free[:, None] & free[None, :]
+    K[~free, ~free] = 1.0
+    got = np.zeros((n, n))
+    got[np.repeat(np.arange(n), np.diff(ia)), ja] = a
+    assert np.abs(got - K).max() <= 1e-11 * np.abs(K).max()
+    assert np.abs(g - f * free).max() <= 1e-11 * np.abs(f).max()

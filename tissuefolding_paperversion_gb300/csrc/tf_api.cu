@@ -110,7 +110,7 @@ tf_status upload(T** p, const std::vector<T>& v) {
 
 void free_all(tf_handle* h) {
     Device& d = h->d;
-    void* ptrs[] = {d.conn, d.gx, d.wdet, d.detdxde, d.Fg, d.invFg, d.rates, d.lam, d.mu, d.eta, d.exposure,
+    void* ptrs[] = {d.conn, d.ginv, d.gx, d.wdet, d.Fg, d.invFg, d.rates, d.lam, d.mu, d.eta, d.exposure,
                     d.aptr, d.alist, d.farea, d.fixed, d.ext_visc, d.area, d.rowptr, d.colidx, d.diag, d.rowof,
                     d.slot, d.bofs, d.wslot0, d.scol, d.val, d.eblk, d.ef, d.gptr, d.glist, d.fptr, d.flist, d.uk, d.un, d.vel, d.g,
                     d.du, d.dinv, d.r, d.p, d.z, d.q, d.rhat, d.s, d.t, d.sh, d.scal, d.part, d.tickets,
@@ -250,7 +250,7 @@ tf_status build(tf_handle* h, const tf_mesh* m, const tf_material* mat, const st
         exposure[e] = ex;
     }
     // ---- reference geometry: dN_X per Gauss point --------------------------
-    std::vector<double> gx(18 * 6 * (size_t)ne), wdet(6 * (size_t)ne), detd(6 * (size_t)ne);
+    std::vector<double> ginv(9 * 6 * (size_t)ne), wdet(6 * (size_t)ne);
     h->h_vref.assign(ne, 0.0);
     double dN[6][3][6];
     for (int gp = 0; gp < 6; ++gp) shape_derivatives(gp, dN[gp]);
@@ -276,14 +276,8 @@ tf_status build(tf_handle* h, const tf_mesh* m, const tf_material* mat, const st
                 return TF_BAD_INPUT;
             }
             const size_t q = 6 * (size_t)e + gp;
-            detd[q] = det;
             wdet[q] = (1.0 / 6.0) * det;
-            for (int a = 0; a < 6; ++a)
-                for (int k = 0; k < 3; ++k) {
-                    double acc = 0.0;
-                    for (int j = 0; j < 3; ++j) acc += inv[3 * j + k] * dN[gp][j][a];
-                    gx[(size_t)(3 * a + k) * (6 * (size_t)ne) + q] = acc;
-                }
+            for (int k = 0; k < 9; ++k) ginv[((size_t)k * 6 + gp) * ne + e] = inv[k];
         }
     }
     // ---- material (Prism::setElasticProperties, Prism.cpp:491-516) ----------
@@ -372,9 +366,10 @@ tf_status build(tf_handle* h, const tf_mesh* m, const tf_material* mat, const st
     }
     // ---- uploads -----------------------------------------------------------------
     TF_TRY(upload(&d.conn, conn_soa));
-    TF_TRY(upload(&d.gx, gx));
+    TF_TRY(upload(&d.ginv, ginv));
     TF_TRY(upload(&d.wdet, wdet));
-    TF_TRY(upload(&d.detdxde, detd));
+    TF_TRY(dev_alloc(&d.gx, 18 * 6 * (size_t)ne));
+    TF_TRY(launch_shape_gradients(h, &dN[0][0][0]));
     TF_TRY(upload(&d.lam, lam));
     TF_TRY(upload(&d.mu, mu));
     TF_TRY(upload(&d.eta, eta));

@@ -9,46 +9,71 @@
 //   calculateImplicitKElastic            ShapeBase.cpp:2619-2639, :2786-2890
 //   calculateImplicitKViscous            ShapeBase.cpp:2641-2705, :2892-3053
 //   write*ToMainKatrix / ge, gv scatter  ShapeBase.cpp:2148-2180, :2707-2758
-// with exact identities that cut FP64 work:
+// with exact identities that cut the work:
 //   * Fe C^-1 Fe^T = I, so sigma = (mu (b - I) + lambda lnJ I) / J with
 //     b = Fe Fe^T, and the 3^6 contraction of integral 1 collapses to
 //     lambda a_i b_k + (mu - lambda lnJ)(delta_ik a.b + a_k b_i);
-//   * dN_x = F^-T dN_X with dN_X = InvdXde^T dN precomputed per element;
-//   * with a = dN_a, b = dN_b, s = a.b and t = a.(sigma' b) the whole 3x3
-//     block (elastic + both viscous integrals) of one Gauss point is
-//       K_ab = u_a b^T + b w_a^T - v_b a^T + s Q + t I
-//     where per node c:  u_c = c1 dN_c + sigma_v' dN_c,
-//                        w_c = c2 dN_c + P^T dN_c,   v_c = sigma_v' dN_c,
-//     and Q = c2 I + P, P = 0.5 eta w dV (I/dt - grad v) (primes: times
-//     w dV).  That is 45 multiply-adds per block and Gauss point instead of
-//     64; without viscosity K_ab = K_ba^T and only the 21 pairs a <= b are
-//     formed.
+//   * with a, b two gradient vectors, s = a.b and t = a.(sigma' b) the whole 3x3
+//     block (elastic + both viscous integrals) of one Gauss point is the
+//     bilinear form
+//       B(a, b) = u_a b^T + b w_a^T - v_b a^T + s Q + t I
+//     with  u_a = c1 a + sigma_v' a,  w_a = Q^T a,  v_b = sigma_v' b,
+//     Q = c2 I + P, P = 0.5 eta w dV (I/dt - grad v) (primes: times w dV);
+//     without viscosity B(a, b) = c1 a b^T + c2 b a^T + (c2 s + t) I = B(b, a)^T;
+//   * the gradient of node (i, layer) is D_i1 L g_1 + D_i2 L g_2 + (+-) N_i/2 g_3
+//     with g_j = grad xi_j the same for all nodes, D constants, L the layer's
+//     weight at the two heights and N_i = 1/6 + delta_it/2 at the three
+//     in-plane points t.  So the 36 node-pair blocks are weighted sums of the nine
+//     blocks B(g_j, g_l) (six without viscosity) of the Gauss points, and the
+//     weights are products of a height and an in-plane factor: the sums are taken
+//     one factor at a time.  That is ~74,000 FP32 operations per prism in
+//     place of ~136,000 for B(dN_a, dN_b) pair by pair;
+//   * dx/dxi_j depends on the height (j = 1, 2) or on the in-plane point (j = 3)
+//     only: formed once per prism and component, not once per Gauss point;
+//     w dV = det(dx/dxi) / 6.
 //
-// Precision split.  GB300 issues FP32 FMAs at about 64 times its FP64 rate,
-// and the tangent's block sums are ~85 % of the kernel's FP64 work.  Phase A
-// (deformation gradient, stress, shape gradients, forces) stays FP64.  The
-// per-Gauss-point vectors the blocks are built from are split into
-// double-float pairs x = hi + lo (two FP32 values, ~48 significant bits) and
-// the block sums run in double-float arithmetic on the FP32 pipe: products by
-// Dekker's exact product (hi*hi and its rounding error by one FMA, plus the
-// cross terms), sums by Knuth's two-sum, the low parts gathered in a second
-// FP32 accumulator and renormalised once per Gauss point (Dekker, "A
-// floating-point technique for extending the available precision", 1971;
-// Knuth, TAOCP vol. 2, 4.2.2).  A block entry carries a relative error of
-// ~1e-13 of its largest term, far inside the 1e-11 parity bound and far
-// below what moves a Newton iterate; the forces and everything the residual
-// depends on stay FP64 (with viscosity the forces use one FP64 stress
-// sigma' + sigma_v', and the tangent's sigma' dN and sigma_v' dN come from
-// the double-float splits of the two stresses).
+// Precision split.  GB300 issues FP32 FMAs at about 64 times its FP64 rate.
+// The Gauss-point algebra (deformation gradient, stress, gradients, forces) is
+// FP64.  The vectors the tangent's blocks are built from are split into
+// double-float pairs x = hi + lo (two FP32 values, 48 significant bits and
+// more) and the block sums run in double-float arithmetic on the FP32 pipe:
+// products by Dekker's exact product (hi*hi and its rounding error by one FMA,
+// plus the cross terms), sums by Knuth's two-sum, the low parts gathered in a
+// second FP32 accumulator and renormalised (Dekker, "A floating-point technique
+// for extending the available precision", 1971; Knuth, TAOCP vol. 2, 4.2.2).  A
+// block entry carries a relative error of ~1e-13 of its largest term, far inside
+// the 1e-11 parity bound and far below what moves a Newton iterate; the forces and
+// everything the residual depends on stay FP64.  The splits and the joins work
+// on the bit patterns: conversion instructions and additions would take the
+// scarce FP64 pipe.
 //
-// Layout: one CTA of 2 x 6 x NE threads handles NE prisms.  Phase A: one
-// thread per (prism, Gauss point) -- the first half of the CTA -- builds the
-// per-point vectors in shared memory.  Phase B: every thread owns 3x3
-// node-pair blocks, sums the six Gauss points and scatters the block.  The matrix assembled is A = K^T, the system the reference
+// Layout: one CTA of 12 x NE threads handles NE prisms, consecutive threads
+// consecutive prisms throughout -- loads, shared memory and the atomics of a
+// warp are then neighbours (with a warp on the node pairs of one prism every
+// atomic went to a sector of its own).  A thread is (slot, prism), slot 0..11:
+//   1. slots 0-5: dx/dxi and dv/dxi, one component each (FP64);
+//   2. slots 0-5: one Gauss point each (FP64), split to shared memory;
+//   3. the double-float vectors of the blocks; the nodal forces (FP64);
+//   4. the blocks B(g_j, g_l) summed over what their weights share, staged in
+//      shared memory;
+//   5. the in-plane and height weights;
+//   6. each node pair's block joined to FP64 and scattered.
+// The loops over a phase's tasks stay rolled: unrolled they overflow the
+// instruction cache.
+// The phases of one CTA use one pipe at a time; three CTAs on an SM overlap them
+// (with the u_j and s_jl kept in shared memory two fit: 2.58 against 1.94 ms).
+// FP64 pipe and issue slots are each half busy: 1,787 FP64 instructions per prism
+// (3,156 before), ~130,000 thread instructions per prism in all; the rest is the barriers
+// between the phases.  320,000 prisms: 3.62 -> 1.89 ms with viscosity, 2.18 -> 1.37 ms
+// without.  K's error against 64 bits, relative (2-norm): 2.0e-15 to 2.4e-15 without
+// viscosity (before 2.1e-15 to 2.2e-15), 2.4e-15 to 2.9e-15 with (2.6e-15 to 3.2e-15).
+// The matrix assembled is A = K^T, the system the reference
 // solves (Pardiso iparm[11] = 1, NewtonRaphsonSolver.cpp:639); in that
 // orientation every element block (a, b) lands at block (conn[a], conn[b])
 // without a transpose.  Fixed DOFs are masked here, which is calcutateFixedK
 // (NewtonRaphsonSolver.cpp:237-255) without a second pass.
+#include <cstring>
+
 #include "tf_internal.cuh"
 
 namespace tf {
@@ -57,19 +82,12 @@ namespace {
 
 enum Mode { kAtomic = 0, kStore = 2 };
 
-// Threads per Gauss point: phase A runs on the first NE x 6 threads of the
-// CTA, the pair phase and the force sums on all of them.  Twice the threads
-// of phase A give the pair phase (FP32 pipe) more warps to hide its latency
-// while other CTAs on the SM run phase A (FP64 pipe): 3.65 against 4.68 ms
-// per 320,000-prism assembly with the merged force stress below and the
-// Gauss loop of the pair phase kept rolled (unrolled it overflows the
-// instruction cache); three threads per Gauss point were slower (registers
-// then allow one CTA per SM).
-constexpr int kTpg = 2;
+constexpr int kSlots = 12;  // threads per prism
 
 struct ElemArgs {
     int ne;
     const int* __restrict__ conn;
+    const double* __restrict__ ginv;  // [9][6][ne] dxi/dX
     const double* __restrict__ gx;
     const double* __restrict__ wdet;
     const double* __restrict__ invFg;
@@ -249,58 +267,44 @@ __device__ __forceinline__ void gauss_point(const ElemArgs& A, int e, int gp, bo
 // reassociates differently (the order-fixed assembly stays bitwise
 // reproducible whatever tile the autotuner picks).
 
-// The FP64 <-> FP32 conversion instructions run on GB300's slow FP64 path,
-// so the split and the join work on the bit patterns (integer pipe) with one
-// FP64 subtraction or addition each.
-
-// float with x's value rounded to 24 significant bits; x must be a double
-// whose low 29 mantissa bits are zero (then the result is exact): sign,
-// exponent rebased 1023 -> 127, the top 23 mantissa bits.  Magnitudes below
-// FP32's normal range become a signed zero; NaN and infinity stay NaN and
-// infinity.
-__device__ __forceinline__ float f32_of_trunc(unsigned hi, unsigned lo) {
-    const unsigned sgn = hi & 0x80000000u;
-    const int e = (int)((hi >> 20) & 0x7ffu);
-    const int fe = e - 896;
-    unsigned f = sgn | ((unsigned)fe << 23) | ((hi & 0xfffffu) << 3) | (lo >> 29);
-    f = (fe > 0) ? f : sgn;
-    f = (e == 0x7ff) ? (sgn | 0x7f800000u | ((hi & 0xfffffu) ? 0x400000u : 0u)) : f;
-    return __uint_as_float(f);
-}
-
-// x rounded to 24 significant bits (round half away from zero on the bit
-// pattern; the carry runs into the exponent), as a double and as a float.
-__device__ __forceinline__ double round24(double x, float* f) {
-    const unsigned lo = __double2loint(x), hi = __double2hiint(x);
-    const unsigned lo2 = lo + (1u << 28);
-    const unsigned hi2 = hi + (lo2 < lo ? 1u : 0u);
-    const unsigned lo3 = lo2 & ~((1u << 29) - 1u);
-    const bool special = ((hi >> 20) & 0x7ffu) == 0x7ffu;
-    *f = f32_of_trunc(special ? hi : hi2, special ? lo : lo3);
-    return special ? x : __hiloint2double(hi2, lo3);
-}
-
-// x = hi + lo, hi and lo FP32 (~48 significant bits in all)
+// x = hi + lo on the bit pattern: hi is x rounded to 24 significant bits (half
+// away from zero; the carry runs into the exponent), lo the rest as an integer
+// of 29 signed bits, scaled.  Magnitudes below FP32's normal range become a
+// signed zero (and the low part below it zero); NaN and infinity stay so.
 __device__ __forceinline__ float2 df_split(double x) {
-    float h, l;
-    const double hd = round24(x, &h);
-    round24(x - hd, &l);
-    return make_float2(h, l);
+    const unsigned l = __double2loint(x), h = __double2hiint(x);
+    const unsigned sgn = h & 0x80000000u;
+    const int e = (int)((h >> 20) & 0x7ffu);
+    const unsigned l2 = l + (1u << 28), h2 = h + (l2 < l ? 1u : 0u);
+    unsigned f = sgn | ((((h2 >> 20) & 0x7ffu) - 896u) << 23) | ((h2 & 0xfffffu) << 3) | (l2 >> 29);
+    f = e > 896 ? f : sgn;
+    f = e == 0x7ff ? (sgn | 0x7f800000u | ((h & 0xfffffu) ? 0x400000u : 0u)) : f;
+    const float scale = __uint_as_float(sgn | ((unsigned)(e - 948) << 23));  // 2^(exponent - 52)
+    const float lo = __int2float_rn((int)(l2 & 0x1fffffffu) - (1 << 28)) * scale;
+    return make_float2(__uint_as_float(f), (e > 948 && e < 0x7ff) ? lo : 0.f);
 }
 
-// float -> double, exact, on the bit pattern (subnormal floats become zero)
-__device__ __forceinline__ double f64_of(float f) {
-    const unsigned u = __float_as_uint(f);
-    const unsigned e = (u >> 23) & 0xffu;
-    const unsigned sgn = u & 0x80000000u;
-    unsigned hi = sgn | ((e + 896u) << 20) | ((u & 0x7fffffu) >> 3);
-    hi = (e == 0u) ? sgn : hi;
-    hi = (e == 0xffu) ? (sgn | 0x7ff00000u | ((u & 0x7fffffu) ? 0x80000u : 0u)) : hi;
-    const unsigned lo = (e == 0u || e == 0xffu) ? 0u : (u << 29);
-    return __hiloint2double(hi, lo);
+// hi + lo as a double on the bit patterns; |lo| at most half an ulp of hi (after
+// df_norm).  The 24 bits of hi, shifted to a double's 53, plus or minus those of
+// lo at their place (bits below a double's last are cut off: an error under one
+// ulp of the double, a hundredth of what the pair carries).
+__device__ __forceinline__ double df_join(float hi, float lo) {
+    const unsigned uh = __float_as_uint(hi), ul = __float_as_uint(lo);
+    const int eh = (int)((uh >> 23) & 0xffu), el = (int)((ul >> 23) & 0xffu);
+    const unsigned long long mh = (unsigned long long)((uh & 0x7fffffu) | 0x800000u) << 29;
+    const unsigned long long ml = el ? (unsigned long long)((ul & 0x7fffffu) | 0x800000u) << 29 : 0ull;
+    const unsigned long long t = ml >> min(eh - el, 63);
+    const unsigned long long m = ((uh ^ ul) & 0x80000000u) ? mh - t : mh + t;
+    // the leading bit of m adds one to the exponent; a difference may have lost it
+    const bool low = m < (1ull << 52);
+    const unsigned long long b = low ? ((unsigned long long)(eh + 894) << 52) + (m << 1)
+                                     : ((unsigned long long)(eh + 895) << 52) + m;
+    const unsigned long long sgn = (unsigned long long)(uh & 0x80000000u) << 32;
+    unsigned long long r = sgn | b;
+    if (eh == 0) r = sgn;
+    if (eh == 0xff) r = sgn | 0x7ff0000000000000ull | ((uh & 0x7fffffu) ? 0x8000000000000ull : 0ull);
+    return __longlong_as_double((long long)r);
 }
-
-__device__ __forceinline__ double df_join(float h, float l) { return f64_of(h) + f64_of(l); }
 
 // (H, L) += x * y: Dekker's product (the rounding error of hi*hi by one FMA,
 // the cross terms into the low word; lo*lo is below the format's precision),
@@ -333,23 +337,165 @@ __device__ __forceinline__ void df_norm(float& H, float& L) {
     H = s;
 }
 
+// c x, c a double-float constant
+__device__ __forceinline__ float2 df_scale(float2 c, float2 x) {
+    float p = __fmul_rn(c.x, x.x);
+    float e = __fmaf_rn(c.x, x.x, -p);
+    e = __fmaf_rn(c.x, x.y, e);
+    e = __fmaf_rn(c.y, x.x, e);
+    df_norm(p, e);
+    return make_float2(p, e);
+}
+// x + y.  FULL: both words by two-sums (the low words' rounding carried too),
+// else the low words simply added.
+template <bool FULL>
+__device__ __forceinline__ float2 df_sum(float2 x, float2 y) {
+    if constexpr (!FULL) {
+        df_add(x.x, x.y, y);
+        df_norm(x.x, x.y);
+        return x;
+    } else {
+        float s = __fadd_rn(x.x, y.x);
+        float bb = __fsub_rn(s, x.x);
+        float e = __fadd_rn(__fsub_rn(x.x, __fsub_rn(s, bb)), __fsub_rn(y.x, bb));
+        const float t = __fadd_rn(x.y, y.y);
+        bb = __fsub_rn(t, x.y);
+        const float ee = __fadd_rn(__fsub_rn(x.y, __fsub_rn(t, bb)), __fsub_rn(y.y, bb));
+        e = __fadd_rn(e, t);
+        df_norm(s, e);
+        e = __fadd_rn(e, ee);
+        df_norm(s, e);
+        return make_float2(s, e);
+    }
+}
+// m + c x, c a small integer (the product's error by one FMA)
+__device__ __forceinline__ float2 df_muladd(float2 m, float c, float2 x) {
+    df_mac(m.x, m.y, make_float2(c, 0.f), x);
+    df_norm(m.x, m.y);
+    return m;
+}
+// (H, L) += s x, s = +-1 (the products are exact).  FULL: the low words' sum by
+// a two-sum too, its rounding gathered in E.
+template <bool FULL>
+__device__ __forceinline__ void df_addmul(float& H, float& L, float& E, float s, float2 x) {
+    const float t = __fmaf_rn(s, x.x, H);
+    float bb = __fsub_rn(t, H);
+    const float err = __fadd_rn(__fsub_rn(H, __fsub_rn(t, bb)), __fmaf_rn(s, x.x, -bb));
+    H = t;
+    if constexpr (!FULL) {
+        L = __fadd_rn(L, __fmaf_rn(s, x.y, err));
+    } else {
+        const float l = __fadd_rn(L, err);
+        bb = __fsub_rn(l, L);
+        E = __fadd_rn(E, __fadd_rn(__fsub_rn(L, __fsub_rn(l, bb)), __fsub_rn(err, bb)));
+        L = __fmaf_rn(s, x.y, l);
+        bb = __fsub_rn(L, l);
+        E = __fadd_rn(E, __fadd_rn(__fsub_rn(l, __fsub_rn(L, bb)), __fmaf_rn(s, x.y, -bb)));
+    }
+}
+// s x, s a power of two or its negative (exact)
+__device__ __forceinline__ float2 df_pow2(float s, float2 x) { return make_float2(s * x.x, s * x.y); }
 __device__ __forceinline__ float2 df_neg(float2 x) { return make_float2(-x.x, -x.y); }
 
-// Shared per-Gauss-point vectors of the fast kernel: the tangent's inputs as
-// double-float pairs, the force terms in FP64.
+constexpr double kSqrt3 = 1.73205080756887729353;
+constexpr float df_hi(double x) { return (float)x; }
+constexpr float df_lo(double x) { return (float)(x - (double)(float)x); }
+#define DF_CONST(x) make_float2(df_hi(x), df_lo(x))
+
+__device__ __forceinline__ bool element_live(const ElemArgs& A, int e) {
+    return e < A.ne && (!A.masked || A.seg_active[A.elem_seg[e]] != 0);
+}
+
+// Index of (j, l) in the order 00 11 22 01 02 12.
+__device__ __forceinline__ int sym_index(int j, int l) { return j == l ? j : j + l + 2; }
+
+// Shared memory of a CTA, the prism fastest everywhere.
+//   gp: double-float vectors of the Gauss points, [value][gp][NE]: the gradients
+//       g_1/sqrt(3), g_2/sqrt(3), g_3/12 (G; the weights of phase 4 are then small
+//       integers but for one factor), their w_j (W) and with viscosity v_j, Q, t_jl
+//       and c1 (u_j and s_jl are formed again in phase 4: their room would cost a
+//       CTA per SM), without it u_j and d_jl = c2 s_jl + t_jl (U, D);
+//   st: staged 3x3 blocks, [block][9][NE]: A_jl(height), j, l in {1, 2}, then
+//       M_jl(layers bb, bt) in their place; B(g_j, g_3)(height, in-plane point)
+//       and with viscosity B(g_3, g_l), then H(layer, node) in their place; and
+//       B(g_3, g_3)(in-plane point), without viscosity per height.  M_jl(tt) and
+//       W(node pair i <= k) go where gp was.
+// st first holds what only the phases before need: dx/dxi and dv/dxi
+// [2][7][3][NE] in FP64 (X), (sigma' + sigma_v') g_j [9][gp][NE] in FP64 for the
+// forces (F), and c1, c2, sigma', sigma_v' [value][gp][NE] (C).
 template <bool VISC>
-struct GpFast;
-template <>
-struct GpFast<false> {
-    float2 dn[18], sdn[18], u[18], w[18];
-    float2 c2;
-    double fs[18];   // sigma' dN (forces)
+struct Lay {
+    static constexpr int G = 0, W = 9, V = 18, Q = 27, T = 36, K1 = 42, U = 18, D = 27;
+    static constexpr int NV = VISC ? 43 : 33;
+    static constexpr int NJL = VISC ? 4 : 3;             // pairs (j, l) of {1, 2}
+    static constexpr int NR = VISC ? 4 : 2;              // (1,3) (2,3) and with viscosity (3,1) (3,2)
+    static constexpr int BA = 0;                         // [NJL][2]
+    static constexpr int BR = 2 * NJL;                   // [NR][2][3]
+    static constexpr int BB = BR + 6 * NR;               // [3], without viscosity [2][3]
+    static constexpr int NB = BB + (VISC ? 3 : 6);
+    static constexpr int XM = 0, XW = NJL;               // blocks in gp's place: [NJL], [6]
+    static constexpr int C1 = 0, C2 = 1, SG = 2, SV = 8; // values of C (with viscosity c1 is in gp, c2 in Q)
+    static constexpr int NC = VISC ? 14 : 8;
 };
-template <>
-struct GpFast<true> {
-    float2 dn[18], sdn[18], u[18], w[18], v[18], Q[9];
-    double fs[18];           // (sigma' + sigma_v') dN (forces)
-};
+template <int NE, bool VISC>
+constexpr size_t elem_smem() {
+    using Y = Lay<VISC>;
+    static_assert(8 * 42 + 8 * 54 + 8 * 6 * Y::NC <= 72 * Y::NB, "X, F and C fit st");
+    return sizeof(float2) * NE * (Y::NV * 6 + Y::NB * 9);
+}
+
+// B(g_j, g_l) of Gauss point gp into (H, L)[9]
+template <int NE, bool VISC>
+__device__ __forceinline__ void gp_block(const float2* __restrict__ sg, int j, int l, int gp, int el, float (&H)[9],
+                                         float (&L)[9]) {
+    using Y = Lay<VISC>;
+    auto at = [&](int v) { return sg[(v * 6 + gp) * NE + el]; };
+    const int jl = sym_index(j, l);
+    const float2 b[3] = {at(Y::G + 3 * l), at(Y::G + 3 * l + 1), at(Y::G + 3 * l + 2)};
+    float2 u[3];
+    if constexpr (VISC) {  // u = c1 g + sigma_v' g
+        const float2 c1 = at(Y::K1);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            u[i] = at(Y::V + 3 * j + i);
+            df_mac(u[i].x, u[i].y, c1, at(Y::G + 3 * j + i));
+            df_norm(u[i].x, u[i].y);
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 3; ++i) u[i] = at(Y::U + 3 * j + i);
+    }
+    const float2 w[3] = {at(Y::W + 3 * j), at(Y::W + 3 * j + 1), at(Y::W + 3 * j + 2)};
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {  // u b^T: the first product needs no sum
+        const float2 x = u[k / 3], y = b[k % 3];
+        H[k] = __fmul_rn(x.x, y.x);
+        L[k] = __fmaf_rn(x.y, y.x, __fmaf_rn(x.x, y.y, __fmaf_rn(x.x, y.x, -H[k])));
+    }
+#pragma unroll
+    for (int k = 0; k < 9; ++k) df_mac(H[k], L[k], b[k / 3], w[k % 3]);
+    if constexpr (VISC) {
+        const float2 a[3] = {at(Y::G + 3 * j), at(Y::G + 3 * j + 1), at(Y::G + 3 * j + 2)};
+        const float2 v[3] = {df_neg(at(Y::V + 3 * l)), df_neg(at(Y::V + 3 * l + 1)), df_neg(at(Y::V + 3 * l + 2))};
+        const float2 t = at(Y::T + jl);
+        float2 s = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) df_mac(s.x, s.y, a[i], b[i]);
+        df_norm(s.x, s.y);
+#pragma unroll
+        for (int k = 0; k < 9; ++k) {
+            df_mac(H[k], L[k], v[k / 3], a[k % 3]);
+            df_mac(H[k], L[k], s, at(Y::Q + k));
+            if (k % 4 == 0) df_add(H[k], L[k], t);
+        }
+    } else {
+        const float2 d = at(Y::D + jl);
+#pragma unroll
+        for (int k = 0; k < 9; k += 4) df_add(H[k], L[k], d);
+    }
+#pragma unroll
+    for (int k = 0; k < 9; ++k) df_norm(H[k], L[k]);
+}
 
 // o = s d for a symmetric s (00 11 22 01 02 12), in double-float
 __device__ __forceinline__ void df_sym_apply(const float2* s, const float2* d, float2* o) {
@@ -368,246 +514,481 @@ __device__ __forceinline__ void df_sym_apply(const float2* s, const float2* d, f
 __constant__ int8_t kPairA[21] = {0, 0, 0, 0, 0, 0, 1, 1, 1, 1, 1, 2, 2, 2, 2, 3, 3, 3, 4, 4, 5};
 __constant__ int8_t kPairB[21] = {0, 1, 2, 3, 4, 5, 1, 2, 3, 4, 5, 2, 3, 4, 5, 3, 4, 5, 4, 5, 5};
 
-__device__ __forceinline__ bool element_live(const ElemArgs& A, int e) {
-    return e < A.ne && (!A.masked || A.seg_active[A.elem_seg[e]] != 0);
-}
-
 template <int NE, int MODE, bool VISC>
-__global__ void __launch_bounds__(NE * kGauss * kTpg) k_element(ElemArgs A) {
+__global__ void __launch_bounds__(NE* kSlots, 48 / NE) k_element(ElemArgs A) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    using Gp = GpFast<VISC>;
-    Gp* sh = reinterpret_cast<Gp*>(smem_raw);  // [NE][6]
-    const int tid = threadIdx.x;
-    constexpr int NT = NE * kGauss * kTpg;
+    using Y = Lay<VISC>;
+    float2* sg = reinterpret_cast<float2*>(smem_raw);     // [NV][6][NE]
+    float2* st = sg + Y::NV * 6 * NE;                     // [NB][9][NE]
+    double* sx = reinterpret_cast<double*>(st);           // X [2][7][3][NE]
+    double* hf = sx + 42 * NE;                            // F [9][6][NE]
+    float2* sc0 = reinterpret_cast<float2*>(hf + 54 * NE);  // C [NC][6][NE]
+    const int el = threadIdx.x % NE, slot = threadIdx.x / NE;
+    const int e = blockIdx.x * NE + el;
+    const bool live = element_live(A, e);
+    if (!__syncthreads_or(live)) return;
+    const int ne = A.ne;
 
-    // ---------------- phase A ----------------------------------------------
-    if (tid < NE * kGauss) {
-        const int el = tid / kGauss;
-        const int gp = tid - el * kGauss;
-        const int e = blockIdx.x * NE + el;
-        if (element_live(A, e)) {
-            const bool visc = VISC && (__ldg(&A.eta[e]) != 0.0);
-            GaussPoint G;
-            gauss_point(A, e, gp, visc, G);
-            Gp& S = sh[el * kGauss + gp];
-            // scalars and matrices the per-node vectors are formed from
-            const float2 c1 = df_split(G.c1), c2 = df_split(G.c2);
-            float2 Pm[9];
+    // ---- 1. dx/dxi_1, dx/dxi_2 at both heights, dx/dxi_3 at the in-plane points
+    // (component slot % 3), and dv/dxi likewise: apical weight (1 + zeta)/2 = b at
+    // the first height, a at the second
+    constexpr double wa = 0.5 - kSqrt3 / 6.0, wb = 0.5 + kSqrt3 / 6.0;
+    if (live && slot < (VISC ? 6 : 3)) {
+        const int c = slot % 3;
+        const double* __restrict__ src = slot < 3 ? A.uk : A.vel;
+        double x[6];
+#pragma unroll
+        for (int a = 0; a < 6; ++a) {
+            int nd = __ldg(&A.conn[a * ne + e]);
+            if (!TF_IN(A.check, nd, A.nn, CK_ELEM_NODE)) nd = 0;
+            x[a] = src[3 * nd + c];
+        }
+        double* o = sx + (size_t)(slot / 3) * 21 * NE + c * NE + el;
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const double lo = x[1 + j] - x[0], up = x[4 + j] - x[3];
+            o[(2 * j) * 3 * NE] = fma(wa, lo, wb * up);
+            o[(2 * j + 1) * 3 * NE] = fma(wb, lo, wa * up);
+        }
+        const double d[3] = {x[3] - x[0], x[4] - x[1], x[5] - x[2]};
+        const double m = (d[0] + d[1] + d[2]) * (1.0 / 12.0);
+#pragma unroll
+        for (int t = 0; t < 3; ++t) o[(4 + t) * 3 * NE] = fma(0.25, d[t], m);
+    }
+    __syncthreads();
+
+    // ---- 2. the Gauss points: Prism::calculateCurrNodalForces (Prism.cpp:749-874)
+    // in closed form.  Every multiply-add is an explicit fma, so the rounding does
+    // not depend on how the compiler contracts expressions in each instantiation
+    // (the order-fixed assembly stays bitwise reproducible whatever tile the
+    // autotuner picks).
+    if (live && slot < kGauss) {
+        const int gp = slot, t = gp % 3, hgt = gp / 3;
+        auto col = [&](int q, int j, int i) {  // dx_i/dxi_j (q = 0), dv_i/dxi_j (1)
+            const int m = j == 2 ? 4 + t : 2 * j + hgt;
+            return sx[((size_t)(q * 7 + m) * 3 + i) * NE + el];
+        };
+        double X[9];  // X[3 j + i] = dx_i / dxi_j
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+#pragma unroll
+            for (int i = 0; i < 3; ++i) X[3 * j + i] = col(0, j, i);
+        double g[9];  // g[3 j + i]: the cofactors, then grad xi_j
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            const double* p = X + 3 * ((j + 1) % 3);
+            const double* q = X + 3 * ((j + 2) % 3);
+            g[3 * j] = fma(p[1], q[2], -(p[2] * q[1]));
+            g[3 * j + 1] = fma(p[2], q[0], -(p[0] * q[2]));
+            g[3 * j + 2] = fma(p[0], q[1], -(p[1] * q[0]));
+        }
+        const double det = fma(X[0], g[0], fma(X[1], g[1], X[2] * g[2]));
+        double Fe[9];
+        {
+            double F[9];  // F[3 i + k] = sum_j dx_i/dxi_j dxi_j/dX_k
+            const double* __restrict__ iv = A.ginv + (size_t)gp * ne + e;
+            const size_t st6 = (size_t)6 * ne;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const double a0 = __ldg(&iv[k * st6]), a1 = __ldg(&iv[(3 + k) * st6]), a2 = __ldg(&iv[(6 + k) * st6]);
+#pragma unroll
+                for (int i = 0; i < 3; ++i) F[3 * i + k] = fma(X[i], a0, fma(X[3 + i], a1, X[6 + i] * a2));
+            }
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const double a0 = __ldg(&A.invFg[k * ne + e]), a1 = __ldg(&A.invFg[(3 + k) * ne + e]),
+                             a2 = __ldg(&A.invFg[(6 + k) * ne + e]);
+#pragma unroll
+                for (int i = 0; i < 3; ++i) Fe[3 * i + k] = fma(F[3 * i], a0, fma(F[3 * i + 1], a1, F[3 * i + 2] * a2));
+            }
+        }
+        const double J = fma(Fe[0], fma(Fe[4], Fe[8], -(Fe[5] * Fe[7])),
+                             fma(-Fe[1], fma(Fe[3], Fe[8], -(Fe[5] * Fe[6])), Fe[2] * fma(Fe[3], Fe[7], -(Fe[4] * Fe[6]))));
+        const double lnJ = log(J);
+        const double rr = 1.0 / (J * det);
+        const double wdV = det * (1.0 / 6.0);
+        const double sc = wdV * (rr * det);  // w dV / J
+        const double rd = rr * J;            // 1 / det
+        float2* out = sg + gp * NE + el;
+        auto put = [&](int v, double x) { out[(size_t)v * 6 * NE] = df_split(x); };
+#pragma unroll
+        for (int k = 0; k < 9; ++k) put(Y::G + k, g[k] * (k < 6 ? rd * (1.0 / kSqrt3) : rd * (1.0 / 12.0)));
+#pragma unroll
+        for (int k = 0; k < 9; ++k) g[k] *= rd;
+        const double lam = __ldg(&A.lam[e]), mu = __ldg(&A.mu[e]);
+        const double dterm = fma(lam, lnJ, -mu);
+        float2* outc = sc0 + gp * NE + el;
+        auto putc = [&](int v, double x) { outc[(size_t)v * 6 * NE] = df_split(x); };
+        // c1 = w dV lambda / J, c2 = w dV (mu - lambda lnJ) / J
+        if constexpr (VISC) put(Y::K1, sc * lam);
+        else putc(Y::C1, sc * lam);
+        const double c2d = -sc * dterm;
+        double sgm[6];  // sigma' = w dV sigma (00 11 22 01 02 12)
+        sgm[0] = sc * fma(mu, fma(Fe[0], Fe[0], fma(Fe[1], Fe[1], Fe[2] * Fe[2])), dterm);
+        sgm[1] = sc * fma(mu, fma(Fe[3], Fe[3], fma(Fe[4], Fe[4], Fe[5] * Fe[5])), dterm);
+        sgm[2] = sc * fma(mu, fma(Fe[6], Fe[6], fma(Fe[7], Fe[7], Fe[8] * Fe[8])), dterm);
+        const double sm = sc * mu;
+        sgm[3] = sm * fma(Fe[0], Fe[3], fma(Fe[1], Fe[4], Fe[2] * Fe[5]));
+        sgm[4] = sm * fma(Fe[0], Fe[6], fma(Fe[1], Fe[7], Fe[2] * Fe[8]));
+        sgm[5] = sm * fma(Fe[3], Fe[6], fma(Fe[4], Fe[7], Fe[5] * Fe[8]));
+#pragma unroll
+        for (int k = 0; k < 6; ++k) putc(Y::SG + k, sgm[k]);
+        if constexpr (VISC) {
+            // grad v = sum_j dv/dxi_j (x) g_j (ShapeBase.cpp:2892-2919); a prism
+            // without viscosity has eta = 0 and these terms vanish
+            double Lg[9];
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                const double v0 = col(1, 0, i), v1 = col(1, 1, i), v2 = col(1, 2, i);
+#pragma unroll
+                for (int k = 0; k < 3; ++k) Lg[3 * i + k] = fma(v0, g[k], fma(v1, g[3 + k], v2 * g[6 + k]));
+            }
+            const double eta = __ldg(&A.eta[e]);
+            const double ew = eta * wdV, hw = 0.5 * ew;
+            const bool visc = eta != 0.0;
+            double sv[6];  // sigma_v' = w dV eta sym(grad v)
+            sv[0] = ew * Lg[0];
+            sv[1] = ew * Lg[4];
+            sv[2] = ew * Lg[8];
+            sv[3] = hw * (Lg[1] + Lg[3]);
+            sv[4] = hw * (Lg[2] + Lg[6]);
+            sv[5] = hw * (Lg[5] + Lg[7]);
+#pragma unroll
+            for (int k = 0; k < 6; ++k) {
+                sv[k] = visc ? sv[k] : 0.0;
+                putc(Y::SV + k, sv[k]);
+                sgm[k] += sv[k];  // one stress for the forces
+            }
+            // Q = c2 I + P, P = 0.5 eta w dV (I/dt - grad v)
+#pragma unroll
+            for (int k = 0; k < 9; ++k) {
+                const double p = visc ? (k % 4 == 0 ? hw * (A.idt - Lg[k]) : -hw * Lg[k]) : 0.0;
+                put(Y::Q + k, k % 4 == 0 ? c2d + p : p);
+            }
+        } else {
+            putc(Y::C2, c2d);
+        }
+        double* ho = hf + gp * NE + el;
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            double h3[3];
+            sym_apply(sgm, g[3 * j], g[3 * j + 1], g[3 * j + 2], h3);
+#pragma unroll
+            for (int i = 0; i < 3; ++i) ho[(size_t)(3 * j + i) * 6 * NE] = h3[i];
+        }
+    }
+    __syncthreads();
+
+    // ---- 3. the double-float vectors of every (Gauss point, g_j): its own ones in
+    // the first 18 tasks, its products with the other gradients in the last 18; then
+    // the nodal forces on slots 6-8
+#pragma unroll 1
+    for (int task = slot; task < 36; task += kSlots) {
+        const int gp = task % 6, j = (task / 6) % 3;
+        auto at = [&](int v) -> float2& { return sg[(v * 6 + gp) * NE + el]; };
+        auto ct = [&](int v) { return sc0[(v * 6 + gp) * NE + el]; };
+        const float2 a[3] = {at(Y::G + 3 * j), at(Y::G + 3 * j + 1), at(Y::G + 3 * j + 2)};
+        float2 s6[6], o[3];
+        if (task < 18) {
             if constexpr (VISC) {
 #pragma unroll
-                for (int k = 0; k < 9; ++k) Pm[k] = df_split(visc ? G.pv[k] : 0.0);
-            }
-            // VISC: one FP64 stress sigma' + sigma_v' for the forces; the
-            // tangent's sigma' dN and sigma_v' dN in double-float from the
-            // splits of the two stresses (54 FP64 multiply-adds and 36 splits
-            // fewer per Gauss point than forming both products in FP64)
-            double st[6];
-            float2 sgs[6], svs[6];
-            if constexpr (VISC) {
+                for (int k = 0; k < 6; ++k) s6[k] = ct(Y::SV + k);
+                df_sym_apply(s6, a, o);
 #pragma unroll
-                for (int k = 0; k < 6; ++k) {
-                    st[k] = visc ? G.sg[k] + G.sv[k] : G.sg[k];
-                    sgs[k] = df_split(G.sg[k]);
-                    svs[k] = df_split(visc ? G.sv[k] : 0.0);
-                }
-            }
+                for (int i = 0; i < 3; ++i) {
+                    at(Y::V + 3 * j + i) = o[i];
+                    float wH = 0.f, wL = 0.f;  // w = Q^T g
 #pragma unroll
-            for (int a = 0; a < 6; ++a) {
-                const double d0 = G.dn[3 * a], d1 = G.dn[3 * a + 1], d2 = G.dn[3 * a + 2];
-                const float2 dn[3] = {df_split(d0), df_split(d1), df_split(d2)};
-                if constexpr (VISC) {
-                    double s3[3];
-                    sym_apply(st, d0, d1, d2, s3);
-                    float2 sd[3];
-                    df_sym_apply(sgs, dn, sd);
-#pragma unroll
-                    for (int i = 0; i < 3; ++i) {
-                        S.dn[3 * a + i] = dn[i];
-                        S.fs[3 * a + i] = s3[i];
-                        S.sdn[3 * a + i] = sd[i];
-                    }
-                } else {
-                    double s3[3];
-                    sym_apply(G.sg, d0, d1, d2, s3);
-#pragma unroll
-                    for (int i = 0; i < 3; ++i) {
-                        S.dn[3 * a + i] = dn[i];
-                        S.fs[3 * a + i] = s3[i];
-                        S.sdn[3 * a + i] = df_split(s3[i]);
-                    }
-                }
-                if constexpr (VISC) {
-                    float2 vs[3];
-                    df_sym_apply(svs, dn, vs);
-#pragma unroll
-                    for (int i = 0; i < 3; ++i) {
-                        const float2 vv = vs[i];
-                        S.v[3 * a + i] = vv;
-                        // u = c1 dN + sigma_v' dN
-                        float uH = 0.0f, uL = 0.0f;
-                        df_mac(uH, uL, c1, dn[i]);
-                        df_add(uH, uL, vv);
-                        df_norm(uH, uL);
-                        S.u[3 * a + i] = make_float2(uH, uL);
-                        // w = c2 dN + P^T dN
-                        float wH = 0.0f, wL = 0.0f;
-                        df_mac(wH, wL, c2, dn[i]);
-#pragma unroll
-                        for (int j = 0; j < 3; ++j) df_mac(wH, wL, Pm[3 * j + i], dn[j]);
-                        df_norm(wH, wL);
-                        S.w[3 * a + i] = make_float2(wH, wL);
-                    }
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 3; ++i) {
-                        float uH = 0.0f, uL = 0.0f, wH = 0.0f, wL = 0.0f;
-                        df_mac(uH, uL, c1, dn[i]);
-                        df_mac(wH, wL, c2, dn[i]);
-                        S.u[3 * a + i] = make_float2(uH, uL);
-                        S.w[3 * a + i] = make_float2(wH, wL);
-                    }
-                }
-            }
-            if constexpr (VISC) {
-                // Q = c2 I + P
-#pragma unroll
-                for (int k = 0; k < 9; ++k) {
-                    float qH = Pm[k].x, qL = Pm[k].y;
-                    if (k == 0 || k == 4 || k == 8) {
-                        df_add(qH, qL, c2);
-                        df_norm(qH, qL);
-                    }
-                    S.Q[k] = make_float2(qH, qL);
+                    for (int k = 0; k < 3; ++k) df_mac(wH, wL, at(Y::Q + 3 * k + i), a[k]);
+                    df_norm(wH, wL);
+                    at(Y::W + 3 * j + i) = make_float2(wH, wL);
                 }
             } else {
-                S.c2 = c2;
+                const float2 c1 = ct(Y::C1), c2 = ct(Y::C2);
+#pragma unroll
+                for (int i = 0; i < 3; ++i) {
+                    at(Y::U + 3 * j + i) = df_scale(c1, a[i]);
+                    at(Y::W + 3 * j + i) = df_scale(c2, a[i]);
+                }
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < 6; ++k) s6[k] = ct(Y::SG + k);
+            df_sym_apply(s6, a, o);
+#pragma unroll 1
+            for (int l = j; l < 3; ++l) {
+                float sH = 0.f, sL = 0.f, tH = 0.f, tL = 0.f;
+#pragma unroll
+                for (int i = 0; i < 3; ++i) {
+                    const float2 b = at(Y::G + 3 * l + i);
+                    df_mac(tH, tL, o[i], b);
+                    if constexpr (!VISC) df_mac(sH, sL, a[i], b);
+                }
+                if constexpr (!VISC) {
+                    df_norm(sH, sL);
+                    df_mac(tH, tL, ct(Y::C2), make_float2(sH, sL));
+                }
+                df_norm(tH, tL);
+                at((VISC ? Y::T : Y::D) + sym_index(j, l)) = make_float2(tH, tL);
+            }
+        }
+    }
+    // component c of the forces: f_a = - sum_g (sigma' + sigma_v') dN_a
+    // (ShapeBase.cpp:2203-2227), the weights one factor at a time
+    if (live && slot >= 6 && slot < 9) {
+        const int c = slot - 6;
+        auto h = [&](int j, int gp) { return hf[((size_t)(3 * j + c) * 6 + gp) * NE + el]; };
+        double T[2][2], z[3];  // T[j][layer]
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const double s0 = h(j, 0) + h(j, 1) + h(j, 2), s1 = h(j, 3) + h(j, 4) + h(j, 5);
+            T[j][0] = fma(wa, s0, wb * s1);
+            T[j][1] = fma(wb, s0, wa * s1);
+        }
+#pragma unroll
+        for (int t = 0; t < 3; ++t) z[t] = h(2, t) + h(2, 3 + t);
+        const double zs = (z[0] + z[1] + z[2]) * (1.0 / 12.0);
+#pragma unroll
+        for (int a = 0; a < 6; ++a) {
+            const int i = a % 3, up = a / 3;
+            const double in = i == 0 ? -(T[0][up] + T[1][up]) : T[i - 1][up];
+            const double zi = fma(0.25, z[i], zs);
+            const double f = up ? -(in + zi) : zi - in;
+            const int node = __ldg(&A.conn[a * ne + e]);
+            if (!TF_IN(A.check, node, A.nn, CK_ELEM_NODE)) continue;
+            const bool fx = A.fixed[3 * node + c] != 0;
+            if (MODE == kStore) A.ef[(size_t)(3 * a + c) * ne + e] = fx ? 0.0 : f;
+            else if (!fx) atomicAdd(&A.g[3 * node + c], f);
+        }
+    }
+    __syncthreads();
+
+    // ---- 4. the blocks B(g_j, g_l), one Gauss point after the other: a unit is
+    // stored by itself or added to the units before it (A_jl over the in-plane
+    // points; B(g_3, g_3) over the heights with viscosity)
+    auto blk = [&](int b) { return st + (size_t)b * 9 * NE + el; };
+    {
+        float SH[9], SL[9];
+        constexpr int kUnits = VISC ? 5 : 3;
+#pragma unroll 1
+        for (int u = 0; u < kUnits; ++u) {
+            int j, l, gp, b;
+            bool first = true, last = true;
+            if (VISC && u < 2) {  // slots 0-5: (j, 3), 6-11: (3, l); both heights
+                const int t = (slot / 2) % 3;
+                j = slot < 6 ? slot % 2 : 2;
+                l = slot < 6 ? 2 : slot % 2;
+                gp = 3 * u + t;
+                b = Y::BR + 6 * (slot < 6 ? slot % 2 : 2 + slot % 2) + gp;
+            } else if (VISC) {
+                if (slot < 8) {
+                    j = slot / 4;
+                    l = (slot / 2) % 2;
+                    gp = 3 * (slot % 2) + u - 2;
+                    b = Y::BA + slot;
+                    first = u == 2;
+                    last = u == 4;
+                } else {
+                    if (slot == 11 || u == 4) break;
+                    j = l = 2;
+                    gp = slot - 8 + 3 * (u - 2);
+                    b = Y::BB + slot - 8;
+                    first = u == 2;
+                    last = u == 3;
+                }
+            } else if (slot < 6) {  // A_jl, pairs 11 12 22
+                j = slot / 4;
+                l = slot < 2 ? 0 : 1;
+                gp = 3 * (slot % 2) + u;
+                b = Y::BA + slot;
+                first = u == 0;
+                last = u == 2;
+            } else if (u < 2) {
+                const int q = slot - 6;
+                j = q % 2;
+                l = 2;
+                gp = 3 * u + q / 2;
+                b = Y::BR + 6 * j + gp;
+            } else {
+                j = l = 2;
+                gp = slot - 6;
+                b = Y::BB + gp;
+            }
+            float H[9], L[9];
+            gp_block<NE, VISC>(sg, j, l, gp, el, H, L);
+#pragma unroll
+            for (int k = 0; k < 9; ++k) {
+                if (!first) {
+                    const float2 x = df_sum<false>(make_float2(SH[k], SL[k]), make_float2(H[k], L[k]));
+                    H[k] = x.x;
+                    L[k] = x.y;
+                }
+                SH[k] = H[k];
+                SL[k] = L[k];
+            }
+            if (last) {
+                float2* o = blk(b);
+#pragma unroll
+                for (int k = 0; k < 9; ++k) o[k * NE] = make_float2(H[k], L[k]);
             }
         }
     }
     __syncthreads();
 
-    // ---------------- element forces: Gauss sum, fixed mask, scatter ------
-    // f_a = - sum_g (sigma' + sigma_v') dN_a  (ShapeBase.cpp:2203-2227)
-    for (int task = tid; task < NE * 18; task += NT) {
-        const int el = task / 18;
-        const int k = task - el * 18;
-        const int e = blockIdx.x * NE + el;
-        if (!element_live(A, e)) continue;
-        double f = 0.0;
+    // ---- 5. the weights, entry by entry -----------------------------------------
+    auto xblk = [&](int b) { return sg + (size_t)b * 9 * NE + el; };
+    constexpr bool kFull = !VISC;
+    {
+        // H(layer, k) = sum over the in-plane points and heights of N_k/2 L_layer B:
+        // S + 3 (k) in the plane, sqrt(3)/2 (B0 + B1) -+ (B0 - B1)/2 over the heights
+        constexpr int kGroups = kSlots / Y::NR;
+        float2* r = blk(Y::BR + 6 * (slot % Y::NR));
+#pragma unroll 1
+        for (int k = slot / Y::NR; k < 9; k += kGroups) {
+            float2 p[3], d[3];
 #pragma unroll
-        for (int gp = 0; gp < kGauss; ++gp) {
-            f -= sh[el * kGauss + gp].fs[k];
+            for (int t = 0; t < 3; ++t) {
+                const float2 x = r[(9 * t + k) * NE], y = r[(9 * (3 + t) + k) * NE];
+                p[t] = df_scale(DF_CONST(0.5 * kSqrt3), df_sum<kFull>(x, y));
+                d[t] = df_pow2(0.5f, df_sum<kFull>(x, df_neg(y)));
+            }
+            const float2 ps = df_sum<kFull>(df_sum<kFull>(p[0], p[1]), p[2]);
+            const float2 ds = df_sum<kFull>(df_sum<kFull>(d[0], d[1]), d[2]);
+#pragma unroll
+            for (int t = 0; t < 3; ++t) {
+                const float2 x = df_muladd(ps, 3.f, p[t]), y = df_muladd(ds, 3.f, d[t]);
+                r[(9 * t + k) * NE] = df_sum<kFull>(x, df_neg(y));
+                r[(9 * (3 + t) + k) * NE] = df_sum<kFull>(x, y);
+            }
         }
-        const int a = k / 3, d = k - 3 * (k / 3);
-        const int node = __ldg(&A.conn[a * A.ne + e]);
-        if (!TF_IN(A.check, node, A.nn, CK_ELEM_NODE)) continue;
-        const bool fx = A.fixed[3 * node + d] != 0;
-        if (MODE == kStore) A.ef[(size_t)k * A.ne + e] = fx ? 0.0 : f;
-        else if (!fx) atomicAdd(&A.g[3 * node + d], f);
     }
+    {
+        // M = sum over the heights of the two layers' weights times A: with
+        // p = A0 + A1 and d = sqrt(3)/2 (A0 - A1), bb p - d, bt p/2, tt p + d
+        constexpr int kGroups = kSlots / Y::NJL;
+        const int q = slot % Y::NJL;
+        float2 *a0 = blk(Y::BA + 2 * q), *a1 = a0 + 9 * NE, *a2 = xblk(Y::XM + q);
+#pragma unroll 1
+        for (int k = slot / Y::NJL; k < 9; k += kGroups) {
+            const float2 x = a0[k * NE], y = a1[k * NE];
+            const float2 p = df_sum<kFull>(x, y);
+            const float2 d = df_scale(DF_CONST(0.5 * kSqrt3), df_sum<kFull>(x, df_neg(y)));
+            a0[k * NE] = df_sum<kFull>(p, df_neg(d));
+            a1[k * NE] = df_pow2(0.5f, p);
+            a2[k * NE] = df_sum<kFull>(p, d);
+        }
+    }
+    {
+        // W(i, k) = sum_t N_i N_k/4 B(t): S + 15 B(i), or S + 3 (B(i) + B(k))
+        const int q = slot % 6;
+        const int i = q < 3 ? q : (q < 5 ? 0 : 1), k2 = q < 3 ? q : (q == 3 ? 1 : 2);
+        float2* o = xblk(Y::XW + q);
+#pragma unroll 1
+        for (int k = slot / 6; k < 9; k += 2) {
+            float2 b[3];
+#pragma unroll
+            for (int t = 0; t < 3; ++t) {
+                b[t] = blk(Y::BB + t)[k * NE];
+                if (!VISC) b[t] = df_sum<kFull>(b[t], blk(Y::BB + 3 + t)[k * NE]);
+            }
+            const float2 s = df_sum<kFull>(df_sum<kFull>(b[0], b[1]), b[2]);
+            const float2 bi = i == 0 ? b[0] : (i == 1 ? b[1] : b[2]), bk = k2 == 1 ? b[1] : b[2];
+            o[k * NE] = i == k2 ? df_muladd(s, 15.f, bi) : df_muladd(s, 3.f, df_sum<kFull>(bi, bk));
+        }
+    }
+    __syncthreads();
+    if (!live) return;
 
-    // ---------------- phase B: 3x3 node-pair blocks ------------------------
+    // ---- 6. the node pairs ------------------------------------------------------
     constexpr int kPairs = VISC ? 36 : 21;
-    for (int task = tid; task < NE * kPairs; task += NT) {
-        const int el = task / kPairs;
-        const int pr = task - el * kPairs;
-        const int e = blockIdx.x * NE + el;
-        if (!element_live(A, e)) continue;
+#pragma unroll 1
+    for (int pr = slot; pr < kPairs; pr += kSlots) {
         const int a = VISC ? pr / 6 : kPairA[pr];
         const int bq = VISC ? pr - 6 * (pr / 6) : kPairB[pr];
-        float aH[9], aL[9];
+        const int i = a % 3, la = a / 3, k2 = bq % 3, lb = bq / 3;
+        // node 0 has both in-plane gradients, negated; node j the j-th
+        const int j0 = i == 2 ? 1 : 0, l0 = k2 == 2 ? 1 : 0, nj = i == 0 ? 2 : 1, nl = k2 == 0 ? 2 : 1;
+        const float si = i == 0 ? -1.f : 1.f, sk = k2 == 0 ? -1.f : 1.f;
+        const float ta = la ? 1.f : -1.f, tb = lb ? 1.f : -1.f;
+        float H[9], L[9], E[9];
 #pragma unroll
-        for (int k = 0; k < 9; ++k) aH[k] = aL[k] = 0.0f;
+        for (int k = 0; k < 9; ++k) H[k] = L[k] = E[k] = 0.f;
 #pragma unroll 1
-        for (int gp = 0; gp < kGauss; ++gp) {
-            const Gp& S = sh[el * kGauss + gp];
-            const float2 a3[3] = {S.dn[3 * a], S.dn[3 * a + 1], S.dn[3 * a + 2]};
-            const float2 b3[3] = {S.dn[3 * bq], S.dn[3 * bq + 1], S.dn[3 * bq + 2]};
-            float sH = 0.0f, sL = 0.0f, tH = 0.0f, tL = 0.0f;
-#pragma unroll
-            for (int j = 0; j < 3; ++j) {
-                df_mac(sH, sL, a3[j], b3[j]);
-                df_mac(tH, tL, a3[j], S.sdn[3 * bq + j]);
-            }
-            const float2 ua[3] = {S.u[3 * a], S.u[3 * a + 1], S.u[3 * a + 2]};
-            const float2 wa[3] = {S.w[3 * a], S.w[3 * a + 1], S.w[3 * a + 2]};
-            if constexpr (VISC) {
-                const float2 s2 = make_float2(sH, sL), t2 = make_float2(tH, tL);
-                const float2 vb[3] = {df_neg(S.v[3 * bq]), df_neg(S.v[3 * bq + 1]), df_neg(S.v[3 * bq + 2])};
-#pragma unroll
-                for (int i = 0; i < 3; ++i)
-#pragma unroll
-                    for (int k = 0; k < 3; ++k) {
-                        float& H = aH[3 * i + k];
-                        float& L = aL[3 * i + k];
-                        df_mac(H, L, ua[i], b3[k]);
-                        df_mac(H, L, b3[i], wa[k]);
-                        df_mac(H, L, vb[i], a3[k]);
-                        df_mac(H, L, s2, S.Q[3 * i + k]);
-                        if (i == k) df_add(H, L, t2);
-                        df_norm(H, L);
-                    }
+        for (int m = 0; m < 1 + nj + nl + nj * nl; ++m) {
+            const float2* x;
+            float s;
+            bool tr = false;  // transposed (the symmetric case stores one triangle)
+            if (m == 0) {
+                x = xblk(Y::XW + sym_index(i, k2));
+                s = ta * tb;
+            } else if (m <= nj) {
+                x = blk(Y::BR + 6 * (j0 + m - 1) + 3 * la + k2);
+                s = si * tb;
+            } else if (m <= nj + nl) {
+                const int l = l0 + m - 1 - nj;
+                x = blk(Y::BR + 6 * (VISC ? 2 + l : l) + 3 * lb + i);
+                s = sk * ta;
+                tr = !VISC;
             } else {
-                // c2 s + t on the diagonal
-                float dH = tH, dL = tL;
-                df_mac(dH, dL, S.c2, make_float2(sH, sL));
-                const float2 dg = make_float2(dH, dL);
-#pragma unroll
-                for (int i = 0; i < 3; ++i)
-#pragma unroll
-                    for (int k = 0; k < 3; ++k) {
-                        float& H = aH[3 * i + k];
-                        float& L = aL[3 * i + k];
-                        df_mac(H, L, ua[i], b3[k]);
-                        df_mac(H, L, b3[i], wa[k]);
-                        if (i == k) df_add(H, L, dg);
-                        df_norm(H, L);
-                    }
+                const int q = m - 1 - nj - nl;
+                const int j = j0 + q / nl, l = l0 + q % nl;
+                const int jl = VISC ? 2 * j + l : j + l;
+                x = la != lb ? blk(Y::BA + 2 * jl + 1) : (la ? xblk(Y::XM + jl) : blk(Y::BA + 2 * jl));
+                s = si * sk;
+                tr = !VISC && j > l;
             }
+            const int s1 = tr ? 3 * NE : NE, s3 = tr ? NE : 3 * NE;
+#pragma unroll
+            for (int k = 0; k < 9; ++k)
+                df_addmul<kFull>(H[k], L[k], E[k], s, x[(k / 3) * s3 + (k % 3) * s1]);
         }
         double acc[9];
 #pragma unroll
-        for (int k = 0; k < 9; ++k) acc[k] = df_join(aH[k], aL[k]);
-        const int na = __ldg(&A.conn[a * A.ne + e]);
-        const int nb = __ldg(&A.conn[bq * A.ne + e]);
+        for (int k = 0; k < 9; ++k) {
+            if (kFull) L[k] = __fadd_rn(L[k], E[k]);
+            df_norm(H[k], L[k]);
+            acc[k] = df_join(H[k], L[k]);
+        }
+        const int na = __ldg(&A.conn[a * ne + e]);
+        const int nb = __ldg(&A.conn[bq * ne + e]);
         if (!TF_IN(A.check, na, A.nn, CK_ELEM_NODE) || !TF_IN(A.check, nb, A.nn, CK_ELEM_NODE)) continue;
         bool fr[3], fc[3];
 #pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            fr[i] = A.fixed[3 * na + i] != 0;
-            fc[i] = A.fixed[3 * nb + i] != 0;
+        for (int q = 0; q < 3; ++q) {
+            fr[q] = A.fixed[3 * na + q] != 0;
+            fc[q] = A.fixed[3 * nb + q] != 0;
         }
         const bool mirror = !VISC && (a != bq);
         if (MODE == kStore) {
-            const size_t stride = (size_t)36 * A.ne;
-            const size_t base = (size_t)(6 * a + bq) * A.ne + e;
-            const size_t baseT = (size_t)(6 * bq + a) * A.ne + e;
+            const size_t stride = (size_t)36 * ne;
+            const size_t base = (size_t)(6 * a + bq) * ne + e;
+            const size_t baseT = (size_t)(6 * bq + a) * ne + e;
 #pragma unroll
-            for (int i = 0; i < 3; ++i)
+            for (int r = 0; r < 3; ++r)
 #pragma unroll
                 for (int k = 0; k < 3; ++k) {
-                    const double v = (fr[i] || fc[k]) ? 0.0 : acc[3 * i + k];
-                    A.eblk[(3 * i + k) * stride + base] = v;
-                    if (mirror) A.eblk[(3 * k + i) * stride + baseT] = v;
+                    const double v = (fr[r] || fc[k]) ? 0.0 : acc[3 * r + k];
+                    A.eblk[(3 * r + k) * stride + base] = v;
+                    if (mirror) A.eblk[(3 * k + r) * stride + baseT] = v;
                 }
         } else {
-            const int off = __ldg(&A.slot[(6 * a + bq) * A.ne + e]);
+            const int off = __ldg(&A.slot[(6 * a + bq) * ne + e]);
             if (!TF_IN(A.check, off, A.nval - 8 * kSlice, CK_ELEM_SLOT)) continue;
             double* dst = A.val + off;
 #pragma unroll
-            for (int i = 0; i < 3; ++i)
+            for (int r = 0; r < 3; ++r)
 #pragma unroll
                 for (int k = 0; k < 3; ++k)
-                    if (!fr[i] && !fc[k]) atomicAdd(dst + kSlice * (3 * i + k), acc[3 * i + k]);
+                    if (!fr[r] && !fc[k]) atomicAdd(dst + kSlice * (3 * r + k), acc[3 * r + k]);
             if (mirror) {
-                const int offT = __ldg(&A.slot[(6 * bq + a) * A.ne + e]);
+                const int offT = __ldg(&A.slot[(6 * bq + a) * ne + e]);
                 if (!TF_IN(A.check, offT, A.nval - 8 * kSlice, CK_ELEM_SLOT)) continue;
                 double* dt = A.val + offT;
 #pragma unroll
-                for (int i = 0; i < 3; ++i)
+                for (int r = 0; r < 3; ++r)
 #pragma unroll
                     for (int k = 0; k < 3; ++k)
-                        if (!fr[i] && !fc[k]) atomicAdd(dt + kSlice * (3 * k + i), acc[3 * i + k]);
+                        if (!fr[r] && !fc[k]) atomicAdd(dt + kSlice * (3 * k + r), acc[3 * r + k]);
             }
         }
     }
@@ -846,6 +1227,7 @@ ElemArgs make_args(tf_handle* h) {
     ElemArgs A{};
     A.ne = d.ne;
     A.conn = d.conn;
+    A.ginv = d.ginv;
     A.gx = d.gx;
     A.wdet = d.wdet;
     A.invFg = d.invFg;
@@ -872,13 +1254,13 @@ ElemArgs make_args(tf_handle* h) {
 
 template <int NE, int MODE, bool VISC>
 tf_status launch_fast(tf_handle* h, const ElemArgs& A) {
-    const size_t smem = sizeof(GpFast<VISC>) * NE * kGauss;
+    constexpr size_t smem = elem_smem<NE, VISC>();
     static int configured_device = -1;
     if (configured_device != h->device) {
         TF_CUDA(cudaFuncSetAttribute(k_element<NE, MODE, VISC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         configured_device = h->device;
     }
-    k_element<NE, MODE, VISC><<<cdiv(A.ne, NE), NE * kGauss * kTpg, smem, h->stream>>>(A);
+    k_element<NE, MODE, VISC><<<cdiv(A.ne, NE), NE * kSlots, smem, h->stream>>>(A);
     TF_LAUNCH_CHECK(h);
     return TF_OK;
 }
@@ -900,13 +1282,40 @@ tf_status launch_with(tf_handle* h, const ElemArgs& A, int ne_per_cta) {
 
 }  // namespace
 
+struct ShapeDerivatives {
+    double dN[6][3][6];
+};
+// dN_X = InvdXde^T dN of every prism and Gauss point (Prism.cpp:705-728)
+__global__ void k_shape_gradients(int ne, ShapeDerivatives S, const double* __restrict__ ginv, double* __restrict__ gx) {
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;  // 6 e + gp
+    if (q >= 6 * ne) return;
+    const int e = q / 6, gp = q - 6 * e;
+    double inv[9];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) inv[k] = ginv[((size_t)k * 6 + gp) * ne + e];
+#pragma unroll
+    for (int a = 0; a < 6; ++a)
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+            gx[(size_t)(3 * a + k) * (6 * (size_t)ne) + q] =
+                inv[k] * S.dN[gp][0][a] + inv[3 + k] * S.dN[gp][1][a] + inv[6 + k] * S.dN[gp][2][a];
+}
+
+tf_status launch_shape_gradients(tf_handle* h, const double* dN) {
+    ShapeDerivatives S;
+    std::memcpy(S.dN, dN, sizeof(S.dN));
+    k_shape_gradients<<<cdiv(6 * (int64_t)h->d.ne, 256), 256, 0, h->stream>>>(h->d.ne, S, h->d.ginv, h->d.gx);
+    TF_LAUNCH_CHECK(h);
+    return TF_OK;
+}
+
 tf_status launch_element(tf_handle* h) {
     const ElemArgs A = make_args(h);
     if (A.ne <= 0) return TF_OK;
     return launch_with(h, A, h->elem_cta);
 }
 
-// Picks the prisms-per-CTA tile (8, 16 or 32 prisms x 6 Gauss points) by
+// Picks the prisms-per-CTA tile (8, 16 or 32 prisms) by
 // timing each candidate on the handle's own mesh; run once per handle before
 // the first assembly.  Results do not depend on the choice.
 tf_status autotune_element(tf_handle* h) {

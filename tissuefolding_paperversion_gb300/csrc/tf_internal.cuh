@@ -56,10 +56,7 @@ __device__ __forceinline__ bool check_in(int* flag, long long i, long long n, in
 constexpr int kSlice = 32;
 constexpr int kSlotDoubles = 9 * kSlice;
 
-// Element-kernel tiling: NE prisms per CTA, one thread per Gauss point.
-constexpr int kGauss = 6;
-constexpr int kElemPerCta = 16;
-constexpr int kCtaThreads = kElemPerCta * kGauss;  // 96
+constexpr int kGauss = 6;  // Gauss points per prism
 
 struct Device {
     // sizes
@@ -68,9 +65,9 @@ struct Device {
     bool any_visc = false;
     // mesh / material (SoA)
     int* conn = nullptr;        // [6][ne]
+    double* ginv = nullptr;     // [9][6][ne] dxi_j/dX_k of each Gauss point (index 3 j + k)
     double* gx = nullptr;       // [18][6*ne] reference shape gradients
     double* wdet = nullptr;     // [6*ne] w * det(dX/dxi)
-    double* detdxde = nullptr;  // [6*ne]
     double* Fg = nullptr;       // [9][ne]
     double* invFg = nullptr;    // [9][ne]
     double* rates = nullptr;    // [3][ne] growth rates (1/s)
@@ -472,6 +469,7 @@ tf_status launch_update_norm(tf_handle* h);   // |du|^2 into S_DU2 without apply
 tf_status newton_device_loop(tf_handle* h, int* it, int* cv, int* capped, int* k, tf_step_stats* st, float* ms_asm,
                              bool* ran, bool* exc);
 tf_status autotune_element(tf_handle* h);
+tf_status launch_shape_gradients(tf_handle* h, const double* dN);  // gx from ginv; dN[6][3][6] on the host
 tf_status amg_build(tf_handle* h, const double* ref_pos);
 tf_status amg_numeric(tf_handle* h);
 void amg_refresh(tf_handle* h);     // launches the level-0 smoother copies of the current assembly
