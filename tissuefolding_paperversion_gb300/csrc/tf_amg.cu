@@ -1026,33 +1026,36 @@ __device__ __forceinline__ void row6_warp(const AmgLevel& L, int i, const float*
         }
 }
 
-// y = S x for row i of a 6-DOF level, S = D^-1 A stored in FP16 (the
-// element blocks only; extra6 adds the coarse image of the extra blocks).
-__device__ __forceinline__ void row6_warp_h(const AmgLevel& L, int i, const float* __restrict__ x, float y[6]) {
+// y_a = (S x)_a on lane a < 6 for a row of a 6-DOF level (blocks p0 .. p1), S =
+// D^-1 A stored in FP16 (the element blocks only; extra6 adds the coarse image of
+// the extra blocks).  Lane 6 k + a (< 30) takes row a of blocks k, k + 5, ...; the
+// columns of up to 30 blocks are loaded before the first is used, so a row costs
+// three dependent loads (range, columns, values) however long it is (two blocks
+// per lane at a time: 7.5 against 6.6 us per sweep of the 8,978-node level).
+__device__ __forceinline__ float row6_warp_h(const AmgLevel& L, int p0, int p1, const float* __restrict__ x) {
     const int lane = threadIdx.x & 31;
     const int kb = lane / 6, a = lane - 6 * kb;
     float acc = 0.f;
-    const int p0 = L.rowptr[i], p1 = L.rowptr[i + 1];
-    if (lane < 30) {
-#pragma unroll 2
-        for (int p = p0 + kb; p < p1; p += 5) {
-            const int j = __ldg(&L.colidx[p]);
-            const __half2* __restrict__ v = reinterpret_cast<const __half2*>(L.valh + 36 * (size_t)p + 6 * a);
-            const float* __restrict__ xj = x + 6 * (size_t)j;
+    for (int pb = p0 + kb; pb - kb < p1; pb += 30) {
+        int j[6];
 #pragma unroll
-            for (int b2 = 0; b2 < 3; ++b2) {
-                const float2 f = __half22float2(__ldg(&v[b2]));
-                acc = fmaf(f.x, xj[2 * b2], fmaf(f.y, xj[2 * b2 + 1], acc));
+        for (int u = 0; u < 6; ++u) j[u] = (lane < 30 && pb + 5 * u < p1) ? __ldg(&L.colidx[pb + 5 * u]) : -1;
+#pragma unroll
+        for (int u = 0; u < 6; ++u) {
+            if (j[u] < 0) continue;
+            const __half2* __restrict__ v = reinterpret_cast<const __half2*>(L.valh + 36 * (size_t)(pb + 5 * u) + 6 * a);
+            const float2* __restrict__ xj = reinterpret_cast<const float2*>(x + 6 * (size_t)j[u]);
+#pragma unroll
+            for (int b = 0; b < 3; ++b) {
+                const float2 f = __half22float2(__ldg(&v[b])), w = xj[b];
+                acc = fmaf(f.x, w.x, fmaf(f.y, w.y, acc));
             }
         }
     }
+    float y = acc;
 #pragma unroll
-    for (int k = 0; k < 6; ++k) {
-        float s2 = 0.f;
-#pragma unroll
-        for (int g = 0; g < 5; ++g) s2 += __shfl_sync(0xffffffffu, acc, 6 * g + k);
-        y[k] = s2;
-    }
+    for (int g = 1; g < 5; ++g) y += __shfl_down_sync(0xffffffffu, acc, 6 * g);
+    return y;
 }
 
 // e = X x for row i: the coarse image of the extra blocks (every lane)
@@ -1592,7 +1595,7 @@ struct V0 {  // level-0 operands
 // and the restricted residual P^T (r - A z) is Q^T r for a symmetric A (the
 // viscous tangent's asymmetry, of the order of eta |grad v| / E, only changes
 // the preconditioner).  So the smoother's matrix is read once instead of twice,
-// and that product does not wait for the coarse levels: k_q_restrict (Q^T r),
+// and that product does not wait for the coarse levels: k_restrict with Q (Q^T r),
 // the coarse levels, k_q_post; k_q_smooth runs beside the coarse levels where
 // those are a chain of launches, and is part of k_q_post where they are one
 // dense product.  Bound by reading S (66 MB at 320,000 prisms) and Q twice (52 MB
@@ -1602,32 +1605,39 @@ struct V0 {  // level-0 operands
 // with extra blocks (packing couples, added entries) keep the kernels that apply
 // the current matrix: k_v0_resid .. k_v0_post below.
 
-// r_C(I) = sum over the blocks (i, I) of Q_iI^T r_i, and the coarse level's first
-// sweep; one CTA of kRestrictThreads per coarse node, its threads striding over
-// the (block, row) pairs of the column, stored contiguously.
-__global__ void __launch_bounds__(kRestrictThreads) k_q_restrict(AmgQ Q, AmgLevel C, int nf, int* check,
-                                                                 const float* __restrict__ r,
-                                                                 const double* __restrict__ scal,
-                                                                 const double* __restrict__ omegaC, int presmooth) {
+// r_C(I) = sum over the blocks (i, I) of P_iI^T t_i (of Q for the folded level-0
+// transfer) and, with presmooth, the coarse level's first sweep x_C = omega_C D_C^-1
+// r_C.  One CTA of kRestrictThreads per coarse node, its threads striding over the
+// (block, row) pairs of the column, stored contiguously (one warp per node: 7.5
+// against 6.0 us from 8,978 to 391 nodes).  V: __half or float values, 6 per pair.
+template <int BS, class V>
+__global__ void __launch_bounds__(kRestrictThreads) k_restrict(const int* __restrict__ cptr,
+                                                               const int* __restrict__ crow,
+                                                               const V* __restrict__ val, AmgLevel C, int nf, int* check,
+                                                               const float* __restrict__ t,
+                                                               const double* __restrict__ scal,
+                                                               const double* __restrict__ omegaC, int presmooth) {
     __shared__ float sm[kRestrictThreads / 32][6];
     pdl_enter();
     const int I = blockIdx.x;
     if (seg_stopped(scal, C.seg[I])) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int q0 = __ldg(&Q.cptr[I]), np = 3 * (__ldg(&Q.cptr[I + 1]) - q0);
+    const int q0 = __ldg(&cptr[I]), np = BS * (__ldg(&cptr[I + 1]) - q0);
     float rc[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll 4
     for (int q = threadIdx.x; q < np; q += kRestrictThreads) {
-        const int m = q / 3, k = q - 3 * m;
-        const int i = __ldg(&Q.crow[q0 + m]);
+        const int m = q / BS, k = q - BS * m;
+        const int i = __ldg(&crow[q0 + m]);
         if (!TF_IN(check, i, nf, CK_RESTRICT_ROW)) continue;
-        const float t = r[3 * (size_t)i + k];
-        const __half2* __restrict__ P = reinterpret_cast<const __half2*>(Q.cval + 9 * (size_t)(q0 + m) + 3 * k);
+        const float tk = t[BS * (size_t)i + k];
+        const V* __restrict__ P = val + 6 * ((size_t)BS * q0 + q);
 #pragma unroll
         for (int b = 0; b < 3; ++b) {
-            const float2 f = __half22float2(__ldg(&P[b]));
-            rc[2 * b] = fmaf(f.x, t, rc[2 * b]);
-            rc[2 * b + 1] = fmaf(f.y, t, rc[2 * b + 1]);
+            float2 f;
+            if constexpr (sizeof(V) == 2) f = __half22float2(__ldg(reinterpret_cast<const __half2*>(P) + b));
+            else f = __ldg(reinterpret_cast<const float2*>(P) + b);
+            rc[2 * b] = fmaf(f.x, tk, rc[2 * b]);
+            rc[2 * b + 1] = fmaf(f.y, tk, rc[2 * b + 1]);
         }
     }
 #pragma unroll
@@ -1799,111 +1809,32 @@ __global__ void k_v0_prolong(V0 a, AmgLevel F, const float* __restrict__ e, floa
     }
 }
 
-// r_C(I) = sum over the prolongator blocks (i, I) of P_iI^T t_i;
-// x_C = omega_C D_C^-1 r_C (pre-smoothing), by one warp: the lanes stride
-// over the (block, row) pairs of column I, stored contiguously.
-template <int BS>
-__device__ __forceinline__ void restrict_node(const AmgLevel& F, const AmgLevel& C, const float* __restrict__ t,
-                                              int I, const double* __restrict__ omegaC, int presmooth) {
-    const int lane = threadIdx.x & 31;
-    float rc[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    const int q0 = F.pcptr[I], np = BS * (F.pcptr[I + 1] - q0);
-    constexpr bool kHalf = BS == 3;  // level 0: the FP16 copy of the prolongator
-    const float* __restrict__ Pc = F.Pc + (size_t)q0 * BS * 6;
-    const __half* __restrict__ Pch = kHalf ? F.Pch + (size_t)q0 * BS * 6 : nullptr;
-    for (int qa = lane; qa < np; qa += 64) {
-        // two (block, row) pairs per lane and pass: their loads overlap
-        float tk[2] = {0.f, 0.f};
-        int qq[2] = {0, 0};
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-            const int q = qa + 32 * u;
-            if (q < np) {
-                const int m = q / BS, k = q - BS * m;
-                const int i = __ldg(&F.pcrow[q0 + m]);
-                if (!TF_IN(F.check, i, F.n, CK_RESTRICT_ROW)) continue;
-                tk[u] = t[BS * (size_t)i + k];
-                qq[u] = q;
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-            if constexpr (kHalf) {
-                const __half2* __restrict__ P2 = reinterpret_cast<const __half2*>(Pch + 6 * (size_t)qq[u]);
-#pragma unroll
-                for (int b = 0; b < 3; ++b) {
-                    const float2 f = __half22float2(__ldg(&P2[b]));
-                    rc[2 * b] = fmaf(f.x, tk[u], rc[2 * b]);
-                    rc[2 * b + 1] = fmaf(f.y, tk[u], rc[2 * b + 1]);
-                }
-            } else {
-                const float* __restrict__ P = Pc + 6 * (size_t)qq[u];
-#pragma unroll
-                for (int b = 0; b < 6; ++b) rc[b] = fmaf(__ldg(&P[b]), tk[u], rc[b]);
-            }
-        }
-    }
-#pragma unroll
-    for (int b = 0; b < 6; ++b)
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) rc[b] += __shfl_xor_sync(0xffffffffu, rc[b], o);
-    if (lane < 6) {
-        C.r[6 * I + lane] = pick6(rc, lane);
-        if (presmooth) C.x[6 * I + lane] = (float)__ldg(omegaC) * lane_mul6(C.dinv + 36 * (size_t)I, rc, lane);
-    }
-}
-
-// Restriction, one warp per coarse node.
-template <int BS>
-__global__ void k_restrict(AmgLevel F, AmgLevel C, const float* __restrict__ t, const double* __restrict__ scal,
-                           const double* __restrict__ omegaC, int presmooth) {
-    pdl_enter();
-    const int I = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (I >= C.n || seg_stopped(scal, C.seg[I])) return;
-    restrict_node<BS>(F, C, t, I, omegaC, presmooth);
-}
-
-// x_i += sum over the prolongator blocks (i, J) of P_iJ e_J (6-DOF level)
-__device__ __forceinline__ void prolong_node(const AmgLevel& F, const float* __restrict__ e, int i, float* x) {
-    float s[6];
-#pragma unroll
-    for (int k = 0; k < 6; ++k) s[k] = x[6 * i + k];
-    for (int b = __ldg(&F.prow[i]); b < __ldg(&F.prow[i + 1]); ++b) {
-        const int J = __ldg(&F.pcol[b]);
-        if (!TF_IN(F.check, J, F.ncoarse, CK_PROLONG_COL)) continue;
-        const float* __restrict__ P = F.Pv + 36 * (size_t)b;
-        float ec[6];
-#pragma unroll
-        for (int c = 0; c < 6; ++c) ec[c] = e[6 * J + c];
-#pragma unroll
-        for (int k = 0; k < 6; ++k)
-#pragma unroll
-            for (int c = 0; c < 6; ++c) s[k] = fmaf(__ldg(&P[6 * k + c]), ec[c], s[k]);
-    }
-#pragma unroll
-    for (int k = 0; k < 6; ++k) x[6 * i + k] = s[k];
-}
-
 // out_i = x_i + omega D_i^-1 (r - A x)_i for row i, by one warp
 __device__ __forceinline__ void post_row(const AmgLevel& L, const double* __restrict__ omega,
                                          const float* __restrict__ x, float* __restrict__ out, int i) {
     // x + omega (D^-1 (r - X x) - S x), S = D^-1 A in FP16, X the extra blocks
     const int lane = threadIdx.x & 31;
-    float y[6], rr[6];
-    row6_warp_h(L, i, x, y);
-    extra6(L, i, x, rr);
+    float rr[6];
 #pragma unroll
-    for (int k = 0; k < 6; ++k) rr[k] = L.r[6 * i + k] - rr[k];
+    for (int k = 0; k < 6; ++k) rr[k] = L.r[6 * i + k];
+    const float y = row6_warp_h(L, __ldg(&L.rowptr[i]), __ldg(&L.rowptr[i + 1]), x);
+    if (L.xrow) {
+        float e[6];
+        extra6(L, i, x, e);
+#pragma unroll
+        for (int k = 0; k < 6; ++k) rr[k] -= e[k];
+    }
     if (lane < 6)
-        out[6 * i + lane] = fmaf((float)__ldg(omega), lane_mul6(L.dinv + 36 * (size_t)i, rr, lane) - pick6(y, lane),
-                                 x[6 * i + lane]);
+        out[6 * i + lane] = fmaf((float)__ldg(omega), lane_mul6(L.dinv + 36 * (size_t)i, rr, lane) - y, x[6 * i + lane]);
 }
 
 // t_i = r_i - (A x)_i with A x = D (S x) + X x, lane k < 6 writing component k
 __device__ __forceinline__ void resid_row(const AmgLevel& L, const float* __restrict__ x, int i) {
     const int lane = threadIdx.x & 31;
+    const float s = row6_warp_h(L, __ldg(&L.rowptr[i]), __ldg(&L.rowptr[i + 1]), x);
     float y[6], e[6];
-    row6_warp_h(L, i, x, y);
+#pragma unroll
+    for (int k = 0; k < 6; ++k) y[k] = __shfl_sync(0xffffffffu, s, k);
     extra6(L, i, x, e);
     if (lane < 6)
         L.t[6 * i + lane] = L.r[6 * i + lane] - lane_mul6(L.val + 36 * (size_t)L.diag[i], y, lane) - pick6(e, lane);
@@ -1926,12 +1857,27 @@ __global__ void k_v6_post(AmgLevel L, const double* __restrict__ scal, const dou
     post_row(L, omega, x, out, i);
 }
 
-// x_i += P_i e  (6-DOF fine level)
+// x_i += sum over the prolongator blocks (i, J) of P_iJ e_J (6-DOF fine level),
+// one thread per DOF (one per node: 7.8 against 5.5 us to 8,978 nodes)
 __global__ void k_v6_prolong(AmgLevel F, const double* __restrict__ scal, const float* __restrict__ e, float* x) {
     pdl_enter();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int q = blockIdx.x * blockDim.x + threadIdx.x, i = q / 6, k = q - 6 * i;
     if (i >= F.n || seg_stopped(scal, F.seg[i])) return;
-    prolong_node(F, e, i, x);
+    float s = x[q];
+    const int b1 = __ldg(&F.prow[i + 1]);
+#pragma unroll 4
+    for (int b = __ldg(&F.prow[i]); b < b1; ++b) {
+        const int J = __ldg(&F.pcol[b]);
+        if (!TF_IN(F.check, J, F.ncoarse, CK_PROLONG_COL)) continue;
+        const float2* __restrict__ P = reinterpret_cast<const float2*>(F.Pv + 36 * (size_t)b + 6 * k);
+        const float2* __restrict__ ej = reinterpret_cast<const float2*>(e + 6 * (size_t)J);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const float2 p = __ldg(&P[c]), v = ej[c];
+            s = fmaf(p.x, v.x, fmaf(p.y, v.y, s));
+        }
+    }
+    x[q] = s;
 }
 
 // Buffers of the damped-Jacobi sweeps of a coarse level (a sweep reads one
@@ -2472,7 +2418,8 @@ void amg_vcycle(tf_handle* h, const double* r, double* out, int dot, double* p) 
             }
             cudaEventRecord(h->join_ev, h->side_stream);
         }
-        launch_pdl(k_q_restrict, a->L[1].n, kRestrictThreads, st, a->Q, a->L[1], L0.n, L0.check, (const float*)L0.t,
+        launch_pdl(k_restrict<3, __half>, a->L[1].n, kRestrictThreads, st, (const int*)a->Q.cptr, (const int*)a->Q.crow,
+                   reinterpret_cast<const __half*>(a->Q.cval), a->L[1], L0.n, L0.check, (const float*)L0.t,
                    (const double*)d.scal, (const double*)(a->omega + 1), presmooth(1));
     } else {
         switch (a->smooth_unroll) {
@@ -2480,8 +2427,9 @@ void amg_vcycle(tf_handle* h, const double* r, double* out, int dot, double* p) 
             case 8: launch_pdl(k_v0_resid<8>, d.ncta, kNodeThreads, st, v0, r, L0.x, L0.t); break;
             default: launch_pdl(k_v0_resid<4>, d.ncta, kNodeThreads, st, v0, r, L0.x, L0.t); break;
         }
-        launch_pdl(k_restrict<3>, cdiv(32 * (int64_t)a->L[1].n, kT), kT, st, L0, a->L[1], (const float*)L0.t,
-                   (const double*)d.scal, (const double*)(a->omega + 1), presmooth(1));
+        launch_pdl(k_restrict<3, __half>, a->L[1].n, kRestrictThreads, st, (const int*)L0.pcptr, (const int*)L0.pcrow,
+                   (const __half*)L0.Pch, a->L[1], L0.n, L0.check, (const float*)L0.t, (const double*)d.scal,
+                   (const double*)(a->omega + 1), presmooth(1));
     }
     float* cur[kAmgMaxLevels] = {};
     for (int l = 1; l < stop; ++l) {
@@ -2496,8 +2444,9 @@ void amg_vcycle(tf_handle* h, const double* r, double* out, int dot, double* p) 
         }
         cur[l] = x;
         launch_pdl(k_v6_resid, nb, kT, st, L, (const double*)d.scal, (const float*)x);
-        launch_pdl(k_restrict<6>, cdiv(32 * (int64_t)a->L[l + 1].n, kT), kT, st, L, a->L[l + 1], (const float*)L.t,
-                   (const double*)d.scal, (const double*)(a->omega + l + 1), presmooth(l + 1));
+        launch_pdl(k_restrict<6, float>, a->L[l + 1].n, kRestrictThreads, st, (const int*)L.pcptr, (const int*)L.pcrow,
+                   (const float*)L.Pc, a->L[l + 1], L.n, L.check, (const float*)L.t, (const double*)d.scal,
+                   (const double*)(a->omega + l + 1), presmooth(l + 1));
     }
     if (a->dense > 0) {
         AmgLevel& LD = a->L[stop];
@@ -2514,7 +2463,7 @@ void amg_vcycle(tf_handle* h, const double* r, double* out, int dot, double* p) 
     for (int l = stop - 1; l >= 1; --l) {
         AmgLevel& L = a->L[l];
         float* x = cur[l];
-        launch_pdl(k_v6_prolong, cdiv(L.n, kT), kT, st, L, d.scal, (const float*)a->L[l + 1].e, x);
+        launch_pdl(k_v6_prolong, cdiv(6 * (int64_t)L.n, kT), kT, st, L, d.scal, (const float*)a->L[l + 1].e, x);
         for (int s = 1; s <= kCoarseSweeps; ++s) {
             float* o = post_sweep_out(L, x, s, kCoarseSweeps);
             launch_pdl(k_v6_post, cdiv(32 * (int64_t)L.n, kT), kT, st, L, (const double*)d.scal,
