@@ -187,3 +187,45 @@ def test_element_tiles(nx, ny, layers, eta, deterministic):
     got[np.repeat(np.arange(n), np.diff(ia)), ja] = a
     assert np.abs(got - K).max() <= 1e-11 * np.abs(K).max()
     assert np.abs(g - f * free).max() <= 1e-11 * np.abs(f).max()
+
+
+# Meshes of up to 65,536 nodes share a row among the warps of a 32-node CTA; larger
+# ones and order-fixed assemblies have a warp per slice.  Node counts with no,
+# one and 31 nodes in the last slice, the largest split mesh and the next, both
+# preconditioners, with and without extra blocks.
+@pytest.mark.parametrize("eta", [0.0, 100.0])
+@pytest.mark.parametrize("precond", [1, 2])
+@pytest.mark.parametrize("nodes,nx,ny,layers", [(128, 7, 7, 1), (225, 8, 4, 4), (255, 16, 4, 2)])
+def test_split_rows_of_small_meshes(nodes, nx, ny, layers, precond, eta):
+    t = _sheet(nx, ny, layers, eta)
+    assert t.n_nodes == nodes
+    uk, un = mesh.perturbed_state(t, seed=5)
+    its = []
+    for deterministic in (False, True):
+        for extra in (False, True):
+            with api.Solver(t, precond=precond, krylov_rtol=RTOL, deterministic=deterministic) as s:
+                s.set_positions(un)
+                s.begin_step(t.dt)
+                s.set_state(uk, un, t.dt)
+                s.assemble()
+                if extra:
+                    s.add_K_triplets([0, 3 * (nodes - 1)], [3 * (nodes - 1), 0], [1e-3, 1e-3])
+                out = s.solve()
+                _check_solution(s, out, [(0, 3 * nodes)])
+                its.append(out["iters"])
+    assert max(its) <= 1.25 * min(its) + 2, its
+
+
+@pytest.mark.parametrize("nodes,nx,ny,layers", [(65536, 127, 127, 3), (65790, 128, 169, 2)])
+def test_largest_split_mesh_and_the_next(nodes, nx, ny, layers):
+    t = _sheet(nx, ny, layers, 100.0)
+    assert t.n_nodes == nodes
+    with api.Solver(t, krylov_rtol=RTOL) as s:
+        assert _solve(s, [t])["iters"] < 200
+
+
+def test_split_rows_of_a_ragged_batch():
+    ts = [_sheet(3, 3, 2, 100.0), _sheet(12, 13, 2, 100.0, 4), _sheet(7, 7, 1, 100.0, 5), _sheet(16, 4, 2, 100.0, 6)]
+    for precond in (1, 2):
+        with api.Batch(ts, precond=precond, krylov_rtol=RTOL) as s:
+            _solve(s, ts)

@@ -232,6 +232,7 @@ struct AmgLevel {
     // vectors (levels >= 1: r input, e output; all levels: x, t work)
     float *r = nullptr, *x = nullptr, *t = nullptr, *e = nullptr;
     int ncoarse = 0;         // nodes of level + 1
+    int single = 0;          // one instance
     int* check = nullptr;    // checked build: failed index checks
 };
 
@@ -364,14 +365,15 @@ static tf_status build_q(const Device& d, AmgQ* q, const std::vector<int>& trowp
     std::vector<int> slot0((size_t)d.ncta * kWarps + 1, 0), tp(nT, -1), pos(nT), cpos(nT), cptr(nc + 1, 0), crow(nT);
     int ns = 0;
     for (int c = 0; c < d.ncta; ++c)
-        for (int w = 0; w < kWarps; ++w) {
+        for (int w = 0; w < (d.split ? 1 : kWarps); ++w) {
             const int r0 = c0[c] + 32 * w, r1 = std::min(r0 + 32, c1[c]);
-            slot0[(size_t)c * kWarps + w] = ns;
             int most = 0;
             for (int i = r0; i < r1; ++i) {
                 most = std::max(most, trowptr[i + 1] - trowptr[i]);
                 for (int t = trowptr[i]; t < trowptr[i + 1]; ++t) pos[t] = (ns + t - trowptr[i]) * 32 + (i - r0);
             }
+            for (int v = w; v < (d.split ? kWarps : w + 1); ++v)  // split: the warps share the slice's slots
+                slot0[(size_t)c * kWarps + v] = ns + (d.split ? most * v / kWarps : 0);
             ns += most;
         }
     slot0[(size_t)d.ncta * kWarps] = ns;
@@ -731,6 +733,7 @@ tf_status amg_build(tf_handle* h, const double* pos) {
     for (int l = 0; l < a->nlev; ++l) {
         a->L[l].ncoarse = l + 1 < a->nlev ? a->L[l + 1].n : 0;
         a->L[l].check = d.check;
+        a->L[l].single = d.nseg == 1;
     }
     AMG_TRY(zeros(&a->omega, (size_t)a->nlev));
     AMG_TRY(zeros(&a->val32, (size_t)d.nval));
@@ -892,6 +895,11 @@ __device__ __forceinline__ bool seg_stopped(const double* scal, int seg) {
     return __ldcg(&scal[(size_t)seg * S_COUNT + S_FLAG]) != 0.0;
 }
 
+// ... and of the instance of node i of a coarse level (one instance: no look-up)
+__device__ __forceinline__ bool level_stopped(const AmgLevel& L, const double* scal, int i) {
+    return seg_stopped(scal, L.single ? 0 : L.seg[i]);
+}
+
 // Sum of one value over the grid: partials per CTA, the last CTA to arrive
 // folds them in a fixed order, all its threads at once (no waiting).  True in
 // thread 0 of that CTA.
@@ -921,12 +929,23 @@ __device__ bool grid_sum(double v, double* part, unsigned* ticket, double* total
 struct Node0 {
     int i, seg;
     bool valid;
+    int row;  // row of this thread's share of a row product (split CTAs: the lane's, whatever the warp)
 };
 __device__ __forceinline__ Node0 node0(const Device& d) {
     Node0 q;
-    q.seg = d.cta_seg[blockIdx.x];
-    q.i = d.cta_node0[blockIdx.x] + threadIdx.x;
-    q.valid = q.i < d.cta_node1[blockIdx.x];
+    int n0, n1;
+    if (d.nseg == 1) {
+        q.seg = 0;
+        n0 = blockIdx.x * d.cta_nodes;
+        n1 = min(n0 + d.cta_nodes, d.nn);
+    } else {
+        q.seg = d.cta_seg[blockIdx.x];
+        n0 = d.cta_node0[blockIdx.x];
+        n1 = d.cta_node1[blockIdx.x];
+    }
+    q.i = n0 + threadIdx.x;
+    q.valid = q.i < n1;
+    q.row = d.split ? min(n0 + (int)(threadIdx.x & 31), n1 - 1) : q.i;
     return q;
 }
 
@@ -936,15 +955,12 @@ __device__ __forceinline__ void mul3(const float* __restrict__ D, const float r[
     z[2] = fmaf(D[6], r[0], fmaf(D[7], r[1], D[8] * r[2]));
 }
 
-// Row of S = D^-1 A (FP16, sliced) times x, FP32 sums; the extra blocks X
-// (FP64) enter as D^-1 (X x).
+// Row of S = D^-1 A (FP16, sliced) times x, FP32 sums: this thread's share of it
+// (split CTAs), from the warp's slots s0 .. s1.
 template <int U = 4>
-__device__ __forceinline__ void row0s(const Device& d, const __half* __restrict__ valh,
-                                      const float* __restrict__ dinv32, const float* __restrict__ x, int i,
-                                      float y[3]) {
+__device__ __forceinline__ void row0_part(const Device& d, int s0, int s1, const __half* __restrict__ valh,
+                                          const float* __restrict__ x, float (&y)[3]) {
     const int lane = threadIdx.x & 31;
-    const int wg = blockIdx.x * kWarps + (threadIdx.x >> 5);
-    const int s0 = __ldg(&d.wslot0[wg]), s1 = __ldg(&d.wslot0[wg + 1]);
     float y0 = 0.f, y1 = 0.f, y2 = 0.f;
     const int* __restrict__ col = d.scol + lane;
     const uint4* __restrict__ p8 = reinterpret_cast<const uint4*>(valh) + lane;
@@ -972,7 +988,18 @@ __device__ __forceinline__ void row0s(const Device& d, const __half* __restrict_
     y[0] = y0;
     y[1] = y1;
     y[2] = y2;
-    if (!d.xrow || d.xrow[i] == d.xrow[i + 1]) return;
+}
+
+// The whole row on its node's thread, the extra blocks X (FP64) entering as
+// D^-1 (X x).  Every thread of the CTA calls it.
+template <int U = 4>
+__device__ __forceinline__ void row0s(const Device& d, const __half* __restrict__ valh,
+                                      const float* __restrict__ dinv32, const float* __restrict__ x, const Node0& q0,
+                                      float (&y)[3]) {
+    const int wg = blockIdx.x * kWarps + (threadIdx.x >> 5), i = q0.i;
+    row0_part<U>(d, __ldg(&d.wslot0[wg]), __ldg(&d.wslot0[wg + 1]), valh, x, y);
+    if (d.split) split_sum(y);
+    if (!q0.valid || !d.xrow || d.xrow[i] == d.xrow[i + 1]) return;
     float e[3] = {0.f, 0.f, 0.f}, z[3];
     for (int q = d.xrow[i]; q < d.xrow[i + 1]; ++q) {
         const int j = d.xcol[q];
@@ -1129,7 +1156,7 @@ __global__ void k_to_h(Device d, const float* __restrict__ val32, const float* _
     const int s0 = d.wslot0[wg], s1 = d.wslot0[wg + 1];
     float D[9];
 #pragma unroll
-    for (int k = 0; k < 9; ++k) D[k] = q.valid ? dinv32[9 * (size_t)q.i + k] : 0.f;
+    for (int k = 0; k < 9; ++k) D[k] = (d.split || q.valid) ? dinv32[9 * (size_t)q.row + k] : 0.f;
     if (q.valid) {
         const float* __restrict__ Dg = val32 + d.diag[q.i];
 #pragma unroll
@@ -1428,7 +1455,7 @@ __global__ void k_pw_step0(Device d, const __half* __restrict__ valh, const floa
     const Node0 q = node0(d);
     double s = 0.0;
     float y[3] = {0.f, 0.f, 0.f};
-    if (q.valid) row0s(d, valh, dinv32, v, q.i, y);  // D^-1 A v = S v, the smoother's operator
+    row0s(d, valh, dinv32, v, q, y);  // D^-1 A v = S v, the smoother's operator
     if (q.valid) {
         const float sc = (float)__ldcg(&scal[0]);
 #pragma unroll
@@ -1620,9 +1647,9 @@ __global__ void __launch_bounds__(kRestrictThreads) k_restrict(const int* __rest
     __shared__ float sm[kRestrictThreads / 32][6];
     pdl_enter();
     const int I = blockIdx.x;
-    if (seg_stopped(scal, C.seg[I])) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int q0 = __ldg(&cptr[I]), np = BS * (__ldg(&cptr[I + 1]) - q0);
+    if (level_stopped(C, scal, I)) return;
     float rc[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll 4
     for (int q = threadIdx.x; q < np; q += kRestrictThreads) {
@@ -1664,19 +1691,19 @@ template <int U>
 __global__ void k_q_smooth(V0 a, const float* __restrict__ z, float* __restrict__ x) {
     pdl_enter();
     const Node0 q = node0(a.d);
-    if (!q.valid || seg_stopped(a.d.scal, q.seg)) return;
+    if (seg_stopped(a.d.scal, q.seg)) return;
     float y[3];
-    row0s<U>(a.d, a.valh, a.dinv32, z, q.i, y);
+    row0s<U>(a.d, a.valh, a.dinv32, z, q, y);
+    if (!q.valid) return;
     const float om = (float)__ldg(a.omega);
 #pragma unroll
     for (int k = 0; k < 3; ++k) x[3 * q.i + k] = fmaf(-om, y[k], 2.f * z[3 * q.i + k]);
 }
 
-// (Q e)_i added to x
-__device__ __forceinline__ void row_q(const AmgQ& Q, const float* __restrict__ e, int nc, int* check, float x[3]) {
+// (Q e)_i added to x: the warp's slots s0 .. s1
+__device__ __forceinline__ void row_q(const AmgQ& Q, int s0, int s1, const float* __restrict__ e, int nc, int* check,
+                                      float (&x)[3]) {
     const int lane = threadIdx.x & 31;
-    const int wg = blockIdx.x * kWarps + (threadIdx.x >> 5);
-    const int s0 = __ldg(&Q.slot0[wg]), s1 = __ldg(&Q.slot0[wg + 1]);
 #pragma unroll 4
     for (int s = s0; s < s1; ++s) {
         const int J = __ldg(&Q.col[32 * (size_t)s + lane]);
@@ -1705,27 +1732,36 @@ __global__ void k_q_post(V0 a, Ctx c, AmgQ Q, int nc, const float* __restrict__ 
                          double* __restrict__ out, const double* __restrict__ r, double* __restrict__ p, int start) {
     pdl_enter();
     const Node0 q = node0(a.d);
-    if (seg_stopped(a.d.scal, q.seg)) return;
-    double v[1] = {0.0};
-    if (q.valid) {
-        float x[3];
-        if constexpr (SMOOTH) {
-            row0s<U>(a.d, a.valh, a.dinv32, zx, q.i, x);
-            const float om = (float)__ldg(a.omega);
+    const double flag = __ldcg(&a.d.scal[(size_t)q.seg * S_COUNT + S_FLAG]);
+    const int wg = blockIdx.x * kWarps + (threadIdx.x >> 5);
+    const int q0 = __ldg(&Q.slot0[wg]), q1 = __ldg(&Q.slot0[wg + 1]);
+    if (flag != 0.0) return;
+    float x[3] = {0.f, 0.f, 0.f}, own[3];
+    double ri[3];
+    float om = 0.f;
+    if constexpr (SMOOTH) {
+        row0_part<U>(a.d, __ldg(&a.d.wslot0[wg]), __ldg(&a.d.wslot0[wg + 1]), a.valh, zx, x);
+        om = (float)__ldg(a.omega);
 #pragma unroll
-            for (int k = 0; k < 3; ++k) x[k] = fmaf(-om, x[k], 2.f * zx[3 * q.i + k]);
-        } else {
-#pragma unroll
-            for (int k = 0; k < 3; ++k) x[k] = zx[3 * q.i + k];
-        }
-        row_q(Q, e, nc, a.d.check, x);
+        for (int k = 0; k < 3; ++k) x[k] *= -om;
+    }
+    row_q(Q, q0, q1, e, nc, a.d.check, x);
+    if (q.valid)
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-            const double o = (double)x[k];
+            own[k] = (SMOOTH ? 2.f : 1.f) * zx[3 * q.i + k];
+            if constexpr (DOT) ri[k] = r[3 * q.i + k];
+        }
+    if (a.d.split) split_sum(x);
+    double v[1] = {0.0};
+    if (q.valid) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const double o = (double)(own[k] + x[k]);
             out[3 * q.i + k] = o;
             if constexpr (DOT) {
                 if (start) p[3 * q.i + k] = o;
-                v[0] = fma(r[3 * q.i + k], o, v[0]);
+                v[0] = fma(ri[k], o, v[0]);
             }
         }
     }
@@ -1743,7 +1779,7 @@ __global__ void k_v0_resid(V0 a, const double* __restrict__ r, const float* __re
     const Node0 q = node0(a.d);
     if (seg_stopped(a.d.scal, q.seg)) return;
     float y[3];
-    if (q.valid) row0s<U>(a.d, a.valh, a.dinv32, x, q.i, y);
+    row0s<U>(a.d, a.valh, a.dinv32, x, q, y);
     if (!q.valid) return;
     // A x = D (S x), D the diagonal block
     const float* __restrict__ Dg = a.diag32 + 9 * (size_t)q.i;
@@ -1760,7 +1796,7 @@ __global__ void k_v0_post(V0 a, const double* __restrict__ r, const float* __res
     const Node0 q = node0(a.d);
     if (seg_stopped(a.d.scal, q.seg)) return;
     float y[3];
-    if (q.valid) row0s<U>(a.d, a.valh, a.dinv32, x, q.i, y);
+    row0s<U>(a.d, a.valh, a.dinv32, x, q, y);
     if (!q.valid) return;
     // x + omega D^-1 (r - A x) = x + omega (D^-1 r - S x)
     const float om = (float)__ldg(a.omega);
@@ -1811,13 +1847,16 @@ __global__ void k_v0_prolong(V0 a, AmgLevel F, const float* __restrict__ e, floa
 
 // out_i = x_i + omega D_i^-1 (r - A x)_i for row i, by one warp
 __device__ __forceinline__ void post_row(const AmgLevel& L, const double* __restrict__ omega,
-                                         const float* __restrict__ x, float* __restrict__ out, int i) {
+                                         const float* __restrict__ x, float* __restrict__ out, int i,
+                                         const double* __restrict__ scal) {
     // x + omega (D^-1 (r - X x) - S x), S = D^-1 A in FP16, X the extra blocks
     const int lane = threadIdx.x & 31;
+    const int p0 = __ldg(&L.rowptr[i]), p1 = __ldg(&L.rowptr[i + 1]);
     float rr[6];
 #pragma unroll
     for (int k = 0; k < 6; ++k) rr[k] = L.r[6 * i + k];
-    const float y = row6_warp_h(L, __ldg(&L.rowptr[i]), __ldg(&L.rowptr[i + 1]), x);
+    if (level_stopped(L, scal, i)) return;
+    const float y = row6_warp_h(L, p0, p1, x);
     if (L.xrow) {
         float e[6];
         extra6(L, i, x, e);
@@ -1829,23 +1868,26 @@ __device__ __forceinline__ void post_row(const AmgLevel& L, const double* __rest
 }
 
 // t_i = r_i - (A x)_i with A x = D (S x) + X x, lane k < 6 writing component k
-__device__ __forceinline__ void resid_row(const AmgLevel& L, const float* __restrict__ x, int i) {
+__device__ __forceinline__ void resid_row(const AmgLevel& L, const float* __restrict__ x, int i,
+                                          const double* __restrict__ scal) {
     const int lane = threadIdx.x & 31;
-    const float s = row6_warp_h(L, __ldg(&L.rowptr[i]), __ldg(&L.rowptr[i + 1]), x);
+    const int p0 = __ldg(&L.rowptr[i]), p1 = __ldg(&L.rowptr[i + 1]), dg = __ldg(&L.diag[i]);
+    if (level_stopped(L, scal, i)) return;
+    const float s = row6_warp_h(L, p0, p1, x);
     float y[6], e[6];
 #pragma unroll
     for (int k = 0; k < 6; ++k) y[k] = __shfl_sync(0xffffffffu, s, k);
     extra6(L, i, x, e);
     if (lane < 6)
-        L.t[6 * i + lane] = L.r[6 * i + lane] - lane_mul6(L.val + 36 * (size_t)L.diag[i], y, lane) - pick6(e, lane);
+        L.t[6 * i + lane] = L.r[6 * i + lane] - lane_mul6(L.val + 36 * (size_t)dg, y, lane) - pick6(e, lane);
 }
 
 // t = r - A x  (one warp per row)
 __global__ void k_v6_resid(AmgLevel L, const double* __restrict__ scal, const float* __restrict__ x) {
     pdl_enter();
     const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (i >= L.n || seg_stopped(scal, L.seg[i])) return;
-    resid_row(L, x, i);
+    if (i >= L.n) return;
+    resid_row(L, x, i, scal);
 }
 
 // out = x + omega D^-1 (r - A x)  (one warp per row)
@@ -1853,8 +1895,8 @@ __global__ void k_v6_post(AmgLevel L, const double* __restrict__ scal, const dou
                           const float* __restrict__ x, float* __restrict__ out) {
     pdl_enter();
     const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (i >= L.n || seg_stopped(scal, L.seg[i])) return;
-    post_row(L, omega, x, out, i);
+    if (i >= L.n) return;
+    post_row(L, omega, x, out, i, scal);
 }
 
 // x_i += sum over the prolongator blocks (i, J) of P_iJ e_J (6-DOF fine level),
@@ -1862,7 +1904,7 @@ __global__ void k_v6_post(AmgLevel L, const double* __restrict__ scal, const dou
 __global__ void k_v6_prolong(AmgLevel F, const double* __restrict__ scal, const float* __restrict__ e, float* x) {
     pdl_enter();
     const int q = blockIdx.x * blockDim.x + threadIdx.x, i = q / 6, k = q - 6 * i;
-    if (i >= F.n || seg_stopped(scal, F.seg[i])) return;
+    if (i >= F.n || level_stopped(F, scal, i)) return;
     float s = x[q];
     const int b1 = __ldg(&F.prow[i + 1]);
 #pragma unroll 4
@@ -1902,12 +1944,13 @@ __global__ void k_dense(AmgLevel L, const double* __restrict__ scal, const int* 
     pdl_enter();
     const int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;  // row over all instances
     if (k >= 6 * L.n) return;
-    const int g = L.seg[k / 6];
+    const int g = L.single ? 0 : L.seg[k / 6];
     if (seg_stopped(scal, g)) return;
     const int lane = threadIdx.x & 31;
-    const int k0 = 6 * L.seg0[g];
-    const int m2 = 3 * (L.seg0[g + 1] - L.seg0[g]);  // pairs of a row: m is even, rows are 8-byte aligned
-    const float2* __restrict__ M = reinterpret_cast<const float2*>(mat + doff[g] + (size_t)(k - k0) * (2 * m2));
+    const int k0 = L.single ? 0 : 6 * L.seg0[g];
+    const int m2 = L.single ? 3 * L.n : 3 * (L.seg0[g + 1] - L.seg0[g]);  // pairs of a row (m is even)
+    const float2* __restrict__ M =
+        reinterpret_cast<const float2*>(mat + (L.single ? 0 : doff[g]) + (size_t)(k - k0) * (2 * m2));
     const float2* __restrict__ r = reinterpret_cast<const float2*>(L.r + k0);
     float s = 0.f;
 #pragma unroll 8
@@ -2226,7 +2269,7 @@ tf_status amg_numeric(tf_handle* h) {
             TF_LAUNCH_CHECK(h);
             for (int it = 0; it < kPowerIters; ++it) {
                 if (l == 0)
-                    k_pw_step0<<<d.ncta, kNodeThreads, 0, st>>>(d, a->valh, a->dinv32, v, w, a->part, a->ticket,
+                    k_pw_step0<<<d.ncta, kNodeThreads, split_bytes<float>(d), st>>>(d, a->valh, a->dinv32, v, w, a->part, a->ticket,
                                                                 scal, a->omega);
                 else
                     k_pw_step6<<<cdiv(32 * (int64_t)L.n, kT), kT, 0, st>>>(L, v, w, a->part, a->ticket, scal,
@@ -2325,9 +2368,9 @@ tf_status amg_autotune(tf_handle* h) {
     for (int u : {2, 4, 8}) {
         for (int r = 0; r < 4; ++r) {  // one warm-up, three timed
             if (r == 1) TF_CUDA(cudaEventRecord(h->ev[4], st));
-            if (u == 2) k_v0_resid<2><<<d.ncta, kNodeThreads, 0, st>>>(v0, d.g, L0.x, L0.t);
-            else if (u == 4) k_v0_resid<4><<<d.ncta, kNodeThreads, 0, st>>>(v0, d.g, L0.x, L0.t);
-            else k_v0_resid<8><<<d.ncta, kNodeThreads, 0, st>>>(v0, d.g, L0.x, L0.t);
+            if (u == 2) k_v0_resid<2><<<d.ncta, kNodeThreads, split_bytes<float>(d), st>>>(v0, d.g, L0.x, L0.t);
+            else if (u == 4) k_v0_resid<4><<<d.ncta, kNodeThreads, split_bytes<float>(d), st>>>(v0, d.g, L0.x, L0.t);
+            else k_v0_resid<8><<<d.ncta, kNodeThreads, split_bytes<float>(d), st>>>(v0, d.g, L0.x, L0.t);
             TF_LAUNCH_CHECK(h);
         }
         TF_CUDA(cudaEventRecord(h->ev[5], st));
@@ -2369,7 +2412,7 @@ int amg_vcycle_kernels(const tf_handle* h) {
 
 template <int U>
 static void launch_q_smooth(tf_handle* h, cudaStream_t st, const V0& v0, const float* z, float* x) {
-    k_q_smooth<U><<<h->d.ncta, kNodeThreads, 0, st>>>(v0, z, x);
+    k_q_smooth<U><<<h->d.ncta, kNodeThreads, split_bytes<float>(h->d), st>>>(v0, z, x);
 }
 
 // The last kernel of a V-cycle through Q.  After k_q_smooth on the side
@@ -2381,14 +2424,17 @@ static void launch_q_post(tf_handle* h, const V0& v0, const float* zx, double* o
     const Ctx c = make_ctx(h);
     const int nb = h->d.ncta, nc = a->L[1].n;
     const float* e = a->L[1].e;
+    const size_t sb = split_bytes<float>(h->d);
+    const int start = dot == kVcycleStart ? 1 : 0;
     if constexpr (SMOOTH) {
-        if (dot) launch_pdl(k_q_post<U, true, true>, nb, kNodeThreads, h->stream, v0, c, a->Q, nc, zx, e, out, r, p,
-                            dot == kVcycleStart ? 1 : 0);
-        else launch_pdl(k_q_post<U, true, false>, nb, kNodeThreads, h->stream, v0, c, a->Q, nc, zx, e, out, r, p, 0);
+        if (dot) launch_pdl_smem(k_q_post<U, true, true>, nb, kNodeThreads, sb, h->stream, v0, c, a->Q, nc, zx, e, out,
+                                 r, p, start);
+        else launch_pdl_smem(k_q_post<U, true, false>, nb, kNodeThreads, sb, h->stream, v0, c, a->Q, nc, zx, e, out, r,
+                             p, 0);
     } else {
-        if (dot) k_q_post<U, false, true><<<nb, kNodeThreads, 0, h->stream>>>(v0, c, a->Q, nc, zx, e, out, r, p,
-                                                                            dot == kVcycleStart ? 1 : 0);
-        else k_q_post<U, false, false><<<nb, kNodeThreads, 0, h->stream>>>(v0, c, a->Q, nc, zx, e, out, r, p, 0);
+        if (dot) k_q_post<U, false, true><<<nb, kNodeThreads, sb, h->stream>>>(v0, c, a->Q, nc, zx, e, out, r, p,
+                                                                             start);
+        else k_q_post<U, false, false><<<nb, kNodeThreads, sb, h->stream>>>(v0, c, a->Q, nc, zx, e, out, r, p, 0);
     }
 }
 
@@ -2423,9 +2469,9 @@ void amg_vcycle(tf_handle* h, const double* r, double* out, int dot, double* p) 
                    (const double*)d.scal, (const double*)(a->omega + 1), presmooth(1));
     } else {
         switch (a->smooth_unroll) {
-            case 2: launch_pdl(k_v0_resid<2>, d.ncta, kNodeThreads, st, v0, r, L0.x, L0.t); break;
-            case 8: launch_pdl(k_v0_resid<8>, d.ncta, kNodeThreads, st, v0, r, L0.x, L0.t); break;
-            default: launch_pdl(k_v0_resid<4>, d.ncta, kNodeThreads, st, v0, r, L0.x, L0.t); break;
+            case 2: launch_pdl_smem(k_v0_resid<2>, d.ncta, kNodeThreads, split_bytes<float>(d), st, v0, r, L0.x, L0.t); break;
+            case 8: launch_pdl_smem(k_v0_resid<8>, d.ncta, kNodeThreads, split_bytes<float>(d), st, v0, r, L0.x, L0.t); break;
+            default: launch_pdl_smem(k_v0_resid<4>, d.ncta, kNodeThreads, split_bytes<float>(d), st, v0, r, L0.x, L0.t); break;
         }
         launch_pdl(k_restrict<3, __half>, a->L[1].n, kRestrictThreads, st, (const int*)L0.pcptr, (const int*)L0.pcrow,
                    (const __half*)L0.Pch, a->L[1], L0.n, L0.check, (const float*)L0.t, (const double*)d.scal,
@@ -2487,9 +2533,9 @@ void amg_vcycle(tf_handle* h, const double* r, double* out, int dot, double* p) 
     launch_pdl_smem(k_v0_prolong, d.ncta, kNodeThreads, (size_t)a->v0_smem, st, v0, L0, (const float*)a->L[1].e,
                     L0.x);
     switch (a->smooth_unroll) {
-        case 2: launch_pdl(k_v0_post<2>, d.ncta, kNodeThreads, st, v0, r, L0.x, out); break;
-        case 8: launch_pdl(k_v0_post<8>, d.ncta, kNodeThreads, st, v0, r, L0.x, out); break;
-        default: launch_pdl(k_v0_post<4>, d.ncta, kNodeThreads, st, v0, r, L0.x, out); break;
+        case 2: launch_pdl_smem(k_v0_post<2>, d.ncta, kNodeThreads, split_bytes<float>(d), st, v0, r, L0.x, out); break;
+        case 8: launch_pdl_smem(k_v0_post<8>, d.ncta, kNodeThreads, split_bytes<float>(d), st, v0, r, L0.x, out); break;
+        default: launch_pdl_smem(k_v0_post<4>, d.ncta, kNodeThreads, split_bytes<float>(d), st, v0, r, L0.x, out); break;
     }
 }
 

@@ -178,19 +178,32 @@ tf_status check_handle(tf_handle* h) {
     return TF_OK;
 }
 
-// CTA tables of the node-parallel kernels: every CTA covers up to
-// kNodeThreads consecutive nodes of one instance.
+// Meshes (batches: in all) of up to this many nodes have CTAs of 32 nodes whose
+// eight warps share each row of a product: with 256 nodes a CTA, 1,323 nodes kept
+// six SMs' FP64 pipes busy and left 146 idle, each lane walking ~27 slots in
+// turn.  Step of 256 / 1,600 / 9,728 (viscous) / 46,208 prisms: 2.27 -> 1.40,
+// 2.71 -> 1.73, 2.9 -> 2.07, 8.1 -> 6.8 ms.  The line: 36,963 nodes 8.4 -> 7.4
+// (viscous 8.9 -> 7.8), 61,605 viscous 11.5 -> 11.0, but 114,005 nodes 13.0 -> 15.9:
+// where whole slices fill the chip, a warp each streams better.  Order-fixed
+// assemblies never split: a batched instance has to sum like its plain run, and
+// large batches are better off whole.
+constexpr int kSplitNodes = 65536;
+
+// CTA tables of the node-parallel kernels: every CTA covers up to cta_nodes
+// consecutive nodes of one instance.
 tf_status setup_instances(tf_handle* h, const std::vector<int>& seg_node0, const std::vector<int>& seg_elem0) {
     Device& d = h->d;
     const int nseg = static_cast<int>(seg_node0.size()) - 1;
     d.nseg = nseg;
+    d.split = !h->opt.deterministic && d.nn <= kSplitNodes;
+    d.cta_nodes = d.split ? 32 : kNodeThreads;
     std::vector<int> cta_seg, cta0, cta1, seg_cta0(nseg + 1, 0), elem_seg(d.ne);
     for (int g = 0; g < nseg; ++g) {
         seg_cta0[g] = static_cast<int>(cta_seg.size());
-        for (int n0 = seg_node0[g]; n0 < seg_node0[g + 1]; n0 += kNodeThreads) {
+        for (int n0 = seg_node0[g]; n0 < seg_node0[g + 1]; n0 += d.cta_nodes) {
             cta_seg.push_back(g);
             cta0.push_back(n0);
-            cta1.push_back(std::min(n0 + kNodeThreads, seg_node0[g + 1]));
+            cta1.push_back(std::min(n0 + d.cta_nodes, seg_node0[g + 1]));
         }
         for (int e = seg_elem0[g]; e < seg_elem0[g + 1]; ++e) elem_seg[e] = g;
     }
@@ -410,19 +423,22 @@ tf_status build(tf_handle* h, const tf_mesh* m, const tf_material* mat, const st
         std::vector<int> cta0;
         std::vector<int> cta1;
         for (size_t g = 0; g + 1 < seg_node0.size(); ++g)
-            for (int n0 = seg_node0[g]; n0 < seg_node0[g + 1]; n0 += kNodeThreads) {
+            for (int n0 = seg_node0[g]; n0 < seg_node0[g + 1]; n0 += d.cta_nodes) {
                 cta0.push_back(n0);
-                cta1.push_back(std::min(n0 + kNodeThreads, seg_node0[g + 1]));
+                cta1.push_back(std::min(n0 + d.cta_nodes, seg_node0[g + 1]));
             }
         const size_t nwarp = cta0.size() * kWarps;
+        const int nslice = d.split ? 1 : kWarps;  // 32-row slices per CTA
         wslot0.assign(nwarp + 1, 0);
         int64_t nslots = 0;
         for (size_t c = 0; c < cta0.size(); ++c)
-            for (int w = 0; w < kWarps; ++w) {
+            for (int w = 0; w < nslice; ++w) {
                 const int r0 = cta0[c] + 32 * w, r1 = std::min(r0 + 32, cta1[c]);
+                const int64_t first = nslots;
                 int W = 0;
                 for (int i = r0; i < r1; ++i) W = std::max(W, rowptr[i + 1] - rowptr[i]);
-                wslot0[c * kWarps + w] = static_cast<int>(nslots);
+                for (int v = w; v < (d.split ? kWarps : w + 1); ++v)  // split: the warps share the slice's slots
+                    wslot0[c * kWarps + v] = static_cast<int>(nslots) + (d.split ? W * v / kWarps : 0);
                 nslots += W;
                 if (nslots * kSlotDoubles > (int64_t)INT32_MAX) {
                     set_error("mesh too large for 32-bit value offsets");
@@ -430,14 +446,14 @@ tf_status build(tf_handle* h, const tf_mesh* m, const tf_material* mat, const st
                 }
                 for (int i = r0; i < r1; ++i)
                     for (int p = rowptr[i]; p < rowptr[i + 1]; ++p)
-                        bofs[p] = (wslot0[c * kWarps + w] + (p - rowptr[i])) * kSlotDoubles + (i - r0);
+                        bofs[p] = static_cast<int>(first + (p - rowptr[i])) * kSlotDoubles + (i - r0);
             }
         wslot0[nwarp] = static_cast<int>(nslots);
         scol.assign(nslots * kSlice, 0);
         for (size_t c = 0; c < cta0.size(); ++c)
-            for (int w = 0; w < kWarps; ++w) {
+            for (int w = 0; w < nslice; ++w) {
                 const int r0 = cta0[c] + 32 * w, r1 = std::min(r0 + 32, cta1[c]);
-                const int s0 = wslot0[c * kWarps + w], s1 = wslot0[c * kWarps + w + 1];
+                const int s0 = wslot0[c * kWarps + w], s1 = wslot0[c * kWarps + (d.split ? kWarps : w + 1)];
                 for (int l = 0; l < 32; ++l) {
                     const int i = r0 + l;
                     const int len = i < r1 ? rowptr[i + 1] - rowptr[i] : 0;

@@ -121,6 +121,11 @@ struct Device {
     // batch of one)
     int nseg = 1;
     int ncta = 0;               // CTAs of the node-parallel kernels
+    // nodes per CTA: kNodeThreads, a warp per 32-row slice of the matrix -- or 32 on
+    // small meshes, the CTA's warps sharing the slots of its one slice (split) and the
+    // kernels without a row product running one warp per CTA
+    int cta_nodes = 256;
+    int split = 0;
     int* seg_node0 = nullptr;   // [nseg+1] node offsets
     int* elem_seg = nullptr;    // [ne] instance of each element
     int* cta_seg = nullptr;     // [ncta] instance of each CTA
@@ -157,8 +162,34 @@ enum Scal {
     S_COUNT = 32
 };
 
-constexpr int kNodeThreads = 256;    // nodes per CTA of the node-parallel kernels
+constexpr int kNodeThreads = 256;    // threads per CTA of the node-parallel kernels
 constexpr int kWarps = kNodeThreads / 32;
+
+// Threads per CTA of the node-parallel kernels without a row product.
+inline int vector_threads(const Device& d) { return d.split ? 32 : kNodeThreads; }
+
+// Split CTAs: the warps' partial row products (lane = row) summed into warp 0, in
+// a fixed order.  Every thread of the CTA calls it; the launch gives
+// split_bytes<T> of shared memory (none, and all of L1, to whole rows).
+template <class T>
+inline size_t split_bytes(const Device& d) {
+    return d.split ? sizeof(T) * (kWarps - 1) * 3 * 32 : 0;
+}
+template <class T>
+__device__ __forceinline__ void split_sum(T (&y)[3]) {
+    extern __shared__ double split_smem[];
+    T(*sm)[3][32] = reinterpret_cast<T(*)[3][32]>(split_smem);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (warp > 0)
+#pragma unroll
+        for (int d = 0; d < 3; ++d) sm[warp - 1][d][lane] = y[d];
+    __syncthreads();
+    if (warp > 0) return;
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+        y[d] = ((y[d] + sm[0][d][lane]) + (sm[1][d][lane] + sm[2][d][lane])) +
+               ((sm[3][d][lane] + sm[4][d][lane]) + (sm[5][d][lane] + sm[6][d][lane]));
+}
 constexpr int kAmgMaxLevels = 10;
 
 struct Amg;      // multigrid hierarchy (tf_amg.cu)
@@ -331,17 +362,15 @@ inline void launch_pdl(void (*kernel)(KArgs...), int grid, int block, cudaStream
 // y = this thread's row of the sliced block matrix times x.  T is the
 // storage type of the values (double for the Krylov operator, float for the
 // copy the multigrid smoother reads); products and sums are FP64.  The thread is
-// node cta_node0[blockIdx.x] + threadIdx.x of a node-parallel kernel (CTAs
-// of kNodeThreads); the warp walks its slots together, each lane reading
-// its own row's block, so every load of a block entry or column is one
-// coalesced access.
+// node cta_node0[blockIdx.x] + threadIdx.x of a node-parallel kernel (split CTAs:
+// node cta_node0[blockIdx.x] + lane, the warp's share of the row); the warp walks
+// its slots s0 .. s1 together, each lane reading its own row's block, so every
+// load of a block entry or column is one coalesced access.
 template <class T, int U = 2>
-__device__ __forceinline__ void sliced_row(const int* __restrict__ wslot0, const int* __restrict__ scol,
-                                           const T* __restrict__ val, const double* __restrict__ x, double y[3],
-                                           int nn = 0, int* check = nullptr) {
+__device__ __forceinline__ void sliced_row(int s0, int s1, const int* __restrict__ scol, const T* __restrict__ val,
+                                           const double* __restrict__ x, double y[3], int nn = 0,
+                                           int* check = nullptr) {
     const int lane = threadIdx.x & 31;
-    const int wg = blockIdx.x * kWarps + (threadIdx.x >> 5);
-    const int s0 = __ldg(&wslot0[wg]), s1 = __ldg(&wslot0[wg + 1]);
     double y0 = 0.0, y1 = 0.0, y2 = 0.0;
     const int* __restrict__ col = scol + lane;
     const T* __restrict__ a = val + lane;

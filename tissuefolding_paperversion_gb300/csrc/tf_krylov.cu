@@ -34,11 +34,28 @@ __device__ __forceinline__ void apply_dinv(const double* __restrict__ D, const d
     z[2] = fma(D[6], r[0], fma(D[7], r[1], D[8] * r[2]));
 }
 
+// y = A x for the rows of the CTA, each on its node's thread: the warps' products
+// (the slots are looked up before the stop flag is tested), then, by every thread
+// of the CTA, their sums and the extra blocks.  Split CTAs load a kernel's other
+// operands between the two, in flight together with the sum; whole rows after
+// it, with 40 registers a thread (6 CTAs per SM).  U: slots in flight per warp, 0 for split CTAs
+// (a warp has a handful of slots).
+struct Slots {
+    int s0, s1;
+};
+__device__ __forceinline__ Slots warp_slots(const Ctx& c) {
+    const int wg = blockIdx.x * kWarps + (threadIdx.x >> 5);
+    return Slots{__ldg(&c.wslot0[wg]), __ldg(&c.wslot0[wg + 1])};
+}
 template <int U = 2>
-__device__ __forceinline__ void bsr_row(const Ctx& c, int i, const double* __restrict__ x, double y[3]) {
-    sliced_row<double, U>(c.wslot0, c.scol, c.val, x, y, c.nn, c.check);
-    if (c.xrow) {
-        for (int p = c.xrow[i]; p < c.xrow[i + 1]; ++p) {
+__device__ __forceinline__ void rows_product(const Ctx& c, Slots s, const double* __restrict__ x, double (&y)[3]) {
+    sliced_row<double, U == 0 ? 2 : U>(s.s0, s.s1, c.scol, c.val, x, y, c.nn, c.check);
+}
+template <int MODE = kEither>
+__device__ __forceinline__ void rows_sum(const Ctx& c, const Where& w, const double* __restrict__ x, double (&y)[3]) {
+    if (MODE == kSplit || (MODE == kEither && c.split)) split_sum(y);
+    if (c.xrow && w.valid) {
+        for (int p = c.xrow[w.node]; p < c.xrow[w.node + 1]; ++p) {
             const int j = c.xcol[p];
             if (!TF_IN(c.check, j, c.nn, CK_EXTRA_COL)) continue;
             const double* __restrict__ a = c.xval + 9 * (size_t)p;
@@ -72,17 +89,32 @@ __device__ __forceinline__ void start_flags(double* s, double bb, double tol2, d
 
 // What the V-cycle starts from, written by the kernel that makes its input v:
 // v in FP32 and the first sweep z = omega D^-1 v (nothing with block-Jacobi).
-__device__ __forceinline__ void pre_smooth(const AmgPre& a, int i, const double v[3]) {
+// Its operands are loaded with the kernel's own (pre_load).
+struct PreD {
+    float om, D[9];
+};
+__device__ __forceinline__ PreD pre_load(const AmgPre& a, int i) {
+    PreD p;
+    if (!a.z) return p;
+    p.om = (float)__ldg(a.omega);
+#pragma unroll
+    for (int k = 0; k < 9; ++k) p.D[k] = __ldg(&a.dinv32[9 * (size_t)i + k]);
+    return p;
+}
+__device__ __forceinline__ void pre_smooth(const AmgPre& a, int i, const double v[3], const PreD& p) {
     if (!a.z) return;
-    const float om = (float)__ldg(a.omega);
     const float f[3] = {(float)v[0], (float)v[1], (float)v[2]};
-    const float* __restrict__ D = a.dinv32 + 9 * (size_t)i;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         a.r[3 * i + k] = f[k];
-        a.z[3 * i + k] =
-            om * fmaf(__ldg(&D[3 * k]), f[0], fmaf(__ldg(&D[3 * k + 1]), f[1], __ldg(&D[3 * k + 2]) * f[2]));
+        a.z[3 * i + k] = p.om * fmaf(p.D[3 * k], f[0], fmaf(p.D[3 * k + 1], f[1], p.D[3 * k + 2] * f[2]));
     }
+}
+
+// The three components of a vector at the thread's node.
+__device__ __forceinline__ void load3(const double* __restrict__ x, int i, double (&v)[3]) {
+#pragma unroll
+    for (int d = 0; d < 3; ++d) v[d] = x[3 * i + d];
 }
 
 // ---- CG -------------------------------------------------------------------
@@ -101,10 +133,14 @@ __global__ void k_cg_init(Ctx c, const double* __restrict__ b, double* __restric
         return;
     }
     double v[3] = {0.0, 0.0, 0.0};  // (r, z), |r|^2, |b|^2
+    double ax[3] = {0.0, 0.0, 0.0};
+    if (x0 && active) {  // start from x0: r = b - A x0
+        rows_product<2>(c, warp_slots(c), x0, ax);
+        rows_sum(c, w, x0, ax);
+    }
     if (w.valid) {
         const int i = w.node;
-        double rr[3], zz[3], ax[3] = {0.0, 0.0, 0.0};
-        if (x0 && active) bsr_row(c, i, x0, ax);  // start from x0: r = b - A x0
+        double rr[3], zz[3];
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
             const double bk = active ? b[3 * i + d] : 0.0;
@@ -123,7 +159,7 @@ __global__ void k_cg_init(Ctx c, const double* __restrict__ b, double* __restric
                 v[0] = fma(rr[d], zz[d], v[0]);
             }
         }
-        pre_smooth(pre, i, rr);
+        pre_smooth(pre, i, rr, pre_load(pre, i));
 #pragma unroll
         for (int d = 0; d < 3; ++d) v[1] = fma(rr[d], rr[d], v[1]);
     }
@@ -136,29 +172,34 @@ __global__ void k_cg_init(Ctx c, const double* __restrict__ b, double* __restric
 
 // q = A p; alpha = rz / (p, q)
 template <int U>
-__global__ void k_cg_spmv(Ctx c, const double* __restrict__ p, double* __restrict__ q) {
+__global__ void __launch_bounds__(kThreads, U == 0 ? 4 : 6)
+    k_cg_spmv(Ctx c, const double* __restrict__ p, double* __restrict__ q) {
     pdl_enter();
     const Where w = where(c);
+    const Slots sl = warp_slots(c);
     if (stopped(w)) return;
-    double v[1] = {0.0};
+    double v[1] = {0.0}, y[3], pi[3];
+    rows_product<U>(c, sl, p, y);
+    const double rz = U == 0 ? __ldcg(&w.s[S_RZ]) : 0.0;
+    if (U == 0 && w.valid) load3(p, w.node, pi);
+    rows_sum<U == 0 ? kSplit : kWhole>(c, w, p, y);
+    if (U != 0 && w.valid) load3(p, w.node, pi);
     if (w.valid) {
-        double y[3];
-        bsr_row<U>(c, w.node, p, y);
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
             q[3 * w.node + d] = y[d];
-            v[0] = fma(p[3 * w.node + d], y[d], v[0]);
+            v[0] = fma(pi[d], y[d], v[0]);
         }
     }
     double tot[1];
-    if (reduce_seg<1>(c, w.seg, v, tot) && threadIdx.x == 0) {
+    if (reduce_seg<1, U == 0 ? kSplit : kWhole>(c, w.seg, v, tot) && threadIdx.x == 0) {
         const double pq = tot[0];
         if (!(pq > 0.0) || !isfinite(pq)) {
             w.s[S_FLAG] = isfinite(pq) ? F_BREAKDOWN : F_NAN;
             w.s[S_WHY] = W_CG_PAP;
         } else {
             w.s[S_PQ] = pq;
-            w.s[S_ALPHA] = w.s[S_RZ] / pq;
+            w.s[S_ALPHA] = (U == 0 ? rz : w.s[S_RZ]) / pq;
         }
     }
 }
@@ -168,17 +209,26 @@ __global__ void k_cg_update(Ctx c, double* __restrict__ x, double* __restrict__ 
                             const double* __restrict__ p, const double* __restrict__ q, int jac, AmgPre pre) {
     pdl_enter();
     const Where w = where(c);
+    const double alpha = __ldcg(&w.s[S_ALPHA]), stop = __ldcg(&w.s[S_TOL2]) * __ldcg(&w.s[S_BB]);
+    const int i = w.node;
+    double pi[3], qi[3], xi[3], ri[3];
+    PreD pd;
+    if (load_now(c, w)) {
+        load3(p, i, pi);
+        load3(q, i, qi);
+        load3(x, i, xi);
+        load3(r, i, ri);
+        pd = pre_load(pre, i);
+    }
     if (stopped(w)) return;
-    const double alpha = __ldcg(&w.s[S_ALPHA]);
     double v[2] = {0.0, 0.0};
     if (w.valid) {
-        const int i = w.node;
         double rr[3], zz[3];
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
             const int k = 3 * i + d;
-            x[k] = fma(alpha, p[k], x[k]);
-            rr[d] = fma(-alpha, q[k], r[k]);
+            x[k] = fma(alpha, pi[d], xi[d]);
+            rr[d] = fma(-alpha, qi[d], ri[d]);
             r[k] = rr[d];
         }
         if (jac) {
@@ -189,7 +239,7 @@ __global__ void k_cg_update(Ctx c, double* __restrict__ x, double* __restrict__ 
                 v[0] = fma(rr[d], zz[d], v[0]);
             }
         }
-        pre_smooth(pre, i, rr);
+        pre_smooth(pre, i, rr, pd);
 #pragma unroll
         for (int d = 0; d < 3; ++d) v[1] = fma(rr[d], rr[d], v[1]);
     }
@@ -204,7 +254,7 @@ __global__ void k_cg_update(Ctx c, double* __restrict__ x, double* __restrict__ 
         s[S_RR] = rr;
         s[S_ITER] += 1.0;
         if (!isfinite(rr)) s[S_FLAG] = F_NAN;
-        else if (rr <= s[S_TOL2] * s[S_BB]) s[S_FLAG] = F_CONVERGED;
+        else if (rr <= stop) s[S_FLAG] = F_CONVERGED;
         else if (jac && !(rz > 0.0)) {
             s[S_FLAG] = F_BREAKDOWN;
             s[S_WHY] = W_CG_RZ;
@@ -236,13 +286,15 @@ __global__ void k_cg_rz(Ctx c, const double* __restrict__ r, const double* __res
 __global__ void k_cg_direction(Ctx c, const double* __restrict__ z, double* __restrict__ p) {
     pdl_enter();
     const Where w = where(c);
-    if (stopped(w) || !w.valid) return;
     const double beta = __ldcg(&w.s[S_BETA]);
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        const int k = 3 * w.node + d;
-        p[k] = fma(beta, p[k], z[k]);
+    double pi[3], zi[3];
+    if (load_now(c, w)) {
+        load3(p, w.node, pi);
+        load3(z, w.node, zi);
     }
+    if (stopped(w) || !w.valid) return;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) p[3 * w.node + d] = fma(beta, pi[d], zi[d]);
 }
 
 // ---- BiCGStab ---------------------------------------------------------------
@@ -258,9 +310,12 @@ __global__ void k_bi_init(Ctx c, const double* __restrict__ b, double* __restric
         return;
     }
     double s[2] = {0.0, 0.0};  // |r|^2, |b|^2
+    double ax[3] = {0.0, 0.0, 0.0};
+    if (x0 && active) {  // start from x0: r = b - A x0
+        rows_product<2>(c, warp_slots(c), x0, ax);
+        rows_sum(c, w, x0, ax);
+    }
     if (w.valid) {
-        double ax[3] = {0.0, 0.0, 0.0};
-        if (x0 && active) bsr_row(c, w.node, x0, ax);  // start from x0: r = b - A x0
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
             const int k = 3 * w.node + d;
@@ -290,17 +345,23 @@ __global__ void k_bi_dir(Ctx c, const double* __restrict__ r, const double* __re
                          double* __restrict__ phat, int jac, AmgPre pre) {
     pdl_enter();
     const Where w = where(c);
-    if (stopped(w) || !w.valid) return;
     const double beta = __ldcg(&w.s[S_BETA]), omega = __ldcg(&w.s[S_OMEGA]);
     const int i = w.node;
-    double pp[3], z[3];
+    double pp[3], z[3], vi[3], pi[3], ri[3];
+    PreD pd;
+    if (load_now(c, w)) {
+        load3(v, i, vi);
+        load3(p, i, pi);
+        load3(r, i, ri);
+        pd = pre_load(pre, i);
+    }
+    if (stopped(w) || !w.valid) return;
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-        const int k = 3 * i + d;
-        pp[d] = fma(beta, fma(-omega, v[k], p[k]), r[k]);
-        p[k] = pp[d];
+        pp[d] = fma(beta, fma(-omega, vi[d], pi[d]), ri[d]);
+        p[3 * i + d] = pp[d];
     }
-    pre_smooth(pre, i, pp);
+    pre_smooth(pre, i, pp, pd);
     if (!jac) return;
     apply_dinv(c.dinv + 9 * (size_t)i, pp, z);
 #pragma unroll
@@ -309,29 +370,34 @@ __global__ void k_bi_dir(Ctx c, const double* __restrict__ r, const double* __re
 
 // v = A phat; alpha = rho / (rhat, v)
 template <int U>
-__global__ void k_bi_spmv1(Ctx c, const double* __restrict__ phat, const double* __restrict__ rhat,
+__global__ void __launch_bounds__(kThreads, U == 0 ? 4 : 6)
+    k_bi_spmv1(Ctx c, const double* __restrict__ phat, const double* __restrict__ rhat,
                            double* __restrict__ v) {
     pdl_enter();
     const Where w = where(c);
+    const Slots sl = warp_slots(c);
     if (stopped(w)) return;
-    double s[1] = {0.0};
+    double s[1] = {0.0}, y[3], rh[3];
+    rows_product<U>(c, sl, phat, y);
+    const double rho = U == 0 ? __ldcg(&w.s[S_RHO]) : 0.0;
+    if (U == 0 && w.valid) load3(rhat, w.node, rh);
+    rows_sum<U == 0 ? kSplit : kWhole>(c, w, phat, y);
+    if (U != 0 && w.valid) load3(rhat, w.node, rh);
     if (w.valid) {
-        double y[3];
-        bsr_row<U>(c, w.node, phat, y);
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
             v[3 * w.node + d] = y[d];
-            s[0] = fma(rhat[3 * w.node + d], y[d], s[0]);
+            s[0] = fma(rh[d], y[d], s[0]);
         }
     }
     double tot[1];
-    if (reduce_seg<1>(c, w.seg, s, tot) && threadIdx.x == 0) {
+    if (reduce_seg<1, U == 0 ? kSplit : kWhole>(c, w.seg, s, tot) && threadIdx.x == 0) {
         const double rv = tot[0];
         if (rv == 0.0 || !isfinite(rv)) {
             w.s[S_FLAG] = isfinite(rv) ? F_BREAKDOWN : F_NAN;
             w.s[S_WHY] = W_BI_RV;
         } else {
-            w.s[S_ALPHA] = w.s[S_RHO] / rv;
+            w.s[S_ALPHA] = (U == 0 ? rho : w.s[S_RHO]) / rv;
         }
     }
 }
@@ -343,17 +409,23 @@ __global__ void k_bi_s(Ctx c, const double* __restrict__ r, const double* __rest
                        double* __restrict__ shat, int jac, AmgPre pre) {
     pdl_enter();
     const Where w = where(c);
+    const double alpha = __ldcg(&w.s[S_ALPHA]), stop = __ldcg(&w.s[S_TOL2]) * __ldcg(&w.s[S_BB]);
+    const int i = w.node;
+    double vi[3], ri[3];
+    PreD pd;
+    if (load_now(c, w)) {
+        load3(v, i, vi);
+        load3(r, i, ri);
+        pd = pre_load(pre, i);
+    }
     if (stopped(w)) return;
-    const double alpha = __ldcg(&w.s[S_ALPHA]);
     double acc[1] = {0.0};
     if (w.valid) {
-        const int i = w.node;
         double ss[3], z[3];
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
-            const int k = 3 * i + d;
-            ss[d] = fma(-alpha, v[k], r[k]);
-            s[k] = ss[d];
+            ss[d] = fma(-alpha, vi[d], ri[d]);
+            s[3 * i + d] = ss[d];
             acc[0] = fma(ss[d], ss[d], acc[0]);
         }
         if (jac) {
@@ -361,12 +433,12 @@ __global__ void k_bi_s(Ctx c, const double* __restrict__ r, const double* __rest
 #pragma unroll
             for (int d = 0; d < 3; ++d) shat[3 * i + d] = z[d];
         }
-        pre_smooth(pre, i, ss);
+        pre_smooth(pre, i, ss, pd);
     }
     double tot[1];
     if (reduce_seg<1>(c, w.seg, acc, tot) && threadIdx.x == 0) {
         if (!isfinite(tot[0])) w.s[S_FLAG] = F_NAN;
-        else if (tot[0] <= w.s[S_TOL2] * w.s[S_BB]) {
+        else if (tot[0] <= stop) {
             w.s[S_RR] = tot[0];  // the residual of x + alpha phat is s
             w.s[S_FLAG] = -1.0;  // half step converged
         }
@@ -376,12 +448,13 @@ __global__ void k_bi_s(Ctx c, const double* __restrict__ r, const double* __rest
 // t = A shat; omega = (t, s) / (t, t).  An instance flagged -1 by k_bi_s takes
 // its half step x += alpha phat here and is marked converged.
 template <int U>
-__global__ void k_bi_spmv2(Ctx c, const double* __restrict__ shat, const double* __restrict__ s,
+__global__ void __launch_bounds__(kThreads, U == 0 ? 4 : 6)
+    k_bi_spmv2(Ctx c, const double* __restrict__ shat, const double* __restrict__ s,
                            double* __restrict__ t, double* __restrict__ x, const double* __restrict__ phat) {
     pdl_enter();
     const Where w = where(c);
-    const double flag = __ldcg(&w.s[S_FLAG]);
-    if (flag == -1.0) {
+    const Slots sl = warp_slots(c);
+    if (w.flag == -1.0) {
         const double alpha = __ldcg(&w.s[S_ALPHA]);
         if (w.valid)
 #pragma unroll
@@ -390,26 +463,28 @@ __global__ void k_bi_spmv2(Ctx c, const double* __restrict__ shat, const double*
                 x[k] = fma(alpha, phat[k], x[k]);
             }
         double none[1] = {0.0}, all[1];
-        if (reduce_seg<1>(c, w.seg, none, all) && threadIdx.x == 0) {
+        if (reduce_seg<1, U == 0 ? kSplit : kWhole>(c, w.seg, none, all) && threadIdx.x == 0) {
             w.s[S_ITER] += 1.0;
             w.s[S_FLAG] = F_CONVERGED;
         }
         return;
     }
-    if (flag != 0.0) return;
-    double acc[2] = {0.0, 0.0};
+    if (stopped(w)) return;
+    double acc[2] = {0.0, 0.0}, y[3], si[3];
+    rows_product<U>(c, sl, shat, y);
+    if (U == 0 && w.valid) load3(s, w.node, si);
+    rows_sum<U == 0 ? kSplit : kWhole>(c, w, shat, y);
+    if (U != 0 && w.valid) load3(s, w.node, si);
     if (w.valid) {
-        double y[3];
-        bsr_row<U>(c, w.node, shat, y);
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
             t[3 * w.node + d] = y[d];
-            acc[0] = fma(y[d], s[3 * w.node + d], acc[0]);
+            acc[0] = fma(y[d], si[d], acc[0]);
             acc[1] = fma(y[d], y[d], acc[1]);
         }
     }
     double tot[2];
-    if (reduce_seg<2>(c, w.seg, acc, tot) && threadIdx.x == 0) {
+    if (reduce_seg<2, U == 0 ? kSplit : kWhole>(c, w.seg, acc, tot) && threadIdx.x == 0) {
         const double ts = tot[0], tt = tot[1];
         if (!isfinite(ts) || !isfinite(tt)) w.s[S_FLAG] = F_NAN;
         else w.s[S_OMEGA] = (tt > 0.0) ? ts / tt : 0.0;
@@ -422,31 +497,42 @@ __global__ void k_bi_x(Ctx c, double* __restrict__ x, double* __restrict__ r, co
                        const double* __restrict__ t) {
     pdl_enter();
     const Where w = where(c);
+    const double alpha = __ldcg(&w.s[S_ALPHA]), omega = __ldcg(&w.s[S_OMEGA]), rho0 = __ldcg(&w.s[S_RHO]);
+    const double stop = __ldcg(&w.s[S_TOL2]) * __ldcg(&w.s[S_BB]);
+    const int i = w.node;
+    double xi[3], ph[3], sh[3], si[3], ti[3], rh[3];
+    if (load_now(c, w)) {
+        load3(x, i, xi);
+        load3(phat, i, ph);
+        load3(shat, i, sh);
+        load3(s, i, si);
+        load3(t, i, ti);
+        load3(rhat, i, rh);
+    }
     if (stopped(w)) return;
-    const double alpha = __ldcg(&w.s[S_ALPHA]), omega = __ldcg(&w.s[S_OMEGA]);
     double acc[2] = {0.0, 0.0};
     if (w.valid) {
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
-            const int k = 3 * w.node + d;
-            x[k] = fma(omega, shat[k], fma(alpha, phat[k], x[k]));
-            const double rk = fma(-omega, t[k], s[k]);
-            r[k] = rk;
-            acc[0] = fma(rhat[k], rk, acc[0]);
+            x[3 * i + d] = fma(omega, sh[d], fma(alpha, ph[d], xi[d]));
+            const double rk = fma(-omega, ti[d], si[d]);
+            r[3 * i + d] = rk;
+            acc[0] = fma(rh[d], rk, acc[0]);
             acc[1] = fma(rk, rk, acc[1]);
         }
     }
+    const double scale = alpha / omega;
     double tot[2];
     if (reduce_seg<2>(c, w.seg, acc, tot) && threadIdx.x == 0) {
         double* q = w.s;
         const double rho = tot[0], rr = tot[1];
-        const double om = q[S_OMEGA];
-        q[S_BETA] = (rho / q[S_RHO]) * (q[S_ALPHA] / om);
+        const double om = omega;
+        q[S_BETA] = (rho / rho0) * scale;
         q[S_RHO] = rho;
         q[S_RR] = rr;
         q[S_ITER] += 1.0;
         if (!isfinite(rr)) q[S_FLAG] = F_NAN;
-        else if (rr <= q[S_TOL2] * q[S_BB]) q[S_FLAG] = F_CONVERGED;
+        else if (rr <= stop) q[S_FLAG] = F_CONVERGED;
         else if (om == 0.0 || rho == 0.0) {
             q[S_FLAG] = F_BREAKDOWN;
             q[S_WHY] = om == 0.0 ? W_BI_OMEGA : W_BI_RHO;
@@ -530,29 +616,31 @@ void issue_iterations_u(tf_handle* h, const Ctx& c, int method, int n) {
     cudaStream_t st = h->stream;
     const int nb = d.ncta;
     const int jac = use_multigrid(h) ? 0 : 1;
+    const int vt = vector_threads(d);
     const AmgPre pre = amg_pre(h);
     for (int it = 0; it < n; ++it) {
         if (method == 1) {
-            launch_pdl(k_cg_spmv<U>, nb, kThreads, st, c, d.p, d.q);
-            launch_pdl(k_cg_update, nb, kThreads, st, c, d.du, d.r, d.z, d.p, d.q, jac, pre);
+            launch_pdl_smem(k_cg_spmv<U>, nb, kThreads, split_bytes<double>(d), st, c, d.p, d.q);
+            launch_pdl(k_cg_update, nb, vt, st, c, d.du, d.r, d.z, d.p, d.q, jac, pre);
             if (!jac) {
                 amg_vcycle(h, d.r, d.z, kVcycleDot, d.p);
-                if (!amg_fuses_dot(h)) launch_pdl(k_cg_rz, nb, kThreads, st, c, d.r, d.z, d.p, 0);
+                if (!amg_fuses_dot(h)) launch_pdl(k_cg_rz, nb, vt, st, c, d.r, d.z, d.p, 0);
             }
-            launch_pdl(k_cg_direction, nb, kThreads, st, c, d.z, d.p);
+            launch_pdl(k_cg_direction, nb, vt, st, c, d.z, d.p);
         } else {
-            launch_pdl(k_bi_dir, nb, kThreads, st, c, d.r, d.q, d.p, d.z, jac, pre);
+            launch_pdl(k_bi_dir, nb, vt, st, c, d.r, d.q, d.p, d.z, jac, pre);
             if (!jac) amg_vcycle(h, d.p, d.z);
-            launch_pdl(k_bi_spmv1<U>, nb, kThreads, st, c, d.z, d.rhat, d.q);
-            launch_pdl(k_bi_s, nb, kThreads, st, c, d.r, d.q, d.s, d.sh, jac, pre);
+            launch_pdl_smem(k_bi_spmv1<U>, nb, kThreads, split_bytes<double>(d), st, c, d.z, d.rhat, d.q);
+            launch_pdl(k_bi_s, nb, vt, st, c, d.r, d.q, d.s, d.sh, jac, pre);
             if (!jac) amg_vcycle(h, d.s, d.sh);
-            launch_pdl(k_bi_spmv2<U>, nb, kThreads, st, c, d.sh, d.s, d.t, d.du, d.z);
-            launch_pdl(k_bi_x, nb, kThreads, st, c, d.du, d.r, d.rhat, d.z, d.sh, d.s, d.t);
+            launch_pdl_smem(k_bi_spmv2<U>, nb, kThreads, split_bytes<double>(d), st, c, d.sh, d.s, d.t, d.du, d.z);
+            launch_pdl(k_bi_x, nb, vt, st, c, d.du, d.r, d.rhat, d.z, d.sh, d.s, d.t);
         }
     }
 }
 
 void issue_iterations(tf_handle* h, const Ctx& c, int method, int n) {
+    if (h->d.split) return issue_iterations_u<0>(h, c, method, n);
     switch (h->spmv_unroll) {
         case 1: issue_iterations_u<1>(h, c, method, n); break;
         case 4: issue_iterations_u<4>(h, c, method, n); break;
@@ -564,9 +652,10 @@ void issue_iterations(tf_handle* h, const Ctx& c, int method, int n) {
 template <int U>
 __global__ void k_spmv_probe(Ctx c, const double* __restrict__ x, double* __restrict__ y) {
     const Where w = where(c);
-    if (!w.valid) return;
     double v[3];
-    bsr_row<U>(c, w.node, x, v);
+    rows_product<U>(c, warp_slots(c), x, v);
+    rows_sum(c, w, x, v);
+    if (!w.valid) return;
 #pragma unroll
     for (int d = 0; d < 3; ++d) y[3 * w.node + d] = v[d];
 }
@@ -591,9 +680,9 @@ tf_status autotune_solve(tf_handle* h) {
     for (int u : {1, 2, 4}) {
         for (int r = 0; r < 4; ++r) {  // one warm-up, three timed
             if (r == 1) TF_CUDA(cudaEventRecord(h->ev[4], st));
-            if (u == 1) k_spmv_probe<1><<<d.ncta, kThreads, 0, st>>>(c, d.du, d.q);
-            else if (u == 2) k_spmv_probe<2><<<d.ncta, kThreads, 0, st>>>(c, d.du, d.q);
-            else k_spmv_probe<4><<<d.ncta, kThreads, 0, st>>>(c, d.du, d.q);
+            if (u == 1) k_spmv_probe<1><<<d.ncta, kThreads, split_bytes<double>(d), st>>>(c, d.du, d.q);
+            else if (u == 2) k_spmv_probe<2><<<d.ncta, kThreads, split_bytes<double>(d), st>>>(c, d.du, d.q);
+            else k_spmv_probe<4><<<d.ncta, kThreads, split_bytes<double>(d), st>>>(c, d.du, d.q);
             TF_LAUNCH_CHECK(h);
         }
         TF_CUDA(cudaEventRecord(h->ev[5], st));
@@ -723,7 +812,7 @@ tf_status krylov_run(tf_handle* h, int method, int keep, int* iters, double* rel
     // test stays relative to |g|, so the accuracy is that of a zero start.
     const double* x0 = (keep == 0 && h->newton_index == 0 && h->have_du0) ? h->du0 : nullptr;
     if (keep == 2) {  // BiCGStab restart: block inverse and x are kept
-        k_bi_restart<<<d.ncta, kThreads, 0, st>>>(c, d.r, d.rhat, d.p, d.q);
+        k_bi_restart<<<d.ncta, vector_threads(d), 0, st>>>(c, d.r, d.rhat, d.p, d.q);
     } else {
         const tf_status sb = launch_block_inverse(h);
         if (sb != TF_OK) return sb;
@@ -736,18 +825,18 @@ tf_status krylov_run(tf_handle* h, int method, int keep, int* iters, double* rel
             if (su != TF_OK) return su;
         }
         if (method == 1) {
-            k_cg_init<<<d.ncta, kThreads, 0, st>>>(c, d.g, d.du, d.r, d.z, d.p, tol2, h->solve_atol, keep, jac, x0,
+            k_cg_init<<<d.ncta, kThreads, split_bytes<double>(d), st>>>(c, d.g, d.du, d.r, d.z, d.p, tol2, h->solve_atol, keep, jac, x0,
                                                    amg_pre(h));
             if (!jac) {
                 amg_vcycle(h, d.r, d.z, kVcycleStart, d.p);
                 h->launches += amg_vcycle_kernels(h);
                 if (!amg_fuses_dot(h)) {
-                    k_cg_rz<<<d.ncta, kThreads, 0, st>>>(c, d.r, d.z, d.p, 1);
+                    k_cg_rz<<<d.ncta, vector_threads(d), 0, st>>>(c, d.r, d.z, d.p, 1);
                     TF_LAUNCH_CHECK(h);
                 }
             }
         } else {
-            k_bi_init<<<d.ncta, kThreads, 0, st>>>(c, d.g, d.du, d.r, d.rhat, d.p, d.q, tol2, h->solve_atol, keep, x0);
+            k_bi_init<<<d.ncta, kThreads, split_bytes<double>(d), st>>>(c, d.g, d.du, d.r, d.rhat, d.p, d.q, tol2, h->solve_atol, keep, x0);
         }
     }
     TF_LAUNCH_CHECK(h);
@@ -921,7 +1010,7 @@ tf_status krylov_solve(tf_handle* h, int* iters, double* relres) {
 tf_status launch_update(tf_handle* h) {
     Device& d = h->d;
     const Ctx c = make_ctx(h);
-    k_update<true><<<d.ncta, kThreads, 0, h->stream>>>(c, d.uk, d.du);
+    k_update<true><<<d.ncta, vector_threads(d), 0, h->stream>>>(c, d.uk, d.du);
     TF_LAUNCH_CHECK(h);
     return TF_OK;
 }
@@ -929,7 +1018,7 @@ tf_status launch_update(tf_handle* h) {
 tf_status launch_update_norm(tf_handle* h) {
     Device& d = h->d;
     const Ctx c = make_ctx(h);
-    k_update<false><<<d.ncta, kThreads, 0, h->stream>>>(c, d.uk, d.du);
+    k_update<false><<<d.ncta, vector_threads(d), 0, h->stream>>>(c, d.uk, d.du);
     TF_LAUNCH_CHECK(h);
     return TF_OK;
 }
@@ -1092,14 +1181,14 @@ bool issue_newton_iteration(tf_handle* h, cudaGraphConditionalHandle newton) {
     const double tol2 = h->opt.krylov_rtol * h->opt.krylov_rtol;
     const int jac = mg ? 0 : 1;
     if (method == 1) {
-        k_cg_init<<<d.ncta, kThreads, 0, st>>>(c, d.g, d.du, d.r, d.z, d.p, tol2, h->opt.update_atol, 0, jac,
+        k_cg_init<<<d.ncta, kThreads, split_bytes<double>(d), st>>>(c, d.g, d.du, d.r, d.z, d.p, tol2, h->opt.update_atol, 0, jac,
                                                 nullptr, amg_pre(h));
         if (mg) {
             amg_vcycle(h, d.r, d.z, kVcycleStart, d.p);
-            if (!amg_fuses_dot(h)) k_cg_rz<<<d.ncta, kThreads, 0, st>>>(c, d.r, d.z, d.p, 1);
+            if (!amg_fuses_dot(h)) k_cg_rz<<<d.ncta, vector_threads(d), 0, st>>>(c, d.r, d.z, d.p, 1);
         }
     } else {
-        k_bi_init<<<d.ncta, kThreads, 0, st>>>(c, d.g, d.du, d.r, d.rhat, d.p, d.q, tol2, h->opt.update_atol, 0,
+        k_bi_init<<<d.ncta, kThreads, split_bytes<double>(d), st>>>(c, d.g, d.du, d.r, d.rhat, d.p, d.q, tol2, h->opt.update_atol, 0,
                                                 nullptr);
     }
     cudaGraphConditionalHandle kc = 0;
@@ -1110,11 +1199,11 @@ bool issue_newton_iteration(tf_handle* h, cudaGraphConditionalHandle newton) {
         k_krylov_ctl<<<1, 32, 0, h->stream>>>(d.scal, d.nseg, h->kloop_ctl, kc);
     });
     if (!ok) return false;
-    k_update<false><<<d.ncta, kThreads, 0, st>>>(c, d.uk, d.du);
+    k_update<false><<<d.ncta, vector_threads(d), 0, st>>>(c, d.uk, d.du);
     int* seg = h->nd_seg;
     k_newton_ctl<<<1, 256, 0, st>>>(d.scal, d.nseg, d.seg_active, seg, seg + d.nseg, seg + 2 * d.nseg, h->nd,
                                      h->opt.newton_tol, tol2, h->opt.newton_max_iter, h->opt.update_atol, newton);
-    k_update<true><<<d.ncta, kThreads, 0, st>>>(c, d.uk, d.du, &h->nd->exc);
+    k_update<true><<<d.ncta, vector_threads(d), 0, st>>>(c, d.uk, d.du, &h->nd->exc);
     return cudaGetLastError() == cudaSuccess;
 }
 

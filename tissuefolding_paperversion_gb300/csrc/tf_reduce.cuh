@@ -24,6 +24,7 @@ struct Ctx {
     double* part;               // [3][ncta]
     unsigned* tickets;          // [nseg]
     int ncta;
+    int single, split, cta_nodes;     // one instance; see Device::split
     const int* __restrict__ cta_seg;
     const int* __restrict__ cta_node0;
     const int* __restrict__ cta_node1;
@@ -37,19 +38,43 @@ struct Ctx {
 };
 
 struct Where {
-    int node;    // node of this thread
-    bool valid;  // node inside this CTA's range
-    int seg;     // instance of this CTA
-    double* s;   // its scalars
+    int node;     // node of this thread
+    bool valid;   // node inside this CTA's range
+    int seg;      // instance of this CTA
+    double* s;    // its scalars
+    double flag;  // its stop flag
 };
 
+// With one instance nothing is looked up: the operands' loads need not wait for
+// the tables', and the kernels below issue them before they test the flag (a
+// batch tests first: its stopped instances would only cost bandwidth).
 __device__ __forceinline__ Where where(const Ctx& c) {
     Where w;
-    w.seg = c.cta_seg[blockIdx.x];
-    w.node = c.cta_node0[blockIdx.x] + threadIdx.x;
-    w.valid = w.node < c.cta_node1[blockIdx.x];
+    int n1;
+    if (c.single) {
+        w.seg = 0;
+        w.node = blockIdx.x * c.cta_nodes + threadIdx.x;
+        n1 = min((int)(blockIdx.x + 1) * c.cta_nodes, c.nn);
+    } else {
+        w.seg = c.cta_seg[blockIdx.x];
+        w.node = c.cta_node0[blockIdx.x] + threadIdx.x;
+        n1 = c.cta_node1[blockIdx.x];
+    }
+    w.valid = w.node < n1;
     w.s = c.scal + (size_t)w.seg * S_COUNT;
+    w.flag = __ldcg(&w.s[S_FLAG]);
     return w;
+}
+__device__ __forceinline__ bool stopped(const Where& w) { return w.flag != 0.0; }
+// The operands of this thread are to be loaded before the flag is tested.
+__device__ __forceinline__ bool load_now(const Ctx& c, const Where& w) { return w.valid && (c.single || !stopped(w)); }
+
+template <int NV>
+__device__ __forceinline__ void warp_sum(double (&v)[NV]) {  // the sums are lane 0's
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int k = 0; k < NV; ++k) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
 }
 
 template <int NV>
@@ -76,13 +101,38 @@ __device__ __forceinline__ void block_sum(double (&v)[NV], double (*sm)[kThreads
 }
 
 // Writes this CTA's partial sums; returns true in the CTA of the instance
-// that arrives last, whose thread 0 then holds the fixed-order totals.
-template <int NV>
+// that arrives last, whose thread 0 then holds the fixed-order totals.  In split
+// CTAs the values are warp 0's, and it works alone: no barrier.  (MODE kSplit or
+// kWhole: the kernel is compiled for one of the two.)
+enum { kWhole = 0, kSplit = 1, kEither = 2 };
+template <int NV, int MODE = kEither>
 __device__ __forceinline__ bool reduce_seg(const Ctx& c, int seg, double (&v)[NV], double (&tot)[NV]) {
     __shared__ double sm[NV][kThreads / 32];
     __shared__ bool last;
+    const int b0 = c.single ? 0 : c.seg_cta0[seg], b1 = c.single ? c.ncta : c.seg_cta0[seg + 1];
+    if (MODE == kSplit || (MODE == kEither && c.split)) {
+        if (threadIdx.x >= 32) return false;
+        warp_sum<NV>(v);
+        unsigned ticket = 0;
+        if (threadIdx.x == 0) {
+#pragma unroll
+            for (int k = 0; k < NV; ++k) c.part[(size_t)k * c.ncta + blockIdx.x] = v[k];
+            __threadfence();
+            ticket = atomicAdd(&c.tickets[seg], 1u);
+        }
+        if (__shfl_sync(0xffffffffu, ticket, 0) != (unsigned)(b1 - b0 - 1)) return false;
+        __threadfence();
+#pragma unroll
+        for (int k = 0; k < NV; ++k) tot[k] = 0.0;
+#pragma unroll 8
+        for (int b = b0 + (int)threadIdx.x; b < b1; b += 32)
+#pragma unroll
+            for (int k = 0; k < NV; ++k) tot[k] += __ldcg(&c.part[(size_t)k * c.ncta + b]);
+        warp_sum<NV>(tot);
+        if (threadIdx.x == 0) c.tickets[seg] = 0u;
+        return true;
+    }
     block_sum<NV>(v, sm);
-    const int b0 = c.seg_cta0[seg], b1 = c.seg_cta0[seg + 1];
     if (threadIdx.x == 0) {
 #pragma unroll
         for (int k = 0; k < NV; ++k) c.part[(size_t)k * c.ncta + blockIdx.x] = v[k];
@@ -105,8 +155,6 @@ __device__ __forceinline__ bool reduce_seg(const Ctx& c, int seg, double (&v)[NV
     if (threadIdx.x == 0) c.tickets[seg] = 0u;
     return true;
 }
-
-__device__ __forceinline__ bool stopped(const Where& w) { return __ldcg(&w.s[S_FLAG]) != 0.0; }
 
 // rz = (r, M^-1 r) of CG: beta = rz / rz_old (not at the start of a solve)
 __device__ __forceinline__ void cg_rz(double* s, double rz, bool start) {
@@ -131,6 +179,9 @@ inline Ctx make_ctx(tf_handle* h) {
     c.part = d.part;
     c.tickets = d.tickets;
     c.ncta = d.ncta;
+    c.single = d.nseg == 1;
+    c.split = d.split;
+    c.cta_nodes = d.cta_nodes;
     c.cta_seg = d.cta_seg;
     c.cta_node0 = d.cta_node0;
     c.cta_node1 = d.cta_node1;
