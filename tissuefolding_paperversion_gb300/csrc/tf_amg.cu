@@ -22,14 +22,15 @@
 //     products that make it (no atomics, reproducible).
 //   Plain aggregation (tf_options.precond 3) keeps P = P_t.
 // Numeric phase, once per time step (all on the device), level by level:
-//   lambda_max of D^-1 A by power iteration (smoother weight and prolongator
+//   lambda_max of D^-1 A by power iteration (smoother weights and prolongator
 //   smoothing weight omega = 4 / (3.15 lambda)); P; T = A P; A_{l+1} = P^T T;
 //   6x6 block inverses; Gauss-Jordan inverse of the coarsest level per
 //   instance (<= 16 nodes); the explicit dense operator of the levels whose
 //   matrices are small enough (k_dense_build).
 // Application (one V-cycle per preconditioner call, all kernels, capturable
-// in a CUDA graph): damped block-Jacobi pre- and post-smoothing (one sweep
-// each way at level 0, kCoarseSweeps on the coarser levels), residual,
+// in a CUDA graph): block-Jacobi pre- and post-smoothing (one damped sweep each
+// way at level 0, kCoarseSweeps with Chebyshev weights on the coarser levels),
+// residual,
 // restriction, coarse correction.  Kernels of an instance whose Krylov
 // solve has stopped return at once.
 // Precision: the preconditioner is any fixed linear operator as far as the
@@ -83,8 +84,31 @@ constexpr int kDenseCycles = 3;   // V-cycles the dense operator stands for
 // wing: 201 / 150 / 128, 177 / 153 / 144 ms) while extra level-0 sweeps,
 // which cost a full-size SpMV each, barely do
 constexpr int kCoarseSweeps = 3;
+// The sweeps of a level >= 1 are those of a Chebyshev polynomial of D^-1 A over
+// [lambda / kChebRatio, lambda]: sweep k takes sweep_weight(k) times the level's
+// weight, the post-sweeps in the reverse order (the cycle stays symmetric).  The
+// same kernels reach further down the spectrum than with equal weights: Krylov
+// iterations per step 38 -> 31 on the 320,000-prism sheet (23.7 -> 20.3 ms), 70 ->
+// 57 on the 1M-prism wing (53.0 -> 46.1 ms), 106 -> 85 for 32 tissues (33.2 -> 28.2
+// ms), 63 -> 50 at 46,208 prisms (7.0 -> 6.0 ms), kLevel0Weight included.  Ratios
+// 4 / 8 / 15: 66 / 65 / 65, 97 / 92 / 84 and 56 / 53 / 50 iterations (wing, tissues,
+// 46,208); the polynomial exceeds one beyond lambda (1 + 1 / ratio), and the power
+// iteration's lambda is some 9 % low on the wing: 25 diverges there.
+constexpr double kChebRatio = 8.0;
+// Level 0 sweeps once each way, with this times its weight: 0.85 / 1 / 1.15 / 1.3
+// give 43 / 41 / 38 / 36 iterations at 1,600 prisms, 25 / 24 / 21 / 20 at 9,728
+// viscous ones, 63 / 62 / 61 / 60 at 46,208.  It converges for eigenvalues up to
+// 1.3 times the estimate.
+constexpr double kLevel0Weight = 1.2;
 
 // ---- host set-up -----------------------------------------------------------------
+
+// 1 / root k of the Chebyshev polynomial of degree n, over the weight 4 / (3 lambda)
+static float sweep_weight(int k, int n) {
+    const double lo = 1.0 / kChebRatio;
+    const double root = 0.5 * (1.0 + lo) + 0.5 * (1.0 - lo) * std::cos(M_PI * (2 * k + 1) / (2.0 * n));
+    return static_cast<float>(0.75 / root);
+}
 
 struct HostLevel {
     int n = 0, bs = 3;
@@ -283,7 +307,8 @@ struct Amg {
     AmgLevel L[kAmgMaxLevels];
     AmgSetup S[kAmgMaxLevels];
     AmgQ Q;
-    double* omega = nullptr;   // [nlev] smoother weights
+    double* omega = nullptr;   // [nlev] smoother weights 4 / (3 lambda)
+    double* omega0 = nullptr;  // level 0's in the V-cycle (omega[0] smooths the prolongator)
     double* pscal = nullptr;   // [nlev][2] power-iteration scalars (scale, lambda)
     float* x1 = nullptr;       // [3 n] the smoothed part of a V-cycle's result (k_q_smooth)
     float* pv = nullptr;       // power-iteration vectors (max n*bs each)
@@ -345,7 +370,7 @@ void amg_free(Amg* a) {
     }
     if (a->dmat != a->cinv && a->dmat) cudaFree(a->dmat);
     if (a->doff != a->cinv0 && a->doff) cudaFree(a->doff);
-    void* ptrs[] = {a->omega, a->pscal, a->pv, a->pw, a->part, a->ticket, a->cnode0, a->cinv0, a->cinv,
+    void* ptrs[] = {a->omega, a->omega0, a->pscal, a->pv, a->pw, a->part, a->ticket, a->cnode0, a->cinv0, a->cinv,
                     a->val32, a->dinv32, a->valh, a->diag32, a->dgroup, a->dwork,
                     a->Q.slot0, a->Q.col, a->Q.v16, a->Q.v2, a->Q.cptr, a->Q.crow, a->Q.cval, a->Q.tp, a->Q.pos,
                     a->Q.cpos, a->x1};
@@ -736,6 +761,7 @@ tf_status amg_build(tf_handle* h, const double* pos) {
         a->L[l].single = d.nseg == 1;
     }
     AMG_TRY(zeros(&a->omega, (size_t)a->nlev));
+    AMG_TRY(zeros(&a->omega0, 1));
     AMG_TRY(zeros(&a->val32, (size_t)d.nval));
     AMG_TRY(zeros(&a->valh, (size_t)d.nval));
     AMG_TRY(zeros(&a->dinv32, 9 * (size_t)d.nn));
@@ -1441,17 +1467,18 @@ __global__ void k_pw_init(int64_t m, float* __restrict__ v, double* part, unsign
     if (grid_sum(s, part, ticket, &tot)) scal[0] = 1.0 / sqrt(tot);
 }
 
-__device__ __forceinline__ void pw_finish(double tot, double* scal, double* omega) {
+__device__ __forceinline__ void pw_finish(double tot, double* scal, double* omega, double* level0 = nullptr) {
     const double lam = sqrt(tot);
     scal[0] = lam > 0.0 ? 1.0 / lam : 1.0;
     scal[1] = lam;
     // 5 % margin: the power iteration approaches lambda_max from below
     *omega = lam > 0.0 ? (4.0 / 3.0) / (1.05 * lam) : 1.0;
+    if (level0) *level0 = kLevel0Weight * *omega;
 }
 
 __global__ void k_pw_step0(Device d, const __half* __restrict__ valh, const float* __restrict__ dinv32,
                            const float* __restrict__ v, float* __restrict__ w, double* part, unsigned* ticket,
-                           double* scal, double* omega) {
+                           double* scal, double* omega, double* level0) {
     const Node0 q = node0(d);
     double s = 0.0;
     float y[3] = {0.f, 0.f, 0.f};
@@ -1466,7 +1493,7 @@ __global__ void k_pw_step0(Device d, const __half* __restrict__ valh, const floa
         }
     }
     double tot;
-    if (grid_sum(s, part, ticket, &tot)) pw_finish(tot, scal, omega);
+    if (grid_sum(s, part, ticket, &tot)) pw_finish(tot, scal, omega, level0);
 }
 
 __global__ void k_pw_step6(AmgLevel L, const float* __restrict__ v, float* __restrict__ w, double* part,
@@ -1633,8 +1660,8 @@ struct V0 {  // level-0 operands
 // the current matrix: k_v0_resid .. k_v0_post below.
 
 // r_C(I) = sum over the blocks (i, I) of P_iI^T t_i (of Q for the folded level-0
-// transfer) and, with presmooth, the coarse level's first sweep x_C = omega_C D_C^-1
-// r_C.  One CTA of kRestrictThreads per coarse node, its threads striding over the
+// transfer) and, with presmooth (the sweep's weight), the coarse level's first sweep
+// x_C = presmooth omega_C D_C^-1 r_C.  One CTA of kRestrictThreads per coarse node, its threads striding over the
 // (block, row) pairs of the column, stored contiguously (one warp per node: 7.5
 // against 6.0 us from 8,978 to 391 nodes).  V: __half or float values, 6 per pair.
 template <int BS, class V>
@@ -1643,7 +1670,7 @@ __global__ void __launch_bounds__(kRestrictThreads) k_restrict(const int* __rest
                                                                const V* __restrict__ val, AmgLevel C, int nf, int* check,
                                                                const float* __restrict__ t,
                                                                const double* __restrict__ scal,
-                                                               const double* __restrict__ omegaC, int presmooth) {
+                                                               const double* __restrict__ omegaC, float presmooth) {
     __shared__ float sm[kRestrictThreads / 32][6];
     pdl_enter();
     const int I = blockIdx.x;
@@ -1682,7 +1709,8 @@ __global__ void __launch_bounds__(kRestrictThreads) k_restrict(const int* __rest
     }
     if (lane < 6) {
         C.r[6 * I + lane] = pick6(rc, lane);
-        if (presmooth) C.x[6 * I + lane] = (float)__ldg(omegaC) * lane_mul6(C.dinv + 36 * (size_t)I, rc, lane);
+        if (presmooth != 0.f)
+            C.x[6 * I + lane] = presmooth * (float)__ldg(omegaC) * lane_mul6(C.dinv + 36 * (size_t)I, rc, lane);
     }
 }
 
@@ -1845,8 +1873,8 @@ __global__ void k_v0_prolong(V0 a, AmgLevel F, const float* __restrict__ e, floa
     }
 }
 
-// out_i = x_i + omega D_i^-1 (r - A x)_i for row i, by one warp
-__device__ __forceinline__ void post_row(const AmgLevel& L, const double* __restrict__ omega,
+// out_i = x_i + weight omega D_i^-1 (r - A x)_i for row i, by one warp
+__device__ __forceinline__ void post_row(const AmgLevel& L, const double* __restrict__ omega, float weight,
                                          const float* __restrict__ x, float* __restrict__ out, int i,
                                          const double* __restrict__ scal) {
     // x + omega (D^-1 (r - X x) - S x), S = D^-1 A in FP16, X the extra blocks
@@ -1864,7 +1892,8 @@ __device__ __forceinline__ void post_row(const AmgLevel& L, const double* __rest
         for (int k = 0; k < 6; ++k) rr[k] -= e[k];
     }
     if (lane < 6)
-        out[6 * i + lane] = fmaf((float)__ldg(omega), lane_mul6(L.dinv + 36 * (size_t)i, rr, lane) - y, x[6 * i + lane]);
+        out[6 * i + lane] =
+            fmaf(weight * (float)__ldg(omega), lane_mul6(L.dinv + 36 * (size_t)i, rr, lane) - y, x[6 * i + lane]);
 }
 
 // t_i = r_i - (A x)_i with A x = D (S x) + X x, lane k < 6 writing component k
@@ -1890,13 +1919,13 @@ __global__ void k_v6_resid(AmgLevel L, const double* __restrict__ scal, const fl
     resid_row(L, x, i, scal);
 }
 
-// out = x + omega D^-1 (r - A x)  (one warp per row)
-__global__ void k_v6_post(AmgLevel L, const double* __restrict__ scal, const double* __restrict__ omega,
+// out = x + weight omega D^-1 (r - A x)  (one warp per row)
+__global__ void k_v6_post(AmgLevel L, const double* __restrict__ scal, const double* __restrict__ omega, float weight,
                           const float* __restrict__ x, float* __restrict__ out) {
     pdl_enter();
     const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (i >= L.n) return;
-    post_row(L, omega, x, out, i, scal);
+    post_row(L, omega, weight, x, out, i, scal);
 }
 
 // x_i += sum over the prolongator blocks (i, J) of P_iJ e_J (6-DOF fine level),
@@ -1977,7 +2006,8 @@ struct DenseBuild {
     const double* omega;
     const int* cinv0;
     const float* cinv;
-    int first, last, sweeps;
+    int first, last;
+    float weight[kDenseSweeps];
     const int2* group;
     int ngroup;
     float* work;
@@ -2085,22 +2115,22 @@ __global__ void __launch_bounds__(kDenseThreads) k_dense_build(DenseBuild B) {
                     const size_t q = (size_t)6 * (i - f0) * kDenseQuads + c;
                     float4 acc[6];
                     load6(r[l] + q, acc);
-                    dense_smooth(F, i, om, acc, nullptr, x[l] + q);
+                    dense_smooth(F, i, om * B.weight[0], acc, nullptr, x[l] + q);
                 }
                 __syncthreads();
                 float4 *cur = x[l], *oth = e[l];
-                for (int s = 2; s <= B.sweeps + 1; ++s) {  // the last pass leaves the residual in t
+                for (int s = 2; s <= kDenseSweeps + 1; ++s) {  // the last pass leaves the residual in t
                     dense_stage(cur, xs, 6 * (f1 - f0));
                     for (int i = f0 + h; i < f1; i += nh) {
                         const size_t q = (size_t)6 * (i - f0) * kDenseQuads + c;
                         float4 acc[6];
                         load6(r[l] + q, acc);
                         dense_row(F, i, f0, f1, xs, c, acc);
-                        if (s <= B.sweeps) dense_smooth(F, i, om, acc, cur + q, oth + q);
+                        if (s <= kDenseSweeps) dense_smooth(F, i, om * B.weight[s - 1], acc, cur + q, oth + q);
                         else store6(t[l] + q, acc);
                     }
                     __syncthreads();
-                    if (s <= B.sweeps) {
+                    if (s <= kDenseSweeps) {
                         float4* sw = cur;
                         cur = oth;
                         oth = sw;
@@ -2153,14 +2183,14 @@ __global__ void __launch_bounds__(kDenseThreads) k_dense_build(DenseBuild B) {
                 }
                 __syncthreads();
                 float4 *cur = x[l], *oth = e[l];
-                for (int s = 1; s <= B.sweeps; ++s) {
+                for (int s = 1; s <= kDenseSweeps; ++s) {
                     dense_stage(cur, xs, 6 * (f1 - f0));
                     for (int i = f0 + h; i < f1; i += nh) {
                         const size_t q = (size_t)6 * (i - f0) * kDenseQuads + c;
                         float4 acc[6];
                         load6(r[l] + q, acc);
                         dense_row(F, i, f0, f1, xs, c, acc);
-                        dense_smooth(F, i, om, acc, cur + q, oth + q);
+                        dense_smooth(F, i, om * B.weight[kDenseSweeps - s], acc, cur + q, oth + q);
                     }
                     __syncthreads();
                     float4* sw = cur;
@@ -2270,7 +2300,7 @@ tf_status amg_numeric(tf_handle* h) {
             for (int it = 0; it < kPowerIters; ++it) {
                 if (l == 0)
                     k_pw_step0<<<d.ncta, kNodeThreads, split_bytes<float>(d), st>>>(d, a->valh, a->dinv32, v, w, a->part, a->ticket,
-                                                                scal, a->omega);
+                                                                scal, a->omega, a->omega0);
                 else
                     k_pw_step6<<<cdiv(32 * (int64_t)L.n, kT), kT, 0, st>>>(L, v, w, a->part, a->ticket, scal,
                                                                             a->omega + l);
@@ -2303,7 +2333,7 @@ tf_status amg_numeric(tf_handle* h) {
             TF_LAUNCH_CHECK(h);
         }
         if (l == 0 && d.nxb == 0) {  // a new extra-block layout rebuilds everything
-            k_make_q<<<cdiv(S.nT, kT), kT, 0, st>>>(a->Q, S, L.Pv, a->dinv32, a->omega);
+            k_make_q<<<cdiv(S.nT, kT), kT, 0, st>>>(a->Q, S, L.Pv, a->dinv32, a->omega0);
             TF_LAUNCH_CHECK(h);
         }
         if (l == 0) k_ptap<3><<<cdiv(C.nnzb * 6, kT), kT, 0, st>>>(L, S, C);
@@ -2338,7 +2368,7 @@ tf_status amg_numeric(tf_handle* h) {
             B.cinv = a->cinv;
             B.first = a->dense;
             B.last = a->nlev - 1;
-            B.sweeps = kDenseSweeps;
+            for (int s = 0; s < kDenseSweeps; ++s) B.weight[s] = sweep_weight(s, kDenseSweeps);
             B.group = a->dgroup;
             B.ngroup = a->ndgroup;
             B.work = a->dwork;
@@ -2363,7 +2393,7 @@ tf_status amg_autotune(tf_handle* h) {
     Device& d = h->d;
     cudaStream_t st = h->stream;
     AmgLevel& L0 = a->L[0];
-    V0 v0{d, a->omega, a->dinv32, a->valh, a->diag32};
+    V0 v0{d, a->omega0, a->dinv32, a->valh, a->diag32};
     float best = 1e30f;
     for (int u : {2, 4, 8}) {
         for (int r = 0; r < 4; ++r) {  // one warm-up, three timed
@@ -2399,7 +2429,7 @@ bool amg_fuses_dot(const tf_handle* h) { return use_multigrid(h) && uses_q(h); }
 AmgPre amg_pre(const tf_handle* h) {
     if (!use_multigrid(h)) return AmgPre{nullptr, nullptr, nullptr, nullptr};
     const Amg* a = h->amg;
-    return AmgPre{a->dinv32, a->omega, a->L[0].x, a->L[0].t};
+    return AmgPre{a->dinv32, a->omega0, a->L[0].x, a->L[0].t};
 }
 
 int amg_vcycle_kernels(const tf_handle* h) {
@@ -2407,7 +2437,7 @@ int amg_vcycle_kernels(const tf_handle* h) {
     const int per = 2 * kCoarseSweeps + 2;  // kernels of a coarse level run kernel by kernel
     const int fine = uses_q(h) ? (forks(a) ? 3 : 2) : 4;
     if (a->dense > 0) return fine + per * (a->dense - 1) + 1;
-    return fine + per * (a->nlev - 2) + 3;
+    return fine + per * (a->nlev - 2) + 2 * kCoarseSweeps - 1;
 }
 
 template <int U>
@@ -2449,9 +2479,11 @@ void amg_vcycle(tf_handle* h, const double* r, double* out, int dot, double* p) 
     cudaStream_t st = h->stream;
     const int nl = a->nlev;
     const int stop = a->dense > 0 ? a->dense : nl - 1;  // first level not handled kernel by kernel
-    V0 v0{d, a->omega, a->dinv32, a->valh, a->diag32};
+    V0 v0{d, a->omega0, a->dinv32, a->valh, a->diag32};
     AmgLevel& L0 = a->L[0];
-    auto presmooth = [&](int l) { return l == a->dense ? 0 : 1; };
+    float weight[kCoarseSweeps];
+    for (int s = 0; s < kCoarseSweeps; ++s) weight[s] = sweep_weight(s, kCoarseSweeps);
+    auto presmooth = [&](int l) { return l == a->dense ? 0.f : weight[0]; };
     const bool q = uses_q(h), fork = q && forks(a);
     if (q) {
         if (fork) {
@@ -2484,7 +2516,7 @@ void amg_vcycle(tf_handle* h, const double* r, double* out, int dot, double* p) 
         float* x = L.x;  // first pre-sweep: fused into the restriction
         for (int s = 2; s <= kCoarseSweeps; ++s) {
             float* o = pre_sweep_out(L, x);
-            launch_pdl(k_v6_post, nb, kT, st, L, (const double*)d.scal, (const double*)(a->omega + l),
+            launch_pdl(k_v6_post, nb, kT, st, L, (const double*)d.scal, (const double*)(a->omega + l), weight[s - 1],
                        (const float*)x, o);
             x = o;
         }
@@ -2499,12 +2531,16 @@ void amg_vcycle(tf_handle* h, const double* r, double* out, int dot, double* p) 
         launch_pdl(k_dense, cdiv(32 * 6 * (int64_t)LD.n, kT), kT, st, LD, (const double*)d.scal, (const int*)a->doff,
                    (const float*)a->dmat);
     } else {
-        // x from the restriction's pre-smoothing; three more sweeps into e
+        // x from the restriction's pre-smoothing; two sweeps more, and three the other way, into e
         AmgLevel& LC = a->L[nl - 1];
         const int nbc = cdiv(32 * (int64_t)LC.n, kT);
-        launch_pdl(k_v6_post, nbc, kT, st, LC, d.scal, a->omega + nl - 1, LC.x, LC.e);
-        launch_pdl(k_v6_post, nbc, kT, st, LC, d.scal, a->omega + nl - 1, LC.e, LC.t);
-        launch_pdl(k_v6_post, nbc, kT, st, LC, d.scal, a->omega + nl - 1, LC.t, LC.e);
+        float* x = LC.x;
+        for (int s = 2; s <= 2 * kCoarseSweeps; ++s) {
+            float* o = s % 2 == 0 ? LC.e : LC.t;
+            launch_pdl(k_v6_post, nbc, kT, st, LC, (const double*)d.scal, (const double*)(a->omega + nl - 1),
+                       weight[s <= kCoarseSweeps ? s - 1 : 2 * kCoarseSweeps - s], (const float*)x, o);
+            x = o;
+        }
     }
     for (int l = stop - 1; l >= 1; --l) {
         AmgLevel& L = a->L[l];
@@ -2513,7 +2549,7 @@ void amg_vcycle(tf_handle* h, const double* r, double* out, int dot, double* p) 
         for (int s = 1; s <= kCoarseSweeps; ++s) {
             float* o = post_sweep_out(L, x, s, kCoarseSweeps);
             launch_pdl(k_v6_post, cdiv(32 * (int64_t)L.n, kT), kT, st, L, (const double*)d.scal,
-                       (const double*)(a->omega + l), (const float*)x, o);
+                       (const double*)(a->omega + l), weight[kCoarseSweeps - s], (const float*)x, o);
             x = o;
         }
     }
