@@ -985,16 +985,14 @@ __device__ __forceinline__ void mul3(const float* __restrict__ D, const float r[
 // (split CTAs), from the warp's slots s0 .. s1.
 template <int U = 4>
 __device__ __forceinline__ void row0_part(const Device& d, int s0, int s1, const __half* __restrict__ valh,
-                                          const float* __restrict__ x, float (&y)[3]) {
+                                          const float* __restrict__ x, float (&y)[3], const Ahead& p = Ahead{}) {
     const int lane = threadIdx.x & 31;
     float y0 = 0.f, y1 = 0.f, y2 = 0.f;
     const int* __restrict__ col = d.scol + lane;
     const uint4* __restrict__ p8 = reinterpret_cast<const uint4*>(valh) + lane;
     const __half* __restrict__ p1 = valh + (size_t)(d.nval / kSlotDoubles) * (kSlice * 8) + lane;
-#pragma unroll U
-    for (int s = s0; s < s1; ++s) {
-        const int j = __ldg(&col[(size_t)s * kSlice]);
-        if (!TF_IN(d.check, j, d.nn, CK_V0_COL)) continue;
+    auto slot = [&](int s, int j) {
+        if (!TF_IN(d.check, j, d.nn, CK_V0_COL)) return;
         const uint4 pk = __ldg(&p8[(size_t)s * kSlice]);
         const float a8 = __half2float(p1[(size_t)s * kSlice]);
         // the low half of each word is the even entry
@@ -1010,7 +1008,14 @@ __device__ __forceinline__ void row0_part(const Device& d, int s0, int s1, const
         y0 = fmaf(a01.x, x0, fmaf(a01.y, x1, fmaf(a23.x, x2, y0)));
         y1 = fmaf(a23.y, x0, fmaf(a45.x, x1, fmaf(a45.y, x2, y1)));
         y2 = fmaf(a67.x, x0, fmaf(a67.y, x1, fmaf(a8, x2, y2)));
+    };
+    if constexpr (U == 0) {
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u)
+            if (p.j[u] >= 0) slot(s0 + u, p.j[u]);
     }
+#pragma unroll (U == 0 ? 1 : U)
+    for (int s = U == 0 ? s0 + kAhead : s0; s < s1; ++s) slot(s, __ldg(&col[(size_t)s * kSlice]));
     y[0] = y0;
     y[1] = y1;
     y[2] = y2;
@@ -1023,7 +1028,10 @@ __device__ __forceinline__ void row0s(const Device& d, const __half* __restrict_
                                       const float* __restrict__ dinv32, const float* __restrict__ x, const Node0& q0,
                                       float (&y)[3]) {
     const int wg = blockIdx.x * kWarps + (threadIdx.x >> 5), i = q0.i;
-    row0_part<U>(d, __ldg(&d.wslot0[wg]), __ldg(&d.wslot0[wg + 1]), valh, x, y);
+    const int s0 = __ldg(&d.wslot0[wg]), s1 = __ldg(&d.wslot0[wg + 1]);
+    Ahead p;
+    if constexpr (U == 0) p = load_ahead(d.scol, s0, s1);
+    row0_part<U>(d, s0, s1, valh, x, y, p);
     if (d.split) split_sum(y);
     if (!q0.valid || !d.xrow || d.xrow[i] == d.xrow[i + 1]) return;
     float e[3] = {0.f, 0.f, 0.f}, z[3];
@@ -1084,27 +1092,54 @@ __device__ __forceinline__ void row6_warp(const AmgLevel& L, int i, const float*
 // the extra blocks).  Lane 6 k + a (< 30) takes row a of blocks k, k + 5, ...; the
 // columns of up to 30 blocks are loaded before the first is used, so a row costs
 // three dependent loads (range, columns, values) however long it is (two blocks
-// per lane at a time: 7.5 against 6.6 us per sweep of the 8,978-node level).
-__device__ __forceinline__ float row6_warp_h(const AmgLevel& L, int p0, int p1, const float* __restrict__ x) {
+// per lane at a time: 7.5 against 6.6 us per sweep of the 8,978-node level); they
+// precede the wait for the kernel before (row6_load), which leaves x's.
+struct Row6 {  // what of a row does not change during a solve, loaded ahead
+    int p0, p1, j[6];
+    __half2 v[6][3];
+};
+__device__ __forceinline__ Row6 row6_load(const AmgLevel& L, int i) {
+    Row6 R;
+    const int lane = threadIdx.x & 31;
+    const int kb = lane / 6, a = lane - 6 * kb;
+    R.p0 = __ldg(&L.rowptr[i]);
+    R.p1 = __ldg(&L.rowptr[i + 1]);
+#pragma unroll
+    for (int u = 0; u < 6; ++u) {
+        const int p = R.p0 + kb + 5 * u;
+        R.j[u] = -1;
+        if (lane >= 30 || p >= R.p1) continue;
+        R.j[u] = __ldg(&L.colidx[p]);
+        const __half2* __restrict__ v = reinterpret_cast<const __half2*>(L.valh + 36 * (size_t)p + 6 * a);
+#pragma unroll
+        for (int b = 0; b < 3; ++b) R.v[u][b] = __ldg(&v[b]);
+    }
+    return R;
+}
+__device__ __forceinline__ float row6_warp_h(const AmgLevel& L, const Row6& R, const float* __restrict__ x) {
     const int lane = threadIdx.x & 31;
     const int kb = lane / 6, a = lane - 6 * kb;
     float acc = 0.f;
-    for (int pb = p0 + kb; pb - kb < p1; pb += 30) {
-        int j[6];
 #pragma unroll
-        for (int u = 0; u < 6; ++u) j[u] = (lane < 30 && pb + 5 * u < p1) ? __ldg(&L.colidx[pb + 5 * u]) : -1;
+    for (int u = 0; u < 6; ++u) {
+        if (R.j[u] < 0) continue;
+        const float2* __restrict__ xj = reinterpret_cast<const float2*>(x + 6 * (size_t)R.j[u]);
 #pragma unroll
-        for (int u = 0; u < 6; ++u) {
-            if (j[u] < 0) continue;
-            const __half2* __restrict__ v = reinterpret_cast<const __half2*>(L.valh + 36 * (size_t)(pb + 5 * u) + 6 * a);
-            const float2* __restrict__ xj = reinterpret_cast<const float2*>(x + 6 * (size_t)j[u]);
+        for (int b = 0; b < 3; ++b) {
+            const float2 f = __half22float2(R.v[u][b]), w = xj[b];
+            acc = fmaf(f.x, w.x, fmaf(f.y, w.y, acc));
+        }
+    }
+    if (lane < 30)
+        for (int p = R.p0 + kb + 30; p < R.p1; p += 5) {
+            const float2* __restrict__ xj = reinterpret_cast<const float2*>(x + 6 * (size_t)__ldg(&L.colidx[p]));
+            const __half2* __restrict__ v = reinterpret_cast<const __half2*>(L.valh + 36 * (size_t)p + 6 * a);
 #pragma unroll
             for (int b = 0; b < 3; ++b) {
                 const float2 f = __half22float2(__ldg(&v[b])), w = xj[b];
                 acc = fmaf(f.x, w.x, fmaf(f.y, w.y, acc));
             }
         }
-    }
     float y = acc;
 #pragma unroll
     for (int g = 1; g < 5; ++g) y += __shfl_down_sync(0xffffffffu, acc, 6 * g);
@@ -1672,10 +1707,11 @@ __global__ void __launch_bounds__(kRestrictThreads) k_restrict(const int* __rest
                                                                const double* __restrict__ scal,
                                                                const double* __restrict__ omegaC, float presmooth) {
     __shared__ float sm[kRestrictThreads / 32][6];
-    pdl_enter();
     const int I = blockIdx.x;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int q0 = __ldg(&cptr[I]), np = BS * (__ldg(&cptr[I + 1]) - q0);
+    pdl_enter();
+    pdl_next();
     if (level_stopped(C, scal, I)) return;
     float rc[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll 4
@@ -1730,12 +1766,10 @@ __global__ void k_q_smooth(V0 a, const float* __restrict__ z, float* __restrict_
 
 // (Q e)_i added to x: the warp's slots s0 .. s1
 __device__ __forceinline__ void row_q(const AmgQ& Q, int s0, int s1, const float* __restrict__ e, int nc, int* check,
-                                      float (&x)[3]) {
+                                      float (&x)[3], const Ahead* p) {
     const int lane = threadIdx.x & 31;
-#pragma unroll 4
-    for (int s = s0; s < s1; ++s) {
-        const int J = __ldg(&Q.col[32 * (size_t)s + lane]);
-        if (!TF_IN(check, J, nc, CK_PROLONG_COL)) continue;
+    auto slot = [&](int s, int J) {
+        if (!TF_IN(check, J, nc, CK_PROLONG_COL)) return;
         const uint4 a = __ldg(&Q.v16[64 * (size_t)s + lane]), b = __ldg(&Q.v16[64 * (size_t)s + 32 + lane]);
         const uint32_t c = __ldg(&Q.v2[32 * (size_t)s + lane]);
         const float2* __restrict__ ej = reinterpret_cast<const float2*>(e + 6 * (size_t)J);
@@ -1749,7 +1783,13 @@ __device__ __forceinline__ void row_q(const AmgQ& Q, int s0, int s1, const float
             x[k] = fmaf(f0.x, e0.x, fmaf(f0.y, e0.y, fmaf(f1.x, e1.x, fmaf(f1.y, e1.y,
                    fmaf(f2.x, e2.x, fmaf(f2.y, e2.y, x[k]))))));
         }
-    }
+    };
+    if (p)
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u)
+            if (p->j[u] >= 0) slot(s0 + u, p->j[u]);
+#pragma unroll 4
+    for (int s = p ? s0 + kAhead : s0; s < s1; ++s) slot(s, __ldg(&Q.col[32 * (size_t)s + lane]));
 }
 
 // out = x + Q e, x = 2 z - omega S z read from k_q_smooth (SMOOTH: formed here
@@ -1758,22 +1798,29 @@ __device__ __forceinline__ void row_q(const AmgQ& Q, int s0, int s1, const float
 template <int U, bool SMOOTH, bool DOT>
 __global__ void k_q_post(V0 a, Ctx c, AmgQ Q, int nc, const float* __restrict__ zx, const float* __restrict__ e,
                          double* __restrict__ out, const double* __restrict__ r, double* __restrict__ p, int start) {
-    pdl_enter();
+    // before the wait: what does not change during a solve
     const Node0 q = node0(a.d);
-    const double flag = __ldcg(&a.d.scal[(size_t)q.seg * S_COUNT + S_FLAG]);
     const int wg = blockIdx.x * kWarps + (threadIdx.x >> 5);
     const int q0 = __ldg(&Q.slot0[wg]), q1 = __ldg(&Q.slot0[wg + 1]);
-    if (flag != 0.0) return;
+    const float om = SMOOTH ? (float)__ldg(a.omega) : 0.f;
+    int s0 = 0, s1 = 0;
+    Ahead ps, pq;
+    if constexpr (SMOOTH) {
+        s0 = __ldg(&a.d.wslot0[wg]);
+        s1 = __ldg(&a.d.wslot0[wg + 1]);
+        if constexpr (U == 0) ps = load_ahead(a.d.scol, s0, s1);
+    }
+    if constexpr (U == 0) pq = load_ahead(Q.col, q0, q1);
+    pdl_enter();
+    if (__ldcg(&a.d.scal[(size_t)q.seg * S_COUNT + S_FLAG]) != 0.0) return;
     float x[3] = {0.f, 0.f, 0.f}, own[3];
     double ri[3];
-    float om = 0.f;
     if constexpr (SMOOTH) {
-        row0_part<U>(a.d, __ldg(&a.d.wslot0[wg]), __ldg(&a.d.wslot0[wg + 1]), a.valh, zx, x);
-        om = (float)__ldg(a.omega);
+        row0_part<U>(a.d, s0, s1, a.valh, zx, x, ps);
 #pragma unroll
         for (int k = 0; k < 3; ++k) x[k] *= -om;
     }
-    row_q(Q, q0, q1, e, nc, a.d.check, x);
+    row_q(Q, q0, q1, e, nc, a.d.check, x, U == 0 ? &pq : nullptr);
     if (q.valid)
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
@@ -1873,71 +1920,78 @@ __global__ void k_v0_prolong(V0 a, AmgLevel F, const float* __restrict__ e, floa
     }
 }
 
-// out_i = x_i + weight omega D_i^-1 (r - A x)_i for row i, by one warp
-__device__ __forceinline__ void post_row(const AmgLevel& L, const double* __restrict__ omega, float weight,
-                                         const float* __restrict__ x, float* __restrict__ out, int i,
-                                         const double* __restrict__ scal) {
-    // x + omega (D^-1 (r - X x) - S x), S = D^-1 A in FP16, X the extra blocks
-    const int lane = threadIdx.x & 31;
-    const int p0 = __ldg(&L.rowptr[i]), p1 = __ldg(&L.rowptr[i + 1]);
+// t = r - A x with A x = D (S x) + X x  (one warp per row, lane k < 6 writing component k)
+__global__ void k_v6_resid(AmgLevel L, const double* __restrict__ scal, const float* __restrict__ x) {
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    Row6 R;
+    float D[6];
+    if (i < L.n) {
+        R = row6_load(L, i);
+        const float* __restrict__ Dg = L.val + 36 * (size_t)__ldg(&L.diag[i]) + 6 * min(lane, 5);
+#pragma unroll
+        for (int k = 0; k < 6; ++k) D[k] = __ldg(&Dg[k]);
+    }
+    pdl_enter();
+    pdl_next();
+    if (i >= L.n || level_stopped(L, scal, i)) return;
+    const float s = row6_warp_h(L, R, x);
+    float y[6], e[6];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) y[k] = __shfl_sync(0xffffffffu, s, k);
+    extra6(L, i, x, e);
+    if (lane >= 6) return;
+    float t = 0.f;
+#pragma unroll
+    for (int k = 0; k < 6; ++k) t = fmaf(D[k], y[k], t);
+    L.t[6 * i + lane] = L.r[6 * i + lane] - t - pick6(e, lane);
+}
+
+// out = x + weight omega D^-1 (r - A x) = x + weight omega (D^-1 (r - X x) - S x),
+// S = D^-1 A in FP16, X the extra blocks  (one warp per row)
+__global__ void k_v6_post(AmgLevel L, const double* __restrict__ scal, const double* __restrict__ omega, float weight,
+                          const float* __restrict__ x, float* __restrict__ out) {
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    Row6 R;
+    float D[6], om = 0.f;
+    if (i < L.n) {
+        R = row6_load(L, i);
+        const float* __restrict__ Dg = L.dinv + 36 * (size_t)i + 6 * min(lane, 5);
+#pragma unroll
+        for (int k = 0; k < 6; ++k) D[k] = __ldg(&Dg[k]);
+        om = weight * (float)__ldg(omega);
+    }
+    pdl_enter();
+    pdl_next();
+    if (i >= L.n) return;
     float rr[6];
 #pragma unroll
     for (int k = 0; k < 6; ++k) rr[k] = L.r[6 * i + k];
     if (level_stopped(L, scal, i)) return;
-    const float y = row6_warp_h(L, p0, p1, x);
+    const float y = row6_warp_h(L, R, x);
     if (L.xrow) {
         float e[6];
         extra6(L, i, x, e);
 #pragma unroll
         for (int k = 0; k < 6; ++k) rr[k] -= e[k];
     }
-    if (lane < 6)
-        out[6 * i + lane] =
-            fmaf(weight * (float)__ldg(omega), lane_mul6(L.dinv + 36 * (size_t)i, rr, lane) - y, x[6 * i + lane]);
-}
-
-// t_i = r_i - (A x)_i with A x = D (S x) + X x, lane k < 6 writing component k
-__device__ __forceinline__ void resid_row(const AmgLevel& L, const float* __restrict__ x, int i,
-                                          const double* __restrict__ scal) {
-    const int lane = threadIdx.x & 31;
-    const int p0 = __ldg(&L.rowptr[i]), p1 = __ldg(&L.rowptr[i + 1]), dg = __ldg(&L.diag[i]);
-    if (level_stopped(L, scal, i)) return;
-    const float s = row6_warp_h(L, p0, p1, x);
-    float y[6], e[6];
+    if (lane >= 6) return;
+    float z = 0.f;
 #pragma unroll
-    for (int k = 0; k < 6; ++k) y[k] = __shfl_sync(0xffffffffu, s, k);
-    extra6(L, i, x, e);
-    if (lane < 6)
-        L.t[6 * i + lane] = L.r[6 * i + lane] - lane_mul6(L.val + 36 * (size_t)dg, y, lane) - pick6(e, lane);
-}
-
-// t = r - A x  (one warp per row)
-__global__ void k_v6_resid(AmgLevel L, const double* __restrict__ scal, const float* __restrict__ x) {
-    pdl_enter();
-    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (i >= L.n) return;
-    resid_row(L, x, i, scal);
-}
-
-// out = x + weight omega D^-1 (r - A x)  (one warp per row)
-__global__ void k_v6_post(AmgLevel L, const double* __restrict__ scal, const double* __restrict__ omega, float weight,
-                          const float* __restrict__ x, float* __restrict__ out) {
-    pdl_enter();
-    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (i >= L.n) return;
-    post_row(L, omega, weight, x, out, i, scal);
+    for (int k = 0; k < 6; ++k) z = fmaf(D[k], rr[k], z);
+    out[6 * i + lane] = fmaf(om, z - y, x[6 * i + lane]);
 }
 
 // x_i += sum over the prolongator blocks (i, J) of P_iJ e_J (6-DOF fine level),
 // one thread per DOF (one per node: 7.8 against 5.5 us to 8,978 nodes)
 __global__ void k_v6_prolong(AmgLevel F, const double* __restrict__ scal, const float* __restrict__ e, float* x) {
-    pdl_enter();
     const int q = blockIdx.x * blockDim.x + threadIdx.x, i = q / 6, k = q - 6 * i;
+    const int b0 = i < F.n ? __ldg(&F.prow[i]) : 0, b1 = i < F.n ? __ldg(&F.prow[i + 1]) : 0;
+    pdl_enter();
+    pdl_next();
     if (i >= F.n || level_stopped(F, scal, i)) return;
     float s = x[q];
-    const int b1 = __ldg(&F.prow[i + 1]);
 #pragma unroll 4
-    for (int b = __ldg(&F.prow[i]); b < b1; ++b) {
+    for (int b = b0; b < b1; ++b) {
         const int J = __ldg(&F.pcol[b]);
         if (!TF_IN(F.check, J, F.ncoarse, CK_PROLONG_COL)) continue;
         const float2* __restrict__ P = reinterpret_cast<const float2*>(F.Pv + 36 * (size_t)b + 6 * k);
@@ -1970,22 +2024,32 @@ __host__ __device__ __forceinline__ float* post_sweep_out(const AmgLevel& L, con
 // levels below.
 __global__ void k_dense(AmgLevel L, const double* __restrict__ scal, const int* __restrict__ doff,
                         const float* __restrict__ mat) {
-    pdl_enter();
     const int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;  // row over all instances
-    if (k >= 6 * L.n) return;
-    const int g = L.single ? 0 : L.seg[k / 6];
-    if (seg_stopped(scal, g)) return;
+    const int g = L.single || k >= 6 * L.n ? 0 : L.seg[k / 6];
     const int lane = threadIdx.x & 31;
     const int k0 = L.single ? 0 : 6 * L.seg0[g];
     const int m2 = L.single ? 3 * L.n : 3 * (L.seg0[g + 1] - L.seg0[g]);  // pairs of a row (m is even)
     const float2* __restrict__ M =
         reinterpret_cast<const float2*>(mat + (L.single ? 0 : doff[g]) + (size_t)(k - k0) * (2 * m2));
+    float2 a[8];  // before the wait: the operator's first entries
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+        a[u] = k < 6 * L.n && lane + 32 * u < m2 ? __ldg(&M[lane + 32 * u]) : make_float2(0.f, 0.f);
+    pdl_enter();
+    pdl_next();
+    if (k >= 6 * L.n || seg_stopped(scal, g)) return;
     const float2* __restrict__ r = reinterpret_cast<const float2*>(L.r + k0);
     float s = 0.f;
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+        if (lane + 32 * u < m2) {
+            const float2 b = r[lane + 32 * u];
+            s = fmaf(a[u].x, b.x, fmaf(a[u].y, b.y, s));
+        }
 #pragma unroll 8
-    for (int q = lane; q < m2; q += 32) {
-        const float2 a = __ldg(&M[q]), b = r[q];
-        s = fmaf(a.x, b.x, fmaf(a.y, b.y, s));
+    for (int q = lane + 256; q < m2; q += 32) {
+        const float2 f = __ldg(&M[q]), b = r[q];
+        s = fmaf(f.x, b.x, fmaf(f.y, b.y, s));
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
@@ -2489,7 +2553,8 @@ void amg_vcycle(tf_handle* h, const double* r, double* out, int dot, double* p) 
         if (fork) {
             cudaEventRecord(h->fork_ev, st);
             cudaStreamWaitEvent(h->side_stream, h->fork_ev, 0);
-            switch (a->smooth_unroll) {
+            switch (d.split ? 0 : a->smooth_unroll) {
+                case 0: launch_q_smooth<0>(h, h->side_stream, v0, L0.x, a->x1); break;
                 case 2: launch_q_smooth<2>(h, h->side_stream, v0, L0.x, a->x1); break;
                 case 8: launch_q_smooth<8>(h, h->side_stream, v0, L0.x, a->x1); break;
                 default: launch_q_smooth<4>(h, h->side_stream, v0, L0.x, a->x1); break;
@@ -2556,9 +2621,11 @@ void amg_vcycle(tf_handle* h, const double* r, double* out, int dot, double* p) 
     if (q) {
         if (fork) {
             cudaStreamWaitEvent(st, h->join_ev, 0);
-            launch_q_post<4, false>(h, v0, a->x1, out, r, p, dot);
+            if (d.split) launch_q_post<0, false>(h, v0, a->x1, out, r, p, dot);
+            else launch_q_post<4, false>(h, v0, a->x1, out, r, p, dot);
         } else {
-            switch (a->smooth_unroll) {
+            switch (d.split ? 0 : a->smooth_unroll) {
+                case 0: launch_q_post<0, true>(h, v0, L0.x, out, r, p, dot); break;
                 case 2: launch_q_post<2, true>(h, v0, L0.x, out, r, p, dot); break;
                 case 8: launch_q_post<8, true>(h, v0, L0.x, out, r, p, dot); break;
                 default: launch_q_post<4, true>(h, v0, L0.x, out, r, p, dot); break;

@@ -331,12 +331,19 @@ __device__ double reference_box_max(int nn, const double* __restrict__ pos, int 
 // Programmatic dependent launch for the chains of short kernels of the
 // linear solve: a kernel launched with launch_pdl may be scheduled as its
 // predecessor's blocks exit, hiding the launch gap; pdl_enter makes it wait
-// for the predecessor's completion (and memory) before anything else.  (An
-// explicit early trigger, letting the next kernel's blocks sit resident
-// while the current one runs, measured 10 % slower on the 320,000-prism
-// step; this form measured ~3 % faster than plain launches.)  A no-op for
+// for the predecessor's completion (and memory).  Before it a kernel may load what
+// does not change during a solve (patterns, matrices, weights: their writers
+// precede the solve's first, ordinary launch), nothing else.  A no-op for
 // ordinary launches.
+// pdl_next lets the next kernel's blocks start while this one still runs: for
+// the coarse levels' kernels, which leave the chip room, so that the next one's
+// indices and matrix rows are in registers when its vector is ready (step of
+// 46,208 prisms 6.0 -> 5.3 ms, 320,000 20.3 -> 19.7, 1M-prism wing 46.1 -> 45.0).
+// In the kernels that fill the chip it costs: 10 % on the 320,000-prism step; in
+// the split kernels of small meshes 5.3 -> 5.5 ms at 46,208 prisms.
 __device__ __forceinline__ void pdl_enter() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+__device__ __forceinline__ void pdl_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 template <typename... KArgs, typename... Args>
 inline void launch_pdl_smem(void (*kernel)(KArgs...), int grid, int block, size_t smem, cudaStream_t st,
@@ -366,16 +373,40 @@ inline void launch_pdl(void (*kernel)(KArgs...), int grid, int block, cudaStream
 // node cta_node0[blockIdx.x] + lane, the warp's share of the row); the warp walks
 // its slots s0 .. s1 together, each lane reading its own row's block, so every
 // load of a block entry or column is one coalesced access.
+// U = 0 (split CTAs): the columns of the first slots come loaded (Ahead).
+constexpr int kAhead = 4;
+struct Ahead {
+    int j[kAhead];  // -1: no such slot
+};
+__device__ __forceinline__ Ahead load_ahead(const int* __restrict__ scol, int s0, int s1) {
+    Ahead p;
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u)
+        p.j[u] = s0 + u < s1 ? __ldg(&scol[(size_t)(s0 + u) * kSlice + (threadIdx.x & 31)]) : -1;
+    return p;
+}
 template <class T, int U = 2>
 __device__ __forceinline__ void sliced_row(int s0, int s1, const int* __restrict__ scol, const T* __restrict__ val,
-                                           const double* __restrict__ x, double y[3], int nn = 0,
-                                           int* check = nullptr) {
+                                           const double* __restrict__ x, double y[3], int nn, int* check,
+                                           const Ahead& p) {
     const int lane = threadIdx.x & 31;
     double y0 = 0.0, y1 = 0.0, y2 = 0.0;
     const int* __restrict__ col = scol + lane;
     const T* __restrict__ a = val + lane;
-#pragma unroll U
-    for (int s = s0; s < s1; ++s) {
+    if constexpr (U == 0) {
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+            const int j = p.j[u];
+            if (j < 0 || !TF_IN(check, j, nn, CK_SPMV_COL)) continue;
+            const T* __restrict__ v = a + (size_t)(s0 + u) * kSlotDoubles;
+            const double x0 = x[3 * j], x1 = x[3 * j + 1], x2 = x[3 * j + 2];
+            y0 = fma((double)__ldg(&v[0]), x0, fma((double)__ldg(&v[32]), x1, fma((double)__ldg(&v[64]), x2, y0)));
+            y1 = fma((double)__ldg(&v[96]), x0, fma((double)__ldg(&v[128]), x1, fma((double)__ldg(&v[160]), x2, y1)));
+            y2 = fma((double)__ldg(&v[192]), x0, fma((double)__ldg(&v[224]), x1, fma((double)__ldg(&v[256]), x2, y2)));
+        }
+    }
+#pragma unroll (U == 0 ? 1 : U)
+    for (int s = U == 0 ? s0 + kAhead : s0; s < s1; ++s) {
         const int j = __ldg(&col[(size_t)s * kSlice]);
         if (!TF_IN(check, j, nn, CK_SPMV_COL)) continue;
         const T* __restrict__ v = a + (size_t)s * kSlotDoubles;

@@ -42,14 +42,21 @@ __device__ __forceinline__ void apply_dinv(const double* __restrict__ D, const d
 // (a warp has a handful of slots).
 struct Slots {
     int s0, s1;
+    Ahead p;  // U = 0
 };
+template <int U = 2>
 __device__ __forceinline__ Slots warp_slots(const Ctx& c) {
+    Slots s;
     const int wg = blockIdx.x * kWarps + (threadIdx.x >> 5);
-    return Slots{__ldg(&c.wslot0[wg]), __ldg(&c.wslot0[wg + 1])};
+    s.s0 = __ldg(&c.wslot0[wg]);
+    s.s1 = __ldg(&c.wslot0[wg + 1]);
+    if constexpr (U == 0) s.p = load_ahead(c.scol, s.s0, s.s1);
+    return s;
 }
 template <int U = 2>
-__device__ __forceinline__ void rows_product(const Ctx& c, Slots s, const double* __restrict__ x, double (&y)[3]) {
-    sliced_row<double, U == 0 ? 2 : U>(s.s0, s.s1, c.scol, c.val, x, y, c.nn, c.check);
+__device__ __forceinline__ void rows_product(const Ctx& c, const Slots& s, const double* __restrict__ x,
+                                             double (&y)[3]) {
+    sliced_row<double, U>(s.s0, s.s1, c.scol, c.val, x, y, c.nn, c.check, s.p);
 }
 template <int MODE = kEither>
 __device__ __forceinline__ void rows_sum(const Ctx& c, const Where& w, const double* __restrict__ x, double (&y)[3]) {
@@ -174,9 +181,9 @@ __global__ void k_cg_init(Ctx c, const double* __restrict__ b, double* __restric
 template <int U>
 __global__ void __launch_bounds__(kThreads, U == 0 ? 4 : 6)
     k_cg_spmv(Ctx c, const double* __restrict__ p, double* __restrict__ q) {
+    const Slots sl = warp_slots<U>(c);  // before the wait: they do not change during a solve
     pdl_enter();
     const Where w = where(c);
-    const Slots sl = warp_slots(c);
     if (stopped(w)) return;
     double v[1] = {0.0}, y[3], pi[3];
     rows_product<U>(c, sl, p, y);
@@ -373,9 +380,9 @@ template <int U>
 __global__ void __launch_bounds__(kThreads, U == 0 ? 4 : 6)
     k_bi_spmv1(Ctx c, const double* __restrict__ phat, const double* __restrict__ rhat,
                            double* __restrict__ v) {
+    const Slots sl = warp_slots<U>(c);  // before the wait: they do not change during a solve
     pdl_enter();
     const Where w = where(c);
-    const Slots sl = warp_slots(c);
     if (stopped(w)) return;
     double s[1] = {0.0}, y[3], rh[3];
     rows_product<U>(c, sl, phat, y);
@@ -451,9 +458,9 @@ template <int U>
 __global__ void __launch_bounds__(kThreads, U == 0 ? 4 : 6)
     k_bi_spmv2(Ctx c, const double* __restrict__ shat, const double* __restrict__ s,
                            double* __restrict__ t, double* __restrict__ x, const double* __restrict__ phat) {
+    const Slots sl = warp_slots<U>(c);  // before the wait: they do not change during a solve
     pdl_enter();
     const Where w = where(c);
-    const Slots sl = warp_slots(c);
     if (w.flag == -1.0) {
         const double alpha = __ldcg(&w.s[S_ALPHA]);
         if (w.valid)
