@@ -358,13 +358,14 @@ TF_API tf_status tf_measure_bandwidth(int32_t device, int64_t bytes, int32_t rep
  * device with block-Jacobi preconditioned BiCGStab in FP64; every pointer is
  * a device pointer the caller owns (rowptr[n+1], colidx[nnzb], val[9*nnzb]
  * row-major blocks, b and x [3n]).  Work space is one static device array of
- * this library (about 4.3 MB, held by every GPU that loads it until exit),
+ * this library (about 4.6 MB, held by every GPU that loads it until exit),
  * so n_block_rows is limited to 16384; larger systems return TF_BAD_INPUT.
  * The first call on a device (and the first after its context changes, e.g.
  * after cudaDeviceReset) looks the array up.  Every call synchronises
  * `stream` and reads scalars back, so it must never be made on a stream that
  * is being captured: it then returns TF_BAD_INPUT.  Calls share the array:
- * overlapping calls race, so serialise them.  `stream` is a cudaStream_t
+ * overlapping calls race, so serialise them (thread blocks that lose each other
+ * that way give up after some seconds and the call returns TF_CUDA_ERROR).  `stream` is a cudaStream_t
  * (NULL: the default stream). */
 TF_API tf_status tf_solve_bsr_static(int32_t n_block_rows, const int32_t* rowptr, const int32_t* colidx,
                                      const double* val, const double* b, double* x, double rtol, int32_t max_iter,

@@ -226,3 +226,48 @@ def test_split_rows_of_a_ragged_batch():
     for precond in (1, 2):
         with api.Batch(ts, precond=precond, krylov_rtol=RTOL) as s:
             _solve(s, ts)
+
+
+# tf_solve_bsr_static, one kernel over all SMs: one row, one group of 32 rows and
+# one more, a group more per block (4,865 = 152 x 32 + 1), the largest system, and
+# rows of up to 120 blocks (more than shared memory holds).  Ragged unsymmetric
+# systems with dominant diagonal blocks; rows 5, 10, .. have a diagonal block only.
+@pytest.mark.parametrize("n,most", [(1, 1), (32, 5), (33, 9), (2000, 30), (4865, 27), (9000, 120), (16384, 27)])
+def test_static_solve_of_ragged_systems(n, most):
+    import ctypes as C
+
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(n)
+    cnt = rng.integers(0, most, size=n)
+    cnt[5::5] = 0
+    rows = np.repeat(np.arange(n), cnt)
+    key = np.unique(np.concatenate([rows * n + rng.integers(0, n, size=rows.size), np.arange(n) * n + np.arange(n)]))
+    br, bc = key // n, key % n
+    val = rng.uniform(-1.0, 1.0, size=(key.size, 3, 3))
+    val[br == bc] += 4.0 * most * np.eye(3)
+    rowptr = np.searchsorted(br, np.arange(n + 1)).astype(np.int32)
+    b = rng.uniform(-1.0, 1.0, size=3 * n)
+    d = {k: torch.from_numpy(np.ascontiguousarray(v)).cuda()
+         for k, v in dict(rowptr=rowptr, col=bc.astype(np.int32), val=val.reshape(-1), b=b).items()}
+    x = torch.full((3 * n,), float("nan"), dtype=torch.float64, device="cuda")
+    it, rr = C.c_int32(0), C.c_double(0.0)
+    p = lambda a: C.c_void_p(a.data_ptr())  # noqa: E731
+    st = api.load().tf_solve_bsr_static(n, p(d["rowptr"]), p(d["col"]), p(d["val"]), p(d["b"]), p(x), RTOL, 500, None,
+                                        C.byref(it), C.byref(rr))
+    assert st == api.TF_OK, api.load().tf_last_error().decode()
+    assert rr.value <= RTOL
+    xs = x.cpu().numpy().reshape(n, 3)
+    prod = np.einsum("kij,kj->ki", val, xs[bc])
+    Ax, mag = np.zeros((n, 3)), np.zeros((n, 3))
+    np.add.at(Ax, br, prod)
+    np.add.at(mag, br, np.einsum("kij,kj->ki", np.abs(val), np.abs(xs[bc])))
+    nb = np.linalg.norm(b)
+    bound = RTOL + 4 * EPS * it.value * np.linalg.norm(mag) / nb
+    assert np.linalg.norm(b - Ax.reshape(-1)) <= bound * nb
+    # a cap is kept, and the second call does not see the first one's state
+    st = api.load().tf_solve_bsr_static(n, p(d["rowptr"]), p(d["col"]), p(d["val"]), p(d["b"]), p(x), 1e-300, 1, None,
+                                        C.byref(it), C.byref(rr))
+    assert it.value <= 1
+    st = api.load().tf_solve_bsr_static(n, p(d["rowptr"]), p(d["col"]), p(d["val"]), p(d["b"]), p(x), RTOL, 500, None,
+                                        C.byref(it), C.byref(rr))
+    assert st == api.TF_OK and np.array_equal(x.cpu().numpy().reshape(n, 3), xs)  # fixed order of sums

@@ -366,6 +366,23 @@ inline void launch_pdl(void (*kernel)(KArgs...), int grid, int block, cudaStream
     launch_pdl_smem(kernel, grid, block, 0, st, args...);
 }
 
+// All CTAs resident at once (they meet at a grid barrier).
+template <typename... KArgs, typename... Args>
+inline void launch_cooperative(void (*kernel)(KArgs...), int grid, int block, size_t smem, cudaStream_t st,
+                               Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
 // y = this thread's row of the sliced block matrix times x.  T is the
 // storage type of the values (double for the Krylov operator, float for the
 // copy the multigrid smoother reads); products and sums are FP64.  The thread is

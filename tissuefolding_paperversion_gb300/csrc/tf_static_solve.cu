@@ -6,22 +6,23 @@
 // routine.  Its work vectors, reduction partials and scalars live in one
 // file-scope device array, g_static_scratch, sized for at most
 // kStaticMaxNodes block rows.  Every GPU that loads this library holds that
-// array (about 4.3 MB) until the process exits.
+// array (about 4.6 MB) until the process exits.
 //
 // Host code cannot use the array's name as a device address, so the first
 // call on each device looks the address up with cudaGetSymbolAddress while
 // that device is current, and caches it together with the CUDA context it
 // came from; a call in another context (after cudaDeviceReset, say) looks it
 // up again.  Every call synchronises its stream and reads scalars back to the
-// host between chunks of iterations, so no call may be made on a stream that
-// is being captured: such a call returns TF_BAD_INPUT and leaves the capture
-// untouched.  All calls on a device share the one array: calls that
-// overlap on the GPU (two streams, two host threads) race on it and give
-// wrong results, so serialise them.  Each call clears the reduction ticket
-// and the scalars it reads before its first kernel, and writes every work
-// vector before reading it, so nothing carries over from the previous call.
+// host, so no call may be made on a stream that is being captured: such a call
+// returns TF_BAD_INPUT and leaves the capture untouched.  All calls on a device
+// share the one array: calls that overlap on the GPU (two streams, two host
+// threads) race on it and give wrong results or an error, so serialise them.
+// Each call clears the scalars and the count of the CTAs' meetings before its
+// kernel, and writes every work vector before reading it, so nothing carries
+// over from the previous call.
 #include <cuda.h>
 
+#include <algorithm>
 #include <mutex>
 
 #include "tf_internal.cuh"
@@ -30,80 +31,180 @@ namespace tf {
 namespace {
 
 constexpr int kStaticMaxNodes = 16384;
-constexpr int kStaticThreads = 256;
-constexpr int kStaticMaxGrid = (kStaticMaxNodes + kStaticThreads - 1) / kStaticThreads;
-constexpr int kNumVec = 8;                    // r, rhat, p, phat, v, s, shat, t
-constexpr size_t kVecLen = 3 * (size_t)kStaticMaxNodes;
-constexpr size_t kOffDinv = kNumVec * kVecLen;            // 9 doubles per node
-constexpr size_t kOffPart = kOffDinv + 9 * (size_t)kStaticMaxNodes;
-constexpr size_t kOffScal = kOffPart + 2 * (size_t)kStaticMaxGrid;
+constexpr int kStaticThreads = 512;
+constexpr int kStaticWarps = kStaticThreads / 32;
+constexpr int kStaticMaxGrid = kStaticMaxNodes / 32;
+constexpr size_t kVecLen = 4 * (size_t)kStaticMaxNodes;  // a row's three entries in one 32-byte load
+// phat and shat, which all CTAs read; then 27 doubles per row that only the
+// row's CTA uses (its vectors and inverse diagonal block), where they do not
+// fit its shared memory
+constexpr size_t kOffLocal = 2 * kVecLen;
+constexpr int kLocal = 27;
+constexpr size_t kOffPart = kOffLocal + kLocal * (size_t)kStaticMaxNodes;
+constexpr int kMaxSums = 2;
+constexpr int kNumSums = 4;                   // reductions of an iteration and the start
+constexpr size_t kOffScal = kOffPart + kNumSums * kMaxSums * (size_t)kStaticMaxGrid;
 constexpr size_t kNumScal = 16;
-constexpr size_t kOffTicket = kOffScal + kNumScal;
-constexpr size_t kScratchDoubles = kOffTicket + 2;
+constexpr size_t kOffBar = kOffScal + kNumScal;
+constexpr size_t kScratchDoubles = kOffBar + 2;
+constexpr int kStaticSmem = 200 * 1024;
+constexpr int kStaticPolls = 1 << 22;         // a wait for the other CTAs gives up after some seconds
 
 __device__ __align__(256) double g_static_scratch[kScratchDoubles];
 
-enum { Q_RHO = 0, Q_ALPHA, Q_OMEGA, Q_BETA, Q_BB, Q_RR, Q_ITER, Q_FLAG, Q_TOL2 };
-enum { QF_RUNNING = 0, QF_CONVERGED = 1, QF_BREAKDOWN = 2, QF_NAN = 3 };
+enum { Q_BB = 0, Q_RR, Q_ITER, Q_FLAG };
+enum { QF_RUNNING = 0, QF_CONVERGED = 1, QF_BREAKDOWN = 2, QF_NAN = 3, QF_STUCK = 4 };
 
 struct SCtx {
     int n;
+    int rows;  // per CTA
+    int max_iter;
+    double tol2;
     const int* __restrict__ rowptr;
     const int* __restrict__ colidx;
     const double* __restrict__ val;
     double* base;  // device address of g_static_scratch
-    __device__ double* vec(int k) const { return base + k * kVecLen; }
-    __device__ double* dinv() const { return base + kOffDinv; }
-    __device__ double* part() const { return base + kOffPart; }
+    __device__ double* phat() const { return base; }
+    __device__ double* shat() const { return base + kVecLen; }
+    __device__ double* part(int k) const { return base + kOffPart + k * kMaxSums * (size_t)kStaticMaxGrid; }
     __device__ double* q() const { return base + kOffScal; }
-    __device__ unsigned* ticket() const { return reinterpret_cast<unsigned*>(base + kOffTicket); }
+    __device__ unsigned* bar() const { return reinterpret_cast<unsigned*>(base + kOffBar); }
 };
 
-template <int NV>
-__device__ bool s_reduce(const SCtx& c, double (&v)[NV], double (&tot)[NV]) {
-    __shared__ double sm[NV][kStaticThreads / 32 + 1];
-    __shared__ bool last;
-    double x[NV];
-#pragma unroll
-    for (int k = 0; k < NV; ++k) x[k] = v[k];
-    cta_sum<kStaticThreads, NV>(x, sm);
+struct SShared {
+    double sums[kMaxSums][kStaticWarps];
+    double rho, rr, bb, alpha, omega, beta;  // the recurrence's scalars
+    int it, flag;
+    double y[kStaticWarps][3][32];
+    int stuck;
+};
+
+// All CTAs meet (they are resident together: a cooperative launch).  False when
+// the wait ran out.
+__device__ __forceinline__ bool s_barrier(const SCtx& c, SShared& sh, unsigned& goal) {
+    goal += gridDim.x;
+    __syncthreads();
     if (threadIdx.x == 0) {
-        for (int k = 0; k < NV; ++k) c.part()[k * gridDim.x + blockIdx.x] = x[k];
-        __threadfence();
-        last = atomicAdd(c.ticket(), 1u) == gridDim.x - 1;
+        unsigned* bar = c.bar();
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
+        unsigned seen;
+        int polls = 0;
+        do {
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(bar) : "memory");
+        } while (seen < goal && ++polls < kStaticPolls);
+        if (seen < goal) sh.stuck = 1;
     }
     __syncthreads();
-    if (!last) return false;
-    __threadfence();
-    // all threads of the last CTA fold the partials (fixed order)
+    return !sh.stuck;
+}
+
+// Sums over all CTAs in a fixed order; thread 0 of every CTA then takes them to
+// the next scalars (`then`), which all threads find in sh.  One thread: a
+// division by all 512 keeps the FP64 pipe busy for 3 us.  `slot`: where this warp's
+// values enter (-1: it has none), `slots`: how many warps have some.  It is a
+// meeting of the CTAs as well.  Reduction k of an iteration has its own partials:
+// they are rewritten an iteration later.
+template <int NV, class F>
+__device__ __forceinline__ bool s_reduce(const SCtx& c, SShared& sh, unsigned& goal, int k, int slot, int slots,
+                                         double (&v)[NV], F then) {
+    const int lane = threadIdx.x & 31;
+    if (slot >= 0) {
 #pragma unroll
-    for (int k = 0; k < NV; ++k) {
-        x[k] = 0.0;
-        for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) x[k] += __ldcg(&c.part()[k * gridDim.x + b]);
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int u = 0; u < NV; ++u) v[u] += __shfl_down_sync(0xffffffffu, v[u], o);
+        if (lane == 0)
+#pragma unroll
+            for (int u = 0; u < NV; ++u) sh.sums[u][slot] = v[u];
     }
-    cta_sum<kStaticThreads, NV>(x, sm);
-    if (threadIdx.x == 0) {
-        for (int k = 0; k < NV; ++k) tot[k] = x[k];
-        *c.ticket() = 0u;
+    __syncthreads();
+    if (threadIdx.x == 0)
+#pragma unroll
+        for (int u = 0; u < NV; ++u) {
+            double s = sh.sums[u][0];
+            for (int w = 1; w < slots; ++w) s += sh.sums[u][w];
+            c.part(k)[u * kStaticMaxGrid + blockIdx.x] = s;
+        }
+    if (!s_barrier(c, sh, goal)) return false;
+    if (threadIdx.x < 32) {
+        double s[NV];
+#pragma unroll
+        for (int u = 0; u < NV; ++u) {
+            s[u] = 0.0;
+#pragma unroll 8
+            for (int b = lane; b < (int)gridDim.x; b += 32) s[u] += __ldcg(&c.part(k)[u * kStaticMaxGrid + b]);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int u = 0; u < NV; ++u) s[u] += __shfl_down_sync(0xffffffffu, s[u], o);
+        if (lane == 0) then(s);
     }
+    __syncthreads();
     return true;
 }
 
-__device__ __forceinline__ bool s_stopped(const SCtx& c) { return __ldcg(&c.q()[Q_FLAG]) != 0.0; }
+// The rows of a CTA: its blocks, in shared memory as far as they fit; a group of
+// warps for 32 rows, each warp a share of every row's blocks.
+struct SRows {
+    int nr, groups, share;  // rows, groups of 32, warps per group
+    int row0;
+    const int* ptr;         // positions of the rows' blocks from the CTA's first (shared)
+    const int* col;
+    const double* val;
+    const double* staged;   // the first nstaged blocks, in shared memory
+    int nstaged;
+};
 
-__device__ __forceinline__ void s_row(const SCtx& c, int i, const double* __restrict__ x, double y[3]) {
+// The entries of a row of phat or shat, written by any CTA before the last meeting
+__device__ __forceinline__ void load_row(const double* x, double (&v)[3]) {
+    double pad;
+    asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(pad) : "l"(x) : "memory");
+}
+
+// y = A x for the rows of a group, summed over its warps, on the group's first
+// warp (returns true there; lane = row of the group).  Every thread calls it.
+__device__ __forceinline__ bool s_rows(const SRows& R, SShared& sh, int g, const double* x, double (&y)[3]) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int w = warp % R.share;
+    const int i = 32 * g + lane;
     double y0 = 0.0, y1 = 0.0, y2 = 0.0;
-    for (int b = c.rowptr[i]; b < c.rowptr[i + 1]; ++b) {
-        const int j = c.colidx[b];
-        const double* a = c.val + 9 * (size_t)b;
-        const double x0 = x[3 * j], x1 = x[3 * j + 1], x2 = x[3 * j + 2];
-        y0 = fma(a[0], x0, fma(a[1], x1, fma(a[2], x2, y0)));
-        y1 = fma(a[3], x0, fma(a[4], x1, fma(a[5], x2, y1)));
-        y2 = fma(a[6], x0, fma(a[7], x1, fma(a[8], x2, y2)));
+    if (g < R.groups && i < R.nr) {
+        const int p1 = R.ptr[i + 1];
+        for (int pb = R.ptr[i] + w; pb < p1; pb += 4 * R.share) {  // four blocks' columns, then their x, then the sums
+            const double* xj[4];
+            double v[4][3];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) xj[u] = pb + u * R.share < p1 ? x + 4 * (size_t)R.col[pb + u * R.share] : nullptr;
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (xj[u]) load_row(xj[u], v[u]);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                if (!xj[u]) continue;
+                const int p = pb + u * R.share;
+                const double* a = (p < R.nstaged ? R.staged : R.val) + 9 * (size_t)p;
+                y0 = fma(a[0], v[u][0], fma(a[1], v[u][1], fma(a[2], v[u][2], y0)));
+                y1 = fma(a[3], v[u][0], fma(a[4], v[u][1], fma(a[5], v[u][2], y1)));
+                y2 = fma(a[6], v[u][0], fma(a[7], v[u][1], fma(a[8], v[u][2], y2)));
+            }
+        }
     }
-    y[0] = y0;
-    y[1] = y1;
-    y[2] = y2;
+    sh.y[warp][0][lane] = y0;
+    sh.y[warp][1][lane] = y1;
+    sh.y[warp][2][lane] = y2;
+    __syncthreads();
+    // pairs of warps, then pairs of pairs: a chain of additions waits for each
+    for (int k = 1; k < R.share; k *= 2) {
+        if (g < R.groups && w % (2 * k) == 0 && w + k < R.share)
+#pragma unroll
+            for (int d = 0; d < 3; ++d) sh.y[warp][d][lane] += sh.y[warp + k][d][lane];
+        __syncthreads();
+    }
+    if (w != 0 || g >= R.groups) return false;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) y[d] = sh.y[warp][d][lane];
+    return i < R.nr;
 }
 
 __device__ __forceinline__ void s_prec(const double* D, const double r[3], double z[3]) {
@@ -112,160 +213,199 @@ __device__ __forceinline__ void s_prec(const double* D, const double r[3], doubl
     z[2] = fma(D[6], r[0], fma(D[7], r[1], D[8] * r[2]));
 }
 
-// inverse diagonal blocks; r = rhat = b; p = v = 0; x = 0; rho = (b, b)
-__global__ void ks_init(SCtx c, const double* __restrict__ b, double* __restrict__ x) {
-    const int i = blockIdx.x * kStaticThreads + threadIdx.x;
-    double acc[1] = {0.0};
-    if (i < c.n) {
-        const double* M = nullptr;
-        for (int p = c.rowptr[i]; p < c.rowptr[i + 1]; ++p)
-            if (c.colidx[p] == i) M = c.val + 9 * (size_t)p;
-        double inv[9] = {1, 0, 0, 0, 1, 0, 0, 0, 1};
-        if (M) {
-            const double c0 = M[4] * M[8] - M[5] * M[7], c1 = M[5] * M[6] - M[3] * M[8], c2 = M[3] * M[7] - M[4] * M[6];
-            const double det = M[0] * c0 + M[1] * c1 + M[2] * c2;
-            if (det != 0.0) {
-                const double r = 1.0 / det;
-                inv[0] = c0 * r;
-                inv[1] = (M[2] * M[7] - M[1] * M[8]) * r;
-                inv[2] = (M[1] * M[5] - M[2] * M[4]) * r;
-                inv[3] = c1 * r;
-                inv[4] = (M[0] * M[8] - M[2] * M[6]) * r;
-                inv[5] = (M[2] * M[3] - M[0] * M[5]) * r;
-                inv[6] = c2 * r;
-                inv[7] = (M[1] * M[6] - M[0] * M[7]) * r;
-                inv[8] = (M[0] * M[4] - M[1] * M[3]) * r;
+// Inverse of a block row's diagonal block (identity where it has none or it is singular)
+__device__ __forceinline__ void s_diag_inverse(const SCtx& c, int i, double* inv) {
+    const double* M = nullptr;
+    for (int p = c.rowptr[i]; p < c.rowptr[i + 1]; ++p)
+        if (c.colidx[p] == i) M = c.val + 9 * (size_t)p;
+    for (int k = 0; k < 9; ++k) inv[k] = k % 4 == 0 ? 1.0 : 0.0;
+    if (!M) return;
+    const double c0 = M[4] * M[8] - M[5] * M[7], c1 = M[5] * M[6] - M[3] * M[8], c2 = M[3] * M[7] - M[4] * M[6];
+    const double det = M[0] * c0 + M[1] * c1 + M[2] * c2;
+    if (det == 0.0) return;
+    const double r = 1.0 / det;
+    inv[0] = c0 * r;
+    inv[1] = (M[2] * M[7] - M[1] * M[8]) * r;
+    inv[2] = (M[1] * M[5] - M[2] * M[4]) * r;
+    inv[3] = c1 * r;
+    inv[4] = (M[0] * M[8] - M[2] * M[6]) * r;
+    inv[5] = (M[2] * M[3] - M[0] * M[5]) * r;
+    inv[6] = c2 * r;
+    inv[7] = (M[1] * M[6] - M[0] * M[7]) * r;
+    inv[8] = (M[0] * M[4] - M[1] * M[3]) * r;
+}
+
+// The whole solve: block-Jacobi BiCGStab over all CTAs, each with the rows
+// blockIdx.x * rows ...  Bound by the meetings of the CTAs (five an iteration, 1.4
+// us each, three of them with a sum) and the FP64 pipe (two products of 27 blocks
+// a row: 4 us each at 56 rows per SM, half the lanes of the last group idle).  As
+// five launches an iteration with a thread per row, 33 of them on 8,405 rows,
+// the products waited for memory: 70 us an iteration against 30 now (19.1 -> 8.3
+// ms to 1e-12; 105 rows 5.0 -> 1.5, 1,200 12.9 -> 4.4, 16,200 19.5 -> 9.8).  The
+// matrix stays in shared memory between the iterations: nothing is allocated.
+__global__ void __launch_bounds__(kStaticThreads, 1) ks_solve(SCtx c, const double* b, double* x) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ SShared sh;
+    const int t = threadIdx.x, warp = t >> 5;
+    SRows R;
+    R.row0 = blockIdx.x * c.rows;
+    R.nr = min(c.rows, c.n - R.row0);
+    const int all = (c.rows + 31) / 32;           // groups of 32 rows
+    R.share = max(1, kStaticWarps / all);         // warps on a group
+    R.groups = (R.nr + 31) / 32;
+    const int passes = (all * R.share + kStaticWarps - 1) / kStaticWarps;  // groups a warp serves in turn
+    const int p0 = c.rowptr[R.row0], nb = c.rowptr[R.row0 + R.nr] - p0;
+    if (t == 0) sh.stuck = 0;
+    // shared memory: row positions, then the CTA's vectors, blocks and columns as far as they fit
+    int* ptr = reinterpret_cast<int*>(smem);
+    size_t used = ((R.nr + 1) * sizeof(int) + 15) / 16 * 16;
+    for (int k = t; k <= R.nr; k += kStaticThreads) ptr[k] = c.rowptr[R.row0 + k] - p0;
+    R.ptr = ptr;
+    double* loc = c.base + kOffLocal + (size_t)kLocal * R.row0;
+    if (used + sizeof(double) * kLocal * R.nr <= kStaticSmem) {
+        loc = reinterpret_cast<double*>(smem + used);
+        used += (sizeof(double) * kLocal * R.nr + 15) / 16 * 16;
+    }
+    R.col = c.colidx + p0;
+    R.val = c.val + 9 * (size_t)p0;
+    if (used + sizeof(int) * nb <= kStaticSmem / 4) {
+        int* col = reinterpret_cast<int*>(smem + used);
+        for (int k = t; k < nb; k += kStaticThreads) col[k] = R.col[k];
+        R.col = col;
+        used += (sizeof(int) * nb + 15) / 16 * 16;
+    }
+    double* staged = reinterpret_cast<double*>(smem + used);
+    R.staged = staged;
+    R.nstaged = min(nb, (int)((kStaticSmem - used) / (9 * sizeof(double))));
+#pragma unroll 8
+    for (int k = t; k < 9 * R.nstaged; k += kStaticThreads) staged[k] = R.val[k];
+    const int n3 = 3 * R.nr;
+    double *r = loc, *rhat = r + n3, *p = rhat + n3, *v = p + n3, *s = v + n3, *tv = s + n3, *dinv = tv + n3;
+    double *phat = c.phat() + 4 * R.row0, *shat = c.shat() + 4 * R.row0;
+    x += 3 * (size_t)R.row0;
+    b += 3 * (size_t)R.row0;
+    // a thread per row, but for the products
+    const int slots_row = min(kStaticWarps, R.groups), slot_row = warp < slots_row ? warp : -1;
+    const int par = kStaticWarps / R.share, slots_mul = min(par, R.groups);
+    const int slot_mul = warp % R.share == 0 && warp / R.share < slots_mul ? warp / R.share : -1;
+    double bb[1] = {0.0};
+    for (int i = t; i < R.nr; i += kStaticThreads) {
+        s_diag_inverse(c, R.row0 + i, dinv + 9 * (size_t)i);
+        for (int d = 3 * i; d < 3 * i + 3; ++d) {
+            const double bk = b[d];
+            r[d] = rhat[d] = bk;
+            p[d] = v[d] = 0.0;
+            x[d] = 0.0;
+            bb[0] = fma(bk, bk, bb[0]);
+        }
+    }
+    unsigned goal = 0;
+    bool ok = s_reduce<1>(c, sh, goal, 0, slot_row, slots_row, bb, [&](const double* q) {
+        sh.rho = sh.rr = sh.bb = q[0];
+        sh.alpha = sh.omega = 1.0;
+        sh.beta = 0.0;
+        sh.it = 0;
+        sh.flag = q[0] == 0.0 ? QF_CONVERGED : (isfinite(q[0]) ? QF_RUNNING : QF_NAN);
+    });
+    while (ok && sh.flag == QF_RUNNING && sh.it < c.max_iter) {
+        // p = r + beta (p - omega v); phat = M^-1 p
+        const double beta = sh.beta, omega0 = sh.omega;
+        for (int i = t; i < R.nr; i += kStaticThreads) {
+            double pp[3], z[3];
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                const int k = 3 * i + d;
+                pp[d] = fma(beta, fma(-omega0, v[k], p[k]), r[k]);
+                p[k] = pp[d];
             }
+            s_prec(dinv + 9 * (size_t)i, pp, z);
+#pragma unroll
+            for (int d = 0; d < 3; ++d) phat[4 * i + d] = z[d];
         }
-        for (int k = 0; k < 9; ++k) c.dinv()[9 * (size_t)i + k] = inv[k];
-        for (int d = 0; d < 3; ++d) {
-            const int k = 3 * i + d;
-            const double bk = b[k];
-            c.vec(0)[k] = bk;     // r
-            c.vec(1)[k] = bk;     // rhat
-            c.vec(2)[k] = 0.0;    // p
-            c.vec(4)[k] = 0.0;    // v
-            x[k] = 0.0;
-            acc[0] = fma(bk, bk, acc[0]);
+        if (!(ok = s_barrier(c, sh, goal))) break;
+        // v = A phat; alpha = rho / (rhat, v)
+        double rv[1] = {0.0}, y[3];
+        for (int k = 0; k < passes; ++k) {
+            const int g = warp / R.share + k * par;
+            if (s_rows(R, sh, g, c.phat(), y))
+#pragma unroll
+                for (int d = 0; d < 3; ++d) {
+                    const int e = 3 * (32 * g + (t & 31)) + d;
+                    v[e] = y[d];
+                    rv[0] = fma(rhat[e], y[d], rv[0]);
+                }
+            if (k + 1 < passes) __syncthreads();
         }
-    }
-    double tot[1];
-    if (s_reduce<1>(c, acc, tot) && threadIdx.x == 0) {
-        double* q = c.q();
-        q[Q_RHO] = tot[0];
-        q[Q_BB] = tot[0];
-        q[Q_RR] = tot[0];
-        q[Q_ALPHA] = 1.0;
-        q[Q_OMEGA] = 1.0;
-        q[Q_BETA] = 0.0;
-        q[Q_ITER] = 0.0;
-        q[Q_FLAG] = tot[0] == 0.0 ? QF_CONVERGED : (isfinite(tot[0]) ? QF_RUNNING : QF_NAN);
-    }
-}
-
-// p = r + beta (p - omega v); phat = M^-1 p
-__global__ void ks_dir(SCtx c) {
-    if (s_stopped(c)) return;
-    const int i = blockIdx.x * kStaticThreads + threadIdx.x;
-    if (i >= c.n) return;
-    const double beta = __ldcg(&c.q()[Q_BETA]), omega = __ldcg(&c.q()[Q_OMEGA]);
-    double pp[3], z[3];
-    for (int d = 0; d < 3; ++d) {
-        const int k = 3 * i + d;
-        pp[d] = fma(beta, fma(-omega, c.vec(4)[k], c.vec(2)[k]), c.vec(0)[k]);
-        c.vec(2)[k] = pp[d];
-    }
-    s_prec(c.dinv() + 9 * (size_t)i, pp, z);
-    for (int d = 0; d < 3; ++d) c.vec(3)[3 * i + d] = z[d];
-}
-
-// v = A phat; alpha = rho / (rhat, v)
-__global__ void ks_spmv1(SCtx c) {
-    if (s_stopped(c)) return;
-    const int i = blockIdx.x * kStaticThreads + threadIdx.x;
-    double acc[1] = {0.0};
-    if (i < c.n) {
-        double y[3];
-        s_row(c, i, c.vec(3), y);
-        for (int d = 0; d < 3; ++d) {
-            c.vec(4)[3 * i + d] = y[d];
-            acc[0] = fma(c.vec(1)[3 * i + d], y[d], acc[0]);
+        ok = s_reduce<1>(c, sh, goal, 1, slot_mul, slots_mul, rv, [&](const double* q) {
+            if (q[0] == 0.0 || !isfinite(q[0])) sh.flag = isfinite(q[0]) ? QF_BREAKDOWN : QF_NAN;
+            else sh.alpha = sh.rho / q[0];
+        });
+        if (!ok || sh.flag != QF_RUNNING) break;
+        // s = r - alpha v; shat = M^-1 s
+        const double alpha = sh.alpha;
+        for (int i = t; i < R.nr; i += kStaticThreads) {
+            double ss[3], z[3];
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                const int k = 3 * i + d;
+                ss[d] = fma(-alpha, v[k], r[k]);
+                s[k] = ss[d];
+            }
+            s_prec(dinv + 9 * (size_t)i, ss, z);
+#pragma unroll
+            for (int d = 0; d < 3; ++d) shat[4 * i + d] = z[d];
         }
-    }
-    double tot[1];
-    if (s_reduce<1>(c, acc, tot) && threadIdx.x == 0) {
-        double* q = c.q();
-        if (tot[0] == 0.0 || !isfinite(tot[0])) q[Q_FLAG] = isfinite(tot[0]) ? QF_BREAKDOWN : QF_NAN;
-        else q[Q_ALPHA] = q[Q_RHO] / tot[0];
-    }
-}
-
-// s = r - alpha v; shat = M^-1 s
-__global__ void ks_s(SCtx c) {
-    if (s_stopped(c)) return;
-    const int i = blockIdx.x * kStaticThreads + threadIdx.x;
-    if (i >= c.n) return;
-    const double alpha = __ldcg(&c.q()[Q_ALPHA]);
-    double ss[3], z[3];
-    for (int d = 0; d < 3; ++d) {
-        const int k = 3 * i + d;
-        ss[d] = fma(-alpha, c.vec(4)[k], c.vec(0)[k]);
-        c.vec(5)[k] = ss[d];
-    }
-    s_prec(c.dinv() + 9 * (size_t)i, ss, z);
-    for (int d = 0; d < 3; ++d) c.vec(6)[3 * i + d] = z[d];
-}
-
-// t = A shat; omega = (t, s) / (t, t)
-__global__ void ks_spmv2(SCtx c) {
-    if (s_stopped(c)) return;
-    const int i = blockIdx.x * kStaticThreads + threadIdx.x;
-    double acc[2] = {0.0, 0.0};
-    if (i < c.n) {
-        double y[3];
-        s_row(c, i, c.vec(6), y);
-        for (int d = 0; d < 3; ++d) {
-            c.vec(7)[3 * i + d] = y[d];
-            acc[0] = fma(y[d], c.vec(5)[3 * i + d], acc[0]);
-            acc[1] = fma(y[d], y[d], acc[1]);
+        if (!(ok = s_barrier(c, sh, goal))) break;
+        // t = A shat; omega = (t, s) / (t, t)
+        double ts[2] = {0.0, 0.0};
+        for (int k = 0; k < passes; ++k) {
+            const int g = warp / R.share + k * par;
+            if (s_rows(R, sh, g, c.shat(), y))
+#pragma unroll
+                for (int d = 0; d < 3; ++d) {
+                    const int e = 3 * (32 * g + (t & 31)) + d;
+                    tv[e] = y[d];
+                    ts[0] = fma(y[d], s[e], ts[0]);
+                    ts[1] = fma(y[d], y[d], ts[1]);
+                }
+            if (k + 1 < passes) __syncthreads();
         }
+        ok = s_reduce<2>(c, sh, goal, 2, slot_mul, slots_mul, ts, [&](const double* q) {
+            if (!isfinite(q[0]) || !isfinite(q[1])) sh.flag = QF_NAN;
+            else sh.omega = q[1] > 0.0 ? q[0] / q[1] : 0.0;
+        });
+        if (!ok || sh.flag != QF_RUNNING) break;
+        // x += alpha phat + omega shat; r = s - omega t; rho' = (rhat, r)
+        const double omega = sh.omega;
+        double ro[2] = {0.0, 0.0};
+        if (t == kStaticThreads - 1) sh.beta = alpha / omega;  // beside the others' work
+        for (int i = t; i < R.nr; i += kStaticThreads)
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                const int k = 3 * i + d;
+                x[k] = fma(omega, shat[4 * i + d], fma(alpha, phat[4 * i + d], x[k]));
+                const double rk = fma(-omega, tv[k], s[k]);
+                r[k] = rk;
+                ro[0] = fma(rhat[k], rk, ro[0]);
+                ro[1] = fma(rk, rk, ro[1]);
+            }
+        ok = s_reduce<2>(c, sh, goal, 3, slot_row, slots_row, ro, [&](const double* q) {
+            sh.beta *= q[0] / sh.rho;
+            sh.rho = q[0];
+            sh.rr = q[1];
+            ++sh.it;
+            if (!isfinite(q[1])) sh.flag = QF_NAN;
+            else if (q[1] <= c.tol2 * sh.bb) sh.flag = QF_CONVERGED;
+            else if (sh.omega == 0.0 || q[0] == 0.0) sh.flag = QF_BREAKDOWN;
+        });
     }
-    double tot[2];
-    if (s_reduce<2>(c, acc, tot) && threadIdx.x == 0) {
-        double* q = c.q();
-        if (!isfinite(tot[0]) || !isfinite(tot[1])) q[Q_FLAG] = QF_NAN;
-        else q[Q_OMEGA] = tot[1] > 0.0 ? tot[0] / tot[1] : 0.0;
-    }
-}
-
-// x += alpha phat + omega shat; r = s - omega t; rho' = (rhat, r)
-__global__ void ks_x(SCtx c, double* __restrict__ x) {
-    if (s_stopped(c)) return;
-    const int i = blockIdx.x * kStaticThreads + threadIdx.x;
-    const double alpha = __ldcg(&c.q()[Q_ALPHA]), omega = __ldcg(&c.q()[Q_OMEGA]);
-    double acc[2] = {0.0, 0.0};
-    if (i < c.n) {
-        for (int d = 0; d < 3; ++d) {
-            const int k = 3 * i + d;
-            x[k] = fma(omega, c.vec(6)[k], fma(alpha, c.vec(3)[k], x[k]));
-            const double rk = fma(-omega, c.vec(7)[k], c.vec(5)[k]);
-            c.vec(0)[k] = rk;
-            acc[0] = fma(c.vec(1)[k], rk, acc[0]);
-            acc[1] = fma(rk, rk, acc[1]);
-        }
-    }
-    double tot[2];
-    if (s_reduce<2>(c, acc, tot) && threadIdx.x == 0) {
-        double* q = c.q();
-        const double om = q[Q_OMEGA];
-        q[Q_BETA] = (tot[0] / q[Q_RHO]) * (q[Q_ALPHA] / om);
-        q[Q_RHO] = tot[0];
-        q[Q_RR] = tot[1];
-        q[Q_ITER] += 1.0;
-        if (!isfinite(tot[1])) q[Q_FLAG] = QF_NAN;
-        else if (tot[1] <= q[Q_TOL2] * q[Q_BB]) q[Q_FLAG] = QF_CONVERGED;
-        else if (om == 0.0 || tot[0] == 0.0) q[Q_FLAG] = QF_BREAKDOWN;
-    }
+    if (t == 0 && !ok) c.q()[Q_FLAG] = QF_STUCK;
+    if (t != 0 || blockIdx.x != 0 || !ok) return;
+    double* q = c.q();
+    q[Q_BB] = sh.bb;
+    q[Q_RR] = sh.rr;
+    q[Q_ITER] = sh.it;
+    q[Q_FLAG] = sh.flag;
 }
 
 std::mutex g_addr_mutex;
@@ -351,35 +491,26 @@ extern "C" TF_API tf_status tf_solve_bsr_static(int32_t n_block_rows, const int3
     double* base = nullptr;
     tf_status s = scratch_address(device, &base);
     if (s != TF_OK) return s;
-    SCtx c{n_block_rows, rowptr, colidx, val, base};
-    const int grid = cdiv(n_block_rows, kStaticThreads);
-    // clear the ticket and scalars, then the tolerance
+    int sms = 0;
+    TF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    const int grid0 = std::min(sms, cdiv(n_block_rows, 32));
+    const int rows = cdiv(n_block_rows, grid0);
+    SCtx c{n_block_rows, rows, max_iter, rtol * rtol, rowptr, colidx, val, base};
+    // clear the scalars and the barrier
     TF_CUDA(cudaMemsetAsync(base + kOffScal, 0, sizeof(double) * (kNumScal + 2), st));
-    const double tol2 = rtol * rtol;
-    TF_CUDA(cudaMemcpyAsync(base + kOffScal + Q_TOL2, &tol2, sizeof(double), cudaMemcpyHostToDevice, st));
-    ks_init<<<grid, kStaticThreads, 0, st>>>(c, b, x);
+    TF_CUDA(cudaFuncSetAttribute(ks_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, kStaticSmem));
+    launch_cooperative(ks_solve, cdiv(n_block_rows, rows), kStaticThreads, kStaticSmem, st, c, b, x);
     TF_CUDA(cudaGetLastError());
     double q[kNumScal];
-    int launched = 0, chunk = 8;
-    while (launched < max_iter) {
-        const int n = chunk < max_iter - launched ? chunk : max_iter - launched;
-        for (int it = 0; it < n; ++it) {
-            ks_dir<<<grid, kStaticThreads, 0, st>>>(c);
-            ks_spmv1<<<grid, kStaticThreads, 0, st>>>(c);
-            ks_s<<<grid, kStaticThreads, 0, st>>>(c);
-            ks_spmv2<<<grid, kStaticThreads, 0, st>>>(c);
-            ks_x<<<grid, kStaticThreads, 0, st>>>(c, x);
-        }
-        TF_CUDA(cudaGetLastError());
-        launched += n;
-        TF_CUDA(cudaMemcpyAsync(q, base + kOffScal, sizeof(q), cudaMemcpyDeviceToHost, st));
-        TF_CUDA(cudaStreamSynchronize(st));
-        if (q[Q_FLAG] != QF_RUNNING) break;
-        if (chunk < 64) chunk *= 2;
-    }
+    TF_CUDA(cudaMemcpyAsync(q, base + kOffScal, sizeof(q), cudaMemcpyDeviceToHost, st));
+    TF_CUDA(cudaStreamSynchronize(st));
     if (iters) *iters = static_cast<int32_t>(q[Q_ITER]);
     if (relres) *relres = q[Q_BB] > 0.0 ? sqrt(q[Q_RR] / q[Q_BB]) : 0.0;
     if (q[Q_FLAG] == QF_CONVERGED) return TF_OK;
+    if (q[Q_FLAG] == QF_STUCK) {
+        set_error("tf_solve_bsr_static: the thread blocks lost each other (overlapping calls?)");
+        return TF_CUDA_ERROR;
+    }
     if (q[Q_FLAG] == QF_NAN) {
         set_error("tf_solve_bsr_static: non-finite value");
         return TF_NAN_DETECTED;
