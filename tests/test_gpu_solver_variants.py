@@ -271,3 +271,31 @@ def test_static_solve_of_ragged_systems(n, most):
     st = api.load().tf_solve_bsr_static(n, p(d["rowptr"]), p(d["col"]), p(d["val"]), p(d["b"]), p(x), RTOL, 500, None,
                                         C.byref(it), C.byref(rr))
     assert st == api.TF_OK and np.array_equal(x.cpu().numpy().reshape(n, 3), xs)  # fixed order of sums
+
+
+# Coarse images of many extra blocks (a lane group takes five at a time; the warps
+# of a split CTA share a row's): a node coupled to 0, 1, 4, 5, 6 and 31 others, its
+# CTA's neighbours to none, split and whole rows, both preconditioners.
+@pytest.mark.parametrize("precond", [1, 2])
+@pytest.mark.parametrize("deterministic", [False, True])
+@pytest.mark.parametrize("many", [1, 4, 5, 6, 31])
+def test_rows_with_many_extra_blocks(many, deterministic, precond):
+    t = _sheet(16, 11, 2, 0.0)
+    uk, un = mesh.perturbed_state(t, seed=5)
+    free = np.flatnonzero(t.fixed.reshape(-1, 3).sum(axis=1) == 0)
+    far = free[free > t.n_nodes // 2][:many]
+    i, j, v = [], [], []
+    for q, n in enumerate(far):  # springs between node free[0] and each of the others
+        for d in range(3):
+            a, b = 3 * free[0] + d, 3 * n + d
+            i += [a, b, a, b]
+            j += [a, b, b, a]
+            v += [1.0 + q, 1.0 + q, -1.0 - q, -1.0 - q]
+    with api.Solver(t, precond=precond, krylov_rtol=RTOL, deterministic=deterministic) as s:
+        s.set_positions(un)
+        s.begin_step(t.dt)
+        s.set_state(uk, un, t.dt)
+        s.assemble()
+        s.add_K_triplets(i, j, v)
+        out = s.solve()
+        _check_solution(s, out, [(0, 3 * t.n_nodes)])

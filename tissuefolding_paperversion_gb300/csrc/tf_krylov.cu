@@ -60,9 +60,11 @@ __device__ __forceinline__ void rows_product(const Ctx& c, const Slots& s, const
 }
 template <int MODE = kEither>
 __device__ __forceinline__ void rows_sum(const Ctx& c, const Where& w, const double* __restrict__ x, double (&y)[3]) {
-    if (MODE == kSplit || (MODE == kEither && c.split)) split_sum(y);
-    if (c.xrow && w.valid) {
-        for (int p = c.xrow[w.node]; p < c.xrow[w.node + 1]; ++p) {
+    const bool split = MODE == kSplit || (MODE == kEither && c.split);
+    const int row = split ? w.node - (int)threadIdx.x + (int)(threadIdx.x & 31) : w.node;
+    if (c.xrow && (split ? row < w.n1 : w.valid)) {  // split CTAs: the warps share the extra blocks of a row too
+        const int p1 = c.xrow[row + 1];
+        for (int p = c.xrow[row] + (split ? (int)(threadIdx.x >> 5) : 0); p < p1; p += split ? kWarps : 1) {
             const int j = c.xcol[p];
             if (!TF_IN(c.check, j, c.nn, CK_EXTRA_COL)) continue;
             const double* __restrict__ a = c.xval + 9 * (size_t)p;
@@ -72,6 +74,7 @@ __device__ __forceinline__ void rows_sum(const Ctx& c, const Where& w, const dou
             y[2] = fma(a[6], x0, fma(a[7], x1, fma(a[8], x2, y[2])));
         }
     }
+    if (split) split_sum(y);
 }
 
 // Sets an instance's stop flag from its first scalars (bb = |b|^2).  With an

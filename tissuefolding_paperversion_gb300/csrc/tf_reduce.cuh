@@ -43,6 +43,7 @@ struct Where {
     int seg;      // instance of this CTA
     double* s;    // its scalars
     double flag;  // its stop flag
+    int n1;       // end of this CTA's nodes
 };
 
 // With one instance nothing is looked up: the operands' loads need not wait for
@@ -50,17 +51,16 @@ struct Where {
 // batch tests first: its stopped instances would only cost bandwidth).
 __device__ __forceinline__ Where where(const Ctx& c) {
     Where w;
-    int n1;
     if (c.single) {
         w.seg = 0;
         w.node = blockIdx.x * c.cta_nodes + threadIdx.x;
-        n1 = min((int)(blockIdx.x + 1) * c.cta_nodes, c.nn);
+        w.n1 = min((int)(blockIdx.x + 1) * c.cta_nodes, c.nn);
     } else {
         w.seg = c.cta_seg[blockIdx.x];
         w.node = c.cta_node0[blockIdx.x] + threadIdx.x;
-        n1 = c.cta_node1[blockIdx.x];
+        w.n1 = c.cta_node1[blockIdx.x];
     }
-    w.valid = w.node < n1;
+    w.valid = w.node < w.n1;
     w.s = c.scal + (size_t)w.seg * S_COUNT;
     w.flag = __ldcg(&w.s[S_FLAG]);
     return w;
