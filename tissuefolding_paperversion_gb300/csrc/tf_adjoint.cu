@@ -308,7 +308,7 @@ tf_status copy_state(tf_handle* h, double* u, double* F, double* iF, const doubl
     TF_CUDA(cudaMemcpyAsync(u, su, n3 * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
     TF_CUDA(cudaMemcpyAsync(F, sF, n9 * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
     TF_CUDA(cudaMemcpyAsync(iF, siF, n9 * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
-    return TF_OK;
+    return iF == d.invFg ? launch_metric(h) : TF_OK;
 }
 
 tf_status adj_forward(tf_handle* h, tf_adjoint* a, const double* rate, const double* logE) {
@@ -329,6 +329,7 @@ tf_status adj_forward(tf_handle* h, tf_adjoint* a, const double* rate, const dou
     TF_LAUNCH_CHECK(h);
     k_reset_Fg<<<cdiv(ne, kT), kT, 0, h->stream>>>(ne, d.Fg, d.invFg);
     TF_LAUNCH_CHECK(h);
+    TFA_TRY(launch_metric(h));
     h->have_rates = true;
     tf_status status = TF_OK;
     for (int n = 0; n < a->n_steps; ++n) {

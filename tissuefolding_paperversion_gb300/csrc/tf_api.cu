@@ -110,7 +110,7 @@ tf_status upload(T** p, const std::vector<T>& v) {
 
 void free_all(tf_handle* h) {
     Device& d = h->d;
-    void* ptrs[] = {d.conn, d.ginv, d.gx, d.wdet, d.Fg, d.invFg, d.rates, d.lam, d.mu, d.eta, d.exposure,
+    void* ptrs[] = {d.conn, d.ginv, d.metric, d.gx, d.wdet, d.Fg, d.invFg, d.rates, d.lam, d.mu, d.eta, d.exposure,
                     d.aptr, d.alist, d.farea, d.fixed, d.ext_visc, d.area, d.rowptr, d.colidx, d.diag, d.rowof,
                     d.slot, d.bofs, d.wslot0, d.scol, d.val, d.eblk, d.ef, d.gptr, d.glist, d.fptr, d.flist, d.uk, d.un, d.vel, d.g,
                     d.du, d.dinv, d.r, d.p, d.z, d.q, d.rhat, d.s, d.t, d.sh, d.scal, d.part, d.tickets,
@@ -403,6 +403,8 @@ tf_status build(tf_handle* h, const tf_mesh* m, const tf_material* mat, const st
         for (int e = 0; e < ne; ++e) ident[(size_t)k * ne + e] = 1.0;
     TF_TRY(upload(&d.Fg, ident));
     TF_TRY(upload(&d.invFg, ident));
+    TF_TRY(dev_alloc(&d.metric, 11 * 6 * (size_t)ne));
+    TF_TRY(launch_metric(h));
     TF_TRY(upload(&d.rates, std::vector<double>(3 * (size_t)ne, 0.0)));
     const size_t n3 = 3 * (size_t)nn;
     std::vector<double> pos(m->node_pos, m->node_pos + n3);
@@ -1483,6 +1485,7 @@ tf_status tf_set_Fg(tf_handle* h, const double* Fg) {
     }
     TF_CUDA(cudaMemcpyAsync(h->d.Fg, f.data(), f.size() * sizeof(double), cudaMemcpyHostToDevice, h->stream));
     TF_CUDA(cudaMemcpyAsync(h->d.invFg, inv.data(), inv.size() * sizeof(double), cudaMemcpyHostToDevice, h->stream));
+    TF_TRY(launch_metric(h));
     amg_mark_stale(h, 2);  // the tangent may differ from the kept coarse levels' by more than a step's change
     return sync(h);
 }

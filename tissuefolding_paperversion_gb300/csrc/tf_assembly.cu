@@ -202,7 +202,7 @@ tf_status launch_growth(tf_handle* h) {
     Device& d = h->d;
     k_growth<<<cdiv(d.ne, 256), 256, 0, h->stream>>>(d.ne, h->dt, d.rates, d.Fg, d.invFg);
     TF_LAUNCH_CHECK(h);
-    return TF_OK;
+    return launch_metric(h);
 }
 
 tf_status launch_viscosity_surfaces(tf_handle* h) {

@@ -62,10 +62,10 @@
 // instruction cache.
 // The phases of one CTA use one pipe at a time; three CTAs on an SM overlap them
 // (with the u_j and s_jl kept in shared memory two fit: 2.58 against 1.94 ms).
-// FP64 pipe and issue slots are each half busy: 1,787 FP64 instructions per prism
+// FP64 pipe and issue slots are each half busy: ~1,450 FP64 instructions per prism
 // (3,156 before), ~130,000 thread instructions per prism in all; the rest is the barriers
-// between the phases.  320,000 prisms: 3.62 -> 1.89 ms with viscosity, 2.18 -> 1.37 ms
-// without.  K's error against 64 bits, relative (2-norm): 2.0e-15 to 2.4e-15 without
+// between the phases (starting the CTAs of an SM in different phases: no change).
+// 320,000 prisms: 3.62 -> 1.81 ms with viscosity, 2.18 -> 1.26 ms without.  K's error against 64 bits, relative (2-norm): 2.0e-15 to 2.4e-15 without
 // viscosity (before 2.1e-15 to 2.2e-15), 2.4e-15 to 2.9e-15 with (2.6e-15 to 3.2e-15).
 // The matrix assembled is A = K^T, the system the reference
 // solves (Pardiso iparm[11] = 1, NewtonRaphsonSolver.cpp:639); in that
@@ -87,7 +87,7 @@ constexpr int kSlots = 12;  // threads per prism
 struct ElemArgs {
     int ne;
     const int* __restrict__ conn;
-    const double* __restrict__ ginv;  // [9][6][ne] dxi/dX
+    const double* __restrict__ metric;  // [11][6][ne] (k_metric)
     const double* __restrict__ gx;
     const double* __restrict__ wdet;
     const double* __restrict__ invFg;
@@ -412,7 +412,8 @@ __device__ __forceinline__ int sym_index(int j, int l) { return j == l ? j : j +
 // Shared memory of a CTA, the prism fastest everywhere.
 //   gp: double-float vectors of the Gauss points, [value][gp][NE]: the gradients
 //       g_1/sqrt(3), g_2/sqrt(3), g_3/12 (G; the weights of phase 4 are then small
-//       integers but for one factor), their w_j (W) and with viscosity v_j, Q, t_jl
+//       integers but for one factor; the forces' weights and the velocities carry
+//       the inverse), their w_j (W) and with viscosity v_j, Q, t_jl
 //       and c1 (u_j and s_jl are formed again in phase 4: their room would cost a
 //       CTA per SM), without it u_j and d_jl = c2 s_jl + t_jl (U, D);
 //   st: staged 3x3 blocks, [block][9][NE]: A_jl(height), j, l in {1, 2}, then
@@ -530,8 +531,9 @@ __global__ void __launch_bounds__(NE* kSlots, 48 / NE) k_element(ElemArgs A) {
     const int ne = A.ne;
 
     // ---- 1. dx/dxi_1, dx/dxi_2 at both heights, dx/dxi_3 at the in-plane points
-    // (component slot % 3), and dv/dxi likewise: apical weight (1 + zeta)/2 = b at
-    // the first height, a at the second
+    // (component slot % 3), and dv/dxi likewise times sqrt(3), sqrt(3) and 12 (the
+    // gradients come divided by these): apical weight (1 + zeta)/2 = b at the first
+    // height, a at the second
     constexpr double wa = 0.5 - kSqrt3 / 6.0, wb = 0.5 + kSqrt3 / 6.0;
     if (live && slot < (VISC ? 6 : 3)) {
         const int c = slot % 3;
@@ -544,16 +546,18 @@ __global__ void __launch_bounds__(NE* kSlots, 48 / NE) k_element(ElemArgs A) {
             x[a] = src[3 * nd + c];
         }
         double* o = sx + (size_t)(slot / 3) * 21 * NE + c * NE + el;
+        const bool vel = slot >= 3;
+        const double a = vel ? kSqrt3 * wa : wa, b = vel ? kSqrt3 * wb : wb;
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
             const double lo = x[1 + j] - x[0], up = x[4 + j] - x[3];
-            o[(2 * j) * 3 * NE] = fma(wa, lo, wb * up);
-            o[(2 * j + 1) * 3 * NE] = fma(wb, lo, wa * up);
+            o[(2 * j) * 3 * NE] = fma(a, lo, b * up);
+            o[(2 * j + 1) * 3 * NE] = fma(b, lo, a * up);
         }
         const double d[3] = {x[3] - x[0], x[4] - x[1], x[5] - x[2]};
-        const double m = (d[0] + d[1] + d[2]) * (1.0 / 12.0);
+        const double m = (d[0] + d[1] + d[2]) * (vel ? 1.0 : 1.0 / 12.0), q = vel ? 3.0 : 0.25;
 #pragma unroll
-        for (int t = 0; t < 3; ++t) o[(4 + t) * 3 * NE] = fma(0.25, d[t], m);
+        for (int t = 0; t < 3; ++t) o[(4 + t) * 3 * NE] = fma(q, d[t], m);
     }
     __syncthreads();
 
@@ -573,7 +577,7 @@ __global__ void __launch_bounds__(NE* kSlots, 48 / NE) k_element(ElemArgs A) {
         for (int j = 0; j < 3; ++j)
 #pragma unroll
             for (int i = 0; i < 3; ++i) X[3 * j + i] = col(0, j, i);
-        double g[9];  // g[3 j + i]: the cofactors, then grad xi_j
+        double g[9];  // g[3 j + i]: the cofactors, then grad xi_j over sqrt(3), sqrt(3), 12
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
             const double* p = X + 3 * ((j + 1) % 3);
@@ -583,38 +587,41 @@ __global__ void __launch_bounds__(NE* kSlots, 48 / NE) k_element(ElemArgs A) {
             g[3 * j + 2] = fma(p[0], q[1], -(p[1] * q[0]));
         }
         const double det = fma(X[0], g[0], fma(X[1], g[1], X[2] * g[2]));
-        double Fe[9];
-        {
-            double F[9];  // F[3 i + k] = sum_j dx_i/dxi_j dxi_j/dX_k
-            const double* __restrict__ iv = A.ginv + (size_t)gp * ne + e;
-            const size_t st6 = (size_t)6 * ne;
+        // Fe = X^T M, M = dxi/dX Fg^-1; b = Fe Fe^T; J = det M det X
+        double Fe[9], b[6];  // b: 00 11 22 01 02 12
+        const double* __restrict__ me = A.metric + (size_t)gp * ne + e;
+        const size_t st6 = (size_t)6 * ne;
 #pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                const double a0 = __ldg(&iv[k * st6]), a1 = __ldg(&iv[(3 + k) * st6]), a2 = __ldg(&iv[(6 + k) * st6]);
+        for (int k = 0; k < 3; ++k) {
+            const double a0 = __ldg(&me[k * st6]), a1 = __ldg(&me[(3 + k) * st6]), a2 = __ldg(&me[(6 + k) * st6]);
 #pragma unroll
-                for (int i = 0; i < 3; ++i) F[3 * i + k] = fma(X[i], a0, fma(X[3 + i], a1, X[6 + i] * a2));
-            }
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                const double a0 = __ldg(&A.invFg[k * ne + e]), a1 = __ldg(&A.invFg[(3 + k) * ne + e]),
-                             a2 = __ldg(&A.invFg[(6 + k) * ne + e]);
-#pragma unroll
-                for (int i = 0; i < 3; ++i) Fe[3 * i + k] = fma(F[3 * i], a0, fma(F[3 * i + 1], a1, F[3 * i + 2] * a2));
-            }
+            for (int i = 0; i < 3; ++i) Fe[3 * i + k] = fma(X[i], a0, fma(X[3 + i], a1, X[6 + i] * a2));
         }
-        const double J = fma(Fe[0], fma(Fe[4], Fe[8], -(Fe[5] * Fe[7])),
-                             fma(-Fe[1], fma(Fe[3], Fe[8], -(Fe[5] * Fe[6])), Fe[2] * fma(Fe[3], Fe[7], -(Fe[4] * Fe[6]))));
-        const double lnJ = log(J);
-        const double rr = 1.0 / (J * det);
+        {
+            auto bij = [&](int i, int k) {
+                return fma(Fe[3 * i], Fe[3 * k], fma(Fe[3 * i + 1], Fe[3 * k + 1], Fe[3 * i + 2] * Fe[3 * k + 2]));
+            };
+            b[0] = bij(0, 0);
+            b[1] = bij(1, 1);
+            b[2] = bij(2, 2);
+            b[3] = bij(0, 1);
+            b[4] = bij(0, 2);
+            b[5] = bij(1, 2);
+        }
+        const double lnJ = log(det * __ldg(&me[9 * st6]));
+        const double sc = __ldg(&me[10 * st6]);  // w dV / J
         const double wdV = det * (1.0 / 6.0);
-        const double sc = wdV * (rr * det);  // w dV / J
-        const double rd = rr * J;            // 1 / det
+        const double rd = 1.0 / det;
         float2* out = sg + gp * NE + el;
         auto put = [&](int v, double x) { out[(size_t)v * 6 * NE] = df_split(x); };
+        {
+            const double r1 = rd * (1.0 / kSqrt3), r3 = rd * (1.0 / 12.0);
 #pragma unroll
-        for (int k = 0; k < 9; ++k) put(Y::G + k, g[k] * (k < 6 ? rd * (1.0 / kSqrt3) : rd * (1.0 / 12.0)));
-#pragma unroll
-        for (int k = 0; k < 9; ++k) g[k] *= rd;
+            for (int k = 0; k < 9; ++k) {
+                g[k] *= k < 6 ? r1 : r3;
+                put(Y::G + k, g[k]);
+            }
+        }
         const double lam = __ldg(&A.lam[e]), mu = __ldg(&A.mu[e]);
         const double dterm = fma(lam, lnJ, -mu);
         float2* outc = sc0 + gp * NE + el;
@@ -624,18 +631,16 @@ __global__ void __launch_bounds__(NE* kSlots, 48 / NE) k_element(ElemArgs A) {
         else putc(Y::C1, sc * lam);
         const double c2d = -sc * dterm;
         double sgm[6];  // sigma' = w dV sigma (00 11 22 01 02 12)
-        sgm[0] = sc * fma(mu, fma(Fe[0], Fe[0], fma(Fe[1], Fe[1], Fe[2] * Fe[2])), dterm);
-        sgm[1] = sc * fma(mu, fma(Fe[3], Fe[3], fma(Fe[4], Fe[4], Fe[5] * Fe[5])), dterm);
-        sgm[2] = sc * fma(mu, fma(Fe[6], Fe[6], fma(Fe[7], Fe[7], Fe[8] * Fe[8])), dterm);
         const double sm = sc * mu;
-        sgm[3] = sm * fma(Fe[0], Fe[3], fma(Fe[1], Fe[4], Fe[2] * Fe[5]));
-        sgm[4] = sm * fma(Fe[0], Fe[6], fma(Fe[1], Fe[7], Fe[2] * Fe[8]));
-        sgm[5] = sm * fma(Fe[3], Fe[6], fma(Fe[4], Fe[7], Fe[5] * Fe[8]));
+#pragma unroll
+        for (int k = 0; k < 3; ++k) sgm[k] = sc * fma(mu, b[k], dterm);
+#pragma unroll
+        for (int k = 3; k < 6; ++k) sgm[k] = sm * b[k];
 #pragma unroll
         for (int k = 0; k < 6; ++k) putc(Y::SG + k, sgm[k]);
         if constexpr (VISC) {
-            // grad v = sum_j dv/dxi_j (x) g_j (ShapeBase.cpp:2892-2919); a prism
-            // without viscosity has eta = 0 and these terms vanish
+            // grad v = sum_j dv/dxi_j (x) g_j (ShapeBase.cpp:2892-2919), the scales of
+            // the two cancelling; a prism without viscosity has eta = 0 and these terms vanish
             double Lg[9];
 #pragma unroll
             for (int i = 0; i < 3; ++i) {
@@ -742,17 +747,17 @@ __global__ void __launch_bounds__(NE* kSlots, 48 / NE) k_element(ElemArgs A) {
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
             const double s0 = h(j, 0) + h(j, 1) + h(j, 2), s1 = h(j, 3) + h(j, 4) + h(j, 5);
-            T[j][0] = fma(wa, s0, wb * s1);
-            T[j][1] = fma(wb, s0, wa * s1);
+            T[j][0] = fma(kSqrt3 * wa, s0, (kSqrt3 * wb) * s1);
+            T[j][1] = fma(kSqrt3 * wb, s0, (kSqrt3 * wa) * s1);
         }
 #pragma unroll
         for (int t = 0; t < 3; ++t) z[t] = h(2, t) + h(2, 3 + t);
-        const double zs = (z[0] + z[1] + z[2]) * (1.0 / 12.0);
+        const double zs = z[0] + z[1] + z[2];
 #pragma unroll
         for (int a = 0; a < 6; ++a) {
             const int i = a % 3, up = a / 3;
             const double in = i == 0 ? -(T[0][up] + T[1][up]) : T[i - 1][up];
-            const double zi = fma(0.25, z[i], zs);
+            const double zi = fma(3.0, z[i], zs);
             const double f = up ? -(in + zi) : zi - in;
             const int node = __ldg(&A.conn[a * ne + e]);
             if (!TF_IN(A.check, node, A.nn, CK_ELEM_NODE)) continue;
@@ -1227,7 +1232,7 @@ ElemArgs make_args(tf_handle* h) {
     ElemArgs A{};
     A.ne = d.ne;
     A.conn = d.conn;
-    A.ginv = d.ginv;
+    A.metric = d.metric;
     A.gx = d.gx;
     A.wdet = d.wdet;
     A.invFg = d.invFg;
@@ -1305,6 +1310,46 @@ tf_status launch_shape_gradients(tf_handle* h, const double* dN) {
     ShapeDerivatives S;
     std::memcpy(S.dN, dN, sizeof(S.dN));
     k_shape_gradients<<<cdiv(6 * (int64_t)h->d.ne, 256), 256, 0, h->stream>>>(h->d.ne, S, h->d.ginv, h->d.gx);
+    TF_LAUNCH_CHECK(h);
+    return TF_OK;
+}
+
+// What the element kernel needs of a Gauss point's reference and growth: M =
+// dxi/dX Fg^-1 (Fe = X^T M for X = dx/dxi), det M (J = det X det M) and 1 / (6 det M)
+// = w dV / J.  They change with the growth, once per time step, and take a matrix
+// product, a determinant and a division out of every Gauss point of every assembly:
+// a sixth of its FP64 instructions (320,000 prisms 1.37 -> 1.26 ms without
+// viscosity, 1.89 -> 1.81 with; one pass over 138 MB per change of the growth).  C = M M^T in place of M would save
+// three loads, but X^T C X loses the digits of a skewed prism's M twice.
+__global__ void k_metric(int ne, const double* __restrict__ ginv, const double* __restrict__ invFg,
+                         double* __restrict__ metric) {
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;  // gp ne + e
+    if (q >= 6 * ne) return;
+    const int e = q % ne;
+    const size_t st6 = (size_t)6 * ne;
+    double G[9], F[9], M[9];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+        G[k] = ginv[k * st6 + q];
+        F[k] = invFg[(size_t)k * ne + e];
+    }
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            M[3 * j + k] = fma(G[3 * j], F[k], fma(G[3 * j + 1], F[3 + k], G[3 * j + 2] * F[6 + k]));
+            metric[(3 * j + k) * st6 + q] = M[3 * j + k];
+        }
+    const double det = fma(M[0], fma(M[4], M[8], -(M[5] * M[7])),
+                           fma(-M[1], fma(M[3], M[8], -(M[5] * M[6])), M[2] * fma(M[3], M[7], -(M[4] * M[6]))));
+    metric[9 * st6 + q] = det;
+    metric[10 * st6 + q] = 1.0 / (6.0 * det);
+}
+
+tf_status launch_metric(tf_handle* h) {
+    const Device& d = h->d;
+    if (d.ne <= 0) return TF_OK;
+    k_metric<<<cdiv(6 * (int64_t)d.ne, 256), 256, 0, h->stream>>>(d.ne, d.ginv, d.invFg, d.metric);
     TF_LAUNCH_CHECK(h);
     return TF_OK;
 }

@@ -862,7 +862,7 @@ tf_status launch_growth_functions(tf_handle* h, bool* done) {
     k_grow<<<cdiv(d.ne, kT), kT, 0, h->stream>>>(A, d.Fg, d.invFg);
     TF_LAUNCH_CHECK(h);
     *done = true;
-    return TF_OK;
+    return launch_metric(h);
 }
 
 // Host copies for the tests: relative z, pinned positions, and the positions

@@ -68,6 +68,7 @@ struct Device {
     double* ginv = nullptr;     // [9][6][ne] dxi_j/dX_k of each Gauss point (index 3 j + k)
     double* gx = nullptr;       // [18][6*ne] reference shape gradients
     double* wdet = nullptr;     // [6*ne] w * det(dX/dxi)
+    double* metric = nullptr;   // [11][6][ne] what the element kernel needs of ginv and invFg (k_metric)
     double* Fg = nullptr;       // [9][ne]
     double* invFg = nullptr;    // [9][ne]
     double* rates = nullptr;    // [3][ne] growth rates (1/s)
@@ -546,6 +547,7 @@ tf_status launch_update_norm(tf_handle* h);   // |du|^2 into S_DU2 without apply
 tf_status newton_device_loop(tf_handle* h, int* it, int* cv, int* capped, int* k, tf_step_stats* st, float* ms_asm,
                              bool* ran, bool* exc);
 tf_status autotune_element(tf_handle* h);
+tf_status launch_metric(tf_handle* h);  // after every change of invFg
 tf_status launch_shape_gradients(tf_handle* h, const double* dN);  // gx from ginv; dN[6][3][6] on the host
 tf_status amg_build(tf_handle* h, const double* ref_pos);
 tf_status amg_numeric(tf_handle* h);
