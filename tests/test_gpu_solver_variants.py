@@ -299,3 +299,27 @@ def test_rows_with_many_extra_blocks(many, deterministic, precond):
         s.add_K_triplets(i, j, v)
         out = s.solve()
         _check_solution(s, out, [(0, 3 * t.n_nodes)])
+
+
+# The device loop runs several iterations a round: caps below, at and between its
+# rounds are kept exactly, on split and whole rows, in a solve and in a Newton step.
+@pytest.mark.parametrize("eta", [0.0, 100.0])
+@pytest.mark.parametrize("deterministic", [False, True])
+@pytest.mark.parametrize("cap", [1, 2, 3, 4, 5, 7])
+def test_iteration_caps_between_the_loops_rounds(cap, deterministic, eta):
+    t = _sheet(12, 12, 2, eta)
+    t.rates = np.tile([4e-6, 3e-6, 0.0], t.n_elems)
+    uk, un = mesh.perturbed_state(t, seed=8)
+    with api.Solver(t, krylov_max_iter=cap, deterministic=deterministic, precond=1) as s:
+        s.set_state(uk, un, t.dt)
+        s.assemble()
+        out = s.solve(allow_not_converged=True)
+        assert out["status"] == api.TF_KRYLOV_NOT_CONVERGED and out["iters"] == cap
+    steps = []
+    for host in (False, True):  # the host-checked loop: the same, but for the solve the device loop hands back
+        with api.Solver(t, krylov_max_iter=cap, deterministic=deterministic, precond=1, host_loops=host) as s:
+            s.set_growth_rates(t.rates)
+            out = s.newton_step(t.dt)
+            steps.append((out["status"], out["iters"], out["krylov_max"]))
+    assert steps[0] == steps[1]
+    assert steps[0][2] <= cap

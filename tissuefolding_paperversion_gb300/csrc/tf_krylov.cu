@@ -740,32 +740,39 @@ tf_status run_chunk(tf_handle* h, const Ctx& c, int method, int ci) {
     return TF_OK;
 }
 
-// Loop control of the device-side Krylov loop (one warp): counts the
-// iteration and keeps the loop going while an instance is still running and
-// the iteration cap is not reached, so the loop always ends.
-__global__ void k_krylov_ctl(const double* __restrict__ scal, int nseg, int* __restrict__ ctl,
+// Iterations in the body of the device-side Krylov loop.  Going round costs ~5 us
+// whatever the mesh; iterations past convergence return at once, but launch.  Step
+// with 1 / 2 / 3 / 4 in the body: 256 prisms 1.19 / 1.11 / 1.09 / 1.09 ms, 1,600 1.41 /
+// 1.32 / 1.28 / 1.29, 9,728 viscous 1.87 / 1.80 / 1.80 / 1.84, 46,208 5.15 / 5.10 / 5.05 /
+// 5.05; whole rows with 1 / 2: 32 tissues 27.5 / 27.3, 320,000 viscous 19.6 / 19.6.
+inline int loop_iterations(const tf_handle* h) { return h->d.split ? 3 : 2; }
+
+// Loop control of the device-side Krylov loop (one warp): counts the body's n
+// iterations and keeps the loop going while an instance is still running and
+// n more are within the iteration cap, so the loop always ends.
+__global__ void k_krylov_ctl(const double* __restrict__ scal, int nseg, int* __restrict__ ctl, int n,
                              cudaGraphConditionalHandle loop) {
     bool running = false;
     for (int g = threadIdx.x; g < nseg; g += 32) running |= __ldcg(&scal[(size_t)g * S_COUNT + S_FLAG]) == F_RUNNING;
     running = __any_sync(0xffffffffu, running);
     if (threadIdx.x == 0) {
-        const int it = ctl[0] + 1;
+        const int it = ctl[0] + n;
         ctl[0] = it;
-        cudaGraphSetConditional(loop, (running && it < ctl[1]) ? 1u : 0u);
+        cudaGraphSetConditional(loop, (running && it + n <= ctl[1]) ? 1u : 0u);
     }
 }
 
 // Resets the iteration count of a device-side Krylov loop (and, inside an
-// enclosing loop, opens the Krylov loop's condition again).
-__global__ void k_krylov_arm(int* __restrict__ ctl, int cap, cudaGraphConditionalHandle loop, int open) {
+// enclosing loop, opens the Krylov loop's condition again if the cap has room for
+// its n iterations).
+__global__ void k_krylov_arm(int* __restrict__ ctl, int cap, cudaGraphConditionalHandle loop, int n) {
     ctl[0] = 0;
     ctl[1] = cap;
-    if (open) cudaGraphSetConditional(loop, 1u);
+    if (n > 0) cudaGraphSetConditional(loop, n <= cap ? 1u : 0u);
 }
 
 // A whole solve's iterations as one graph: a conditional while node whose
-// body is one iteration followed by k_krylov_ctl; no host round trip and no
-// iteration past convergence.  Returns false when the graph cannot be built
+// body is loop_iterations iterations followed by k_krylov_ctl; no host round trip.  Returns false when the graph cannot be built
 // (the caller then runs host-checked chunks).
 bool build_krylov_loop(tf_handle* h, const Ctx& c, int method) {
     cudaGraph_t g = nullptr;
@@ -786,8 +793,8 @@ bool build_krylov_loop(tf_handle* h, const Ctx& c, int method) {
         ok = cudaStreamBeginCaptureToGraph(h->stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal) ==
              cudaSuccess;
         if (ok) {
-            issue_iterations(h, c, method, 1);
-            k_krylov_ctl<<<1, 32, 0, h->stream>>>(h->d.scal, h->d.nseg, h->kloop_ctl, hc);
+            issue_iterations(h, c, method, loop_iterations(h));
+            k_krylov_ctl<<<1, 32, 0, h->stream>>>(h->d.scal, h->d.nseg, h->kloop_ctl, loop_iterations(h), hc);
             cudaGraph_t out = nullptr;
             ok = cudaStreamEndCapture(h->stream, &out) == cudaSuccess;
         }
@@ -871,8 +878,9 @@ tf_status krylov_run(tf_handle* h, int method, int keep, int* iters, double* rel
         TF_CUDA(cudaMallocHost(&h->kloop_host, sizeof(int)));
     }
     if (!h->kloop_off && !h->kloop[method - 1] && !build_krylov_loop(h, c, method)) h->kloop_off = true;
-    if (!h->kloop_off) {
-        // the device-side loop: every iteration until convergence (or the cap)
+    if (!h->kloop_off && maxit >= loop_iterations(h)) {
+        // the device-side loop: every iteration until convergence (or less than a
+        // body's iterations from the cap: the rest is issued below)
         k_krylov_arm<<<1, 1, 0, st>>>(h->kloop_ctl, maxit, 0, 0);
         TF_LAUNCH_CHECK(h);
         TF_CUDA(cudaGraphLaunch(h->kloop[method - 1], st));
@@ -880,8 +888,11 @@ tf_status krylov_run(tf_handle* h, int method, int keep, int* iters, double* rel
         TF_CUDA(cudaMemcpyAsync(d.host_scal, d.scal, sizeof(double) * nscal, cudaMemcpyDeviceToHost, st));
         TF_CUDA(cudaStreamSynchronize(st));
         launched = *h->kloop_host;
-        h->launches += (int64_t)launched * (kernels_per_iteration(h, method) + 1);
+        h->launches += (int64_t)launched * kernels_per_iteration(h, method) + launched / loop_iterations(h);
         done = true;
+        for (int g = 0; g < d.nseg && done; ++g)
+            if (d.host_scal[(size_t)g * S_COUNT + S_FLAG] == F_RUNNING) done = false;
+        planned = 0;
     }
     while (launched < maxit && !done) {
         int target = planned > 0 ? planned : (fixed ? kChunk0 : (kChunk0 << ci));
@@ -1203,10 +1214,11 @@ bool issue_newton_iteration(tf_handle* h, cudaGraphConditionalHandle newton) {
     }
     cudaGraphConditionalHandle kc = 0;
     if (!capture_handle(h, &kc)) return false;
-    k_krylov_arm<<<1, 1, 0, st>>>(h->kloop_ctl, krylov_cap(h), kc, 1);
+    const int n = loop_iterations(h);
+    k_krylov_arm<<<1, 1, 0, st>>>(h->kloop_ctl, krylov_cap(h), kc, n);
     bool ok = capture_while(h, kc, [&] {
-        issue_iterations(h, c, method, 1);
-        k_krylov_ctl<<<1, 32, 0, h->stream>>>(d.scal, d.nseg, h->kloop_ctl, kc);
+        issue_iterations(h, c, method, n);
+        k_krylov_ctl<<<1, 32, 0, h->stream>>>(d.scal, d.nseg, h->kloop_ctl, n, kc);
     });
     if (!ok) return false;
     k_update<false><<<d.ncta, vector_threads(d), 0, st>>>(c, d.uk, d.du);
@@ -1332,10 +1344,12 @@ tf_status newton_device_loop(tf_handle* h, int* it, int* cv, int* capped, int* k
     st->krylov_iters_max = std::max(st->krylov_iters_max, nh.krylov_max);
     *ms_asm += (float)(nh.t_asm * 1e-6);
     // kernels the graph ran: the fixed ones of each Newton iteration (an
-    // iteration handed back ran all but the update) and one control kernel
-    // more than the solver's own per Krylov iteration
+    // iteration handed back ran all but the update), the solver's own per Krylov
+    // iteration (those that ran past convergence not counted) and a control kernel
+    // per body of the Krylov loop
     h->launches += (int64_t)(done + (*exc ? 1 : 0)) * h->nloop_kernels +
-                   (int64_t)nh.krylov_total * (kernels_per_iteration(h, h->method) + 1);
+                   (int64_t)nh.krylov_total * kernels_per_iteration(h, h->method) +
+                   nh.krylov_total / loop_iterations(h);
     if (use_multigrid(h)) amg_refreshed(h);
     h->assembled = true;
     return TF_OK;
