@@ -118,17 +118,17 @@ def algorithmic_bytes(nn, ne, nnz):
 
 # Instruction mix of one element-kernel launch, counted with ncu on the
 # 135,200-prism sheet with internal viscosity (per prism): FP64 flops
-# (2 x DFMA + DADD + DMUL thread instructions; phase A and the joins) and
+# (2 x DFMA + DADD + DMUL thread instructions; the Gauss points and the forces) and
 # FP32 thread instructions (FADD + FFMA + FMUL; the double-float block sums),
 # with the FP64 pipe's busy fraction ncu reported.  The elastic-only counts
 # apply when every eta is 0 (not captured).
-FP64_FLOPS_PER_PRISM = {"viscous": 4644, "elastic": None}
-FP32_INST_PER_PRISM = {"viscous": 136492, "elastic": None}
-FP64_PIPE_PCT_NCU = {"viscous": 44.1, "elastic": None}
+FP64_FLOPS_PER_PRISM = {"viscous": 2171, "elastic": None}
+FP32_INST_PER_PRISM = {"viscous": 66498, "elastic": None}
+FP64_PIPE_PCT_NCU = {"viscous": 43.3, "elastic": None}
 # DRAM bytes (read + write) per prism of one element-kernel launch, from the
-# same ncu capture (333.1 MB at 135,200 prisms); the kernel's traffic grows
+# same ncu capture (258.2 MB at 135,200 prisms); the kernel's traffic grows
 # with the number of prisms, so a full launch is scaled from it.
-DRAM_BYTES_PER_PRISM = {"viscous": 333.1e6 / 135200, "elastic": None}
+DRAM_BYTES_PER_PRISM = {"viscous": 258.2e6 / 135200, "elastic": None}
 FP64_PEAK_TFLOPS = 304 * 2 * 2.07e9 / 1e12
 
 

@@ -62,9 +62,10 @@
 // instruction cache.
 // The phases of one CTA use one pipe at a time; three CTAs on an SM overlap them
 // (with the u_j and s_jl kept in shared memory two fit: 2.58 against 1.94 ms).
-// FP64 pipe and issue slots are each half busy: ~1,450 FP64 instructions per prism
-// (3,156 before), ~130,000 thread instructions per prism in all; the rest is the barriers
-// between the phases (starting the CTAs of an SM in different phases: no change).
+// FP64 pipe and issue slots are each half busy: 1,496 FP64 instructions per prism
+// (3,156 before), ~120,000 thread instructions per prism in all; the rest is the barriers
+// between the phases (starting the CTAs of an SM in different phases: no change; two
+// threads per Gauss point: 1.77 ms with viscosity, but 1.29 without).
 // 320,000 prisms: 3.62 -> 1.81 ms with viscosity, 2.18 -> 1.26 ms without.  K's error against 64 bits, relative (2-norm): 2.0e-15 to 2.4e-15 without
 // viscosity (before 2.1e-15 to 2.2e-15), 2.4e-15 to 2.9e-15 with (2.6e-15 to 3.2e-15).
 // The matrix assembled is A = K^T, the system the reference
@@ -1319,7 +1320,7 @@ tf_status launch_shape_gradients(tf_handle* h, const double* dN) {
 // = w dV / J.  They change with the growth, once per time step, and take a matrix
 // product, a determinant and a division out of every Gauss point of every assembly:
 // a sixth of its FP64 instructions (320,000 prisms 1.37 -> 1.26 ms without
-// viscosity, 1.89 -> 1.81 with; one pass over 138 MB per change of the growth).  C = M M^T in place of M would save
+// viscosity, 1.89 -> 1.81 with; 0.15 ms per change of the growth).  C = M M^T in place of M would save
 // three loads, but X^T C X loses the digits of a skewed prism's M twice.
 __global__ void k_metric(int ne, const double* __restrict__ ginv, const double* __restrict__ invFg,
                          double* __restrict__ metric) {
