@@ -619,6 +619,30 @@ __global__ void k_update(Ctx c, double* __restrict__ uk, const double* __restric
     }
 }
 
+// The residual of a converged solve, formed again from x: b - A x.  Near a loss of
+// stability the multigrid's coarse matrix comes close to singular, its answers to
+// vectors of any size, and BiCGStab's recurrence then converges on a residual that x
+// no longer has (a grown 192-prism sheet: one run in nine ended in a tangled
+// shape, none with block-Jacobi).  An instance whose residual is ten times the tolerance
+// asked for (and 1e-9 of |b|: the rounding of A x at tight ones) is flagged F_DRIFT.
+// Costs a product; run where block-Jacobi stands by (verifies).
+__global__ void k_verify(Ctx c, const double* __restrict__ b, const double* __restrict__ x) {
+    const Where w = where(c);
+    if (w.flag != F_CONVERGED || __ldcg(&w.s[S_BB]) == 0.0) return;
+    double y[3], bi[3], v[1] = {0.0};
+    rows_product<2>(c, warp_slots(c), x, y);
+    if (w.valid) load3(b, w.node, bi);
+    rows_sum(c, w, x, y);
+    if (w.valid)
+#pragma unroll
+        for (int d = 0; d < 3; ++d) v[0] = fma(bi[d] - y[d], bi[d] - y[d], v[0]);
+    double tot[1];
+    if (reduce_seg<1>(c, w.seg, v, tot) && threadIdx.x == 0 &&
+        !(tot[0] <= fmax(100.0 * __ldcg(&w.s[S_TOL2]), 1e-18) * __ldcg(&w.s[S_BB])))
+        w.s[S_FLAG] = F_DRIFT;
+}
+bool verifies(const tf_handle* h) { return h->amg_trial && use_multigrid(h); }
+
 // Issues n iterations of `method` on the stream (no host interaction).
 template <int U>
 void issue_iterations_u(tf_handle* h, const Ctx& c, int method, int n) {
@@ -884,6 +908,10 @@ tf_status krylov_run(tf_handle* h, int method, int keep, int* iters, double* rel
         k_krylov_arm<<<1, 1, 0, st>>>(h->kloop_ctl, maxit, 0, 0);
         TF_LAUNCH_CHECK(h);
         TF_CUDA(cudaGraphLaunch(h->kloop[method - 1], st));
+        if (verifies(h)) {
+            k_verify<<<d.ncta, kThreads, split_bytes<double>(d), st>>>(c, d.g, d.du);
+            TF_LAUNCH_CHECK(h);
+        }
         TF_CUDA(cudaMemcpyAsync(h->kloop_host, h->kloop_ctl, sizeof(int), cudaMemcpyDeviceToHost, st));
         TF_CUDA(cudaMemcpyAsync(d.host_scal, d.scal, sizeof(double) * nscal, cudaMemcpyDeviceToHost, st));
         TF_CUDA(cudaStreamSynchronize(st));
@@ -913,6 +941,10 @@ tf_status krylov_run(tf_handle* h, int method, int keep, int* iters, double* rel
             issued = target;
         }
         launched += issued;
+        if (verifies(h)) {
+            k_verify<<<d.ncta, kThreads, split_bytes<double>(d), st>>>(c, d.g, d.du);
+            TF_LAUNCH_CHECK(h);
+        }
         TF_CUDA(cudaMemcpyAsync(d.host_scal, d.scal, sizeof(double) * nscal, cudaMemcpyDeviceToHost, st));
         TF_CUDA(cudaStreamSynchronize(st));
         done = true;
@@ -935,6 +967,7 @@ tf_status krylov_run(tf_handle* h, int method, int keep, int* iters, double* rel
         if (s[S_BB] > 0.0) rmax = std::max(rmax, std::sqrt(s[S_RR] / s[S_BB]));
         if (f == F_NAN) worst = F_NAN;
         else if (f == F_BREAKDOWN && worst != F_NAN) worst = F_BREAKDOWN;
+        else if (f == F_DRIFT && (worst == F_CONVERGED || worst == F_RUNNING)) worst = F_DRIFT;
         else if (f == F_RUNNING && worst == F_CONVERGED) worst = F_RUNNING;
     }
     *iters = itmax;
@@ -957,7 +990,8 @@ tf_status krylov_run(tf_handle* h, int method, int keep, int* iters, double* rel
         set_error("Krylov breakdown" + where);
         return TF_KRYLOV_BREAKDOWN;
     }
-    set_error("linear solve reached its iteration cap");
+    set_error(worst == F_DRIFT ? "the linear solve's residual drifted from its recurrence"
+                               : "linear solve reached its iteration cap");
     return TF_KRYLOV_NOT_CONVERGED;
 }
 
@@ -1221,6 +1255,7 @@ bool issue_newton_iteration(tf_handle* h, cudaGraphConditionalHandle newton) {
         k_krylov_ctl<<<1, 32, 0, h->stream>>>(d.scal, d.nseg, h->kloop_ctl, n, kc);
     });
     if (!ok) return false;
+    if (verifies(h)) k_verify<<<d.ncta, kThreads, split_bytes<double>(d), st>>>(c, d.g, d.du);
     k_update<false><<<d.ncta, vector_threads(d), 0, st>>>(c, d.uk, d.du);
     int* seg = h->nd_seg;
     k_newton_ctl<<<1, 256, 0, st>>>(d.scal, d.nseg, d.seg_active, seg, seg + d.nseg, seg + 2 * d.nseg, h->nd,
@@ -1253,12 +1288,12 @@ bool build_newton_loop(tf_handle* h) {
             // kernels of one iteration outside the Krylov loop: two time
             // stamps, prepare, element (+2 order-fixed gathers), block
             // inverse, the multigrid refresh (3), the solver's start (CG with
-            // multigrid: init, a V-cycle, rz), the loop arm, |du|, the Newton
-            // test and the update
+            // multigrid: init, a V-cycle, rz), the loop arm, the check of the
+            // residual, |du|, the Newton test and the update
             const bool mg = use_multigrid(h);
             h->nloop_kernels = 2 + 2 + (h->opt.deterministic ? 2 : 0) + 1 + (mg ? 3 : 0) +
                                (h->method == 1 && mg ? 1 + (amg_fuses_dot(h) ? 0 : 1) + amg_vcycle_kernels(h) : 1) +
-                               1 + 3;
+                               1 + (verifies(h) ? 1 : 0) + 3;
             cudaGraph_t out = nullptr;
             ok = (cudaStreamEndCapture(h->stream, &out) == cudaSuccess) && ok;
         }

@@ -9,7 +9,7 @@ namespace tf {
 
 constexpr int kThreads = kNodeThreads;
 
-enum Flag { F_RUNNING = 0, F_CONVERGED = 1, F_BREAKDOWN = 2, F_NAN = 3 };
+enum Flag { F_RUNNING = 0, F_CONVERGED = 1, F_BREAKDOWN = 2, F_NAN = 3, F_DRIFT = 4 };
 // Cause of a breakdown (S_WHY): which denominator vanished.
 enum Why { W_NONE = 0, W_CG_PAP = 1, W_CG_RZ = 2, W_BI_RV = 3, W_BI_OMEGA = 4, W_BI_RHO = 5 };
 static const char* const kWhy[] = {"", "(p, Ap) <= 0", "(r, M^-1 r) <= 0", "(rhat, A phat) = 0", "omega = 0",
