@@ -77,7 +77,8 @@ typedef struct tf_options {
     int32_t autotune_off;    /* 1: keep 16 prisms per CTA instead of timing 8/16/32 on the mesh */
     int32_t precond;         /* 0 auto (smoothed-aggregation multigrid from 20,000 nodes on
                                 and, with the atomic assembly, on smaller meshes too, there
-                                with block-Jacobi in its place once a solve with it fails;
+                                with block-Jacobi in its place once a solve with it fails
+                                or leaves a residual ten times the one its recurrence shows;
                                 else block-Jacobi), 1 block-Jacobi, 2 smoothed-aggregation
                                 multigrid, 3 plain-aggregation multigrid (no reference
                                 counterpart for 2 and 3); other values: TF_BAD_INPUT */
@@ -127,7 +128,8 @@ typedef struct tf_step_stats {
     int32_t device_handback;    /* why that loop handed an iteration back to the host: 0 it did not,
                                    1 a loosened solve's |du| near newton_tol, 3 a non-finite update,
                                    10 + the Krylov flag (11 converged is not used, 12 breakdown, 13 NaN,
-                                   10 still running at the iteration cap) for a solve that did not converge */
+                                   14 a residual that drifted from its recurrence, 10 still running at
+                                   the iteration cap) for a solve that did not converge */
 } tf_step_stats;
 
 TF_API const char* tf_status_string(tf_status s);
