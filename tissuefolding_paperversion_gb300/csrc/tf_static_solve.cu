@@ -17,14 +17,15 @@
 // returns TF_BAD_INPUT and leaves the capture untouched.  All calls on a device
 // share the one array: calls that overlap on the GPU (two streams, two host
 // threads) race on it and give wrong results or an error, so serialise them.
-// Each call clears the scalars and the count of the CTAs' meetings before its
-// kernel, and writes every work vector before reading it, so nothing carries
+// Each call sets the count of the CTAs' meetings before its kernel, and writes
+// the scalars and every work vector before reading it, so nothing carries
 // over from the previous call.
 #include <cuda.h>
 
 #include <algorithm>
 #include <mutex>
 
+#include "tf_count.h"
 #include "tf_internal.cuh"
 
 namespace tf {
@@ -49,6 +50,9 @@ constexpr size_t kOffBar = kOffScal + kNumScal;
 constexpr size_t kScratchDoubles = kOffBar + 2;
 constexpr int kStaticSmem = 200 * 1024;
 constexpr int kStaticPolls = 1 << 22;         // a wait for the other CTAs gives up after some seconds
+// The count of the CTAs' arrivals wraps after 5.65 M iterations on 152 SMs.  It
+// starts one below the wrap (a memset's pattern), so every solve crosses it.
+constexpr unsigned kCountStart = 0xffffffffu;
 
 __device__ __align__(256) double g_static_scratch[kScratchDoubles];
 
@@ -91,8 +95,8 @@ __device__ __forceinline__ bool s_barrier(const SCtx& c, SShared& sh, unsigned& 
         int polls = 0;
         do {
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(bar) : "memory");
-        } while (seen < goal && ++polls < kStaticPolls);
-        if (seen < goal) sh.stuck = 1;
+        } while (!count_reached(seen, goal) && ++polls < kStaticPolls);
+        if (!count_reached(seen, goal)) sh.stuck = 1;
     }
     __syncthreads();
     return !sh.stuck;
@@ -299,7 +303,7 @@ __global__ void __launch_bounds__(kStaticThreads, 1) ks_solve(SCtx c, const doub
             bb[0] = fma(bk, bk, bb[0]);
         }
     }
-    unsigned goal = 0;
+    unsigned goal = kCountStart;
     bool ok = s_reduce<1>(c, sh, goal, 0, slot_row, slots_row, bb, [&](const double* q) {
         sh.rho = sh.rr = sh.bb = q[0];
         sh.alpha = sh.omega = 1.0;
@@ -496,18 +500,19 @@ extern "C" TF_API tf_status tf_solve_bsr_static(int32_t n_block_rows, const int3
     const int grid0 = std::min(sms, cdiv(n_block_rows, 32));
     const int rows = cdiv(n_block_rows, grid0);
     SCtx c{n_block_rows, rows, max_iter, rtol * rtol, rowptr, colidx, val, base};
-    // clear the scalars and the barrier
-    TF_CUDA(cudaMemsetAsync(base + kOffScal, 0, sizeof(double) * (kNumScal + 2), st));
+    // the count to kCountStart; the scalars are the kernel's to write
+    TF_CUDA(cudaMemsetAsync(base + kOffScal, 0xff, sizeof(double) * (kNumScal + 2), st));
     TF_CUDA(cudaFuncSetAttribute(ks_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, kStaticSmem));
     launch_cooperative(ks_solve, cdiv(n_block_rows, rows), kStaticThreads, kStaticSmem, st, c, b, x);
     TF_CUDA(cudaGetLastError());
     double q[kNumScal];
     TF_CUDA(cudaMemcpyAsync(q, base + kOffScal, sizeof(q), cudaMemcpyDeviceToHost, st));
     TF_CUDA(cudaStreamSynchronize(st));
-    if (iters) *iters = static_cast<int32_t>(q[Q_ITER]);
-    if (relres) *relres = q[Q_BB] > 0.0 ? sqrt(q[Q_RR] / q[Q_BB]) : 0.0;
+    const bool stuck = !(q[Q_FLAG] < QF_STUCK);  // or not written: an overlapping call's memset
+    if (iters) *iters = stuck ? 0 : static_cast<int32_t>(q[Q_ITER]);
+    if (relres) *relres = !stuck && q[Q_BB] > 0.0 ? sqrt(q[Q_RR] / q[Q_BB]) : 0.0;
     if (q[Q_FLAG] == QF_CONVERGED) return TF_OK;
-    if (q[Q_FLAG] == QF_STUCK) {
+    if (stuck) {
         set_error("tf_solve_bsr_static: the thread blocks lost each other (overlapping calls?)");
         return TF_CUDA_ERROR;
     }
