@@ -347,3 +347,36 @@ def test_solves_near_a_loss_of_stability_keep_their_residual(run):
         for i in range(900):
             out = s.newton_step(t.dt, allow_not_converged=False)
             assert out["iters"] <= 4, (i, out["dunorm"])
+
+
+# The static solve where fewer thread blocks than SMs can be resident together: one
+# block, a few (their vectors in global memory, several groups of rows a warp),
+# and 512, which no GPU of this kind takes together: it then runs with fewer.
+@pytest.mark.parametrize("blocks", [1, 3, 17, 60, 512])
+@pytest.mark.parametrize("n,most", [(33, 9), (2000, 30), (16384, 27)])
+def test_static_solve_on_fewer_blocks(n, most, blocks):
+    import ctypes as C
+
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(n)
+    rows = np.repeat(np.arange(n), rng.integers(0, most, size=n))
+    key = np.unique(np.concatenate([rows * n + rng.integers(0, n, size=rows.size), np.arange(n) * n + np.arange(n)]))
+    br, bc = key // n, key % n
+    val = rng.uniform(-1.0, 1.0, size=(key.size, 3, 3))
+    val[br == bc] += 4.0 * most * np.eye(3)
+    b = rng.uniform(-1.0, 1.0, size=3 * n)
+    d = [torch.from_numpy(np.ascontiguousarray(v)).cuda()
+         for v in (np.searchsorted(br, np.arange(n + 1)).astype(np.int32), bc.astype(np.int32), val.reshape(-1), b)]
+    x = torch.full((3 * n,), float("nan"), dtype=torch.float64, device="cuda")
+    it, rr = C.c_int32(0), C.c_double(0.0)
+    p = [C.c_void_p(a.data_ptr()) for a in d]
+    L = api.load()
+    st = L.tf_static_solve_blocks(blocks, n, *p, C.c_void_p(x.data_ptr()), C.c_double(RTOL), 500, None, C.byref(it),
+                                  C.byref(rr))
+    assert st == api.TF_OK, L.tf_last_error().decode()
+    xs = x.cpu().numpy().reshape(n, 3)
+    Ax, mag = np.zeros((n, 3)), np.zeros((n, 3))
+    np.add.at(Ax, br, np.einsum("kij,kj->ki", val, xs[bc]))
+    np.add.at(mag, br, np.einsum("kij,kj->ki", np.abs(val), np.abs(xs[bc])))
+    bound = RTOL + 4 * EPS * it.value * np.linalg.norm(mag) / np.linalg.norm(b)
+    assert rr.value <= RTOL and np.linalg.norm(b - Ax.reshape(-1)) <= bound * np.linalg.norm(b)

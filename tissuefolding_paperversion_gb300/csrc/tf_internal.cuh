@@ -369,8 +369,8 @@ inline void launch_pdl(void (*kernel)(KArgs...), int grid, int block, cudaStream
 
 // All CTAs resident at once (they meet at a grid barrier).
 template <typename... KArgs, typename... Args>
-inline void launch_cooperative(void (*kernel)(KArgs...), int grid, int block, size_t smem, cudaStream_t st,
-                               Args... args) {
+inline cudaError_t launch_cooperative(void (*kernel)(KArgs...), int grid, int block, size_t smem, cudaStream_t st,
+                                      Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(block);
@@ -381,7 +381,7 @@ inline void launch_cooperative(void (*kernel)(KArgs...), int grid, int block, si
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
 // y = this thread's row of the sliced block matrix times x.  T is the

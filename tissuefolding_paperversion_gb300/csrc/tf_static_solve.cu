@@ -470,10 +470,14 @@ tf_status scratch_address(int device, double** out) {
 
 using namespace tf;
 
-extern "C" TF_API tf_status tf_solve_bsr_static(int32_t n_block_rows, const int32_t* rowptr, const int32_t* colidx,
-                                                const double* val, const double* b, double* x, double rtol,
-                                                int32_t max_iter, void* stream, int32_t* iters, double* relres) {
-    if (n_block_rows <= 0 || !rowptr || !colidx || !val || !b || !x || !(rtol > 0.0) || max_iter <= 0) {
+// With up to max_blocks thread blocks (tests; tf_solve_bsr_static asks for one per
+// SM, max_blocks = 0).
+extern "C" TF_API tf_status tf_static_solve_blocks(int32_t max_blocks, int32_t n_block_rows, const int32_t* rowptr,
+                                                   const int32_t* colidx, const double* val, const double* b,
+                                                   double* x, double rtol, int32_t max_iter, void* stream,
+                                                   int32_t* iters, double* relres) {
+    if (n_block_rows <= 0 || !rowptr || !colidx || !val || !b || !x || !(rtol > 0.0) || max_iter <= 0 ||
+        max_blocks < 0) {
         set_error("tf_solve_bsr_static: bad arguments");
         return TF_BAD_INPUT;
     }
@@ -495,16 +499,25 @@ extern "C" TF_API tf_status tf_solve_bsr_static(int32_t n_block_rows, const int3
     double* base = nullptr;
     tf_status s = scratch_address(device, &base);
     if (s != TF_OK) return s;
-    int sms = 0;
-    TF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-    const int grid0 = std::min(sms, cdiv(n_block_rows, 32));
-    const int rows = cdiv(n_block_rows, grid0);
-    SCtx c{n_block_rows, rows, max_iter, rtol * rtol, rowptr, colidx, val, base};
+    int sms = max_blocks;
+    if (max_blocks == 0) TF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    SCtx c{n_block_rows, 0, max_iter, rtol * rtol, rowptr, colidx, val, base};
     // the count to kCountStart; the scalars are the kernel's to write
     TF_CUDA(cudaMemsetAsync(base + kOffScal, 0xff, sizeof(double) * (kNumScal + 2), st));
     TF_CUDA(cudaFuncSetAttribute(ks_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, kStaticSmem));
-    launch_cooperative(ks_solve, cdiv(n_block_rows, rows), kStaticThreads, kStaticSmem, st, c, b, x);
-    TF_CUDA(cudaGetLastError());
+    // One block per SM.  Where not all of them can be resident together (a stream
+    // that owns a part of the SMs only), half as many until they can: one always fits.
+    int blocks = std::min(sms, cdiv(n_block_rows, 32));
+    while (true) {
+        c.rows = cdiv(n_block_rows, blocks);
+        blocks = cdiv(n_block_rows, c.rows);
+        const cudaError_t e =
+            launch_cooperative(ks_solve, blocks, kStaticThreads, kStaticSmem, st, c, b, x);
+        if (e == cudaSuccess) break;
+        (void)cudaGetLastError();
+        if (e != cudaErrorCooperativeLaunchTooLarge || blocks == 1) return cuda_fail(e, "tf_solve_bsr_static");
+        blocks /= 2;
+    }
     double q[kNumScal];
     TF_CUDA(cudaMemcpyAsync(q, base + kOffScal, sizeof(q), cudaMemcpyDeviceToHost, st));
     TF_CUDA(cudaStreamSynchronize(st));
@@ -526,4 +539,11 @@ extern "C" TF_API tf_status tf_solve_bsr_static(int32_t n_block_rows, const int3
     }
     set_error("tf_solve_bsr_static: iteration cap reached");
     return TF_KRYLOV_NOT_CONVERGED;
+}
+
+extern "C" TF_API tf_status tf_solve_bsr_static(int32_t n_block_rows, const int32_t* rowptr, const int32_t* colidx,
+                                                const double* val, const double* b, double* x, double rtol,
+                                                int32_t max_iter, void* stream, int32_t* iters, double* relres) {
+    return tf_static_solve_blocks(0, n_block_rows, rowptr, colidx, val, b, x, rtol, max_iter, stream, iters,
+                                  relres);
 }
