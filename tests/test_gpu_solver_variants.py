@@ -380,3 +380,34 @@ def test_static_solve_on_fewer_blocks(n, most, blocks):
     np.add.at(mag, br, np.einsum("kij,kj->ki", np.abs(val), np.abs(xs[bc])))
     bound = RTOL + 4 * EPS * it.value * np.linalg.norm(mag) / np.linalg.norm(b)
     assert rr.value <= RTOL and np.linalg.norm(b - Ax.reshape(-1)) <= bound * np.linalg.norm(b)
+
+
+def _bending_sheet():
+    """192 viscous prisms in eight layers, the apical half growing half as fast
+    again: past some 800 steps it comes near a loss of stability."""
+    rng = np.random.default_rng(3)
+    pos, conn, pl = mesh.rect_sheet(5, 4, 5.0, 8, 40.0, 0.5, rng)
+    ne, nn = conn.size // 6, pl.size
+    fixed = np.zeros((nn, 3), dtype=np.uint8)
+    fixed[pl == 0, 2] = 1
+    ev = np.zeros((nn, 3))
+    ev[pl != 2] = 10.0
+    t = mesh.Tissue(pos=pos, conn=conn, fixed=fixed.reshape(-1), ext_visc=ev.reshape(-1), node_placement=pl,
+                    E=1000.0 * rng.uniform(0.98, 1.02, size=ne), nu=np.full(ne, 0.3), eta=np.full(ne, 100.0),
+                    rates=np.zeros(3 * ne))
+    g = (0.01 + 0.005 * (t.centroids()[:, 2] >= 20.0)) * 1.02 / mesh.HOUR
+    t.rates = np.stack([g, g, np.zeros(ne)], axis=1).reshape(-1)
+    return t
+
+
+# A batch of 20,000 nodes of such sheets keeps the multigrid whatever happens: a
+# drifted solve goes on from its own residual, at the 4 Newton iterations a step of
+# block-Jacobi (without the check both of two runs ended in non-finite values).
+def test_batch_near_a_loss_of_stability_keeps_its_residuals():
+    ts = [_bending_sheet() for _ in range(112)]
+    with api.Batch(ts) as s:
+        assert s.multigrid_info()[0][0] == 20160
+        s.set_growth_rates()
+        for i in range(840):
+            out = s.step(ts[0].dt)
+            assert np.all(out["converged"]) and np.max(out["iters"]) <= 4, i

@@ -272,6 +272,32 @@ __global__ void k_cg_update(Ctx c, double* __restrict__ x, double* __restrict__ 
     }
 }
 
+// Starts CG again from x: r = b - A x is in place (k_verify), z and p follow from the
+// V-cycle.  |b|, the tolerance and the iteration count carry over.  Instances
+// outside seg_solve keep their result and are flagged done.
+__global__ void k_cg_restart(Ctx c, const double* __restrict__ r, AmgPre pre) {
+    const Where w = where(c);
+    if (c.seg_solve[w.seg] == 0) {
+        if (threadIdx.x == 0) w.s[S_FLAG] = F_CONVERGED;
+        return;
+    }
+    double v[1] = {0.0};
+    if (w.valid) {
+        double rr[3];
+        load3(r, w.node, rr);
+        pre_smooth(pre, w.node, rr, pre_load(pre, w.node));
+#pragma unroll
+        for (int d = 0; d < 3; ++d) v[0] = fma(rr[d], rr[d], v[0]);
+    }
+    double tot[1];
+    if (reduce_seg<1>(c, w.seg, v, tot) && threadIdx.x == 0) {
+        w.s[S_RR] = tot[0];
+        w.s[S_WHY] = W_NONE;
+        if (!isfinite(tot[0])) w.s[S_FLAG] = F_NAN;
+        else w.s[S_FLAG] = (tot[0] <= w.s[S_TOL2] * w.s[S_BB]) ? F_CONVERGED : F_RUNNING;
+    }
+}
+
 // With the multigrid preconditioner (z = M^-1 r computed between kernels), where
 // its last kernel does not do it (systems with extra blocks):
 // rz = (r, z), beta = rz / rz_old; start != 0 also sets p = z (first step).
@@ -619,14 +645,14 @@ __global__ void k_update(Ctx c, double* __restrict__ uk, const double* __restric
     }
 }
 
-// The residual of a converged solve, formed again from x: b - A x.  Near a loss of
-// stability the multigrid's coarse matrix comes close to singular, its answers to
+// The residual of a converged solve, formed again from x: r = b - A x.  Near a loss
+// of stability the multigrid's coarse matrix comes close to singular, its answers to
 // vectors of any size, and BiCGStab's recurrence then converges on a residual that x
-// no longer has (a grown 192-prism sheet: one run in nine ended in a tangled
-// shape, none with block-Jacobi).  An instance whose residual is ten times the tolerance
-// asked for (and 1e-9 of |b|: the rounding of A x at tight ones) is flagged F_DRIFT.
-// Costs a product; run where block-Jacobi stands by (verifies).
-__global__ void k_verify(Ctx c, const double* __restrict__ b, const double* __restrict__ x) {
+// no longer has (a grown 192-prism sheet ended in a tangled shape, never with
+// block-Jacobi).  An instance whose residual is ten times the tolerance
+// asked for (and 1e-9 of |b|: the rounding of A x at tight ones) is flagged F_DRIFT
+// and solved on from its x (settle).  Costs a product.
+__global__ void k_verify(Ctx c, const double* __restrict__ b, const double* __restrict__ x, double* __restrict__ r) {
     const Where w = where(c);
     if (w.flag != F_CONVERGED || __ldcg(&w.s[S_BB]) == 0.0) return;
     double y[3], bi[3], v[1] = {0.0};
@@ -635,13 +661,22 @@ __global__ void k_verify(Ctx c, const double* __restrict__ b, const double* __re
     rows_sum(c, w, x, y);
     if (w.valid)
 #pragma unroll
-        for (int d = 0; d < 3; ++d) v[0] = fma(bi[d] - y[d], bi[d] - y[d], v[0]);
+        for (int d = 0; d < 3; ++d) {
+            const double rd = bi[d] - y[d];
+            r[3 * w.node + d] = rd;
+            v[0] = fma(rd, rd, v[0]);
+        }
     double tot[1];
     if (reduce_seg<1>(c, w.seg, v, tot) && threadIdx.x == 0 &&
-        !(tot[0] <= fmax(100.0 * __ldcg(&w.s[S_TOL2]), 1e-18) * __ldcg(&w.s[S_BB])))
+        !(tot[0] <= fmax(100.0 * __ldcg(&w.s[S_TOL2]), 1e-18) * __ldcg(&w.s[S_BB]))) {
+        w.s[S_RR] = tot[0];
         w.s[S_FLAG] = F_DRIFT;
+    }
 }
-bool verifies(const tf_handle* h) { return h->amg_trial && use_multigrid(h); }
+void launch_verify(tf_handle* h, const Ctx& c) {
+    Device& d = h->d;
+    k_verify<<<d.ncta, kThreads, split_bytes<double>(d), h->stream>>>(c, d.g, d.du, d.r);
+}
 
 // Issues n iterations of `method` on the stream (no host interaction).
 template <int U>
@@ -852,8 +887,9 @@ tf_status krylov_run(tf_handle* h, int method, int keep, int* iters, double* rel
     // first Newton iteration changes by ~0.1 % from step to step); the stop
     // test stays relative to |g|, so the accuracy is that of a zero start.
     const double* x0 = (keep == 0 && h->newton_index == 0 && h->have_du0) ? h->du0 : nullptr;
-    if (keep == 2) {  // BiCGStab restart: block inverse and x are kept
-        k_bi_restart<<<d.ncta, vector_threads(d), 0, st>>>(c, d.r, d.rhat, d.p, d.q);
+    if (keep == 2) {  // restart: block inverse and x are kept
+        if (method == 1) k_cg_restart<<<d.ncta, vector_threads(d), 0, st>>>(c, d.r, amg_pre(h));
+        else k_bi_restart<<<d.ncta, vector_threads(d), 0, st>>>(c, d.r, d.rhat, d.p, d.q);
     } else {
         const tf_status sb = launch_block_inverse(h);
         if (sb != TF_OK) return sb;
@@ -868,19 +904,19 @@ tf_status krylov_run(tf_handle* h, int method, int keep, int* iters, double* rel
         if (method == 1) {
             k_cg_init<<<d.ncta, kThreads, split_bytes<double>(d), st>>>(c, d.g, d.du, d.r, d.z, d.p, tol2, h->solve_atol, keep, jac, x0,
                                                    amg_pre(h));
-            if (!jac) {
-                amg_vcycle(h, d.r, d.z, kVcycleStart, d.p);
-                h->launches += amg_vcycle_kernels(h);
-                if (!amg_fuses_dot(h)) {
-                    k_cg_rz<<<d.ncta, vector_threads(d), 0, st>>>(c, d.r, d.z, d.p, 1);
-                    TF_LAUNCH_CHECK(h);
-                }
-            }
         } else {
             k_bi_init<<<d.ncta, kThreads, split_bytes<double>(d), st>>>(c, d.g, d.du, d.r, d.rhat, d.p, d.q, tol2, h->solve_atol, keep, x0);
         }
     }
     TF_LAUNCH_CHECK(h);
+    if (method == 1 && !jac) {
+        amg_vcycle(h, d.r, d.z, kVcycleStart, d.p);
+        h->launches += amg_vcycle_kernels(h);
+        if (!amg_fuses_dot(h)) {
+            k_cg_rz<<<d.ncta, vector_threads(d), 0, st>>>(c, d.r, d.z, d.p, 1);
+            TF_LAUNCH_CHECK(h);
+        }
+    }
     const int maxit = krylov_cap(h);
     const size_t nscal = (size_t)d.nseg * S_COUNT;
     // Iterations run in graph chunks of 4/8/16/32/64 with a flag check after
@@ -908,8 +944,8 @@ tf_status krylov_run(tf_handle* h, int method, int keep, int* iters, double* rel
         k_krylov_arm<<<1, 1, 0, st>>>(h->kloop_ctl, maxit, 0, 0);
         TF_LAUNCH_CHECK(h);
         TF_CUDA(cudaGraphLaunch(h->kloop[method - 1], st));
-        if (verifies(h)) {
-            k_verify<<<d.ncta, kThreads, split_bytes<double>(d), st>>>(c, d.g, d.du);
+        if (!jac) {
+            launch_verify(h, c);
             TF_LAUNCH_CHECK(h);
         }
         TF_CUDA(cudaMemcpyAsync(h->kloop_host, h->kloop_ctl, sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -941,8 +977,8 @@ tf_status krylov_run(tf_handle* h, int method, int keep, int* iters, double* rel
             issued = target;
         }
         launched += issued;
-        if (verifies(h)) {
-            k_verify<<<d.ncta, kThreads, split_bytes<double>(d), st>>>(c, d.g, d.du);
+        if (!jac) {
+            launch_verify(h, c);
             TF_LAUNCH_CHECK(h);
         }
         TF_CUDA(cudaMemcpyAsync(d.host_scal, d.scal, sizeof(double) * nscal, cudaMemcpyDeviceToHost, st));
@@ -997,6 +1033,28 @@ tf_status krylov_run(tf_handle* h, int method, int keep, int* iters, double* rel
 
 }  // namespace
 
+// A solve; the instances whose residual drifted from the recurrence (k_verify) go
+// on from their x with the residual that it has.
+static tf_status settle(tf_handle* h, int method, int keep, int* iters, double* relres) {
+    Device& d = h->d;
+    tf_status s = krylov_run(h, method, keep, iters, relres);
+    for (int restart = 0; restart < 3 && s == TF_KRYLOV_NOT_CONVERGED; ++restart) {
+        std::vector<int> redo(d.nseg, 0);
+        bool drift = false, running = false;
+        for (int g = 0; g < d.nseg; ++g) {
+            const double f = d.host_scal[(size_t)g * S_COUNT + S_FLAG];
+            redo[g] = f == F_DRIFT ? 1 : 0;
+            drift = drift || f == F_DRIFT;
+            running = running || f == F_RUNNING;
+        }
+        if (!drift || running) break;  // a solve at its iteration cap stays one
+        TF_CUDA(cudaMemcpyAsync(d.seg_solve, redo.data(), sizeof(int) * (size_t)d.nseg, cudaMemcpyHostToDevice,
+                                h->stream));
+        s = krylov_run(h, method, 2, iters, relres);  // the iteration counts carry over
+    }
+    return s;
+}
+
 // Auto mode picks CG when the tangent is symmetric; CG needs a positive
 // definite operator, which large compressive growth can take away (the
 // geometric stiffness term), so the instances whose CG breaks down are solved
@@ -1006,7 +1064,7 @@ static tf_status krylov_attempt(tf_handle* h, int* iters, double* relres) {
     Device& d = h->d;
     TF_CUDA(cudaMemcpyAsync(d.seg_solve, d.seg_active, sizeof(int) * (size_t)d.nseg, cudaMemcpyDeviceToDevice,
                             h->stream));
-    tf_status s = krylov_run(h, h->method, 0, iters, relres);
+    tf_status s = settle(h, h->method, 0, iters, relres);
     if (s != TF_OK && use_multigrid(h) && amg_reused(h)) {
         // the coarse levels came from an earlier Newton iteration: rebuild
         // them for this matrix and solve again
@@ -1014,7 +1072,7 @@ static tf_status krylov_attempt(tf_handle* h, int* iters, double* relres) {
         TF_CUDA(cudaMemcpyAsync(d.seg_solve, d.seg_active, sizeof(int) * (size_t)d.nseg, cudaMemcpyDeviceToDevice,
                                 h->stream));
         int it2 = 0;
-        s = krylov_run(h, h->method, 0, &it2, relres);
+        s = settle(h, h->method, 0, &it2, relres);
         *iters += it2;
     }
     if (s == TF_KRYLOV_BREAKDOWN && h->method == 1 && h->opt.krylov_method == 0) {
@@ -1024,7 +1082,7 @@ static tf_status krylov_attempt(tf_handle* h, int* iters, double* relres) {
         TF_CUDA(cudaMemcpyAsync(d.seg_solve, redo.data(), sizeof(int) * (size_t)d.nseg, cudaMemcpyHostToDevice,
                                 h->stream));
         int it2 = 0;
-        s = krylov_run(h, 2, 1, &it2, relres);
+        s = settle(h, 2, 1, &it2, relres);
         *iters += it2;
     }
     // BiCGStab breakdowns: restart the instances concerned from their
@@ -1037,7 +1095,7 @@ static tf_status krylov_attempt(tf_handle* h, int* iters, double* relres) {
         TF_CUDA(cudaMemcpyAsync(d.seg_solve, redo.data(), sizeof(int) * (size_t)d.nseg, cudaMemcpyHostToDevice,
                                 h->stream));
         int it2 = 0;
-        s = krylov_run(h, 2, 2, &it2, relres);
+        s = settle(h, 2, 2, &it2, relres);
         *iters += it2;
     }
     return s;
@@ -1255,7 +1313,7 @@ bool issue_newton_iteration(tf_handle* h, cudaGraphConditionalHandle newton) {
         k_krylov_ctl<<<1, 32, 0, h->stream>>>(d.scal, d.nseg, h->kloop_ctl, n, kc);
     });
     if (!ok) return false;
-    if (verifies(h)) k_verify<<<d.ncta, kThreads, split_bytes<double>(d), st>>>(c, d.g, d.du);
+    if (mg) launch_verify(h, c);
     k_update<false><<<d.ncta, vector_threads(d), 0, st>>>(c, d.uk, d.du);
     int* seg = h->nd_seg;
     k_newton_ctl<<<1, 256, 0, st>>>(d.scal, d.nseg, d.seg_active, seg, seg + d.nseg, seg + 2 * d.nseg, h->nd,
@@ -1293,7 +1351,7 @@ bool build_newton_loop(tf_handle* h) {
             const bool mg = use_multigrid(h);
             h->nloop_kernels = 2 + 2 + (h->opt.deterministic ? 2 : 0) + 1 + (mg ? 3 : 0) +
                                (h->method == 1 && mg ? 1 + (amg_fuses_dot(h) ? 0 : 1) + amg_vcycle_kernels(h) : 1) +
-                               1 + (verifies(h) ? 1 : 0) + 3;
+                               1 + (mg ? 1 : 0) + 3;
             cudaGraph_t out = nullptr;
             ok = (cudaStreamEndCapture(h->stream, &out) == cudaSuccess) && ok;
         }
