@@ -76,12 +76,13 @@ typedef struct tf_options {
     int32_t device;          /* CUDA device ordinal */
     int32_t autotune_off;    /* 1: keep 16 prisms per CTA instead of timing 8/16/32 on the mesh */
     int32_t precond;         /* 0 auto (smoothed-aggregation multigrid from 20,000 nodes on
-                                and, with the atomic assembly, on smaller meshes too, there
-                                with block-Jacobi in its place once a solve with it fails
-                                or leaves a residual ten times the one its recurrence shows;
-                                else block-Jacobi), 1 block-Jacobi, 2 smoothed-aggregation
+                                and, with the atomic assembly, on smaller meshes too, which
+                                stay with block-Jacobi once a solve with it failed; else
+                                block-Jacobi), 1 block-Jacobi, 2 smoothed-aggregation
                                 multigrid, 3 plain-aggregation multigrid (no reference
-                                counterpart for 2 and 3); other values: TF_BAD_INPUT */
+                                counterpart for 2 and 3); other values: TF_BAD_INPUT.
+                                A multigrid solve that fails, or leaves a residual ten times
+                                the tolerance, is done again with block-Jacobi */
     double update_atol;      /* tf_newton_step / tf_batch_step only: absolute accuracy (um, 2-norm)
                                 each Newton update needs.  A linear solve stops at the looser of
                                 krylov_rtol and the relative residual that bounds the update's

@@ -411,3 +411,17 @@ def test_batch_near_a_loss_of_stability_keeps_its_residuals():
         for i in range(840):
             out = s.step(ts[0].dt)
             assert np.all(out["converged"]) and np.max(out["iters"]) <= 4, i
+
+
+# The multigrid asked for, one sheet: BiCGStab with it diverges at step 811 (as it did
+# in every run before, with non-finite values); block-Jacobi then solves the step and
+# the handle goes back to the multigrid.
+@pytest.mark.parametrize("run", range(2))
+def test_multigrid_solves_near_a_loss_of_stability_keep_their_residual(run):
+    t = _bending_sheet()
+    with api.Solver(t, precond=2) as s:
+        s.set_growth_rates(t.rates)
+        for i in range(840):
+            out = s.newton_step(t.dt, allow_not_converged=False)
+            assert out["iters"] <= 4, (i, out["dunorm"])
+        assert s.multigrid_info()[0]

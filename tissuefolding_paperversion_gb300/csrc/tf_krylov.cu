@@ -1101,17 +1101,26 @@ static tf_status krylov_attempt(tf_handle* h, int* iters, double* relres) {
     return s;
 }
 
-// A solve with the multigrid on trial (chosen by size where block-Jacobi is
-// the general path) that fails is done again with block-Jacobi, which then
-// stays for the handle; where that fails too, the system is to blame and its
-// answer is the one block-Jacobi gives.
+// Whether the last solve stopped at its iteration cap: slow, not failed.
+static bool capped(const tf_handle* h) {
+    for (int g = 0; g < h->d.nseg; ++g)
+        if (h->d.host_scal[(size_t)g * S_COUNT + S_FLAG] == F_RUNNING) return true;
+    return false;
+}
+
+// A multigrid solve that fails is done again with block-Jacobi, whose answer
+// then counts: near a loss of stability BiCGStab with the multigrid can diverge
+// where block-Jacobi converges.  A handle with the multigrid on trial (chosen by size
+// where block-Jacobi is the general path) stays with block-Jacobi once that
+// converged; others go back to the multigrid, and at their iteration cap they stop.
 tf_status krylov_solve(tf_handle* h, int* iters, double* relres) {
     const tf_status s = krylov_attempt(h, iters, relres);
-    if (s == TF_OK || !h->amg_trial || !use_multigrid(h) || s == TF_CUDA_ERROR || s == TF_OUT_OF_MEMORY) return s;
+    if (s == TF_OK || !use_multigrid(h) || s == TF_CUDA_ERROR || s == TF_OUT_OF_MEMORY) return s;
+    if (!h->amg_trial && s == TF_KRYLOV_NOT_CONVERGED && capped(h)) return s;
     destroy_graphs(h);  // they hold the multigrid's kernels
     h->amg_off = true;
     const tf_status t = krylov_attempt(h, iters, relres);
-    if (t == TF_OK) {
+    if (t == TF_OK && h->amg_trial) {
         h->amg_failed = true;
     } else {
         destroy_graphs(h);
