@@ -81,8 +81,9 @@ typedef struct tf_options {
                                 block-Jacobi), 1 block-Jacobi, 2 smoothed-aggregation
                                 multigrid, 3 plain-aggregation multigrid (no reference
                                 counterpart for 2 and 3); other values: TF_BAD_INPUT.
-                                A multigrid solve that fails, or leaves a residual ten times
-                                the tolerance, is done again with block-Jacobi */
+                                A multigrid solve that fails, or leaves a residual of more
+                                than ten times the tolerance (at a tight one: more than its
+                                rounding leaves), is done again with block-Jacobi */
     double update_atol;      /* tf_newton_step / tf_batch_step only: absolute accuracy (um, 2-norm)
                                 each Newton update needs.  A linear solve stops at the looser of
                                 krylov_rtol and the relative residual that bounds the update's
@@ -120,7 +121,7 @@ typedef struct tf_step_stats {
     int32_t krylov_iters_max;
     int32_t converged;          /* 1 if |du| <= tol before the cap */
     double dunorm[32];          /* |du|_2 of each Newton iteration (first 32) */
-    double final_relres;        /* relative residual of the last linear solve */
+    double final_relres;        /* relative residual of the last linear solve, by its recurrence */
     float ms_assemble;          /* device time spent in assembly (all iterations) */
     float ms_solve;             /* device time spent in linear solves */
     float ms_total;             /* device time of the whole step */

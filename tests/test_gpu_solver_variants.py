@@ -425,3 +425,40 @@ def test_multigrid_solves_near_a_loss_of_stability_keep_their_residual(run):
             out = s.newton_step(t.dt, allow_not_converged=False)
             assert out["iters"] <= 4, (i, out["dunorm"])
         assert s.multigrid_info()[0]
+
+
+@pytest.fixture(scope="module")
+def bending_states():
+    """Positions and growth of the bending sheet at steps 760, 762, .. 838."""
+    t = _bending_sheet()
+    out = []
+    with api.Solver(t) as s:
+        s.set_growth_rates(t.rates)
+        for i in range(840):
+            s.newton_step(t.dt)
+            if i >= 760 and i % 2 == 0:
+                out.append((s.positions(), s.get_Fg()[0]))
+    return t, out
+
+
+# Every solve that reports success has the residual it was asked for: at most ten
+# times the tolerance, or what the rounding of its iterations leaves at a tight one.
+@pytest.mark.parametrize("rtol", [1e-8, 1e-10, 1e-13])
+@pytest.mark.parametrize("precond", [0, 2])
+def test_residuals_near_a_loss_of_stability_follow_the_tolerance(bending_states, precond, rtol):
+    t, states = bending_states
+    for x, Fg in states:
+        with api.Solver(t, precond=precond, krylov_rtol=rtol) as s:
+            s.set_Fg(Fg)
+            s.set_positions(x)
+            s.set_growth_rates(t.rates)
+            s.begin_step(t.dt)
+            for _ in range(3):
+                s.assemble()
+                out = s.solve()
+                ia, ja, a = s.export_csr(0.0)
+                g, p = s.residual(), a * s.delta_u()[np.repeat(np.arange(3 * t.n_nodes), np.diff(ia))]
+                r = np.linalg.norm(g - np.bincount(ja, weights=p, minlength=g.size))
+                mag = np.linalg.norm(np.bincount(ja, weights=np.abs(p), minlength=g.size))
+                assert r <= max(10 * rtol * np.linalg.norm(g), 4 * EPS * max(out["iters"], 1) * mag)
+                s.update()

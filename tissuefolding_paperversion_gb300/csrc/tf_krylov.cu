@@ -645,32 +645,79 @@ __global__ void k_update(Ctx c, double* __restrict__ uk, const double* __restric
     }
 }
 
+// y = A x and m = |A| |x| (entry by entry) for the rows of the CTA, each on its
+// node's thread.  Every thread of the CTA calls it.
+__device__ __forceinline__ void rows_product_abs(const Ctx& c, const Where& w, const double* __restrict__ x,
+                                                 double (&y)[3], double (&m)[3]) {
+    const Slots sl = warp_slots<2>(c);
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) y[d] = m[d] = 0.0;
+    auto block = [&](int j, auto at) {
+        const double xj[3] = {x[3 * j], x[3 * j + 1], x[3 * j + 2]};
+#pragma unroll
+        for (int k = 0; k < 9; ++k) {
+            const double a = at(k);
+            y[k / 3] = fma(a, xj[k % 3], y[k / 3]);
+            m[k / 3] = fma(fabs(a), fabs(xj[k % 3]), m[k / 3]);
+        }
+    };
+#pragma unroll 2
+    for (int s = sl.s0; s < sl.s1; ++s) {
+        const int j = __ldcs(&c.scol[(size_t)s * kSlice + lane]);
+        if (!TF_IN(c.check, j, c.nn, CK_SPMV_COL)) continue;
+        const double* __restrict__ v = c.val + (size_t)s * kSlotDoubles + lane;
+        block(j, [&](int k) { return __ldcs(&v[kSlice * k]); });
+    }
+    const int row = c.split ? w.node - (int)threadIdx.x + lane : w.node;
+    if (c.xrow && (c.split ? row < w.n1 : w.valid)) {
+        const int p1 = c.xrow[row + 1];
+        for (int p = c.xrow[row] + (c.split ? (int)(threadIdx.x >> 5) : 0); p < p1; p += c.split ? kWarps : 1) {
+            const int j = c.xcol[p];
+            if (!TF_IN(c.check, j, c.nn, CK_EXTRA_COL)) continue;
+            const double* __restrict__ v = c.xval + 9 * (size_t)p;
+            block(j, [&](int k) { return v[k]; });
+        }
+    }
+    if (c.split) {
+        split_sum(y);
+        __syncthreads();  // its shared memory again
+        split_sum(m);
+    }
+}
+
 // The residual of a converged solve, formed again from x: r = b - A x.  Near a loss
 // of stability the multigrid's coarse matrix comes close to singular, its answers to
 // vectors of any size, and BiCGStab's recurrence then converges on a residual that x
 // no longer has (a grown 192-prism sheet ended in a tangled shape, never with
-// block-Jacobi).  An instance whose residual is ten times the tolerance
-// asked for (and 1e-9 of |b|: the rounding of A x at tight ones) is flagged F_DRIFT
-// and solved on from its x (settle).  Costs a product.
+// block-Jacobi).  An instance whose residual is more than ten times the tolerance asked
+// for is flagged F_DRIFT and solved on from its x (settle).  Where that is less than what
+// rounding leaves, the limit is eps x iterations x ||A| |x||, four times over (each
+// iteration rounds its update and its product once at that scale), up to 1e-9 of |b|:
+// an x far too large has a large |A| |x| as well.  Costs a product.
 __global__ void k_verify(Ctx c, const double* __restrict__ b, const double* __restrict__ x, double* __restrict__ r) {
     const Where w = where(c);
     if (w.flag != F_CONVERGED || __ldcg(&w.s[S_BB]) == 0.0) return;
-    double y[3], bi[3], v[1] = {0.0};
-    rows_product<2>(c, warp_slots(c), x, y);
-    if (w.valid) load3(b, w.node, bi);
-    rows_sum(c, w, x, y);
-    if (w.valid)
+    double y[3], m[3], bi[3], v[2] = {0.0, 0.0};
+    rows_product_abs(c, w, x, y, m);
+    if (w.valid) {
+        load3(b, w.node, bi);
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
             const double rd = bi[d] - y[d];
             r[3 * w.node + d] = rd;
             v[0] = fma(rd, rd, v[0]);
+            v[1] = fma(m[d], m[d], v[1]);
         }
-    double tot[1];
-    if (reduce_seg<1>(c, w.seg, v, tot) && threadIdx.x == 0 &&
-        !(tot[0] <= fmax(100.0 * __ldcg(&w.s[S_TOL2]), 1e-18) * __ldcg(&w.s[S_BB]))) {
-        w.s[S_RR] = tot[0];
-        w.s[S_FLAG] = F_DRIFT;
+    }
+    double tot[2];
+    if (reduce_seg<2>(c, w.seg, v, tot) && threadIdx.x == 0) {
+        const double rounding = 4.0 * 2.220446049250313e-16 * fmax(w.s[S_ITER], 1.0);
+        const double bb = w.s[S_BB];
+        if (!(tot[0] <= fmax(100.0 * w.s[S_TOL2] * bb, fmin(rounding * rounding * tot[1], 1e-18 * bb)))) {
+            w.s[S_RR] = tot[0];
+            w.s[S_FLAG] = F_DRIFT;
+        }
     }
 }
 void launch_verify(tf_handle* h, const Ctx& c) {
