@@ -462,3 +462,34 @@ def test_residuals_near_a_loss_of_stability_follow_the_tolerance(bending_states,
                 mag = np.linalg.norm(np.bincount(ja, weights=np.abs(p), minlength=g.size))
                 assert r <= max(10 * rtol * np.linalg.norm(g), 4 * EPS * max(out["iters"], 1) * mag)
                 s.update()
+
+
+# A caller's iteration cap that ends the solve with either preconditioner: both are
+# tried at the first such solve, later ones cost a single attempt with the one that
+# came closer (block-Jacobi on a sheet with displaced nodes, the multigrid on one that grew).
+@pytest.mark.parametrize("grown", [False, True])
+@pytest.mark.parametrize("eta", [0.0, 100.0])
+@pytest.mark.parametrize("cap", [2, 5])
+def test_capped_solves_are_not_repeated(cap, eta, grown):
+    t = _sheet(20, 20, 2, eta)
+    uk, un = mesh.perturbed_state(t, seed=5)
+    launches = {}
+    for pc in (1, 0):
+        with api.Solver(t, krylov_max_iter=cap, precond=pc) as s:
+            if grown:
+                s.set_growth_rates(np.tile([4e-6, 3e-6, 0.0], t.n_elems))
+                s.begin_step(t.dt)
+            launches[pc] = []
+            for _ in range(3):
+                if not grown:
+                    s.set_state(uk, un, t.dt)
+                s.assemble()
+                before = s.launch_count()
+                out = s.solve(allow_not_converged=True)
+                launches[pc].append(s.launch_count() - before)
+                assert out["status"] == api.TF_KRYLOV_NOT_CONVERGED and out["iters"] == cap
+            if pc == 0:
+                assert bool(s.multigrid_info()[0]) == grown
+    assert launches[0][2] <= launches[0][0] - launches[1][2], launches
+    if not grown:
+        assert launches[0][2] == launches[1][2]

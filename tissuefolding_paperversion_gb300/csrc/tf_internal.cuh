@@ -508,6 +508,7 @@ struct tf_handle {
     bool amg_off = false;                       // ... built, but block-Jacobi is used
     bool amg_trial = false;                     // ... chosen by size: block-Jacobi where a solve with it fails
     bool amg_failed = false;                    // ... and one has: block-Jacobi from then on
+    bool amg_capped = false;                    // ... and the caller's iteration cap ended both: one attempt each
     bool amg_adjoint = false;                   // ... built for the adjoint's solves only
     tf::Packing* pk = nullptr;                  // packing between tissue surfaces (null: off)
     tf::Growth* growth = nullptr;               // growth functions (null: none added yet)

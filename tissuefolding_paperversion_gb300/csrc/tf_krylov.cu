@@ -1080,6 +1080,18 @@ tf_status krylov_run(tf_handle* h, int method, int keep, int* iters, double* rel
 
 }  // namespace
 
+// Whether the last solve stopped at its iteration cap: slow, not failed.
+static bool capped(const tf_handle* h) {
+    for (int g = 0; g < h->d.nseg; ++g)
+        if (h->d.host_scal[(size_t)g * S_COUNT + S_FLAG] == F_RUNNING) return true;
+    return false;
+}
+
+// The caller's own iteration cap ended a trial solve.
+static bool capped_by_caller(const tf_handle* h, tf_status s) {
+    return s == TF_KRYLOV_NOT_CONVERGED && h->opt.krylov_max_iter <= kTrialIters && capped(h);
+}
+
 // A solve; the instances whose residual drifted from the recurrence (k_verify) go
 // on from their x with the residual that it has.
 static tf_status settle(tf_handle* h, int method, int keep, int* iters, double* relres) {
@@ -1112,7 +1124,8 @@ static tf_status krylov_attempt(tf_handle* h, int* iters, double* relres) {
     TF_CUDA(cudaMemcpyAsync(d.seg_solve, d.seg_active, sizeof(int) * (size_t)d.nseg, cudaMemcpyDeviceToDevice,
                             h->stream));
     tf_status s = settle(h, h->method, 0, iters, relres);
-    if (s != TF_OK && use_multigrid(h) && amg_reused(h)) {
+    const bool once = h->amg_capped && capped_by_caller(h, s);  // a capped solve is not repeated (krylov_solve)
+    if (s != TF_OK && use_multigrid(h) && amg_reused(h) && !once) {
         // the coarse levels came from an earlier Newton iteration: rebuild
         // them for this matrix and solve again
         amg_mark_stale(h, 2);
@@ -1148,28 +1161,28 @@ static tf_status krylov_attempt(tf_handle* h, int* iters, double* relres) {
     return s;
 }
 
-// Whether the last solve stopped at its iteration cap: slow, not failed.
-static bool capped(const tf_handle* h) {
-    for (int g = 0; g < h->d.nseg; ++g)
-        if (h->d.host_scal[(size_t)g * S_COUNT + S_FLAG] == F_RUNNING) return true;
-    return false;
-}
-
 // A multigrid solve that fails is done again with block-Jacobi, whose answer
 // then counts: near a loss of stability BiCGStab with the multigrid can diverge
 // where block-Jacobi converges.  A handle with the multigrid on trial (chosen by size
 // where block-Jacobi is the general path) stays with block-Jacobi once that
 // converged; others go back to the multigrid, and at their iteration cap they stop.
+// Where the caller's cap ends both, the handle stays with the one that came closer
+// and does not try the other again: a caller who uses capped solves pays for
+// one (1,323 nodes, a cap of 10: 237 launches a solve before, 38 now, as with block-Jacobi).
 tf_status krylov_solve(tf_handle* h, int* iters, double* relres) {
     const tf_status s = krylov_attempt(h, iters, relres);
     if (s == TF_OK || !use_multigrid(h) || s == TF_CUDA_ERROR || s == TF_OUT_OF_MEMORY) return s;
     if (!h->amg_trial && s == TF_KRYLOV_NOT_CONVERGED && capped(h)) return s;
+    const bool cap = h->amg_trial && capped_by_caller(h, s);
+    if (cap && h->amg_capped) return s;
+    const double rel = *relres;
     destroy_graphs(h);  // they hold the multigrid's kernels
     h->amg_off = true;
     const tf_status t = krylov_attempt(h, iters, relres);
-    if (t == TF_OK && h->amg_trial) {
+    if (h->amg_trial && (t == TF_OK || (cap && capped_by_caller(h, t) && *relres < rel))) {
         h->amg_failed = true;
     } else {
+        h->amg_capped = h->amg_capped || (cap && capped_by_caller(h, t));
         destroy_graphs(h);
         h->amg_off = false;
     }
