@@ -493,3 +493,29 @@ def test_capped_solves_are_not_repeated(cap, eta, grown):
     assert launches[0][2] <= launches[0][0] - launches[1][2], launches
     if not grown:
         assert launches[0][2] == launches[1][2]
+
+
+# The element kernel's double-float pairs over FP32's range: moduli from 1e-26 to 1e34
+# times those of a tissue, K against the element routine's FP64 sums as in
+# test_element_tiles (1e-11 of the largest entry).
+@pytest.mark.parametrize("scale", [1e-26, 1e-24, 1e-20, 1e20, 1e34])
+@pytest.mark.parametrize("eta", [0.0, 100.0])
+def test_element_kernel_over_the_range_of_moduli(eta, scale):
+    t = mesh.config_tiny(seed=5, n=4, n_layers=2, eta=eta)
+    t.E, t.eta = t.E * scale, t.eta * scale
+    uk, un = mesh.perturbed_state(t, seed=9, amp=0.8)
+    with api.Solver(t) as s:
+        s.set_state(uk, un, t.dt)
+        s.assemble()
+        ia, ja, a = s.export_csr(0.0)
+        ev = s.element_eval()
+    n = 3 * t.n_nodes
+    K = np.zeros((n, n))
+    for e, nodes in enumerate(t.conn.reshape(-1, 6)):
+        dof = (3 * nodes[:, None] + np.arange(3)).reshape(-1)
+        K[np.ix_(dof, dof)] += ev["Ke"][e] + ev["Kv"][e]
+    got = np.zeros((n, n))
+    got[np.repeat(np.arange(n), np.diff(ia)), ja] = a
+    free = np.flatnonzero(t.fixed == 0)
+    d = (got - K)[np.ix_(free, free)]
+    assert np.abs(d).max() <= 1e-11 * np.abs(K[np.ix_(free, free)]).max()
