@@ -519,3 +519,17 @@ def test_element_kernel_over_the_range_of_moduli(eta, scale):
     free = np.flatnonzero(t.fixed == 0)
     d = (got - K)[np.ix_(free, free)]
     assert np.abs(d).max() <= 1e-11 * np.abs(K[np.ix_(free, free)]).max()
+
+
+@pytest.mark.parametrize("scale", [1e36, 1e40, 1e60, 1e100])
+@pytest.mark.parametrize("eta", [0.0, 100.0])
+def test_moduli_beyond_the_element_kernels_range_are_reported(eta, scale):
+    t = mesh.config_tiny(seed=5, n=4, n_layers=2, eta=eta)
+    t.E, t.eta = t.E * scale, t.eta * scale
+    uk, un = mesh.perturbed_state(t, seed=9, amp=0.05)
+    with api.Solver(t) as s:
+        s.set_state(uk, un, t.dt)
+        s.assemble()
+        with pytest.raises(api.TfError) as e:
+            s.solve()
+        assert e.value.status == api.TF_NAN_DETECTED
