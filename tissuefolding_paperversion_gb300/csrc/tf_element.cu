@@ -270,8 +270,8 @@ __device__ __forceinline__ void gauss_point(const ElemArgs& A, int e, int gp, bo
 
 // x = hi + lo on the bit pattern: hi is x rounded to 24 significant bits (half
 // away from zero; the carry runs into the exponent), lo the rest as an integer
-// of 29 signed bits, scaled (in two factors where the scale is below FP32's normal
-// range).  Magnitudes below FP32's normal range become a signed zero, those above
+// of 29 signed bits, scaled (in two factors: 2^(exponent - 52) itself can lie below
+// FP32's normal range).  Magnitudes below FP32's normal range become a signed zero, those above
 // it infinity; NaN and infinity stay so.
 __device__ __forceinline__ float2 df_split(double x) {
     const unsigned l = __double2loint(x), h = __double2hiint(x);
@@ -281,9 +281,8 @@ __device__ __forceinline__ float2 df_split(double x) {
     unsigned f = sgn | ((((h2 >> 20) & 0x7ffu) - 896u) << 23) | ((h2 & 0xfffffu) << 3) | (l2 >> 29);
     f = e > 896 ? f : sgn;
     f = e > 1150 ? (sgn | 0x7f800000u | ((e == 0x7ff && (h & 0xfffffu)) ? 0x400000u : 0u)) : f;
-    const bool low = e <= 948;
-    const float scale = __uint_as_float(sgn | ((unsigned)(e - (low ? 884 : 948)) << 23));  // 2^(exponent - 52)
-    const float lo = __int2float_rn((int)(l2 & 0x1fffffffu) - (1 << 28)) * scale * (low ? 0x1p-64f : 1.f);
+    const float scale = __uint_as_float(sgn | ((unsigned)(e - 896) << 23));  // 2^exponent
+    const float lo = __int2float_rn((int)(l2 & 0x1fffffffu) - (1 << 28)) * 0x1p-52f * scale;
     return make_float2(__uint_as_float(f), (e > 896 && e <= 1150) ? lo : 0.f);
 }
 
