@@ -425,7 +425,8 @@ __device__ __forceinline__ int sym_index(int j, int l) { return j == l ? j : j +
 //       W(node pair i <= k) go where gp was.
 // st first holds what only the phases before need: dx/dxi and dv/dxi
 // [2][7][3][NE] in FP64 (X), (sigma' + sigma_v') g_j [9][gp][NE] in FP64 for the
-// forces (F), and c1, c2, sigma', sigma_v' [value][gp][NE] (C).
+// forces (F), and [value][gp][NE] (C): with viscosity sigma', sigma_v', without it c1,
+// c2 and sigma' g_j, formed in FP64 for the forces anyway.
 template <bool VISC>
 struct Lay {
     static constexpr int G = 0, W = 9, V = 18, Q = 27, T = 36, K1 = 42, U = 18, D = 27;
@@ -437,8 +438,9 @@ struct Lay {
     static constexpr int BB = BR + 6 * NR;               // [3], without viscosity [2][3]
     static constexpr int NB = BB + (VISC ? 3 : 6);
     static constexpr int XM = 0, XW = NJL;               // blocks in gp's place: [NJL], [6]
-    static constexpr int C1 = 0, C2 = 1, SG = 2, SV = 8; // values of C (with viscosity c1 is in gp, c2 in Q)
-    static constexpr int NC = VISC ? 14 : 8;
+    static constexpr int SG = 0, SV = 6;                 // values of C with viscosity (c1 is in gp, c2 in Q)
+    static constexpr int C1 = 0, C2 = 1, SF = 2;         // ... and without
+    static constexpr int NC = VISC ? 12 : 11;
 };
 template <int NE, bool VISC>
 constexpr size_t elem_smem() {
@@ -638,9 +640,9 @@ __global__ void __launch_bounds__(NE* kSlots, 48 / NE) k_element(ElemArgs A) {
         for (int k = 0; k < 3; ++k) sgm[k] = sc * fma(mu, b[k], dterm);
 #pragma unroll
         for (int k = 3; k < 6; ++k) sgm[k] = sm * b[k];
-#pragma unroll
-        for (int k = 0; k < 6; ++k) putc(Y::SG + k, sgm[k]);
         if constexpr (VISC) {
+#pragma unroll
+            for (int k = 0; k < 6; ++k) putc(Y::SG + k, sgm[k]);
             // grad v = sum_j dv/dxi_j (x) g_j (ShapeBase.cpp:2892-2919), the scales of
             // the two cancelling; a prism without viscosity has eta = 0 and these terms vanish
             double Lg[9];
@@ -681,7 +683,10 @@ __global__ void __launch_bounds__(NE* kSlots, 48 / NE) k_element(ElemArgs A) {
             double h3[3];
             sym_apply(sgm, g[3 * j], g[3 * j + 1], g[3 * j + 2], h3);
 #pragma unroll
-            for (int i = 0; i < 3; ++i) ho[(size_t)(3 * j + i) * 6 * NE] = h3[i];
+            for (int i = 0; i < 3; ++i) {
+                ho[(size_t)(3 * j + i) * 6 * NE] = h3[i];
+                if constexpr (!VISC) putc(Y::SF + 3 * j + i, h3[i]);
+            }
         }
     }
     __syncthreads();
@@ -719,9 +724,14 @@ __global__ void __launch_bounds__(NE* kSlots, 48 / NE) k_element(ElemArgs A) {
                 }
             }
         } else {
+            if constexpr (VISC) {
 #pragma unroll
-            for (int k = 0; k < 6; ++k) s6[k] = ct(Y::SG + k);
-            df_sym_apply(s6, a, o);
+                for (int k = 0; k < 6; ++k) s6[k] = ct(Y::SG + k);
+                df_sym_apply(s6, a, o);
+            } else {
+#pragma unroll
+                for (int i = 0; i < 3; ++i) o[i] = ct(Y::SF + 3 * j + i);
+            }
 #pragma unroll 1
             for (int l = j; l < 3; ++l) {
                 float sH = 0.f, sL = 0.f, tH = 0.f, tL = 0.f;
