@@ -61,6 +61,7 @@ constexpr int kRestrictThreads = 128;  // per coarse node in the level-0 restric
 constexpr int kCoarseNodes = 16;  // nodes per instance at the coarsest level (96 DOFs)
 constexpr int kCoarseDofs = 6 * kCoarseNodes;
 constexpr int kInvThreads = 512;  // of the coarsest level's inverse
+constexpr int kSmemOptIn = 227 * 1024;  // the most a CTA may ask for: no handle lowers another's limit
 constexpr int kPowerIters = 16;
 // The first level whose dense operators (one m x m FP32 matrix per instance,
 // m = 6 nodes) fit these bytes, and every level below it, is applied as one
@@ -433,6 +434,11 @@ static tf_status build_q(const Device& d, AmgQ* q, const std::vector<int>& trowp
     return TF_OK;
 }
 
+namespace {
+__global__ void k_coarse_invert(AmgLevel L, const int* __restrict__ cnode0, const int* __restrict__ cinv0,
+                                float* __restrict__ cinv);
+}
+
 // Symbolic set-up from the level-0 pattern, the reference positions and the
 // fixed DOFs.  Level 0 uses the handle's own matrix, block inverses and
 // sliced storage.
@@ -794,6 +800,8 @@ tf_status amg_build(tf_handle* h, const double* pos) {
     AMG_TRY(up(&a->cinv0, cinv0));
     AMG_TRY(zeros(&a->cinv, (size_t)std::max(cinv0[d.nseg], 1)));
     if (!a->coarse_exact) return TF_OK;
+    TF_CUDA(cudaFuncSetAttribute(k_coarse_invert, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)(sizeof(double) * kCoarseDofs * kCoarseDofs)));
     // the dense operator: from the finest level that fits down (the coarsest
     // level's inverse exists anyway)
     a->dense = a->nlev - 1;
@@ -2362,7 +2370,7 @@ tf_status amg_numeric(tf_handle* h) {
     Amg* a = h->amg;
     if (a->stale == 0) return TF_OK;
     if (a->v0_smem > 48 * 1024)  // outside any stream capture: the V-cycles launched later need it
-        TF_CUDA(cudaFuncSetAttribute(k_v0_prolong, cudaFuncAttributeMaxDynamicSharedMemorySize, a->v0_smem));
+        TF_CUDA(cudaFuncSetAttribute(k_v0_prolong, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemOptIn));
     Device& d = h->d;
     cudaStream_t st = h->stream;
     amg_refresh(h);
@@ -2440,12 +2448,6 @@ tf_status amg_numeric(tf_handle* h) {
     if (a->coarse_exact) {
         AmgLevel& L = a->L[a->nlev - 1];
         const size_t smem = sizeof(double) * (size_t)a->max_cm * a->max_cm;
-        static bool configured = false;
-        if (!configured) {
-            TF_CUDA(cudaFuncSetAttribute(k_coarse_invert, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)(sizeof(double) * kCoarseDofs * kCoarseDofs)));
-            configured = true;
-        }
         k_coarse_invert<<<a->nseg, kInvThreads, smem, st>>>(L, a->cnode0, a->cinv0, a->cinv);
         TF_LAUNCH_CHECK(h);
         if (a->dense < a->nlev - 1) {

@@ -1272,10 +1272,10 @@ ElemArgs make_args(tf_handle* h) {
 template <int NE, int MODE, bool VISC>
 tf_status launch_fast(tf_handle* h, const ElemArgs& A) {
     constexpr size_t smem = elem_smem<NE, VISC>();
-    static int configured_device = -1;
-    if (configured_device != h->device) {
+    constexpr unsigned bit = 1u << (2 * (NE / 8) + (VISC ? 1 : 0));  // the assembly mode is the handle's
+    if (!(h->elem_smem & bit)) {
         TF_CUDA(cudaFuncSetAttribute(k_element<NE, MODE, VISC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        configured_device = h->device;
+        h->elem_smem |= bit;
     }
     k_element<NE, MODE, VISC><<<cdiv(A.ne, NE), NE * kSlots, smem, h->stream>>>(A);
     TF_LAUNCH_CHECK(h);
@@ -1423,11 +1423,7 @@ tf_status launch_element_eval(tf_handle* h, int e0, int count, double* Ke, doubl
     if (count <= 0) return TF_OK;
     constexpr int NE = 8;
     const size_t smem = sizeof(GpEval) * NE * kGauss;
-    static bool configured = false;
-    if (!configured) {
-        TF_CUDA(cudaFuncSetAttribute(k_element_eval<NE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        configured = true;
-    }
+    TF_CUDA(cudaFuncSetAttribute(k_element_eval<NE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     k_element_eval<NE><<<cdiv(count, NE), NE * kGauss, smem, h->stream>>>(A);
     TF_LAUNCH_CHECK(h);
     return TF_OK;

@@ -478,6 +478,7 @@ struct tf_handle {
     std::vector<int> h_seg_node0, h_seg_elem0;  // host copies of the instance offsets
     std::vector<int> h_active;                  // host mirror of seg_active
     int elem_cta = 16;                          // prisms per CTA of the element kernel (autotuned)
+    unsigned elem_smem = 0;                     // its variants whose shared memory this handle's device has granted
     bool tuned = false;
     cudaGraphExec_t graph[2][5] = {};           // Krylov chunks [method-1][log2(chunk/4)]
     int64_t graph_kernels[2][5] = {};
