@@ -533,3 +533,26 @@ def test_moduli_beyond_the_element_kernels_range_are_reported(eta, scale):
         with pytest.raises(api.TfError) as e:
             s.solve()
         assert e.value.status == api.TF_NAN_DETECTED
+
+
+# A small mesh on a device with little memory left gets a handle wherever block-Jacobi
+# fits: without a hierarchy, if that does not.
+@pytest.mark.parametrize("deterministic", [False, True])
+def test_small_meshes_do_without_the_multigrid_where_memory_is_short(deterministic):
+    torch = pytest.importorskip("torch")
+    t = _sheet(60, 60, 2, 100.0)
+    t.rates = np.tile([4e-6, 3e-6, 0.0], t.n_elems)
+    lp = np.array([100.0, 100.0, 5.0, 40.0])
+    hog = torch.empty(torch.cuda.mem_get_info()[0] - (130 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        with api.Solver(t, deterministic=deterministic) as s:
+            assert s.multigrid_info()[0] == []
+            s.set_growth_rates(t.rates)
+            s.newton_step(t.dt, allow_not_converged=False)
+            if deterministic:  # whose hierarchy is built at the first adjoint call
+                _, saved = s.adjoint_forward(np.full(t.n_elems, 1e-6), np.log(t.E), 1, t.dt, 1, lp)
+                s.adjoint_backward(saved)
+                saved.free()
+    finally:
+        del hog
+        torch.cuda.empty_cache()

@@ -498,10 +498,8 @@ TF_API tf_status tf_adj_forward(tf_handle* h, const double* rate, const double* 
     a->device = h->device;
     std::memcpy(a->params, loss_params, sizeof(a->params));
     if (h->amg_trial && !h->amg) {
-        const tf_status b = amg_build(h, h->h_pos0.data());
+        const tf_status b = amg_build_trial(h, h->h_pos0.data());
         if (b != TF_OK) {
-            amg_free(h->amg);
-            h->amg = nullptr;
             tf_adj_free(a);
             return b;
         }

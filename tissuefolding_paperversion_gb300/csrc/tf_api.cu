@@ -611,7 +611,7 @@ tf_status create_handle(const tf_mesh* mesh, const tf_material* mat, const tf_op
     const bool large = mesh->n_nodes >= kAutoMultigridNodes;
     const bool amg = h->opt.precond >= 2 || (h->opt.precond == 0 && (large || !h->opt.deterministic));
     h->amg_trial = h->opt.precond == 0 && !large;
-    if (s == TF_OK && amg) s = amg_build(h, mesh->node_pos);
+    if (s == TF_OK && amg) s = h->amg_trial ? amg_build_trial(h, mesh->node_pos) : amg_build(h, mesh->node_pos);
     if (s != TF_OK) {
         free_all(h);
         delete h;

@@ -556,6 +556,7 @@ tf_status autotune_element(tf_handle* h);
 tf_status launch_metric(tf_handle* h);  // after every change of invFg
 tf_status launch_shape_gradients(tf_handle* h, const double* dN);  // gx from ginv; dN[6][3][6] on the host
 tf_status amg_build(tf_handle* h, const double* ref_pos);
+tf_status amg_build_trial(tf_handle* h, const double* ref_pos);  // no hierarchy (block-Jacobi) where memory is short
 tf_status amg_numeric(tf_handle* h);
 void amg_refresh(tf_handle* h);     // launches the level-0 smoother copies of the current assembly
 tf_status amg_autotune(tf_handle* h);  // picks the level-0 smoother's row-product variant by timing
