@@ -556,3 +556,72 @@ def test_small_meshes_do_without_the_multigrid_where_memory_is_short(determinist
     finally:
         del hog
         torch.cuda.empty_cache()
+
+
+def _floating_sheet(nx, ny, layers):
+    """No external viscosity: the in-plane rigid motions have no stiffness, and the
+    multigrid's coarsest matrix is singular.  The systems are consistent."""
+    t = _sheet(nx, ny, layers, 0.0)
+    t.ext_visc[:] = 0.0
+    t.rates = np.tile([4e-6, 3e-6, 0.0], t.n_elems)
+    return t
+
+
+def _residuals(s, out, rows, rtol=1e-8):
+    """Every instance's true residual against the tolerance and its rounding."""
+    ia, ja, a = s.export_csr(0.0)
+    g, n = s.residual(), len(ia) - 1
+    p = a * s.delta_u()[np.repeat(np.arange(n), np.diff(ia))]
+    r = g - np.bincount(ja, weights=p, minlength=n)
+    mag = np.bincount(ja, weights=np.abs(p), minlength=n)
+    for lo, hi in rows:
+        assert np.linalg.norm(r[lo:hi]) <= (rtol * np.linalg.norm(g[lo:hi])
+                                            + 4 * EPS * max(out["iters"], 1) * np.linalg.norm(mag[lo:hi]))
+
+
+# A solve that the multigrid does not finish is block-Jacobi's: its du solves the
+# assembled system, the handle then shows no hierarchy, and later solves and steps work.
+@pytest.mark.parametrize("nx,ny,layers", [(12, 12, 2), (20, 20, 2)])
+def test_small_handle_goes_to_block_jacobi_and_stays(nx, ny, layers):
+    t = _floating_sheet(nx, ny, layers)
+    uk, un = mesh.perturbed_state(t, seed=8, amp=0.005)
+    with api.Solver(t) as s:
+        assert s.multigrid_info()[0]
+        s.set_state(uk, un, t.dt)
+        for _ in range(2):
+            s.assemble()
+            _residuals(s, s.solve(), [(0, 3 * t.n_nodes)])
+            assert s.multigrid_info()[0] == []
+        s.set_growth_rates(t.rates)
+        s.set_positions(t.pos)
+        s.newton_step(t.dt, allow_not_converged=False)
+        assert s.multigrid_info()[0] == []
+
+
+def test_batch_goes_to_block_jacobi_with_one_instance():
+    ts = [_sheet(9, 7, 2, 0.0), _floating_sheet(12, 12, 2), _sheet(5, 8, 3, 0.0, 4)]
+    states = [mesh.perturbed_state(t, seed=8, amp=0.005) for t in ts]
+    off = np.cumsum([0] + [3 * t.n_nodes for t in ts])
+    with api.Batch(ts) as s:
+        assert s.multigrid_info()[0]
+        s.set_positions(np.concatenate([v[1] for v in states]))
+        s.begin_step(ts[0].dt)
+        s.set_state(np.concatenate([v[0] for v in states]), np.concatenate([v[1] for v in states]), ts[0].dt)
+        for _ in range(2):
+            s.assemble()
+            _residuals(s, s.solve(), list(zip(off[:-1], off[1:])))
+            assert s.multigrid_info()[0] == []
+
+
+def test_adjoint_forward_goes_to_block_jacobi():
+    """The order-fixed handle takes the multigrid for the adjoint's solves only; the
+    loss is that of block-Jacobi to the accuracy of the solves."""
+    t = _floating_sheet(12, 12, 2)
+    lp, loss = np.array([30.0, 30.0, 5.0, 20.0]), []
+    for pc in (0, 1):
+        with api.Solver(t, deterministic=True, precond=pc) as s:
+            lv, saved = s.adjoint_forward(np.full(t.n_elems, 1e-5), np.log(t.E), 2, t.dt, 1, lp)
+            saved.free()
+            assert s.multigrid_info()[0] == []
+            loss.append(lv)
+    assert abs(loss[0] - loss[1]) <= 1e-7 * abs(loss[1])
