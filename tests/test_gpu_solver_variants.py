@@ -371,7 +371,7 @@ def test_static_solve_on_fewer_blocks(n, most, blocks):
     it, rr = C.c_int32(0), C.c_double(0.0)
     p = [C.c_void_p(a.data_ptr()) for a in d]
     L = api.load()
-    st = L.tf_static_solve_blocks(blocks, n, *p, C.c_void_p(x.data_ptr()), C.c_double(RTOL), 500, None, C.byref(it),
+    st = L.tf_static_solve_blocks(blocks, 0, n, *p, C.c_void_p(x.data_ptr()), C.c_double(RTOL), 500, None, C.byref(it),
                                   C.byref(rr))
     assert st == api.TF_OK, L.tf_last_error().decode()
     xs = x.cpu().numpy().reshape(n, 3)
@@ -625,3 +625,23 @@ def test_adjoint_forward_goes_to_block_jacobi():
             assert s.multigrid_info()[0] == []
             loss.append(lv)
     assert abs(loss[0] - loss[1]) <= 1e-7 * abs(loss[1])
+
+
+def test_static_solve_gives_up_on_a_block_that_does_not_come():
+    """The thread blocks wait for one more than there are: every wait runs out, the
+    call returns an error, and the next call is right."""
+    import ctypes as C
+
+    torch = pytest.importorskip("torch")
+    n = 100
+    d = [torch.from_numpy(v).cuda() for v in (np.arange(n + 1, dtype=np.int32), np.arange(n, dtype=np.int32),
+                                              np.tile((2.0 * np.eye(3)).reshape(-1), n), np.ones(3 * n))]
+    x = torch.zeros(3 * n, dtype=torch.float64, device="cuda")
+    it, rr = C.c_int32(7), C.c_double(7.0)
+    args = [C.c_void_p(a.data_ptr()) for a in d] + [C.c_void_p(x.data_ptr()), C.c_double(RTOL), 500, None, C.byref(it),
+                                                   C.byref(rr)]
+    L = api.load()
+    assert L.tf_static_solve_blocks(0, 1, n, *args) == api.TF_CUDA_ERROR
+    assert "lost each other" in L.tf_last_error().decode() and (it.value, rr.value) == (0, 0.0)
+    assert L.tf_static_solve_blocks(0, 0, n, *args) == api.TF_OK
+    assert np.array_equal(x.cpu().numpy(), np.full(3 * n, 0.5))

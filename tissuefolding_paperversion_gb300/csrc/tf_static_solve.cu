@@ -62,6 +62,7 @@ enum { QF_RUNNING = 0, QF_CONVERGED = 1, QF_BREAKDOWN = 2, QF_NAN = 3, QF_STUCK 
 struct SCtx {
     int n;
     int rows;  // per CTA
+    int meet;  // CTAs at a meeting
     int max_iter;
     double tol2;
     const int* __restrict__ rowptr;
@@ -86,7 +87,7 @@ struct SShared {
 // All CTAs meet (they are resident together: a cooperative launch).  False when
 // the wait ran out.
 __device__ __forceinline__ bool s_barrier(const SCtx& c, SShared& sh, unsigned& goal) {
-    goal += gridDim.x;
+    goal += c.meet;
     __syncthreads();
     if (threadIdx.x == 0) {
         unsigned* bar = c.bar();
@@ -470,14 +471,14 @@ tf_status scratch_address(int device, double** out) {
 
 using namespace tf;
 
-// With up to max_blocks thread blocks (tests; tf_solve_bsr_static asks for one per
-// SM, max_blocks = 0).
-extern "C" TF_API tf_status tf_static_solve_blocks(int32_t max_blocks, int32_t n_block_rows, const int32_t* rowptr,
+// With up to max_blocks thread blocks, which wait for `absent` more at their meetings
+// (tests; tf_solve_bsr_static asks for one per SM, max_blocks = 0, and none absent).
+extern "C" TF_API tf_status tf_static_solve_blocks(int32_t max_blocks, int32_t absent, int32_t n_block_rows, const int32_t* rowptr,
                                                    const int32_t* colidx, const double* val, const double* b,
                                                    double* x, double rtol, int32_t max_iter, void* stream,
                                                    int32_t* iters, double* relres) {
     if (n_block_rows <= 0 || !rowptr || !colidx || !val || !b || !x || !(rtol > 0.0) || max_iter <= 0 ||
-        max_blocks < 0) {
+        max_blocks < 0 || absent < 0) {
         set_error("tf_solve_bsr_static: bad arguments");
         return TF_BAD_INPUT;
     }
@@ -501,7 +502,7 @@ extern "C" TF_API tf_status tf_static_solve_blocks(int32_t max_blocks, int32_t n
     if (s != TF_OK) return s;
     int sms = max_blocks;
     if (max_blocks == 0) TF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-    SCtx c{n_block_rows, 0, max_iter, rtol * rtol, rowptr, colidx, val, base};
+    SCtx c{n_block_rows, 0, 0, max_iter, rtol * rtol, rowptr, colidx, val, base};
     // the count to kCountStart; the scalars are the kernel's to write
     TF_CUDA(cudaMemsetAsync(base + kOffScal, 0xff, sizeof(double) * (kNumScal + 2), st));
     TF_CUDA(cudaFuncSetAttribute(ks_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, kStaticSmem));
@@ -511,6 +512,7 @@ extern "C" TF_API tf_status tf_static_solve_blocks(int32_t max_blocks, int32_t n
     while (true) {
         c.rows = cdiv(n_block_rows, blocks);
         blocks = cdiv(n_block_rows, c.rows);
+        c.meet = blocks + absent;
         const cudaError_t e =
             launch_cooperative(ks_solve, blocks, kStaticThreads, kStaticSmem, st, c, b, x);
         if (e == cudaSuccess) break;
@@ -544,6 +546,6 @@ extern "C" TF_API tf_status tf_static_solve_blocks(int32_t max_blocks, int32_t n
 extern "C" TF_API tf_status tf_solve_bsr_static(int32_t n_block_rows, const int32_t* rowptr, const int32_t* colidx,
                                                 const double* val, const double* b, double* x, double rtol,
                                                 int32_t max_iter, void* stream, int32_t* iters, double* relres) {
-    return tf_static_solve_blocks(0, n_block_rows, rowptr, colidx, val, b, x, rtol, max_iter, stream, iters,
+    return tf_static_solve_blocks(0, 0, n_block_rows, rowptr, colidx, val, b, x, rtol, max_iter, stream, iters,
                                   relres);
 }
