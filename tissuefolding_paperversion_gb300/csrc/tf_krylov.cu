@@ -645,22 +645,52 @@ __global__ void k_update(Ctx c, double* __restrict__ uk, const double* __restric
     }
 }
 
-// y = A x and m = |A| |x| (entry by entry) for the rows of the CTA, each on its
-// node's thread.  Every thread of the CTA calls it.
+// The residual of a converged solve, formed again from x: r = b - A x.  Near a loss
+// of stability the multigrid's coarse matrix comes close to singular, its answers to
+// vectors of any size, and BiCGStab's recurrence then converges on a residual that x
+// no longer has (a grown 192-prism sheet ended in a tangled shape, never with
+// block-Jacobi).  An instance whose residual is more than ten times the tolerance asked
+// for is flagged F_DRIFT and solved on from its x (settle), unless that is what
+// rounding leaves (k_rounding).  Bound by the FP64 pipe, like every product: a step of
+// 320,000 prisms takes 0.2 ms more, one of 46,208 prisms 0.1 ms.
+template <int U>
+__global__ void __launch_bounds__(kThreads, U == 0 ? 4 : 6)
+    k_verify(Ctx c, const double* __restrict__ b, const double* __restrict__ x, double* __restrict__ r) {
+    const Slots sl = warp_slots<U>(c);
+    const Where w = where(c);
+    if (w.flag != F_CONVERGED || __ldcg(&w.s[S_BB]) == 0.0) return;
+    double y[3], bi[3], v[1] = {0.0};
+    rows_product<U>(c, sl, x, y);
+    if (U == 0 && w.valid) load3(b, w.node, bi);
+    rows_sum<U == 0 ? kSplit : kWhole>(c, w, x, y);
+    if (U != 0 && w.valid) load3(b, w.node, bi);
+    if (w.valid)
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const double rd = bi[d] - y[d];
+            r[3 * w.node + d] = rd;
+            v[0] = fma(rd, rd, v[0]);
+        }
+    double tot[1];
+    if (reduce_seg<1, U == 0 ? kSplit : kWhole>(c, w.seg, v, tot) && threadIdx.x == 0 &&
+        !(tot[0] <= 100.0 * w.s[S_TOL2] * w.s[S_BB])) {
+        w.s[S_RR] = tot[0];
+        w.s[S_FLAG] = F_DRIFT;
+    }
+}
+
+// y = |A| |x|, entry by entry, for the rows of the CTA, each on its node's thread.
+// Every thread of the CTA calls it.
 __device__ __forceinline__ void rows_product_abs(const Ctx& c, const Where& w, const double* __restrict__ x,
-                                                 double (&y)[3], double (&m)[3]) {
+                                                 double (&y)[3]) {
     const Slots sl = warp_slots<2>(c);
     const int lane = threadIdx.x & 31;
 #pragma unroll
-    for (int d = 0; d < 3; ++d) y[d] = m[d] = 0.0;
+    for (int d = 0; d < 3; ++d) y[d] = 0.0;
     auto block = [&](int j, auto at) {
-        const double xj[3] = {x[3 * j], x[3 * j + 1], x[3 * j + 2]};
+        const double xj[3] = {fabs(x[3 * j]), fabs(x[3 * j + 1]), fabs(x[3 * j + 2])};
 #pragma unroll
-        for (int k = 0; k < 9; ++k) {
-            const double a = at(k);
-            y[k / 3] = fma(a, xj[k % 3], y[k / 3]);
-            m[k / 3] = fma(fabs(a), fabs(xj[k % 3]), m[k / 3]);
-        }
+        for (int k = 0; k < 9; ++k) y[k / 3] = fma(fabs(at(k)), xj[k % 3], y[k / 3]);
     };
 #pragma unroll 2
     for (int s = sl.s0; s < sl.s1; ++s) {
@@ -679,50 +709,34 @@ __device__ __forceinline__ void rows_product_abs(const Ctx& c, const Where& w, c
             block(j, [&](int k) { return v[k]; });
         }
     }
-    if (c.split) {
-        split_sum(y);
-        __syncthreads();  // its shared memory again
-        split_sum(m);
-    }
+    if (c.split) split_sum(y);
 }
 
-// The residual of a converged solve, formed again from x: r = b - A x.  Near a loss
-// of stability the multigrid's coarse matrix comes close to singular, its answers to
-// vectors of any size, and BiCGStab's recurrence then converges on a residual that x
-// no longer has (a grown 192-prism sheet ended in a tangled shape, never with
-// block-Jacobi).  An instance whose residual is more than ten times the tolerance asked
-// for is flagged F_DRIFT and solved on from its x (settle).  Where that is less than what
-// rounding leaves, the limit is eps x iterations x ||A| |x||, four times over (each
-// iteration rounds its update and its product once at that scale), up to 1e-9 of |b|:
-// an x far too large has a large |A| |x| as well.  Costs a product.
-__global__ void k_verify(Ctx c, const double* __restrict__ b, const double* __restrict__ x, double* __restrict__ r) {
+// Of the instances that k_verify flagged: a residual of up to eps x iterations x
+// ||A| |x||, four times over, is rounding (each iteration rounds its update and its
+// product once at that scale), as far as 1e-9 of |b|: an x far too large has a large
+// |A| |x| as well.  Returns at once where none is flagged.
+__global__ void k_rounding(Ctx c, const double* __restrict__ x) {
     const Where w = where(c);
-    if (w.flag != F_CONVERGED || __ldcg(&w.s[S_BB]) == 0.0) return;
-    double y[3], m[3], bi[3], v[2] = {0.0, 0.0};
-    rows_product_abs(c, w, x, y, m);
-    if (w.valid) {
-        load3(b, w.node, bi);
+    if (w.flag != F_DRIFT) return;
+    double y[3], v[1] = {0.0};
+    rows_product_abs(c, w, x, y);
+    if (w.valid)
 #pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            const double rd = bi[d] - y[d];
-            r[3 * w.node + d] = rd;
-            v[0] = fma(rd, rd, v[0]);
-            v[1] = fma(m[d], m[d], v[1]);
-        }
-    }
-    double tot[2];
-    if (reduce_seg<2>(c, w.seg, v, tot) && threadIdx.x == 0) {
+        for (int d = 0; d < 3; ++d) v[0] = fma(y[d], y[d], v[0]);
+    double tot[1];
+    if (reduce_seg<1>(c, w.seg, v, tot) && threadIdx.x == 0) {
         const double rounding = 4.0 * 2.220446049250313e-16 * fmax(w.s[S_ITER], 1.0);
-        const double bb = w.s[S_BB];
-        if (!(tot[0] <= fmax(100.0 * w.s[S_TOL2] * bb, fmin(rounding * rounding * tot[1], 1e-18 * bb)))) {
-            w.s[S_RR] = tot[0];
-            w.s[S_FLAG] = F_DRIFT;
-        }
+        if (w.s[S_RR] <= fmin(rounding * rounding * tot[0], 1e-18 * w.s[S_BB])) w.s[S_FLAG] = F_CONVERGED;
     }
 }
+constexpr int kVerifyKernels = 2;
 void launch_verify(tf_handle* h, const Ctx& c) {
     Device& d = h->d;
-    k_verify<<<d.ncta, kThreads, split_bytes<double>(d), h->stream>>>(c, d.g, d.du, d.r);
+    const size_t sb = split_bytes<double>(d);
+    if (d.split) k_verify<0><<<d.ncta, kThreads, sb, h->stream>>>(c, d.g, d.du, d.r);
+    else k_verify<2><<<d.ncta, kThreads, sb, h->stream>>>(c, d.g, d.du, d.r);
+    k_rounding<<<d.ncta, kThreads, sb, h->stream>>>(c, d.du);
 }
 
 // Issues n iterations of `method` on the stream (no host interaction).
@@ -993,6 +1007,7 @@ tf_status krylov_run(tf_handle* h, int method, int keep, int* iters, double* rel
         TF_CUDA(cudaGraphLaunch(h->kloop[method - 1], st));
         if (!jac) {
             launch_verify(h, c);
+            h->launches += kVerifyKernels - 1;
             TF_LAUNCH_CHECK(h);
         }
         TF_CUDA(cudaMemcpyAsync(h->kloop_host, h->kloop_ctl, sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -1026,6 +1041,7 @@ tf_status krylov_run(tf_handle* h, int method, int keep, int* iters, double* rel
         launched += issued;
         if (!jac) {
             launch_verify(h, c);
+            h->launches += kVerifyKernels - 1;
             TF_LAUNCH_CHECK(h);
         }
         TF_CUDA(cudaMemcpyAsync(d.host_scal, d.scal, sizeof(double) * nscal, cudaMemcpyDeviceToHost, st));
@@ -1420,7 +1436,7 @@ bool build_newton_loop(tf_handle* h) {
             const bool mg = use_multigrid(h);
             h->nloop_kernels = 2 + 2 + (h->opt.deterministic ? 2 : 0) + 1 + (mg ? 3 : 0) +
                                (h->method == 1 && mg ? 1 + (amg_fuses_dot(h) ? 0 : 1) + amg_vcycle_kernels(h) : 1) +
-                               1 + (mg ? 1 : 0) + 3;
+                               1 + (mg ? kVerifyKernels : 0) + 3;
             cudaGraph_t out = nullptr;
             ok = (cudaStreamEndCapture(h->stream, &out) == cudaSuccess) && ok;
         }
