@@ -645,3 +645,21 @@ def test_static_solve_gives_up_on_a_block_that_does_not_come():
     assert "lost each other" in L.tf_last_error().decode() and (it.value, rr.value) == (0, 0.0)
     assert L.tf_static_solve_blocks(0, 0, n, *args) == api.TF_OK
     assert np.array_equal(x.cpu().numpy(), np.full(3 * n, 0.5))
+
+
+# Split rows have one form of the FP64 product, so a handle's first solve times none:
+# with block-Jacobi it launches what it launches without the autotuner.  Whole rows
+# time three forms, four launches each.
+@pytest.mark.parametrize("deterministic,probes", [(False, 0), (True, 12)])
+def test_split_rows_have_no_product_forms_to_time(deterministic, probes):
+    t = _sheet(12, 12, 2, 0.0)
+    uk, un = mesh.perturbed_state(t, seed=5)
+    launches = []
+    for autotune in (True, False):
+        with api.Solver(t, precond=1, krylov_max_iter=4, deterministic=deterministic, autotune=autotune) as s:
+            s.set_state(uk, un, t.dt)
+            s.assemble()
+            before = s.launch_count()
+            assert s.solve(allow_not_converged=True)["iters"] == 4
+            launches.append(s.launch_count() - before)
+    assert launches[0] - launches[1] == probes, launches

@@ -2,7 +2,6 @@
 // reference's Pardiso phases 11/22/33 (NewtonRaphsonSolver.cpp:418-683,
 // transposed solve iparm[11] = 1 at :639).
 //
-//   * block-Jacobi preconditioner on the 3x3 diagonal blocks;
 //   * CG when every element has zero internal viscosity (A symmetric),
 //     BiCGStab otherwise (the viscous tangent is not symmetric);
 //   * a batch of independent instances is one block-diagonal system, solved
@@ -14,8 +13,13 @@
 //     partial sums and the last CTA of the instance to finish (atomic ticket,
 //     no waiting) folds them in a fixed order, so results are bitwise
 //     reproducible;
-//   * iterations run in chunks of 8-64 replayed from CUDA graphs; the host
-//     reads the flags once per chunk.
+//   * a solve's iterations are one graph whose device-side while loop ends when
+//     every instance has stopped (build_krylov_loop); the host reads the flags once,
+//     after it.  Where that graph cannot be built, or tf_options.host_loops asks
+//     for it, they run in chunks of 4-64 with a read after each;
+//   * the preconditioner is the multigrid (tf_amg.cu) or block-Jacobi; a converged
+//     multigrid solve has its residual formed again (k_verify), one that failed is
+//     done again with block-Jacobi (krylov_solve).
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -792,9 +796,11 @@ __global__ void k_spmv_probe(Ctx c, const double* __restrict__ x, double* __rest
 
 // Picks the solve's kernel variants by timing them on the handle's own
 // matrix, once per handle before its first solve builds any graph: the
-// FP64 block SpMV with 1, 2 or 4 slots in flight per lane, and (multigrid)
-// the level-0 smoother's row product with 2, 4 or 8.  Results do not depend
-// on the choice (the same products in the same order).
+// FP64 block SpMV with 1, 2 or 4 slots in flight per lane (whole rows; split
+// ones have a single form), and (multigrid) the level-0 smoother's row product
+// with 2, 4 or 8 (split rows too: systems with extra blocks use it, and couples
+// may come later).  Results do not depend on the choice (the same products in
+// the same order).
 tf_status autotune_solve(tf_handle* h) {
     if (h->solve_tuned) return TF_OK;
     h->solve_tuned = true;
@@ -808,6 +814,7 @@ tf_status autotune_solve(tf_handle* h) {
     TF_CUDA(cudaMemsetAsync(d.scal, 0, sizeof(double) * (size_t)d.nseg * S_COUNT, st));
     float best = 1e30f;
     for (int u : {1, 2, 4}) {
+        if (d.split) break;  // issue_iterations has one form
         for (int r = 0; r < 4; ++r) {  // one warm-up, three timed
             if (r == 1) TF_CUDA(cudaEventRecord(h->ev[4], st));
             if (u == 1) k_spmv_probe<1><<<d.ncta, kThreads, split_bytes<double>(d), st>>>(c, d.du, d.q);
