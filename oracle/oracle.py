@@ -25,8 +25,8 @@ import numpy as np
 HERE = os.path.dirname(os.path.abspath(__file__))
 PORT_LIB = os.path.join(HERE, "_build", "libtforacle.so")
 REF_LIB = os.path.join(HERE, "_ref", "libtfref.so")
-# root of the reference checkout (read only); TF_REFERENCE_DIR overrides it
-REF_ROOT = os.environ.get("TF_REFERENCE_DIR", "/root/reference")
+# root of the reference checkout (read only): TF_REFERENCE_DIR, or "reference" beside this repository
+REF_ROOT = os.environ.get("TF_REFERENCE_DIR", os.path.join(os.path.dirname(os.path.dirname(HERE)), "reference"))
 REF_SRC = os.path.join(REF_ROOT, "TissueFolding", "TissueFolding", "SourceCode")
 
 LITERAL = 0
