@@ -72,12 +72,13 @@ constexpr int64_t kDenseBytes = 64 << 20;
 constexpr int kDenseThreads = 512;
 constexpr int kDenseCols = 16;    // columns of the dense operator built together by one CTA
 constexpr int kDenseQuads = kDenseCols / 4;  // lanes per row, four columns each
-// Three V-cycles instead of one cost nothing per application and leave the
-// coarse levels nearly solved: 95 -> 70 CG iterations per 1.0M-prism wing step,
-// 42 -> 39 BiCGStab iterations on the 320,000-prism sheet (two cycles: 78 and 41).
 constexpr int kDenseRows = 3600;  // rows of an instance: its vectors have to fit shared memory, 64 bytes a row
+// V-cycles the dense operator stands for.  Three instead of one cost nothing per
+// application and leave the coarse levels nearly solved: 95 -> 70 CG iterations per
+// 1.0M-prism wing step, 42 -> 39 BiCGStab iterations on the 320,000-prism sheet (two
+// cycles: 78 and 41).
+constexpr int kDenseCycles = 3;
 constexpr int kDenseSweeps = 3;  // their sweeps each way
-constexpr int kDenseCycles = 3;   // V-cycles the dense operator stands for
 // damped block-Jacobi sweeps before and after the coarse correction on the
 // levels >= 1 (level 0 sweeps once each way): more sweeps on the small,
 // launch-bound coarse levels cut the Krylov iterations (320,000-prism sheet:
@@ -2519,7 +2520,8 @@ tf_status amg_autotune(tf_handle* h) {
 
 int amg_smoother_unroll(const tf_handle* h) { return use_multigrid(h) ? h->amg->smooth_unroll : 0; }
 
-// Level 0 through Q (k_q_restrict ..): every system without extra blocks.
+// Level 0 through Q (k_restrict<3> on Q by column, k_q_smooth, k_q_post): every system
+// without extra blocks.
 static bool uses_q(const tf_handle* h) { return h->d.nxb == 0; }
 
 // k_q_smooth beside the coarse levels: where those are a chain of launches

@@ -467,6 +467,10 @@ tf_status build(tf_handle* h, const tf_mesh* m, const tf_material* mat, const st
                 }
             }
         d.nval = nslots * kSlotDoubles;
+        d.matrix_bytes = nslots * (int64_t)(kSlotDoubles * sizeof(double) + kSlice * sizeof(int));
+        int l2 = 0;
+        TF_CUDA(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, h->device));
+        d.l2_bytes = l2;
     }
     std::vector<int> slot_ofs(slot.size()), diag_ofs(nn);
     for (size_t q = 0; q < slot.size(); ++q) slot_ofs[q] = bofs[slot[q]];

@@ -127,6 +127,8 @@ struct Device {
     // kernels without a row product running one warp per CTA
     int cta_nodes = 256;
     int split = 0;
+    int64_t matrix_bytes = 0;   // of the sliced FP64 matrix and its columns
+    int64_t l2_bytes = 0;
     int* seg_node0 = nullptr;   // [nseg+1] node offsets
     int* elem_seg = nullptr;    // [ne] instance of each element
     int* cta_seg = nullptr;     // [ncta] instance of each CTA
@@ -392,6 +394,7 @@ inline cudaError_t launch_cooperative(void (*kernel)(KArgs...), int grid, int bl
 // its slots s0 .. s1 together, each lane reading its own row's block, so every
 // load of a block entry or column is one coalesced access.
 // U = 0 (split CTAs): the columns of the first slots come loaded (Ahead).
+// stream: the matrix passes L2 by (stream_matrix; whole rows only).
 constexpr int kAhead = 4;
 struct Ahead {
     int j[kAhead];  // -1: no such slot
@@ -406,7 +409,7 @@ __device__ __forceinline__ Ahead load_ahead(const int* __restrict__ scol, int s0
 template <class T, int U = 2>
 __device__ __forceinline__ void sliced_row(int s0, int s1, const int* __restrict__ scol, const T* __restrict__ val,
                                            const double* __restrict__ x, double y[3], int nn, int* check,
-                                           const Ahead& p) {
+                                           bool stream, const Ahead& p) {
     const int lane = threadIdx.x & 31;
     double y0 = 0.0, y1 = 0.0, y2 = 0.0;
     const int* __restrict__ col = scol + lane;
@@ -423,20 +426,20 @@ __device__ __forceinline__ void sliced_row(int s0, int s1, const int* __restrict
             y2 = fma((double)__ldg(&v[192]), x0, fma((double)__ldg(&v[224]), x1, fma((double)__ldg(&v[256]), x2, y2)));
         }
     }
-    // streamed: a whole-row product reads its matrix once an iteration, and L2 (129 MB)
-    // should keep the vectors and the coarse levels instead (32 tissues 27.6 -> 26.9 ms a
-    // step, 114,005 nodes 10.74 -> 10.58, 320,000 prisms 19.85 -> 19.75; the FP16 sweep's
-    // operator streamed as well: 27.6, 10.64, 19.8)
+    auto rest = [&](auto load) {
 #pragma unroll (U == 0 ? 1 : U)
-    for (int s = U == 0 ? s0 + kAhead : s0; s < s1; ++s) {
-        const int j = __ldcs(&col[(size_t)s * kSlice]);
-        if (!TF_IN(check, j, nn, CK_SPMV_COL)) continue;
-        const T* __restrict__ v = a + (size_t)s * kSlotDoubles;
-        const double x0 = x[3 * j], x1 = x[3 * j + 1], x2 = x[3 * j + 2];
-        y0 = fma((double)__ldcs(&v[0]), x0, fma((double)__ldcs(&v[32]), x1, fma((double)__ldcs(&v[64]), x2, y0)));
-        y1 = fma((double)__ldcs(&v[96]), x0, fma((double)__ldcs(&v[128]), x1, fma((double)__ldcs(&v[160]), x2, y1)));
-        y2 = fma((double)__ldcs(&v[192]), x0, fma((double)__ldcs(&v[224]), x1, fma((double)__ldcs(&v[256]), x2, y2)));
-    }
+        for (int s = U == 0 ? s0 + kAhead : s0; s < s1; ++s) {
+            const int j = load(&col[(size_t)s * kSlice]);
+            if (!TF_IN(check, j, nn, CK_SPMV_COL)) continue;
+            const T* __restrict__ v = a + (size_t)s * kSlotDoubles;
+            const double x0 = x[3 * j], x1 = x[3 * j + 1], x2 = x[3 * j + 2];
+            y0 = fma((double)load(&v[0]), x0, fma((double)load(&v[32]), x1, fma((double)load(&v[64]), x2, y0)));
+            y1 = fma((double)load(&v[96]), x0, fma((double)load(&v[128]), x1, fma((double)load(&v[160]), x2, y1)));
+            y2 = fma((double)load(&v[192]), x0, fma((double)load(&v[224]), x1, fma((double)load(&v[256]), x2, y2)));
+        }
+    };
+    if (U != 0 && stream) rest([](const auto* p) { return __ldcs(p); });
+    else rest([](const auto* p) { return __ldg(p); });
     y[0] = y0;
     y[1] = y1;
     y[2] = y2;

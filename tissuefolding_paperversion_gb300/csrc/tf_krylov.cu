@@ -60,7 +60,7 @@ __device__ __forceinline__ Slots warp_slots(const Ctx& c) {
 template <int U = 2>
 __device__ __forceinline__ void rows_product(const Ctx& c, const Slots& s, const double* __restrict__ x,
                                              double (&y)[3]) {
-    sliced_row<double, U>(s.s0, s.s1, c.scol, c.val, x, y, c.nn, c.check, s.p);
+    sliced_row<double, U>(s.s0, s.s1, c.scol, c.val, x, y, c.nn, c.check, c.stream, s.p);
 }
 template <int MODE = kEither>
 __device__ __forceinline__ void rows_sum(const Ctx& c, const Where& w, const double* __restrict__ x, double (&y)[3]) {

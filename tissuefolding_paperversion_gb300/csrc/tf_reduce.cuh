@@ -4,6 +4,7 @@
 #pragma once
 
 #include "tf_internal.cuh"
+#include "tf_stream.h"
 
 namespace tf {
 
@@ -25,6 +26,7 @@ struct Ctx {
     unsigned* tickets;          // [nseg]
     int ncta;
     int single, split, cta_nodes;     // one instance; see Device::split
+    int stream;                       // the matrix is read past L2 (stream_matrix)
     const int* __restrict__ cta_seg;
     const int* __restrict__ cta_node0;
     const int* __restrict__ cta_node1;
@@ -181,6 +183,7 @@ inline Ctx make_ctx(tf_handle* h) {
     c.ncta = d.ncta;
     c.single = d.nseg == 1;
     c.split = d.split;
+    c.stream = !d.split && stream_matrix(d.matrix_bytes, use_multigrid(h), d.l2_bytes);
     c.cta_nodes = d.cta_nodes;
     c.cta_seg = d.cta_seg;
     c.cta_node0 = d.cta_node0;
