@@ -307,10 +307,11 @@ TF_API tf_status tf_get_instances(tf_handle* h, int32_t* n_instances, int32_t* n
 TF_API int32_t tf_elements_per_cta(tf_handle* h);
 /* The solve's kernel variants the autotuner chose by timing them on the
  * handle's own matrix before its first solve: block rows' slots in flight per
- * lane in the FP64 SpMV (1, 2, 4) and in the multigrid's level-0 smoother
- * (2, 4, 8; 0 without multigrid).  Meshes of up to 65,536 nodes with the atomic
- * assembly have one form of the SpMV, timed against nothing (2 is reported), and
- * use the smoother's only with extra blocks.  No reference counterpart. */
+ * lane in the multigrid's level-0 smoother (2, 4, 8; 0 without multigrid), and
+ * those in the FP64 SpMV, which follow the method (4 with CG, 2 with BiCGStab).
+ * Meshes of up to 65,536 nodes with the atomic assembly have one form of the
+ * SpMV (2 is reported) and use the smoother's only with extra blocks.  No
+ * reference counterpart. */
 TF_API tf_status tf_solve_variants(tf_handle* h, int32_t* spmv_unroll, int32_t* smoother_unroll);
 
 /* --- inspection (parity tests) ------------------------------------------ */

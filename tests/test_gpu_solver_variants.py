@@ -647,12 +647,12 @@ def test_static_solve_gives_up_on_a_block_that_does_not_come():
     assert np.array_equal(x.cpu().numpy(), np.full(3 * n, 0.5))
 
 
-# Split rows have one form of the FP64 product, so a handle's first solve times none:
-# with block-Jacobi it launches what it launches without the autotuner.  Whole rows
-# time three forms, four launches each.
-@pytest.mark.parametrize("deterministic,probes", [(False, 0), (True, 12)])
-def test_split_rows_have_no_product_forms_to_time(deterministic, probes):
-    t = _sheet(12, 12, 2, 0.0)
+# The form of the FP64 product follows from the rows and the method, so a handle's first
+# solve times none: with block-Jacobi it launches what it launches without the autotuner.
+@pytest.mark.parametrize("eta", [0.0, 100.0])
+@pytest.mark.parametrize("deterministic", [False, True])
+def test_first_solve_times_no_forms_of_the_product(deterministic, eta):
+    t = _sheet(12, 12, 2, eta)
     uk, un = mesh.perturbed_state(t, seed=5)
     launches = []
     for autotune in (True, False):
@@ -662,4 +662,5 @@ def test_split_rows_have_no_product_forms_to_time(deterministic, probes):
             before = s.launch_count()
             assert s.solve(allow_not_converged=True)["iters"] == 4
             launches.append(s.launch_count() - before)
-    assert launches[0] - launches[1] == probes, launches
+            assert s.tiles()["spmv_unroll"] == (4 if deterministic and eta == 0.0 else 2)
+    assert launches[0] == launches[1], launches

@@ -1442,7 +1442,7 @@ int32_t tf_elements_per_cta(tf_handle* h) { return h ? h->elem_cta : 0; }
 
 tf_status tf_solve_variants(tf_handle* h, int32_t* spmv_unroll, int32_t* smoother_unroll) {
     TF_TRY(check_handle(h));
-    if (spmv_unroll) *spmv_unroll = h->spmv_unroll;
+    if (spmv_unroll) *spmv_unroll = spmv_unroll_of(h);
     if (smoother_unroll) *smoother_unroll = amg_smoother_unroll(h);
     return TF_OK;
 }

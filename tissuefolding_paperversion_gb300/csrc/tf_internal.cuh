@@ -502,8 +502,7 @@ struct tf_handle {
     int* kloop_ctl = nullptr;                   // device: [iterations run, iteration cap]
     int* kloop_host = nullptr;                  // pinned copy of the iterations run
     int last_iters[2] = {0, 0};                 // iterations of the last solve per method (chunk planning)
-    bool solve_tuned = false;                   // the solve's kernel variants below were chosen by timing
-    int spmv_unroll = 2;                        // slots in flight per lane in the FP64 block SpMV (1, 2, 4)
+    bool solve_tuned = false;                   // the smoother's variant was chosen by timing
     int plan_iters[2][8] = {};                  // the same per Newton iteration of a step (0-6, 7: later ones)
     int newton_index = -1;                      // Newton iteration of the current solve (-1: outside a step)
     double* du0 = nullptr;                      // the first Newton update of the last step (start of the next)
@@ -564,6 +563,7 @@ tf_status amg_numeric(tf_handle* h);
 void amg_refresh(tf_handle* h);     // launches the level-0 smoother copies of the current assembly
 tf_status amg_autotune(tf_handle* h);  // picks the level-0 smoother's row-product variant by timing
 int amg_smoother_unroll(const tf_handle* h);
+int spmv_unroll_of(const tf_handle* h);  // slots in flight per lane in the FP64 products of whole rows
 void amg_refreshed(tf_handle* h);   // records that amg_refresh ran for the current assembly
 // out = M^-1 r; dot: what the last kernel does besides (CG): (r, out) with beta,
 // or the same at the start of a solve with p = out (amg_fuses_dot).

@@ -743,9 +743,19 @@ void launch_verify(tf_handle* h, const Ctx& c) {
     k_rounding<<<d.ncta, kThreads, sb, h->stream>>>(c, d.du);
 }
 
+// Slots in flight per lane in the FP64 products: 0 for split rows (they have a handful);
+// of whole rows four in CG and two in BiCGStab.  All keep to 40 registers without
+// spills; with four, BiCGStab's kernels, which read and write more vectors, get slower.
+// us an iteration with 2 / 4, order-fixed block-Jacobi: 1,323 nodes CG 29.7 / 29.4, BiCGStab
+// 58.2 / 62.6; 6,125 31.5 / 30.8 and 61.3 / 64.9; 18,605 32.0 / 31.4 and 63.7 / 67.8; multigrid
+// 99,405 nodes 205 / 203 and 423 / 432, 567,009 741 / 740 and 1,551 / 1,559 (one slot: 747
+// and 1,556).  Timing a product by itself took four for both.
+constexpr int slots_in_flight(int method, bool split) { return split ? 0 : (method == 1 ? 4 : 2); }
+
 // Issues n iterations of `method` on the stream (no host interaction).
-template <int U>
-void issue_iterations_u(tf_handle* h, const Ctx& c, int method, int n) {
+template <bool SPLIT>
+void issue_iterations_in(tf_handle* h, const Ctx& c, int method, int n) {
+    constexpr int UC = slots_in_flight(1, SPLIT), UB = slots_in_flight(2, SPLIT);
     Device& d = h->d;
     cudaStream_t st = h->stream;
     const int nb = d.ncta;
@@ -754,7 +764,7 @@ void issue_iterations_u(tf_handle* h, const Ctx& c, int method, int n) {
     const AmgPre pre = amg_pre(h);
     for (int it = 0; it < n; ++it) {
         if (method == 1) {
-            launch_pdl_smem(k_cg_spmv<U>, nb, kThreads, split_bytes<double>(d), st, c, d.p, d.q);
+            launch_pdl_smem(k_cg_spmv<UC>, nb, kThreads, split_bytes<double>(d), st, c, d.p, d.q);
             launch_pdl(k_cg_update, nb, vt, st, c, d.du, d.r, d.z, d.p, d.q, jac, pre);
             if (!jac) {
                 amg_vcycle(h, d.r, d.z, kVcycleDot, d.p);
@@ -764,75 +774,34 @@ void issue_iterations_u(tf_handle* h, const Ctx& c, int method, int n) {
         } else {
             launch_pdl(k_bi_dir, nb, vt, st, c, d.r, d.q, d.p, d.z, jac, pre);
             if (!jac) amg_vcycle(h, d.p, d.z);
-            launch_pdl_smem(k_bi_spmv1<U>, nb, kThreads, split_bytes<double>(d), st, c, d.z, d.rhat, d.q);
+            launch_pdl_smem(k_bi_spmv1<UB>, nb, kThreads, split_bytes<double>(d), st, c, d.z, d.rhat, d.q);
             launch_pdl(k_bi_s, nb, vt, st, c, d.r, d.q, d.s, d.sh, jac, pre);
             if (!jac) amg_vcycle(h, d.s, d.sh);
-            launch_pdl_smem(k_bi_spmv2<U>, nb, kThreads, split_bytes<double>(d), st, c, d.sh, d.s, d.t, d.du, d.z);
+            launch_pdl_smem(k_bi_spmv2<UB>, nb, kThreads, split_bytes<double>(d), st, c, d.sh, d.s, d.t, d.du, d.z);
             launch_pdl(k_bi_x, nb, vt, st, c, d.du, d.r, d.rhat, d.z, d.sh, d.s, d.t);
         }
     }
 }
 
 void issue_iterations(tf_handle* h, const Ctx& c, int method, int n) {
-    if (h->d.split) return issue_iterations_u<0>(h, c, method, n);
-    switch (h->spmv_unroll) {
-        case 1: issue_iterations_u<1>(h, c, method, n); break;
-        case 4: issue_iterations_u<4>(h, c, method, n); break;
-        default: issue_iterations_u<2>(h, c, method, n); break;
-    }
+    if (h->d.split) issue_iterations_in<true>(h, c, method, n);
+    else issue_iterations_in<false>(h, c, method, n);
 }
 
-// y = A x alone (no dot, no flags): the SpMV variants the solve autotuner times
-template <int U>
-__global__ void k_spmv_probe(Ctx c, const double* __restrict__ x, double* __restrict__ y) {
-    const Where w = where(c);
-    double v[3];
-    rows_product<U>(c, warp_slots(c), x, v);
-    rows_sum(c, w, x, v);
-    if (!w.valid) return;
-#pragma unroll
-    for (int d = 0; d < 3; ++d) y[3 * w.node + d] = v[d];
-}
-
-// Picks the solve's kernel variants by timing them on the handle's own
-// matrix, once per handle before its first solve builds any graph: the
-// FP64 block SpMV with 1, 2 or 4 slots in flight per lane (whole rows; split
-// ones have a single form), and (multigrid) the level-0 smoother's row product
-// with 2, 4 or 8 (split rows too: systems with extra blocks use it, and couples
-// may come later).  Results do not depend on the choice (the same products in
-// the same order).
+// Picks the multigrid's level-0 smoother by timing it on the handle's own matrix,
+// once per handle before its first solve builds any graph: the row product with 2, 4
+// or 8 slots in flight per lane (split rows too: systems with extra blocks use it, and
+// couples may come later).  Results do not depend on the choice (the same products
+// in the same order).
 tf_status autotune_solve(tf_handle* h) {
     if (h->solve_tuned) return TF_OK;
     h->solve_tuned = true;
-    if (h->opt.autotune_off) return TF_OK;
-    Device& d = h->d;
-    const Ctx c = make_ctx(h);
-    cudaStream_t st = h->stream;
+    if (h->opt.autotune_off || !use_multigrid(h)) return TF_OK;
     // every instance "running" while the variants are timed (the solver's
     // start writes all the scalars afterwards; nothing is kept across solves
     // before the first one)
-    TF_CUDA(cudaMemsetAsync(d.scal, 0, sizeof(double) * (size_t)d.nseg * S_COUNT, st));
-    float best = 1e30f;
-    for (int u : {1, 2, 4}) {
-        if (d.split) break;  // issue_iterations has one form
-        for (int r = 0; r < 4; ++r) {  // one warm-up, three timed
-            if (r == 1) TF_CUDA(cudaEventRecord(h->ev[4], st));
-            if (u == 1) k_spmv_probe<1><<<d.ncta, kThreads, split_bytes<double>(d), st>>>(c, d.du, d.q);
-            else if (u == 2) k_spmv_probe<2><<<d.ncta, kThreads, split_bytes<double>(d), st>>>(c, d.du, d.q);
-            else k_spmv_probe<4><<<d.ncta, kThreads, split_bytes<double>(d), st>>>(c, d.du, d.q);
-            TF_LAUNCH_CHECK(h);
-        }
-        TF_CUDA(cudaEventRecord(h->ev[5], st));
-        TF_CUDA(cudaEventSynchronize(h->ev[5]));
-        float ms = 0.f;
-        TF_CUDA(cudaEventElapsedTime(&ms, h->ev[4], h->ev[5]));
-        if (ms < best) {
-            best = ms;
-            h->spmv_unroll = u;
-        }
-    }
-    if (use_multigrid(h)) return amg_autotune(h);
-    return TF_OK;
+    TF_CUDA(cudaMemsetAsync(h->d.scal, 0, sizeof(double) * (size_t)h->d.nseg * S_COUNT, h->stream));
+    return amg_autotune(h);
 }
 
 int kernels_per_iteration(const tf_handle* h, int method) {
@@ -1102,6 +1071,8 @@ tf_status krylov_run(tf_handle* h, int method, int keep, int* iters, double* rel
 }
 
 }  // namespace
+
+int spmv_unroll_of(const tf_handle* h) { return h->d.split ? 2 : slots_in_flight(h->method, false); }
 
 // Whether the last solve stopped at its iteration cap: slow, not failed.
 static bool capped(const tf_handle* h) {
