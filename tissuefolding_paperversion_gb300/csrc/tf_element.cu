@@ -66,8 +66,12 @@
 // (3,156 before), ~120,000 thread instructions per prism in all; the rest is the barriers
 // between the phases (starting the CTAs of an SM in different phases: no change; two
 // threads per Gauss point: 1.77 ms with viscosity, but 1.29 without).
-// 320,000 prisms: 3.62 -> 1.81 ms with viscosity, 2.18 -> 1.26 ms without.  K's error against 64 bits, relative (2-norm): 2.0e-15 to 2.4e-15 without
-// viscosity (before 2.1e-15 to 2.2e-15), 2.4e-15 to 2.9e-15 with (2.6e-15 to 3.2e-15).
+// 320,000 prisms: 3.61 -> 1.84 ms with viscosity, 2.16 -> 1.25 ms without.  K's error,
+// against sums in extended precision and against the pairwise form's (before), relative
+// 2-norm: without viscosity 1.9e-15 to 2.9e-15 over 240 sheets of three shapes, 2.29e-15
+// on average (before 2.0e-15 to 2.8e-15, 2.29e-15), the largest entry's 3.2e-15 of the
+// largest entry (3.9e-15); with viscosity 2.3e-15 to 3.0e-15 over 12 sheets, 2.61e-15 on
+// average (2.6e-15 to 3.2e-15, 2.81e-15), the largest entry's 3.7e-15 (4.4e-15).
 // The matrix assembled is A = K^T, the system the reference
 // solves (Pardiso iparm[11] = 1, NewtonRaphsonSolver.cpp:639); in that
 // orientation every element block (a, b) lands at block (conn[a], conn[b])
