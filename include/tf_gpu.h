@@ -273,7 +273,9 @@ TF_API tf_status tf_grid_growth_positions(tf_handle* h, double* rel_z, double* r
 TF_API tf_status tf_set_time(tf_handle* h, double time_sec);
 TF_API tf_status tf_get_time(tf_handle* h, double* time_sec);
 /* solveForDeltaU (NewtonRaphsonSolver.cpp:382-404): solves K^T du = g, the
- * transposed system Pardiso is asked for (iparm[11] = 1, :639). */
+ * transposed system Pardiso is asked for (iparm[11] = 1, :639).  relres is the
+ * recurrence's; with the multigrid the residual of du itself is checked too
+ * (tf_options.precond). */
 TF_API tf_status tf_solve(tf_handle* h, int32_t* iters, double* relres);
 /* checkConvergenceViaDeltaU + updateUkInIteration (:727-761). */
 TF_API tf_status tf_update(tf_handle* h, int32_t* converged, double* dunorm);
@@ -372,8 +374,11 @@ TF_API tf_status tf_measure_bandwidth(int32_t device, int64_t bytes, int32_t rep
  * `stream` and reads scalars back, so it must never be made on a stream that
  * is being captured: it then returns TF_BAD_INPUT.  Calls share the array:
  * overlapping calls race, so serialise them (thread blocks that lose each other
- * that way give up after some seconds and the call returns TF_CUDA_ERROR).  `stream` is a cudaStream_t
- * (NULL: the default stream). */
+ * that way give up after some seconds and the call returns TF_CUDA_ERROR).  The
+ * solve is one kernel whose thread blocks, one per SM, are resident together: it
+ * starts once the kernels of other streams leave it 200 KB of each SM's shared
+ * memory, so no kernel may stay resident until this call is done.  `stream` is a
+ * cudaStream_t (NULL: the default stream). */
 TF_API tf_status tf_solve_bsr_static(int32_t n_block_rows, const int32_t* rowptr, const int32_t* colidx,
                                      const double* val, const double* b, double* x, double rtol, int32_t max_iter,
                                      void* stream, int32_t* iters, double* relres);
