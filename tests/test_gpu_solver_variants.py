@@ -664,3 +664,27 @@ def test_first_solve_times_no_forms_of_the_product(deterministic, eta):
             launches.append(s.launch_count() - before)
             assert s.tiles()["spmv_unroll"] == (4 if deterministic and eta == 0.0 else 2)
     assert launches[0] == launches[1], launches
+
+
+# A tolerance that no solve reaches, so the caller's cap ends both preconditioners'
+# attempts and the multigrid comes closer (it halves the residual: 1e-28 after 80, well
+# inside FP32's range).  With a cap of 40 later solves are the multigrid's attempt
+# alone; with 80 block-Jacobi still gets its turn.
+@pytest.mark.parametrize("cap,both", [(40, False), (80, True)])
+def test_block_jacobi_keeps_its_turn_under_large_caps(cap, both):
+    t = _sheet(20, 20, 2, 0.0)
+    launches = {}
+    for pc in (1, 0):
+        with api.Solver(t, krylov_rtol=1e-200, krylov_max_iter=cap, precond=pc) as s:
+            s.set_growth_rates(np.tile([4e-6, 3e-6, 0.0], t.n_elems))
+            s.begin_step(t.dt)
+            for _ in range(2):
+                s.assemble()
+                before = s.launch_count()
+                assert s.solve(allow_not_converged=True)["status"] == api.TF_KRYLOV_NOT_CONVERGED
+                launches[pc] = s.launch_count() - before
+            if pc == 0:
+                assert s.multigrid_info()[0]
+    # 3 launches an iteration with block-Jacobi, 6 with the multigrid here, 1 every third for
+    # the loop: the multigrid's attempt alone is 1.9 times block-Jacobi's, both are 2.9 or more
+    assert both == (launches[0] > 2.4 * launches[1]), launches

@@ -908,6 +908,10 @@ bool build_krylov_loop(tf_handle* h, const Ctx& c, int method) {
 // systems it suits have needed (packed sheets to 1e-12: 1,400), so a solve that
 // will not converge does not run to the caller's cap first.
 constexpr int kTrialIters = 2000;
+// Caps up to which a solve that both preconditioners leave at the cap is taken for one
+// that the caller means to cut short: what the multigrid needs on the systems it suits
+// (20 to 85), a fraction of what block-Jacobi needs (200 to 1,600).
+constexpr int kFewIters = 50;
 
 int krylov_cap(const tf_handle* h) {
     return h->amg_trial && use_multigrid(h) ? std::min(h->opt.krylov_max_iter, kTrialIters) : h->opt.krylov_max_iter;
@@ -1161,8 +1165,10 @@ static tf_status krylov_attempt(tf_handle* h, int* iters, double* relres) {
 // where block-Jacobi is the general path) stays with block-Jacobi once that
 // converged; others go back to the multigrid, and at their iteration cap they stop.
 // Where the caller's cap ends both, the handle stays with the one that came closer
-// and does not try the other again: a caller who uses capped solves pays for
-// one (1,323 nodes, a cap of 10: 237 launches a solve before, 38 now, as with block-Jacobi).
+// and, with a cap of kFewIters or less, does not try the other again: a caller who uses
+// capped solves pays for one (1,323 nodes, a cap of 10: 237 launches a solve before, 38
+// now, as with block-Jacobi).  With more iterations allowed, a later solve that the
+// multigrid cannot do may be one that block-Jacobi can.
 tf_status krylov_solve(tf_handle* h, int* iters, double* relres) {
     const tf_status s = krylov_attempt(h, iters, relres);
     if (s == TF_OK || !use_multigrid(h) || s == TF_CUDA_ERROR || s == TF_OUT_OF_MEMORY) return s;
@@ -1176,7 +1182,7 @@ tf_status krylov_solve(tf_handle* h, int* iters, double* relres) {
     if (h->amg_trial && (t == TF_OK || (cap && capped_by_caller(h, t) && *relres < rel))) {
         h->amg_failed = true;
     } else {
-        h->amg_capped = h->amg_capped || (cap && capped_by_caller(h, t));
+        h->amg_capped = h->amg_capped || (cap && capped_by_caller(h, t) && h->opt.krylov_max_iter <= kFewIters);
         destroy_graphs(h);
         h->amg_off = false;
     }
